@@ -6,11 +6,11 @@
 // then costs one phase multiply, one inverse FFT and |.| per A-scan
 // (dispersion.py:88-102), and a sharpness metric per B-scan over the depth
 // pixels z >= 20 (dispersion.py:46-63).
-//   k_disp_mag    one launch for a whole list of betas: 128 threads per
-//                 A-scan load X and the beta's phase row straight into the
-//                 registers of the first FFT stage, then the shared-memory
-//                 Stockham FFT of the reconstruction kernel; |X| is averaged
-//                 over the B-scan repeats (dispersion.py:101).
+//   k_disp_mag    one launch for a whole list of betas: a warp per A-scan
+//                 loads X and the beta's phase row straight into the registers
+//                 of the first FFT stage (64 points a lane), one exchange
+//                 through its own shared memory; |X| is averaged over the
+//                 B-scan repeats (dispersion.py:101).
 //   k_top_sum     top_percentile: one CTA per (beta, B-scan) finds the exact
 //                 k-th largest magnitude by a three-digit radix select on the
 //                 float bits (12 + 11 + 8 bits, histograms in shared memory),
@@ -32,88 +32,91 @@
 namespace octgb {
 namespace {
 
+// One warp an A-scan (ifft2048_low_mag_warp), four warps a CTA, three CTAs an
+// SM (168 registers a thread: 64 complex points a lane).  Bound by latency and
+// issue: 2 835 warp instructions an A-scan, issue active 56 %, FMA pipe 50 %,
+// shared-memory path 54 %, DRAM 32 % (205 000 transforms, 41 betas).  There it
+// takes 823 us; with 128 threads an A-scan, two exchanges and four group
+// barriers the same arithmetic took 967 us.  The next line is prefetched into
+// L2 only: holding it in registers behind the last stage spilled.
+constexpr int kDispWarps = 4;
+
 struct DispSmem {
-    alignas(16) float2 spec[kPerCta][kSpecStride];  // FFT work line per group
-    alignas(16) float2 tw2[16][16];
-    alignas(16) float2 tw3[8][256];
+    alignas(16) float2 tw2[256];
+    alignas(16) float2 tw3[kTw3];
+    alignas(16) float2 ex[kDispWarps][kWarpExchange];
+    // followed by [kDispWarps][kHalf] floats (a line's magnitudes) with pooling or repeats
 };
 
-__global__ void __launch_bounds__(kThreads, 2) k_disp_mag(const DispArgs a) {
+// streamed once: keep L1 for the phase row
+__device__ __forceinline__ float ld_stream(const float* p) {
+    float v;
+    asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
+// Rep: several B-scan repeats (a.rep > 1)
+template <bool Pool, bool Rep>
+__global__ void __launch_bounds__(kDispWarps * 32, 3) k_disp_mag(const DispArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     DispSmem& S = *reinterpret_cast<DispSmem*>(smem_raw);
-    const int tid = threadIdx.x;
-    const int g = tid / kGroup, lt = tid % kGroup;
-    for (int k = tid; k < 16 * 16; k += kThreads) {
-        const int r = k / 16, j = k % 16;
-        S.tw2[r][j] = __ldg(a.tw + (r * j * (kN / 256)) % kN);
-    }
-    for (int k = tid; k < 8 * 256; k += kThreads) {
-        const int r = k / 256, j = k % 256;
-        S.tw3[r][j] = __ldg(a.tw + (r * j) % kN);
-    }
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int k = tid; k < 256; k += kDispWarps * 32) S.tw2[k] = __ldg(a.tw + ((k >> 4) * (k & 15) * (kN / 256)) % kN);   // symmetric in its indices
+    for (int k = tid; k < kTw3; k += kDispWarps * 32) S.tw3[k] = __ldg(a.tw + (((k >> 8) + 1) * (k & 255)) % kN);
     __syncthreads();
-    // items < 2^32 - 2 kPerCta gridDim (the launcher checks): 32-bit item arithmetic
+    float2* ex = S.ex[warp];
+    float* sums = reinterpret_cast<float*>(&S + 1) + warp * kHalf;
+    // items < 2^32 - the grid's warps (the launcher checks): 32-bit item arithmetic
     const unsigned int nbx = static_cast<unsigned int>(a.nb) * static_cast<unsigned int>(a.nx);
-    const unsigned int n_items = static_cast<unsigned int>(a.n_beta) * nbx;
-    for (unsigned int item = blockIdx.x * kPerCta + g; item < n_items; item += gridDim.x * kPerCta) {
-        const unsigned int gu = item / nbx, bx = item - gu * nbx;
+    const unsigned int n_items = static_cast<unsigned int>(a.n_beta) * nbx, step = gridDim.x * kDispWarps;
+    // repeat 0 of an item: B-scan b0 + bu, A-scan x; repeat rp is rp * nx lines further
+    auto line_of = [&](unsigned int item) -> const float* {
+        const unsigned int bx = item % nbx;
         const unsigned int bu = bx / static_cast<unsigned int>(a.nx);
         const unsigned int x = bx - bu * static_cast<unsigned int>(a.nx);
-        const float2* ph = a.phase + static_cast<int64_t>(gu) * kN;
-        // repeat rp of A-scan x of B-scan b0 + bu: line0 + rp * nx * kN
-        const float* line0 =
-            a.X + ((static_cast<int64_t>(a.b0 + static_cast<int>(bu)) * a.rep) * a.nx + x) * kN;
-        float acc[2][4];
+        return a.X + ((static_cast<int64_t>(a.b0 + static_cast<int>(bu)) * a.rep) * a.nx + x) * kN;
+    };
+    for (unsigned int item = blockIdx.x * kDispWarps + warp; item < n_items; item += step) {
+        const float2* ph = a.phase + static_cast<int64_t>(item / nbx) * kN + lane;
+        const float* line = line_of(item) + lane;
+        float* out = Pool ? sums : a.A + static_cast<int64_t>(item) * kHalf;
+        // the warp's next line into L2 behind this one's transform
+        if (!Rep && lane == 0 && item + step < n_items) bulk_prefetch_l2(line_of(item + step), kN * sizeof(float));
+        for (int rp = 0; rp < (Rep ? a.rep : 1); ++rp, line += static_cast<int64_t>(a.nx) * kN) {
+            float2 v[64];
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+            for (int r = 0; r < 64; ++r) v[r].x = ld_stream(line + 32 * r);
 #pragma unroll
-            for (int r = 0; r < 4; ++r) acc[h][r] = 0.f;
-        for (int rp = 0; rp < a.rep; ++rp) {
-            const float* line = line0 + static_cast<int64_t>(rp) * a.nx * kN;
-            float2 v[16];
-#pragma unroll
-            for (int r = 0; r < 16; ++r) {
-                const int j = lt + 128 * r;
-                const float xv = __ldg(line + j);
-                const float2 p = __ldg(ph + j);
+            for (int r = 0; r < 64; ++r) {
+                const float2 p = __ldg(ph + 32 * r);
                 // complex64 (xv + 0i) * p, as numpy multiplies (dispersion.py:94)
-                v[r] = make_float2(xv * p.x, xv * p.y);
+                v[r] = make_float2(v[r].x * p.x, v[r].x * p.y);
             }
-            float mag[2][4];
-            ifft2048_low_mag_regs(v, S.spec[g], S.tw2, S.tw3, g, lt, mag);
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int r = 0; r < 4; ++r) acc[h][r] += mag[h][r];
+            ifft2048_low_mag_warp(v, ex, S.tw2, S.tw3, lane, [&](int k, float m) {
+                if (!Rep) {
+                    out[k] = m;
+                    return;
+                }
+                // numpy's float32 mean over the repeats: sum, then divide
+                const float t = (rp == 0 ? 0.f : sums[k]) + m;
+                if (rp + 1 == a.rep)
+                    out[k] = __fdiv_rn(t, static_cast<float>(a.rep));
+                else
+                    sums[k] = t;
+            });
         }
-        if (a.zcol != nullptr) {
-            // probe images: |X| into the group's (now free) line, then per image
-            // row zi the sum over depths [zi z_keep / 256, ceil((zi + 1) z_keep / 256))
-            float* M = reinterpret_cast<float*>(S.spec[g]);
-            group_sync(g);                              // every thread has read the line's last stage
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int r = 0; r < 4; ++r)
-                    M[lt + 128 * h + 256 * r] = a.rep == 1 ? acc[h][r] : __fdiv_rn(acc[h][r], static_cast<float>(a.rep));
-            group_sync(g);
-            for (int zi = lt; zi < 256; zi += kGroup) {
+        if (Pool) {
+            // probe images: per image row zi the sum over depths
+            // [zi z_keep / 256, ceil((zi + 1) z_keep / 256))
+            __syncwarp();
+            for (int zi = lane; zi < 256; zi += 32) {
                 const int z0 = zi * a.z_keep / 256, z1 = ((zi + 1) * a.z_keep + 255) / 256;
                 float sum = 0.f;
-                for (int z = z0; z < z1; ++z) sum += M[z];
+                for (int z = z0; z < z1; ++z) sum += sums[z];
                 a.zcol[static_cast<int64_t>(item) * 256 + zi] = sum;
             }
-            continue;                                   // the next transform writes the line after a group barrier
+            __syncwarp();
         }
-        float* out = a.A + static_cast<int64_t>(item) * kHalf;
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int k = lt + 128 * h + 256 * r;
-                // numpy's float32 mean over the repeats: sum, then divide
-                out[k] = a.rep == 1 ? acc[h][r] : __fdiv_rn(acc[h][r], static_cast<float>(a.rep));
-            }
     }
 }
 
@@ -395,15 +398,16 @@ __global__ void __launch_bounds__(kMedCols * 32) k_xmedian(const float* __restri
 }  // namespace
 
 cudaError_t launch_disp_mag(const DispArgs& a, int num_sms, cudaStream_t st) {
-    const size_t smem = sizeof(DispSmem);
-    cudaError_t e = cudaFuncSetAttribute(k_disp_mag, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+    const size_t smem = sizeof(DispSmem) + (a.zcol != nullptr || a.rep > 1 ? kDispWarps * kHalf * sizeof(float) : 0);
+    const auto kernel = a.zcol != nullptr ? (a.rep > 1 ? k_disp_mag<true, true> : k_disp_mag<true, false>)
+                                          : (a.rep > 1 ? k_disp_mag<false, true> : k_disp_mag<false, false>);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
     const int64_t items = static_cast<int64_t>(a.n_beta) * a.nb * a.nx;
-    if (items >= (int64_t(1) << 32) - 2 * kPerCta * num_sms) return cudaErrorInvalidValue;   // 32-bit item index
-    int64_t grid = (items + kPerCta - 1) / kPerCta;
-    if (grid > 2 * num_sms) grid = 2 * num_sms;
-    k_disp_mag<<<static_cast<int>(grid), kThreads, smem, st>>>(a);
+    if (items >= (int64_t(1) << 32) - 3 * kDispWarps * num_sms) return cudaErrorInvalidValue;   // 32-bit item index
+    int64_t grid = (items + kDispWarps - 1) / kDispWarps;
+    if (grid > 3 * num_sms) grid = 3 * num_sms;
+    kernel<<<static_cast<int>(grid), kDispWarps * 32, smem, st>>>(a);
     return cudaGetLastError();
 }
 

@@ -128,6 +128,11 @@ __device__ __forceinline__ void tma_bulk_g2s(void* dst, const void* src, uint32_
         : "memory");
 }
 
+// copy `bytes` (a multiple of 16) from a 16-byte aligned global address into L2
+__device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+
 // one arrival on the mbarrier once every cp.async this thread issued so far
 // has landed (counted against the barrier's expected arrivals)
 // asynchronous global -> shared copy of 16 bytes (both addresses 16-byte
@@ -385,6 +390,92 @@ __device__ __forceinline__ void ifft2048_low_mag(float2* X, const float2 (*tw2)[
 #pragma unroll
     for (int r = 0; r < 16; ++r) v[r] = X[pad(lt + 128 * r)];
     ifft2048_low_mag_regs(v, X, tw2, tw3, g, lt, mag);
+}
+
+// Inverse FFT of one 2048-point line by one warp, 64 points a lane, with one
+// exchange through the warp's own shared memory and no block barrier.  The
+// arithmetic is that of the radix 16, 16, 8 transform above, operation for
+// operation (the same bits); only the grouping differs.  With n = a + 8 b +
+// 128 n1 (a < 8, b = b1 + 4 b2 < 16, n1 < 16) lane a + 8 b1 holds every n1 and
+// b2: the first radix-16 stage (over n1) and the first radix-4 layer of the
+// second (over b2) need no exchange.  The result c = k0 + 16 k2 (< 64) then
+// moves to lane c mod 32, which holds every a and b1: the second radix-4
+// layer (over b1) and the radix-8 stage (over a) need none either.  The
+// exchange runs in two halves (c < 32, c >= 32) through 32 x 33 complex
+// values, the odd pitch keeping both sides free of bank conflicts, so the
+// second half waits in registers while the first is read.
+// v[r] = x[lane + 32 r] on entry; emit(k, |X[k]|) for the lane's 32 bins
+// k < N/2.
+// tw2[16 j + r] = w^(r j N/256), tw3[256 (r - 1) + j] = w^(r j) for r >= 1.
+constexpr int kWarpPitch = 33;
+constexpr int kWarpExchange = 32 * kWarpPitch;            // float2 of a warp's exchange buffer
+constexpr int kTw3 = 7 * 256;
+
+template <typename Emit>
+__device__ __forceinline__ void ifft2048_low_mag_warp(float2 (&v)[64], float2* ex, const float2* tw2,
+                                                      const float2* tw3, int lane, Emit&& emit) {
+    const int b1 = lane >> 3;
+    // v[b2 + 4 n1] -> v[b2 + 4 k0]
+#pragma unroll
+    for (int b2 = 0; b2 < 4; ++b2) {
+        float2 t[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) t[i] = v[b2 + 4 * i];
+        dft16(t);
+        const float2* tw = tw2 + b1 + 4 * b2;             // four addresses a warp, in four banks
+        v[b2] = t[0];
+#pragma unroll
+        for (int i = 1; i < 16; ++i) v[b2 + 4 * i] = cmul(t[i], tw[16 * i]);
+    }
+    // the inner twiddles w16^(b1 k2) of the second radix-16 stage, k2 = 1..3,
+    // as dft16 has them (b1 = 0 and the exact i give the same values)
+    const float2 wi1 = b1 == 0 ? make_float2(1.f, 0.f) : b1 == 1 ? make_float2(kC1, kS1)
+                     : b1 == 2 ? make_float2(kC2, kC2) : make_float2(kS1, kC1);
+    const float2 wi2 = b1 == 0 ? make_float2(1.f, 0.f) : b1 == 1 ? make_float2(kC2, kC2)
+                     : b1 == 2 ? make_float2(0.f, 1.f) : make_float2(-kC2, kC2);
+    const float2 wi3 = b1 == 0 ? make_float2(1.f, 0.f) : b1 == 1 ? make_float2(kS1, kC1)
+                     : b1 == 2 ? make_float2(-kC2, kC2) : make_float2(-kC1, -kS1);
+#pragma unroll
+    for (int k0 = 0; k0 < 16; ++k0) {
+        float2 (&q)[64] = v;
+        dft4(q[4 * k0], q[4 * k0 + 1], q[4 * k0 + 2], q[4 * k0 + 3]);
+        q[4 * k0 + 1] = cmul(q[4 * k0 + 1], wi1);
+        q[4 * k0 + 2] = cmul(q[4 * k0 + 2], wi2);
+        q[4 * k0 + 3] = cmul(q[4 * k0 + 3], wi3);
+    }
+    __syncwarp();                                         // the buffer's last readers are done
+#pragma unroll
+    for (int c = 0; c < 32; ++c) ex[c * kWarpPitch + lane] = v[4 * (c & 15) + (c >> 4)];
+    __syncwarp();
+    float2 u[32];                                         // u[a + 8 b1] of c = lane (then c = lane + 32)
+#pragma unroll
+    for (int i = 0; i < 32; ++i) u[i] = ex[lane * kWarpPitch + i];
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < 32; ++c) ex[c * kWarpPitch + lane] = v[4 * (c & 15) + (c >> 4) + 2];
+    __syncwarp();
+    // one copy of the code for both halves: the whole kernel stays near 32 KB
+    // of instructions, which the warps at different points of it share
+#pragma unroll 1
+    for (int c = lane;; c += 32) {
+#pragma unroll
+        for (int a = 0; a < 8; ++a) dft4(u[a], u[a + 8], u[a + 16], u[a + 24]);
+#pragma unroll
+        for (int k1 = 0; k1 < 4; ++k1) {
+            const int K = c + 64 * k1;
+            float2 w[8];
+            w[0] = u[8 * k1];
+#pragma unroll
+            for (int a = 1; a < 8; ++a) w[a] = cmul(u[8 * k1 + a], tw3[256 * (a - 1) + K]);
+            float2 X[4];
+            dft8_low(w, X);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) emit(K + 256 * p, __fsqrt_rn(fmaf(X[p].x, X[p].x, X[p].y * X[p].y)));
+        }
+        if (c >= 32) break;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) u[i] = ex[lane * kWarpPitch + i];
+    }
 }
 
 }  // namespace
