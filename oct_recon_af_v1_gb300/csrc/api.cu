@@ -173,9 +173,9 @@ struct octgb_ctx {
     DevBuf wgrad_part;                       // CNN training: per-CTA sums of the tensor-core weight gradient
     // dispersion scorer and focus profiles
     bool win_is_one = false;                 // geometry window is exactly 1 (plain linearisation)
-    DevBuf disp_x, disp_hann, disp_phase, disp_a, disp_score, xmed;
+    DevBuf disp_x, disp_hann, disp_dk2, disp_betas, disp_phase, disp_a, disp_score, xmed;
     int disp_b = 0, disp_rep = 0, disp_nx = 0;
-    std::vector<double> dk2;
+    bool has_dk2 = false;
     std::vector<QTable*> qtables;            // batched form: device tile tables by content
     uint64_t qtable_clock = 0;
     std::vector<SlotTable*> slot_tables;
@@ -500,7 +500,7 @@ int octgb_destroy(octgb_ctx* c) {
     }
     for (DevBuf* b : {&c->w, &c->start, &c->win, &c->tw, &c->wsh, &c->s0, &c->raw, &c->apod, &c->out, &c->mm, &c->frames, &c->num,
                       &c->den, &c->plan_table, &c->run_mm, &c->magbuf, &c->dbbuf, &c->planemm, &c->segs, &c->qtable,
-                      &c->qcounter, &c->disp_x, &c->disp_hann, &c->disp_phase, &c->disp_a, &c->disp_score, &c->xmed,
+                      &c->qcounter, &c->disp_x, &c->disp_hann, &c->disp_dk2, &c->disp_betas, &c->disp_phase, &c->disp_a, &c->disp_score, &c->xmed,
                       &c->prec_w, &c->prec_kb, &c->prec_hi, &c->prec_lo, &c->prec_m, &c->prec_x, &c->ex_w, &c->ex_win, &c->ex_tw, &c->bias_part, &c->wgrad_part, &c->prep,
                       &c->prep_apod, &c->magrep, &c->srr, &c->gemm_part, &c->enc_bits, &c->enc_lut, &c->enc_slots, &c->enc_sizes})
         b->release();
@@ -1266,7 +1266,7 @@ int octgb_graph_end(octgb_ctx* c, int* graph_id) {
         // a buffer that grows keeps its old allocation until octgb_destroy
         for (DevBuf* b : {&c->raw, &c->apod, &c->out, &c->mm, &c->frames, &c->num, &c->den, &c->plan_table,
                           &c->run_mm, &c->magbuf, &c->dbbuf, &c->planemm, &c->segs, &c->qtable, &c->qcounter,
-                          &c->disp_x, &c->disp_hann, &c->disp_phase, &c->disp_a, &c->disp_score, &c->xmed,
+                          &c->disp_x, &c->disp_hann, &c->disp_dk2, &c->disp_betas, &c->disp_phase, &c->disp_a, &c->disp_score, &c->xmed,
                           &c->prec_hi, &c->prec_lo, &c->prec_m, &c->prec_x, &c->prep, &c->prep_apod,
                           &c->magrep, &c->srr, &c->gemm_part, &c->enc_bits, &c->enc_lut, &c->enc_slots, &c->enc_sizes})
             b->keep_old = true;
@@ -1436,21 +1436,24 @@ int octgb_disp_lines(octgb_ctx* c, float* out, int out_loc) {
 int octgb_disp_set_dk2(octgb_ctx* c, const double* dk2) {
     return guarded(c, [&] {
         require(dk2 != nullptr, "dk2 is NULL");
-        c->dk2.assign(dk2, dk2 + kN);
+        ck(c->disp_dk2.ensure(kN * sizeof(double)), "cudaMalloc(dk2)");
+        ck(cudaMemcpyAsync(c->disp_dk2.p, dk2, kN * sizeof(double), cudaMemcpyHostToDevice, c->stream), "H2D dk2");
+        ck(cudaStreamSynchronize(c->stream), "sync dk2");
+        c->has_dk2 = true;
     });
 }
 
 namespace {
-// exp(-i beta dk^2) in float64, rounded to complex64 (dispersion.py:88-89), times 1/N
-void disp_phase_rows(const octgb_ctx* c, const double* betas, int n, float2* ph) {
-    for (int gi = 0; gi < n; ++gi) {
-        const double beta = betas[gi];
-        for (int j = 0; j < kN; ++j) {
-            const double t = beta * c->dk2[j];
-            ph[static_cast<size_t>(gi) * kN + j] = make_float2(static_cast<float>(std::cos(t)) * (1.0f / kN),
-                                                               static_cast<float>(-std::sin(t)) * (1.0f / kN));
-        }
-    }
+// phase rows of `n` betas into c->disp_phase (sized for `cap` rows)
+void disp_phase_rows(octgb_ctx* c, const double* betas, int n, int cap) {
+    ck(c->disp_betas.ensure(static_cast<size_t>(cap) * sizeof(double)), "cudaMalloc(betas)");
+    ck(c->disp_phase.ensure(static_cast<size_t>(cap) * kN * sizeof(float2)), "cudaMalloc(phase)");
+    ck(cudaMemcpyAsync(c->disp_betas.p, betas, static_cast<size_t>(n) * sizeof(double), cudaMemcpyHostToDevice,
+                       c->stream),
+       "H2D betas");
+    ck(launch_phase(c->disp_betas.as<double>(), c->disp_dk2.as<double>(), n, c->disp_phase.as<float2>(), c->stream),
+       "phase kernel");
+    c->launches++;
 }
 }  // namespace
 
@@ -1458,7 +1461,7 @@ int octgb_disp_eval(octgb_ctx* c, int n_beta, const double* betas, int b0, int n
                     int z_min, double* scores, float* mag, int mag_loc) {
     return guarded(c, [&] {
         require(c->disp_b > 0, "octgb_disp_load has not been called");
-        require(static_cast<int>(c->dk2.size()) == kN, "octgb_disp_set_dk2 has not been called");
+        require(c->has_dk2, "octgb_disp_set_dk2 has not been called");
         require(n_beta >= 1 && betas != nullptr, "no betas");
         require(b0 >= 0 && nb >= 1 && b0 + nb <= c->disp_b, "B-scan range outside the loaded B-scans");
         require(metric >= 0 && metric <= 4, "metric must be 0 (none) .. 4");
@@ -1474,15 +1477,10 @@ int octgb_disp_eval(octgb_ctx* c, int n_beta, const double* betas, int b0, int n
         const int per = mag != nullptr && mag_loc == OCTGB_DEVICE
                             ? n_beta
                             : std::max(1, static_cast<int>((size_t(1) << 30) / (seg_floats * nb * sizeof(float))));
-        std::vector<float2> ph(static_cast<size_t>(std::min(per, n_beta)) * kN);
         ck(c->disp_score.ensure(static_cast<size_t>(n_beta) * nb * sizeof(double)), "cudaMalloc(scores)");
         for (int g0 = 0; g0 < n_beta; g0 += per) {
             const int ng = std::min(per, n_beta - g0);
-            disp_phase_rows(c, betas + g0, ng, ph.data());
-            ck(c->disp_phase.ensure(static_cast<size_t>(per) * kN * sizeof(float2)), "cudaMalloc(phase)");
-            ck(cudaMemcpyAsync(c->disp_phase.p, ph.data(), static_cast<size_t>(ng) * kN * sizeof(float2),
-                               cudaMemcpyHostToDevice, c->stream),
-               "H2D phase");
+            disp_phase_rows(c, betas + g0, ng, std::min(per, n_beta));
             float* A = nullptr;
             if (mag != nullptr && mag_loc == OCTGB_DEVICE) {
                 A = mag + static_cast<size_t>(g0) * nb * seg_floats;
@@ -1504,7 +1502,7 @@ int octgb_disp_eval(octgb_ctx* c, int n_beta, const double* betas, int b0, int n
             c->launches++;
             if (metric != 0) {
                 ck(launch_disp_metric(A, ng * nb, nx, z_min, metric, static_cast<unsigned int>(top_k),
-                                      c->disp_score.as<double>() + static_cast<size_t>(g0) * nb, c->stream),
+                                      c->disp_score.as<double>() + static_cast<size_t>(g0) * nb, c->num_sms, c->stream),
                    "dispersion metric kernel");
                 c->launches++;
             }
@@ -1963,18 +1961,14 @@ int octgb_disp_images(octgb_ctx* c, int n_beta, const double* betas, int b0, int
                       int normalise) {
     return guarded(c, [&] {
         require(c->disp_b > 0, "octgb_disp_load has not been called");
-        require(static_cast<int>(c->dk2.size()) == kN, "octgb_disp_set_dk2 has not been called");
+        require(c->has_dk2, "octgb_disp_set_dk2 has not been called");
         require(n_beta >= 1 && betas != nullptr, "no betas");
         require(b0 >= 0 && nb >= 1 && b0 + nb <= c->disp_b, "B-scan range outside the loaded B-scans");
         require(z_keep >= 1 && z_keep <= kHalf, "z_keep must be in [1, N/2]");
         require(img != nullptr, "img is NULL");
         if (c->cancel.load()) throw Error(OCTGB_ERR_CANCELLED, "cancelled");
         const int nx = c->disp_nx;
-        std::vector<float2> ph(static_cast<size_t>(n_beta) * kN);
-        disp_phase_rows(c, betas, n_beta, ph.data());
-        ck(c->disp_phase.ensure(ph.size() * sizeof(float2)), "cudaMalloc(phase)");
-        ck(cudaMemcpyAsync(c->disp_phase.p, ph.data(), ph.size() * sizeof(float2), cudaMemcpyHostToDevice, c->stream),
-           "H2D phase");
+        disp_phase_rows(c, betas, n_beta, n_beta);
         const size_t cols = static_cast<size_t>(n_beta) * nb * nx * 256;
         ck(c->disp_a.ensure(cols * sizeof(float)), "cudaMalloc(columns)");
         DispArgs a{};

@@ -11,7 +11,8 @@
 //                 of the first FFT stage (64 points a lane), one exchange
 //                 through its own shared memory; |X| is averaged over the
 //                 B-scan repeats (dispersion.py:101).
-//   k_top_sum     top_percentile: one CTA per (beta, B-scan) finds the exact
+//   k_phase       the phase rows of a list of betas, in float64.
+//   k_top_sum     top_percentile: 1 to 8 CTAs per (beta, B-scan) find the exact
 //                 k-th largest magnitude by a three-digit radix select on the
 //                 float bits (12 + 11 + 8 bits, histograms in shared memory),
 //                 then sums I = float32(A^2) in float64 over the top k
@@ -23,6 +24,7 @@
 // float64, optionally ignoring NaN (nanmedian), by a bitonic sort per column
 // in shared memory (one warp per column); or, in mean mode, the float64 mean
 // of the column's non-NaN values.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -120,10 +122,23 @@ __global__ void __launch_bounds__(kDispWarps * 32, 3) k_disp_mag(const DispArgs 
     }
 }
 
-// ---------------------------------------------------------------- block helpers (1024 threads)
-constexpr int kSelThreads = 1024;
+// Phase rows exp(-i beta dk^2), formed in float64, rounded to complex64
+// (dispersion.py:88-89) and scaled by 1/N, one thread a sample.
+__global__ void __launch_bounds__(256) k_phase(const double* __restrict__ betas, const double* __restrict__ dk2,
+                                               int n, float2* __restrict__ phase) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= n * kN) return;
+    double s, c;
+    sincos(betas[i / kN] * dk2[i % kN], &s, &c);
+    phase[i] = make_float2(static_cast<float>(c) * (1.0f / kN), static_cast<float>(-s) * (1.0f / kN));
+}
+
+// ---------------------------------------------------------------- block helpers
+constexpr int kSelThreads = 1024;                // k_moments
+constexpr int kTopThreads = 512;                 // k_top_sum
 
 // Inclusive prefix sum of one value per thread over the block.
+template <int kThr>
 __device__ __forceinline__ unsigned int block_inclusive_scan(unsigned int v, unsigned int* warp_tot) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
@@ -134,7 +149,7 @@ __device__ __forceinline__ unsigned int block_inclusive_scan(unsigned int v, uns
     if (lane == 31) warp_tot[w] = v;
     __syncthreads();
     if (w == 0) {
-        unsigned int t = warp_tot[lane];
+        unsigned int t = lane < kThr / 32 ? warp_tot[lane] : 0u;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const unsigned int u = __shfl_up_sync(0xffffffffu, t, o);
@@ -150,15 +165,16 @@ __device__ __forceinline__ unsigned int block_inclusive_scan(unsigned int v, uns
 
 // The bin (counted from the top) holding the need-th largest element, and the
 // number of elements in the bins above it.  hist has nbins entries.
+template <int kThr>
 __device__ __forceinline__ void find_from_top(const unsigned int* hist, int nbins, unsigned int need,
                                               unsigned int* warp_tot, int* bin_out, unsigned int* above_out) {
-    const int chunk = (nbins + kSelThreads - 1) / kSelThreads;
+    const int chunk = (nbins + kThr - 1) / kThr;
     const int lo = threadIdx.x * chunk, hi = min(lo + chunk, nbins);
     unsigned int c = 0;
     for (int b = lo; b < hi; ++b) c += hist[b];
-    const unsigned int incl = block_inclusive_scan(c, warp_tot);
+    const unsigned int incl = block_inclusive_scan<kThr>(c, warp_tot);
     __shared__ unsigned int total_s;
-    if (threadIdx.x == kSelThreads - 1) total_s = incl;
+    if (threadIdx.x == kThr - 1) total_s = incl;
     __syncthreads();
     const unsigned int above = total_s - incl;     // elements in bins >= hi
     if (c > 0 && above < need && above + c >= need) {
@@ -183,7 +199,7 @@ __device__ __forceinline__ double block_sum_f64(double v, double* red) {
     __syncthreads();
     double t = 0.0;
     if (w == 0) {
-        t = red[lane];
+        t = lane < static_cast<int>(blockDim.x >> 5) ? red[lane] : 0.0;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
         if (lane == 0) red[0] = t;
@@ -213,65 +229,138 @@ __device__ __forceinline__ double block_max_f64(double v, double* red) {
     return t;
 }
 
-// One CTA per segment (beta, B-scan) of A (nx rows of kHalf magnitudes);
-// thread t reads depth z_min + t of every row (z_min + 1024 >= kHalf).
-__global__ void __launch_bounds__(kSelThreads, 1) k_top_sum(const float* __restrict__ A, int nx, int z_min,
+// top_percentile of a segment (beta, B-scan) of A (nx rows of kHalf
+// magnitudes): a cluster of C CTAs, each with its share of the rows, counts
+// the first digit, collects the elements of the digit's bin (each thread its
+// own, in its own slots, so that the order of every sum is fixed) while it sums
+// the larger ones, and decides the other two digits among the collected ones:
+// two passes over the magnitudes.  Rank 0's histogram gathers the cluster's
+// through distributed shared memory.  C (set by the launcher) fills the GPU
+// when there are few segments (the search's refinement rounds have 1 to 9).
+// Bound by DRAM: 410 segments of 500 rows (840 MB, read twice) in 315 us =
+// 5.3 TB/s; one CTA a segment reading four times, a float a load, took 1304 us.
+constexpr int kTopSlots = 24;                     // collected elements of a thread; past them it reads A again
+
+struct TopSmem {
+    unsigned int hist[4096];
+    unsigned int warp_tot[32];
+    double red[32];
+    int bin;
+    unsigned int above;
+    double part[8];                               // rank 0: the CTAs' sums
+    unsigned int cand[kTopSlots][kTopThreads];
+};
+
+__global__ void __launch_bounds__(kTopThreads, 3) k_top_sum(const float* __restrict__ A, int nx, int z_min,
                                                             unsigned int k, double* __restrict__ score) {
-    __shared__ unsigned int hist[4096];
-    __shared__ unsigned int warp_tot[32];
-    __shared__ double red[32];
-    __shared__ int bin_s;
-    __shared__ unsigned int above_s;
-    const float* seg = A + static_cast<int64_t>(blockIdx.x) * nx * kHalf;
-    const int z = z_min + threadIdx.x;
-    const bool act = z < kHalf;
-    // pass 1: bits 31..19
-    for (int b = threadIdx.x; b < 4096; b += kSelThreads) hist[b] = 0u;
-    __syncthreads();
-    if (act)
-        for (int x = 0; x < nx; ++x) atomicAdd(&hist[__float_as_uint(seg[static_cast<int64_t>(x) * kHalf + z]) >> 19], 1u);
-    __syncthreads();
-    find_from_top(hist, 4096, k, warp_tot, &bin_s, &above_s);
-    const unsigned int p1 = static_cast<unsigned int>(bin_s);
-    unsigned int gt = above_s;
-    __syncthreads();
-    // pass 2: bits 18..8 among prefix p1
-    for (int b = threadIdx.x; b < 2048; b += kSelThreads) hist[b] = 0u;
-    __syncthreads();
-    if (act)
-        for (int x = 0; x < nx; ++x) {
-            const unsigned int key = __float_as_uint(seg[static_cast<int64_t>(x) * kHalf + z]);
-            if ((key >> 19) == p1) atomicAdd(&hist[(key >> 8) & 0x7ffu], 1u);
+    namespace cg = cooperative_groups;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    TopSmem& S = *reinterpret_cast<TopSmem*>(smem_raw);
+    cg::cluster_group cl = cg::this_cluster();
+    const int C = static_cast<int>(cl.num_blocks()), rank = static_cast<int>(cl.block_rank());
+    TopSmem& S0 = *cl.map_shared_rank(&S, 0);
+    const int tid = threadIdx.x;
+    const int x0 = static_cast<int>(static_cast<int64_t>(nx) * rank / C);
+    const int x1 = static_cast<int>(static_cast<int64_t>(nx) * (rank + 1) / C);
+    const float* seg = A + (static_cast<int64_t>(blockIdx.x / C) * nx + x0) * kHalf;
+    const bool vec = (reinterpret_cast<uintptr_t>(A) & 15u) == 0;   // a caller's buffer may be aligned to a float only
+    // four depths a load: group q = i % 256 of row i / 256
+    const int n4 = (x1 - x0) * (kHalf / 4);
+    auto each = [&](auto&& f) {
+        constexpr int kU = 4;                     // loads in flight
+        for (int i0 = tid; i0 < n4; i0 += kU * kTopThreads) {
+            float4 v[kU];
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                const int i = i0 + u * kTopThreads;
+                if (i >= n4) continue;
+                const float* p = seg + 4 * static_cast<int64_t>(i);
+                v[u] = vec ? __ldg(reinterpret_cast<const float4*>(p))
+                           : make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+            }
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                const int i = i0 + u * kTopThreads;
+                const int z = 4 * (i & (kHalf / 4 - 1));
+                if (i >= n4 || z + 3 < z_min) continue;
+                if (z >= z_min) f(__float_as_uint(v[u].x) & 0x7fffffffu);
+                if (z + 1 >= z_min) f(__float_as_uint(v[u].y) & 0x7fffffffu);
+                if (z + 2 >= z_min) f(__float_as_uint(v[u].z) & 0x7fffffffu);
+                f(__float_as_uint(v[u].w) & 0x7fffffffu);
+            }
         }
-    __syncthreads();
-    find_from_top(hist, 2048, k - gt, warp_tot, &bin_s, &above_s);
-    const unsigned int p2 = (p1 << 11) | static_cast<unsigned int>(bin_s);
-    gt += above_s;
-    __syncthreads();
-    // pass 3: bits 7..0 among prefix p2
-    for (int b = threadIdx.x; b < 256; b += kSelThreads) hist[b] = 0u;
-    __syncthreads();
-    if (act)
-        for (int x = 0; x < nx; ++x) {
-            const unsigned int key = __float_as_uint(seg[static_cast<int64_t>(x) * kHalf + z]);
-            if ((key >> 8) == p2) atomicAdd(&hist[key & 0xffu], 1u);
+    };
+    // the digit's bin holding the need-th largest element of the cluster's
+    // histograms, and the elements above it
+    auto decide = [&](int nbins, unsigned int need, unsigned int& above) -> unsigned int {
+        if (rank != 0) {
+            __syncthreads();
+            for (int b = tid; b < nbins; b += kTopThreads)
+                if (S.hist[b] != 0u) atomicAdd(&S0.hist[b], S.hist[b]);
         }
-    __syncthreads();
-    find_from_top(hist, 256, k - gt, warp_tot, &bin_s, &above_s);
-    const unsigned int thr = (p2 << 8) | static_cast<unsigned int>(bin_s);
-    gt += above_s;
-    // pass 4: float64 sum of I = float32(A^2) above the threshold, in row order
+        cl.sync();
+        if (rank == 0) find_from_top<kTopThreads>(S.hist, nbins, need, S.warp_tot, &S.bin, &S.above);
+        cl.sync();
+        const unsigned int bin = static_cast<unsigned int>(S0.bin);
+        above = S0.above;
+        cl.sync();                                // read before the next digit's decision
+        return bin;
+    };
+    auto clear = [&](int nbins) {
+        for (int b = tid; b < nbins; b += kTopThreads) S.hist[b] = 0u;
+        cl.sync();                                // rank 0's is clear before the others add to it
+    };
+    unsigned int above;
+    clear(4096);
+    each([&](unsigned int key) { atomicAdd(&S.hist[key >> 19], 1u); });
+    const unsigned int p1 = decide(4096, k, above);        // bits 30..19
+    unsigned int gt = above;
+    // float64 sum of I = float32(A^2), in row order
+    auto square = [](unsigned int key) {
+        const float v = __uint_as_float(key);
+        return static_cast<double>(__fmul_rn(v, v));
+    };
     double s = 0.0;
-    if (act)
-        for (int x = 0; x < nx; ++x) {
-            const float v = seg[static_cast<int64_t>(x) * kHalf + z];
-            if (__float_as_uint(v) > thr) s += static_cast<double>(__fmul_rn(v, v));
+    int n = 0;
+    each([&](unsigned int key) {
+        const unsigned int p = key >> 19;
+        if (p < p1) return;
+        if (p > p1) {
+            s += square(key);
+        } else {
+            if (n < kTopSlots) S.cand[n][tid] = key;
+            ++n;
         }
-    s = block_sum_f64(s, red);
-    if (threadIdx.x == 0) {
-        const float tv = __uint_as_float(thr);
-        const double top = s + static_cast<double>(k - gt) * static_cast<double>(__fmul_rn(tv, tv));
-        score[blockIdx.x] = log(top / static_cast<double>(k));
+    });
+    auto each_cand = [&](auto&& f) {
+        if (n <= kTopSlots) {
+            for (int i = 0; i < n; ++i) f(S.cand[i][tid]);
+        } else {
+            each([&](unsigned int key) {
+                if ((key >> 19) == p1) f(key);
+            });
+        }
+    };
+    clear(2048);
+    each_cand([&](unsigned int key) { atomicAdd(&S.hist[(key >> 8) & 0x7ffu], 1u); });
+    const unsigned int p2 = (p1 << 11) | decide(2048, k - gt, above);
+    gt += above;
+    clear(256);
+    each_cand([&](unsigned int key) {
+        if ((key >> 8) == p2) atomicAdd(&S.hist[key & 0xffu], 1u);
+    });
+    const unsigned int thr = (p2 << 8) | decide(256, k - gt, above);
+    gt += above;
+    each_cand([&](unsigned int key) {
+        if (key > thr) s += square(key);
+    });
+    s = block_sum_f64(s, S.red);
+    if (tid == 0) S0.part[rank] = s;
+    cl.sync();
+    if (rank == 0 && tid == 0) {
+        double top = static_cast<double>(k - gt) * square(thr);
+        for (int r = 0; r < C; ++r) top += S.part[r];
+        score[blockIdx.x / C] = log(top / static_cast<double>(k));
     }
 }
 
@@ -411,11 +500,33 @@ cudaError_t launch_disp_mag(const DispArgs& a, int num_sms, cudaStream_t st) {
     return cudaGetLastError();
 }
 
+cudaError_t launch_phase(const double* betas, const double* dk2, int n, float2* phase, cudaStream_t st) {
+    k_phase<<<n * (kN / 256), 256, 0, st>>>(betas, dk2, n, phase);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_disp_metric(const float* A, int n_seg, int nx, int z_min, int metric, unsigned int top_k,
-                               double* score, cudaStream_t st) {
-    if (metric == 1)
-        k_top_sum<<<n_seg, kSelThreads, 0, st>>>(A, nx, z_min, top_k, score);
-    else
+                               double* score, int num_sms, cudaStream_t st) {
+    if (metric == 1) {
+        // three CTAs an SM: the widest cluster (1 to 8 CTAs a segment) that one wave holds
+        int C = 8;
+        while (C > 1 && (static_cast<int64_t>(n_seg) * C > 3 * num_sms || nx < C)) C >>= 1;
+        cudaError_t e = cudaFuncSetAttribute(k_top_sum, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             static_cast<int>(sizeof(TopSmem)));
+        if (e != cudaSuccess) return e;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = static_cast<unsigned int>(C);
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(static_cast<unsigned int>(n_seg * C));
+        cfg.blockDim = dim3(kTopThreads);
+        cfg.dynamicSmemBytes = sizeof(TopSmem);
+        cfg.stream = st;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, k_top_sum, A, nx, z_min, top_k, score);
+    } else
         k_moments<<<n_seg, kSelThreads, 0, st>>>(A, nx, z_min, metric, score);
     return cudaGetLastError();
 }

@@ -180,7 +180,9 @@ cudaError_t launch_disp_mag(const DispArgs& a, int num_sms, cudaStream_t st);
 // per segment (n_seg rows of nx x kHalf magnitudes): metric 1 top_percentile
 // (top_k elements), 2 kurtosis, 3 entropy, 4 legacy_peak, depths >= z_min
 cudaError_t launch_disp_metric(const float* A, int n_seg, int nx, int z_min, int metric, unsigned int top_k,
-                               double* score, cudaStream_t st);
+                               double* score, int num_sms, cudaStream_t st);
+// n phase rows exp(-i beta dk2) / N (complex64 of the float64 value)
+cudaError_t launch_phase(const double* betas, const double* dk2, int n, float2* phase, cudaStream_t st);
 // median over x of every (frame, z) column of (n_frames, nx, nz) float32, as float64
 cudaError_t launch_xmedian(const float* mag, int n_frames, int nx, int nz, int ignore_nan, int mean_mode,
                            double* out, cudaStream_t st);

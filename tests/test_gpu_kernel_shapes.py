@@ -31,3 +31,31 @@ def test_transform_of_loaded_lines(gpu_ctx, bscans, rep, nx):
         phase = np.exp(-1j * beta * dk2).astype(np.complex64).astype(np.complex128)
         ref = np.abs(np.fft.ifft(lines * phase)[..., :1024]).mean(1)
         assert np.abs(got - ref).max() < 1e-6 * ref.max()
+
+
+@pytest.mark.parametrize("bscans,nx,betas,z_min", [(1, 1, 1, 20), (1, 3, 1, 0), (1, 37, 2, 21), (2, 130, 3, 1000),
+                                                   (1, 900, 1, 20), (40, 9, 13, 20)])
+def test_top_percentile_of_returned_magnitudes(gpu_ctx, bscans, nx, betas, z_min):
+    """The score is the log of the mean of the k largest squared magnitudes:
+    against the magnitudes the same call returns (in a buffer aligned to one
+    float only), for clusters of 1 to 8 blocks, all elements equal included
+    (k of them tie).  Both sides sum float64 values of the same float32 squares:
+    1e-12."""
+    torch = pytest.importorskip("torch")
+    from oct_recon_af_v1_gb300 import estimation as E
+    from oct_recon_af_v1_gb300 import geometry as G
+    from oct_recon_af_v1_gb300 import synthetic
+    sg = G.build_spectral_geometry(synthetic.lambda_nm(), 0.0, 1.33)
+    gpu_ctx.set_geometry(sg.sinc_idx, sg.sinc_w, np.ones(2048, np.complex128))
+    gpu_ctx.disp_set_dk2(G.dispersion_dk2(sg))
+    raw = synthetic.generate_numpy(bscans, nx, 25, seed=6)
+    if nx == 9:
+        raw[:, 25:] = raw[:, 25:26]                     # identical A-scans: every value repeats nine times
+    gpu_ctx.disp_load(raw, 25, bscans, 1, E.hann_rms(2048))
+    n = nx * (1024 - z_min)
+    buf = torch.empty(betas * bscans * nx * 1024 + 1, dtype=torch.float32, device="cuda")
+    mag = buf[1:].view(betas, bscans, nx, 1024)
+    for k in (1, max(1, n // 100), n):
+        got = gpu_ctx.disp_eval(np.linspace(-2e7, 2e7, betas), 0, bscans, 1, k, z_min, mag=mag)
+        sq = np.sort((mag * mag).cpu().numpy()[..., z_min:].reshape(betas, bscans, n).astype(np.float64))[..., n - k:]
+        np.testing.assert_allclose(got, np.log(sq.mean(-1)), rtol=1e-12, atol=1e-12)
