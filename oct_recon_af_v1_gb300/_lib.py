@@ -177,6 +177,7 @@ class Context:
         self.device = int(device)
         self.n = None
         self.taps = None
+        self._pack = None                                    # packbits: host buffer of the largest image so far
 
     def close(self):
         if getattr(self, "h", None):
@@ -444,7 +445,9 @@ class Context:
             img = np.ascontiguousarray(img, dtype=np.uint16)
         p, loc = _ptr(img)
         cap = rows * (2 * cols + (2 * cols + 127) // 128 + 1)
-        out = np.empty(max(cap, 1), np.uint8)
+        if self._pack is None or self._pack.size < cap:      # touched pages are reused by the next plane
+            self._pack = np.empty(max(cap, 1), np.uint8)
+        out = self._pack
         sizes = np.empty(max(rows, 1), np.int32)
         total = ctypes.c_int64(0)
         self._check(self.lib.octgb_packbits(self.h, p, loc, rows, cols, out.ctypes.data, cap, sizes.ctypes.data,

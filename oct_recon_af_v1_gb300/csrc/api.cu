@@ -161,7 +161,7 @@ struct octgb_ctx {
     DevBuf magbuf, dbbuf, planemm, segs, qtable;
     DevBuf qcounter;                         // batched form: queue head
     // legacy TIFF encoding
-    DevBuf enc_bits, enc_lut, enc_slots, enc_sizes;
+    DevBuf enc_bits, enc_lut, enc_slots, enc_sizes, enc_offsets, enc_packed;
     // rare raw formats: prepared batch, frame-mean lines, per-file magnitudes
     DevBuf prep, prep_apod, magrep, srr, gemm_part;
     // precision form (tensor-core sinc)
@@ -502,7 +502,7 @@ int octgb_destroy(octgb_ctx* c) {
                       &c->den, &c->plan_table, &c->run_mm, &c->magbuf, &c->dbbuf, &c->planemm, &c->segs, &c->qtable,
                       &c->qcounter, &c->disp_x, &c->disp_hann, &c->disp_dk2, &c->disp_betas, &c->disp_phase, &c->disp_a, &c->disp_score, &c->xmed,
                       &c->prec_w, &c->prec_kb, &c->prec_hi, &c->prec_lo, &c->prec_m, &c->prec_x, &c->ex_w, &c->ex_win, &c->ex_tw, &c->bias_part, &c->wgrad_part, &c->prep,
-                      &c->prep_apod, &c->magrep, &c->srr, &c->gemm_part, &c->enc_bits, &c->enc_lut, &c->enc_slots, &c->enc_sizes})
+                      &c->prep_apod, &c->magrep, &c->srr, &c->gemm_part, &c->enc_bits, &c->enc_lut, &c->enc_slots, &c->enc_sizes, &c->enc_offsets, &c->enc_packed})
         b->release();
     for (QTable* t : c->qtables) {
         t->buf.release();
@@ -1268,7 +1268,7 @@ int octgb_graph_end(octgb_ctx* c, int* graph_id) {
                           &c->run_mm, &c->magbuf, &c->dbbuf, &c->planemm, &c->segs, &c->qtable, &c->qcounter,
                           &c->disp_x, &c->disp_hann, &c->disp_dk2, &c->disp_betas, &c->disp_phase, &c->disp_a, &c->disp_score, &c->xmed,
                           &c->prec_hi, &c->prec_lo, &c->prec_m, &c->prec_x, &c->prep, &c->prep_apod,
-                          &c->magrep, &c->srr, &c->gemm_part, &c->enc_bits, &c->enc_lut, &c->enc_slots, &c->enc_sizes})
+                          &c->magrep, &c->srr, &c->gemm_part, &c->enc_bits, &c->enc_lut, &c->enc_slots, &c->enc_sizes, &c->enc_offsets, &c->enc_packed})
             b->keep_old = true;
         for (int k = 0; k < octgb_ctx::kRing; ++k) c->ring[k].keep_old = true;
         c->launches.store(c->capture_launch0);
@@ -1604,27 +1604,26 @@ int octgb_packbits(octgb_ctx* c, const uint16_t* img, int img_loc, int rows, int
                "H2D image");
             src = c->enc_bits.as<uint16_t>();
         }
-        const int slot = packbits_slot(cols);
-        ck(c->enc_slots.ensure(static_cast<size_t>(rows) * slot), "cudaMalloc(slots)");
+        const size_t cap = static_cast<size_t>(rows) * packbits_slot(cols);
+        ck(c->enc_slots.ensure(cap), "cudaMalloc(slots)");
+        ck(c->enc_packed.ensure(cap), "cudaMalloc(packed rows)");
         ck(c->enc_sizes.ensure(static_cast<size_t>(rows) * sizeof(int)), "cudaMalloc(sizes)");
-        ck(launch_packbits(src, rows, cols, c->enc_slots.as<uint8_t>(), c->enc_sizes.as<int>(), c->stream),
-           "packbits kernel");
-        c->launches++;
-        std::vector<uint8_t> h(static_cast<size_t>(rows) * slot);
+        ck(c->enc_offsets.ensure((static_cast<size_t>(rows) + 1) * sizeof(long long)), "cudaMalloc(row offsets)");
+        ck(launch_packbits(src, rows, cols, c->enc_slots.as<uint8_t>(), c->enc_sizes.as<int>(),
+                           c->enc_offsets.as<long long>(), c->enc_packed.as<uint8_t>(), c->stream),
+           "packbits kernels");
+        c->launches += 3;
         ck(cudaMemcpyAsync(row_sizes, c->enc_sizes.p, static_cast<size_t>(rows) * sizeof(int), cudaMemcpyDeviceToHost,
                            c->stream),
            "D2H sizes");
-        ck(cudaMemcpyAsync(h.data(), c->enc_slots.p, h.size(), cudaMemcpyDeviceToHost, c->stream), "D2H slots");
         check_status(c);
-        int64_t off = 0;
-        for (int r = 0; r < rows; ++r) off += row_sizes[r];
-        require(off <= capacity, "output capacity too small for the packed image");
-        off = 0;
-        for (int r = 0; r < rows; ++r) {
-            memcpy(out + off, h.data() + static_cast<size_t>(r) * slot, row_sizes[r]);
-            off += row_sizes[r];
-        }
-        *total = off;
+        int64_t bytes = 0;
+        for (int r = 0; r < rows; ++r) bytes += row_sizes[r];
+        require(bytes <= capacity, "output capacity too small for the packed image");
+        ck(cudaMemcpyAsync(out, c->enc_packed.p, static_cast<size_t>(bytes), cudaMemcpyDeviceToHost, c->stream),
+           "D2H packed rows");
+        check_status(c);
+        *total = bytes;
     });
 }
 

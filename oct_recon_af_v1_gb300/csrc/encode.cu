@@ -8,11 +8,13 @@
 //                   operations (bits_to_db then db_to_bits, :33-45), replaces
 //                   the per-voxel float64 work; k_apply_lut maps the codes.
 //   k_packbits_rows PackBits (TIFF compression 32773) of every image row on
-//                   its own (TIFF 6.0 packs rows separately), one thread per
+//                   its own (TIFF 6.0 packs rows separately), one warp per
 //                   row, little-endian sample bytes: a run of >= 3 equal bytes
 //                   (up to 128) becomes a repeat packet, everything else
 //                   literal packets of up to 128 bytes.  Each row is written to
 //                   its own worst-case slot; its byte count goes to sizes[].
+//   k_row_offsets, k_pack_rows   the rows' bytes without gaps, so that only
+//                   they cross to the host.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -49,41 +51,110 @@ __global__ void k_apply_lut(uint16_t* __restrict__ bits, int64_t n, const uint16
         bits[i] = lut[bits[i]];
 }
 
-__device__ __forceinline__ uint8_t row_byte(const uint16_t* row, int k) {
-    return static_cast<uint8_t>(row[k >> 1] >> ((k & 1) * 8));
-}
-
-__global__ void k_packbits_rows(const uint16_t* __restrict__ img, int rows, int cols, uint8_t* __restrict__ out,
-                                int slot, int* __restrict__ sizes) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+// The row is a chain of packets, so a warp walks it packet by packet: lane l
+// holds the bytes i + 4 l .. + 3 of the 128 that a packet starting at i can
+// cover, and one ballot finds where the run or the literal ends.  Bound by the
+// latency of that chain (about 35 packets of 128 bytes a row of 1900 codes);
+// 1767 such rows take 32 us, and one thread a row (14 CTAs) took 1183.
+constexpr int kPackWarps = 4;
+__global__ void __launch_bounds__(kPackWarps * 32) k_packbits_rows(const uint16_t* __restrict__ img, int rows,
+                                                                   int cols, uint8_t* __restrict__ out, int slot,
+                                                                   int* __restrict__ sizes) {
+    const int r = blockIdx.x * kPackWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (r >= rows) return;
-    const uint16_t* row = img + static_cast<int64_t>(r) * cols;
+    const uint8_t* row = reinterpret_cast<const uint8_t*>(img + static_cast<int64_t>(r) * cols);   // little-endian
     uint8_t* o = out + static_cast<int64_t>(r) * slot;
     const int n = 2 * cols;
-    int i = 0, w = 0;
-    while (i < n) {
-        const uint8_t b = row_byte(row, i);
-        int run = 1;
-        while (i + run < n && run < 128 && row_byte(row, i + run) == b) ++run;
-        if (run >= 3) {
-            o[w++] = static_cast<uint8_t>(1 - run);       // -(run - 1)
-            o[w++] = b;
-            i += run;
-            continue;
+    int w = 0;
+    for (int i = 0; i < n;) {
+        const int j0 = i + 4 * lane;
+        // bytes j0 .. j0 + 5; past the row: distinct values that equal nothing
+        int c[6];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) c[e] = j0 + e < n ? __ldg(row + j0 + e) : 256 + e;
+#pragma unroll
+        for (int e = 4; e < 6; ++e) {
+            c[e] = __shfl_down_sync(0xffffffffu, c[e - 4], 1);
+            if (lane == 31) c[e] = j0 + e < n ? __ldg(row + j0 + e) : 260 + e;
         }
-        int j = i;
-        while (j < n && j - i < 128) {
-            if (j + 2 < n) {
-                const uint8_t c = row_byte(row, j);
-                if (row_byte(row, j + 1) == c && row_byte(row, j + 2) == c) break;
+        // first place of the lane's four where the run of b[i] ends, and where three equal bytes start
+        int ends = 4, three = 4;
+#pragma unroll
+        for (int e = 3; e >= 0; --e) {
+            if (c[e] != c[e + 1]) ends = e;
+            if (c[e] == c[e + 1] && c[e] == c[e + 2]) three = e;
+        }
+        const bool repeat = __shfl_sync(0xffffffffu, three, 0) == 0;
+        const int mine = repeat ? ends : three;
+        const unsigned int found = __ballot_sync(0xffffffffu, mine < 4);
+        const int at = found ? __ffs(static_cast<int>(found)) - 1 : 0;
+        const int first = 4 * at + __shfl_sync(0xffffffffu, mine, at);
+        if (repeat) {
+            const int run = found && first < 127 ? first + 1 : 128;
+            if (lane == 0) {
+                o[w] = static_cast<uint8_t>(1 - run);     // -(run - 1)
+                o[w + 1] = static_cast<uint8_t>(c[0]);
             }
-            ++j;
+            w += 2;
+            i += run;
+        } else {
+            const int left = n - i < 128 ? n - i : 128;
+            const int len = found && first < left ? first : left;
+            if (lane == 0) o[w] = static_cast<uint8_t>(len - 1);
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (4 * lane + e < len) o[w + 1 + 4 * lane + e] = static_cast<uint8_t>(c[e]);
+            w += 1 + len;
+            i += len;
         }
-        o[w++] = static_cast<uint8_t>(j - i - 1);
-        for (int k = i; k < j; ++k) o[w++] = row_byte(row, k);
-        i = j;
     }
-    sizes[r] = w;
+    if (lane == 0) sizes[r] = w;
+}
+
+// offsets[r] = bytes of the rows before r (offsets[rows]: of all); one CTA
+__global__ void __launch_bounds__(1024) k_row_offsets(const int* __restrict__ sizes, int rows,
+                                                      long long* __restrict__ offsets) {
+    __shared__ long long tot[32];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    long long base = 0;
+    for (int r0 = 0; r0 < rows; r0 += 1024) {
+        const int r = r0 + tid;
+        const long long v = r < rows ? sizes[r] : 0;
+        long long t = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long u = __shfl_up_sync(0xffffffffu, t, o);
+            if (lane >= o) t += u;
+        }
+        if (lane == 31) tot[w] = t;
+        __syncthreads();
+        long long before = 0, all = 0;
+        for (int k = 0; k < 32; ++k) {
+            if (k < w) before += tot[k];
+            all += tot[k];
+        }
+        if (r < rows) offsets[r] = base + before + t - v;
+        base += all;
+        __syncthreads();
+    }
+    if (tid == 0) offsets[rows] = base;
+}
+
+// one CTA a row: whole destination words, each from two source words
+__global__ void __launch_bounds__(128) k_pack_rows(const uint8_t* __restrict__ slots, int slot,
+                                                   const int* __restrict__ sizes,
+                                                   const long long* __restrict__ offsets, uint8_t* __restrict__ out) {
+    const int r = blockIdx.x, n = sizes[r];
+    const uint8_t* src = slots + static_cast<int64_t>(r) * slot;      // slot: a multiple of 4, with 4 bytes to spare
+    uint8_t* dst = out + offsets[r];
+    const int head = static_cast<int>((4 - (reinterpret_cast<uintptr_t>(dst) & 3u)) & 3u);
+    const int h = head < n ? head : n, words = (n - h) / 4;
+    const uint32_t* s4 = reinterpret_cast<const uint32_t*>(src);
+    uint32_t* d4 = reinterpret_cast<uint32_t*>(dst + h);
+    for (int i = threadIdx.x; i < words; i += 128) d4[i] = __funnelshift_r(s4[i], s4[i + 1], 8 * h);
+    if (static_cast<int>(threadIdx.x) < h) dst[threadIdx.x] = src[threadIdx.x];
+    const int tail = h + 4 * words;
+    if (static_cast<int>(threadIdx.x) < n - tail) dst[tail + threadIdx.x] = src[tail + threadIdx.x];
 }
 
 int grid_n(int64_t n) {
@@ -100,10 +171,16 @@ cudaError_t launch_requant(uint16_t* bits, int64_t n, double p1, double p2, doub
     return cudaGetLastError();
 }
 
-int packbits_slot(int cols) { return 2 * cols + (2 * cols + 127) / 128 + 1; }
+// the worst case of a row (whole words, and one that k_pack_rows may read past the last byte)
+int packbits_slot(int cols) { return ((2 * cols + (2 * cols + 127) / 128 + 1 + 3) & ~3) + 4; }
 
-cudaError_t launch_packbits(const uint16_t* img, int rows, int cols, uint8_t* out, int* sizes, cudaStream_t st) {
-    k_packbits_rows<<<(rows + 127) / 128, 128, 0, st>>>(img, rows, cols, out, packbits_slot(cols), sizes);
+cudaError_t launch_packbits(const uint16_t* img, int rows, int cols, uint8_t* slots, int* sizes, long long* offsets,
+                            uint8_t* out, cudaStream_t st) {
+    const int slot = packbits_slot(cols);
+    k_packbits_rows<<<(rows + kPackWarps - 1) / kPackWarps, kPackWarps * 32, 0, st>>>(img, rows, cols, slots, slot,
+                                                                                      sizes);
+    k_row_offsets<<<1, 1024, 0, st>>>(sizes, rows, offsets);
+    k_pack_rows<<<rows, 128, 0, st>>>(slots, slot, sizes, offsets, out);
     return cudaGetLastError();
 }
 

@@ -207,7 +207,9 @@ cudaError_t launch_avg_repeats(const float* mag, int n_frames, int nb, int size_
 cudaError_t launch_requant(uint16_t* bits, int64_t n, double p1, double p2, double c1, double c2, uint16_t* lut,
                            cudaStream_t st);
 int packbits_slot(int cols);
-cudaError_t launch_packbits(const uint16_t* img, int rows, int cols, uint8_t* out, int* sizes, cudaStream_t st);
+// slots: rows x packbits_slot(cols) bytes of scratch; offsets: rows + 1; out: the rows' bytes, one after the other
+cudaError_t launch_packbits(const uint16_t* img, int rows, int cols, uint8_t* slots, int* sizes, long long* offsets,
+                            uint8_t* out, cudaStream_t st);
 
 // precision form (precision.cu): tensor-core sinc
 constexpr int kPM = 128;                 // A-scans per tile (MMA M)

@@ -59,3 +59,24 @@ def test_top_percentile_of_returned_magnitudes(gpu_ctx, bscans, nx, betas, z_min
         got = gpu_ctx.disp_eval(np.linspace(-2e7, 2e7, betas), 0, bscans, 1, k, z_min, mag=mag)
         sq = np.sort((mag * mag).cpu().numpy()[..., z_min:].reshape(betas, bscans, n).astype(np.float64))[..., n - k:]
         np.testing.assert_allclose(got, np.log(sq.mean(-1)), rtol=1e-12, atol=1e-12)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 1), (3, 2), (5, 63), (4, 64), (2, 65), (130, 129), (1030, 7), (3, 5001)])
+def test_packbits_rows(gpu_ctx, rows, cols):
+    """Packets around the 128-byte limit, runs that end at a packet's or a
+    row's end, more rows than one scan block: the oracle's bytes exactly."""
+    from oracle import numerics as O
+    rng = np.random.default_rng(rows * 7919 + cols)
+    img = rng.integers(0, 65536, size=(rows, cols)).astype(np.uint16)
+    for r in range(rows):
+        x = 0
+        while x < cols:                                    # literals and runs of every length, byte runs of two kinds
+            n = int(rng.integers(1, 140))
+            v = rng.integers(0, 4)
+            if v < 2:
+                img[r, x:x + n] = (0, 0x4141, 0x0041, 0xffff)[int(rng.integers(0, 4))]
+            x += n
+    packed, sizes = gpu_ctx.packbits(img)
+    ref = [O.packbits_encode_row(img[r].astype("<u2").tobytes()) for r in range(rows)]
+    assert [int(s) for s in sizes] == [len(b) for b in ref]
+    assert packed == b"".join(ref)
