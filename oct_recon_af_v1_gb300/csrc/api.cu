@@ -1035,15 +1035,19 @@ bool prep_args(PrepArgs& a, const void* raw, int B, int n_lines, int apod, int b
 }
 
 // prepared batch on the device (c->prep, float32 (B, a_out + n_kept, N))
-void run_prepare(octgb_ctx* c, const PrepArgs& a0, int dtype, int loc) {
+// into c->prep, or into `out` (device, 16-byte aligned)
+void run_prepare(octgb_ctx* c, const PrepArgs& a0, int dtype, int loc, float* out = nullptr) {
     PrepArgs a = a0;
     const size_t bytes = static_cast<size_t>(a.B) * a.n_lines * kN * raw_elem(dtype);
     a.raw = stage_raw(c, a.raw, dtype, loc, bytes);
-    ck(c->prep.ensure(static_cast<size_t>(a.B) * (a.a_out + a.n_kept) * kN * sizeof(float) + 16),
-       "cudaMalloc(prepared)");
+    if (out == nullptr) {
+        ck(c->prep.ensure(static_cast<size_t>(a.B) * (a.a_out + a.n_kept) * kN * sizeof(float) + 16),
+           "cudaMalloc(prepared)");
+        out = c->prep.as<float>();
+    }
     if (a.mode == 1)
         ck(c->prep_apod.ensure(static_cast<size_t>(a.B / a.group) * kN * sizeof(float)), "cudaMalloc(frame mean)");
-    ck(launch_prepare(a, dtype, c->prep_apod.as<float>(), c->prep.as<float>(), c->stream), "prepare kernel");
+    ck(launch_prepare(a, dtype, c->prep_apod.as<float>(), out, c->stream), "prepare kernel");
     c->launches += a.mode == 1 ? 2 : 1;
 }
 }  // namespace
@@ -1639,8 +1643,10 @@ int octgb_prepare_raw(octgb_ctx* c, const void* raw, int dtype, int loc, int B, 
         prep_args(a, raw, B, n_lines, apod, binning, apod_mode, apod_group);
         *out_lines = a.a_out + a.n_kept;
         if (B == 0) return;
-        run_prepare(c, a, dtype, loc);
-        copy_out(c, out, out_loc, c->prep.p, static_cast<size_t>(B) * (a.a_out + a.n_kept) * kN * sizeof(float));
+        const bool direct = out_loc == OCTGB_DEVICE && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+        run_prepare(c, a, dtype, loc, direct ? out : nullptr);
+        if (!direct)
+            copy_out(c, out, out_loc, c->prep.p, static_cast<size_t>(B) * (a.a_out + a.n_kept) * kN * sizeof(float));
         check_status(c);
     });
 }

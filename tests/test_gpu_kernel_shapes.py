@@ -80,3 +80,26 @@ def test_packbits_rows(gpu_ctx, rows, cols):
     ref = [O.packbits_encode_row(img[r].astype("<u2").tobytes()) for r in range(rows)]
     assert [int(s) for s in sizes] == [len(b) for b in ref]
     assert packed == b"".join(ref)
+
+
+@pytest.mark.parametrize("nx,nz", [(1, 1), (2, 17), (31, 16), (32, 5), (33, 40), (256, 20), (257, 20), (512, 9),
+                                   (1024, 33), (1025, 9), (4096, 3)])
+def test_x_profiles_equal_numpy(gpu_ctx, nx, nz):
+    """Median, nanmedian and mean over x at the edges of the kernel's register
+    forms: ties, negative values, infinities and NaN, odd and even counts.
+    The medians are exact; a float64 mean of up to 4096 values: 1e-12."""
+    rng = np.random.default_rng(nx * 31 + nz)
+    mag = rng.normal(size=(2, nx, nz)).astype(np.float32)
+    mag[0] = np.round(mag[0])                                   # many ties, both zeros
+    np.testing.assert_array_equal(gpu_ctx.xmedian(mag), np.median(mag.astype(np.float64), axis=1))
+    np.testing.assert_allclose(gpu_ctx.xmean(mag), mag.astype(np.float64).mean(1), rtol=1e-12, atol=1e-12)
+    mag[1, rng.integers(0, nx, nx // 3), rng.integers(0, nz, nx // 3)] = np.nan
+    mag[0, nx // 2, 0] = np.inf
+    mag[1, 0, nz - 1] = -np.inf
+    mag[1, :, nz // 2] = np.nan
+    with np.errstate(all="ignore"):
+        import warnings
+        warnings.simplefilter("ignore", RuntimeWarning)
+        np.testing.assert_array_equal(gpu_ctx.xmedian(mag), np.median(mag.astype(np.float64), axis=1))
+        np.testing.assert_array_equal(gpu_ctx.xmedian(mag, ignore_nan=True),
+                                      np.nanmedian(mag.astype(np.float64), axis=1))
