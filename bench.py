@@ -14,8 +14,8 @@ legacy uint16 quantisation of the volume.
 spectral stage to dB, global clim, quantisation.
 `--config 2`: the config-1 tiles through the precision form of the spectral
 stage (exact background, tcgen05 split-FP16 sinc), beside the float32 form.
-`--config 3`: 64 tiles of uneven size in one persistent launch (device work
-queue, CUDA graph, autotuned grab / order), beside per-tile launches.
+`--config 3`: 64 tiles of uneven size in one call (CUDA graph, autotuned
+order), beside per-tile calls.
 `--config 4`: the learned beta/focus estimator trained on the device (20 k
 probe images), timed on 500 held-out B-scans against the GPU plain search.
 
@@ -381,7 +381,7 @@ def gpu_arm(args, rank, world):
         "gpu_launches": int(launches),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                      "traffic": SPECTRAL_DRAM_BYTES_PER_ASCAN * kascans,
-                     "kernel": "spectral stage (apod mean + k_spectral, magnitude out)",
+                     "kernel": "spectral stage (apod mean + k_lines + k_disp_mag, magnitude out)",
                      "bytes_per_launch": kbytes, "ms_per_launch": kms, "a_scans_per_launch": kascans,
                      "peak_source": src + " (burst copy)",
                      # the arithmetic intensity (~21 flop/B) is above the FP32 ridge: the same
@@ -507,7 +507,7 @@ def config3_specs(seed=3, n_tiles=64):
 def config3_desc(specs):
     a = sum(b * nx for b, nx, _ in specs)
     return {"workload": f"config3: {len(specs)} tiles of uneven size (A-scans U[300,1200], B-scans U[50,300], "
-                        "z-crop U[400,1500] px at 1 um), 2048 uint16 spectra, one persistent launch",
+                        "z-crop U[400,1500] px at 1 um), 2048 uint16 spectra, one call",
             "a_scans_per_step": a, "tiles": len(specs), "l2_flush": "inputs larger than L2"}
 
 
@@ -581,7 +581,7 @@ def gpu_arm_config3(args, rank, world, torch, ctx, stream, dev):
         torch.cuda.synchronize()
         return e0.elapsed_time(e1) / steps, ctx.launches - n0
 
-    # the last tuning choice: the persistent queue launch or one launch per
+    # the last tuning choice: one call for all tiles or one call per
     # tile, both captured in a graph (the same kernels and results)
     # (five interleaved rounds of 3 steps each, medians, with the SM clock
     # sampled meanwhile: the two forms differ by a few per cent)
@@ -660,12 +660,12 @@ def gpu_arm_config3(args, rank, world, torch, ctx, stream, dev):
             "gpu_launches": int(launches),
             "roofline": {"bound": "hbm", "achieved": alg / (ms * 1e-3) / 1e9, "peak": hbm, "unit": "GB/s",
                          "frac": alg / (ms * 1e-3) / 1e9 / hbm, "traffic": None,
-                         "kernel": "whole step (apod + persistent spectral/resample + quantise)",
+                         "kernel": "whole step (apod + lines + transform + resample + quantise)",
                          "bytes_per_launch": alg, "peak_source": src + " (burst copy)"},
             "clocks": clk,
             "forms": {"chosen": form, "queue_ms": ms_queue, "per_tile_ms": ms_tiles,
                       "queue_ms_rounds": q_ms, "per_tile_ms_rounds": t_ms, "clocks": choice_clock,
-                      "note": "both CUDA graphs: the persistent queue launch over all tiles, or one apodisation "
+                      "note": "both CUDA graphs: one call over all tiles, or one apodisation "
                               "+ one spectral launch per tile; medians of 5 interleaved rounds, the faster one "
                               "is timed"},
             "e2e": {"value": ascans / (ms_e2e * 1e-3), "unit": "A-scans/s", "ms_per_step": ms_e2e,

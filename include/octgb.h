@@ -284,7 +284,7 @@ int octgb_graph_begin(octgb_ctx *ctx);
 int octgb_graph_end(octgb_ctx *ctx, int *graph_id);
 int octgb_graph_launch(octgb_ctx *ctx, int graph_id);
 /* Self-test of the bounded device waits (no counterpart in the reference):
- * runs the spectral kernel (which = 0) or the precision form's tensor-core
+ * runs the lines kernel (which = 0) or the precision form's tensor-core
  * sinc (which = 1, integer raws; needs a geometry with precision tiles) on a
  * small internal batch of zero raws, with the waits' limit cut to
  * wait_limit_us (100 .. 2 000 000) and each CTA's first row-copy barrier
@@ -322,13 +322,15 @@ typedef struct octgb_tile {
     float *db;
 } octgb_tile;
 
-/* Reconstruct n_tiles (<= 256) independent tiles of uneven sizes in ONE
- * persistent launch: every CTA takes `grab` groups of 4 A-scans at a time
- * from a device work queue spanning all tiles, runs the spectral stage and
- * resamples each depth profile with its tile's plan, finalising to dB
- * (threshold -> NaN, 20*log10(num/den), pipeline.py:296-300).  The finite
- * [min, max] folds into the running clim.  One apodisation launch precedes
- * it.  No host sync; graph-capturable once the same tile table has been run. */
+/* Reconstruct n_tiles (<= 256) independent tiles of uneven sizes, their
+ * A-scans numbered through and taken in passes of whole B-scans: lines,
+ * transform, then each depth profile resampled with its tile's plan and
+ * finalised to dB (threshold -> NaN, 20*log10(num/den), pipeline.py:296-300).
+ * The finite [min, max] folds into the running clim.  One apodisation launch
+ * precedes the passes.  `grab` (1 .. 4096) is accepted for callers of the
+ * earlier work queue and changes nothing: every block takes an equal,
+ * contiguous share.  No host sync; graph-capturable once the same tile table
+ * has been run. */
 int octgb_batch_process(octgb_ctx *ctx, int n_tiles, const octgb_tile *tiles, int raw_dtype, float threshold,
                         int grab);
 
@@ -449,10 +451,11 @@ int octgb_cnn_adam(octgb_ctx *ctx, float *p, const float *g, float *m, float *v,
  * synchronise the device and stall acquisition, or a process whose GPU
  * memory belongs to another framework's pool).  This entry point has no
  * counterpart in the reference.  raw (B, interf, n) and mag (B, interf-apod,
- * n/2) must be device pointers owned by the caller; the only scratch (the
- * apodisation mean) lives in a fixed array of 64 B-scans x n floats
- * (512 KiB) in the library image, held by every GPU that loads the library
- * until the process exits; B > 64 is rejected with OCTGB_ERR_ARG.  The call
+ * n/2) must be device pointers owned by the caller; the scratch is a fixed
+ * array of 64 B-scans x n floats (512 KiB, the apodisation mean) in the
+ * library image, held by every GPU that loads the library until the process
+ * exits, and 30 MiB of the context (lines of 3648 A-scans) allocated by
+ * octgb_set_geometry; B > 64 is rejected with OCTGB_ERR_ARG.  The call
  * makes no cudaMalloc/cudaFree.  The first call on a device looks up the
  * array's device address (cudaGetSymbolAddress); make that first call before
  * any stream capture.  All calls on a device share the array, so calls that

@@ -151,17 +151,22 @@ def _ptr(a):
     raise TypeError(f"unsupported array type {type(a)!r}")
 
 
+_TORCH_DTYPE: dict = {}          # torch dtype -> raw_dtype, filled when the first tensor comes
+
+
 def _raw_dtype(a) -> int:
     if isinstance(a, np.ndarray):
-        dt = a.dtype
+        code = _DTYPE.get(a.dtype)
     else:
-        import torch
-        dt = {torch.int16: np.dtype(np.int16), torch.float32: np.dtype(np.float32)}.get(a.dtype)
-        if dt is None and str(a.dtype) == "torch.uint16":
-            dt = np.dtype(np.uint16)
-    if dt not in _DTYPE:
-        raise TypeError(f"raw spectra must be uint16, int16 or float32, got {dt}")
-    return _DTYPE[dt]
+        if not _TORCH_DTYPE:
+            import torch
+            _TORCH_DTYPE.update({torch.int16: I16, torch.float32: F32})
+            if hasattr(torch, "uint16"):
+                _TORCH_DTYPE[torch.uint16] = U16
+        code = _TORCH_DTYPE.get(a.dtype)
+    if code is None:
+        raise TypeError(f"raw spectra must be uint16, int16 or float32, got {a.dtype}")
+    return code
 
 
 class Context:

@@ -1,11 +1,9 @@
-"""Launch-shape autotuners: the batched form's work queue (octgb_batch_process)
-and the frame API's stitch tile shape (octgb_set_stitch_rows).
+"""Launch-shape autotuners: the batched form (octgb_batch_process) and the
+frame API's stitch tile shape (octgb_set_stitch_rows).
 
-The persistent spectral kernel takes `grab` groups of 4 A-scans per atomic
-operation on the work queue: small grabs balance load across SMs at the end
-of the batch, large grabs cut queue traffic and keep each CTA on one tile
-(fewer tile switches and depth-table reloads).  The order of the tile table
-decides which tiles meet at the end of the queue.  `tune_batch` times every
+The order of the tile table decides which tiles share a pass of the batched
+form.  (`grab` belonged to an earlier work queue; the kernels' blocks now take
+equal shares, and its candidates time alike.)  `tune_batch` times every
 candidate (grab, order) on the actual batch with CUDA events on the launching
 stream, keeps the fastest, and caches it per batch signature (tile count and
 total A-scans, bucketed) for the life of the process.

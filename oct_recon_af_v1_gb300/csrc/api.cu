@@ -60,7 +60,7 @@ struct Plan {
     int cblk_first = 0, n_cblk = 0, xs_max = 1, rs_max = 1;
     std::vector<int2> zblk_h, cblk_h;   // host copies of the block tables
     bool lateral_identity = false;      // WxT is the identity (single-tile output grid)
-    bool lateral_quad_local = false;    // every non-zero lateral weight stays inside the column's B-scan quad
+    bool lateral_quad_local = false;    // every non-zero lateral weight stays inside the column's group of four
     DevBuf zr, wz0, wz1, xr, wx0, wx1, fz, shift, lo, hi, zblk, cblk, zrow, zf, xcol;
     bool opc = false;
     StitchDev dev() const {
@@ -140,13 +140,17 @@ struct octgb_ctx {
     std::string err;
     std::atomic<int> cancel{0};
     std::atomic<int64_t> launches{0};
+    uint64_t ready = 0;                      // kernels that have their shared memory (kernel_ready)
     // geometry
     bool has_geom = false;
     int taps = 0;
     int U = 0;
-    DevBuf w, start, win, tw, wsh, s0;
+    DevBuf start, win, tw, wsh, s0;
+    DevBuf lines;                // linearised lines of one pass (up to kMaxPass), grown by the calls
+    DevBuf lines_fixed;          // the allocation-free entry point's own (kMinPass), allocated with the geometry
     // work buffers
     DevBuf raw, apod, out, mm, frames;
+    DevBuf mm_empty;             // the range of no values (ordered uint [max, 0]), copied to reset a range
     int* status_host = nullptr;  // mapped pinned status word
     int* status_dev = nullptr;
     // plans and row state
@@ -159,7 +163,6 @@ struct octgb_ctx {
     bool capturing = false;
     int64_t capture_launch0 = 0;
     DevBuf magbuf, dbbuf, planemm, segs, qtable;
-    DevBuf qcounter;                         // batched form: queue head
     // legacy TIFF encoding
     DevBuf enc_bits, enc_lut, enc_slots, enc_sizes, enc_offsets, enc_packed;
     // rare raw formats: prepared batch, frame-mean lines, per-file magnitudes
@@ -255,57 +258,117 @@ void validate_raw(const void* raw, int dtype, int loc, int B, int interf, int ap
     if (loc == OCTGB_DEVICE) require((reinterpret_cast<uintptr_t>(raw) & 15u) == 0, "device raw must be 16-byte aligned");
 }
 
-// Launch apod mean + fused spectral kernel over n_seg device batches (same B, interf, apod).
-void launch_spectral_segs(octgb_ctx* c, const void* const* segs, int n_seg, int dtype, int B, int interf, int apod,
-                          int mode, float* out_dev, int z0, int nz, unsigned int* mm_dev,
-                          const double* hann = nullptr, const float2* hann2 = nullptr) {
-    if (B == 0 || n_seg == 0) return;
-    ck(c->apod.ensure(static_cast<size_t>(n_seg) * B * kN * sizeof(float) + 16), "cudaMalloc(apod)");
-    SpectralArgs a{};
-    a.raw = segs[0];
+// Arguments of the lines kernel over n_seg device batches (same B, interf, apod).
+LinesArgs lines_args(octgb_ctx* c, const void* const* segs, int n_seg, int B, int interf, int apod,
+                     const float* apod_mean) {
+    LinesArgs a{};
     for (int i = 0; i < n_seg; ++i) a.seg[i] = segs[i];
-    a.n_seg = n_seg;
     a.B = B;
     a.interf = interf;
     a.apod = apod;
     a.nx = interf - apod;
-    a.n_ascans = static_cast<int64_t>(n_seg) * B * (interf - apod);
-    a.apod_mean = c->apod.as<float>();
-    a.g.w = c->w.as<float>();
-    a.g.start = c->start.as<int>();
-    a.g.taps = c->taps;
+    a.apod_mean = apod_mean;
     a.g.win = c->win.as<float2>();
     a.g.tw = c->tw.as<float2>();
-    a.g.wsh = c->wsh.as<float>();
+    a.g.wsh = c->wsh.as<float2>();
     a.g.s0 = c->s0.as<int>();
     a.g.U = c->U;
-    a.out = out_dev;
-    a.z0 = z0;
-    a.nz = nz;
-    a.minmax = mm_dev;
-    a.hann = hann;
-    a.hann2 = hann2;
     a.status = c->status_dev;
-    ck(launch_apod_mean(a, dtype, c->stream), "apod kernel");
-    c->launches++;
-    const int64_t pairs = (a.n_ascans + kPerCta - 1) / kPerCta;
-    int64_t grid = static_cast<int64_t>(c->num_sms) * spectral_max_ctas_per_sm(dtype, mode);
-    if (grid > pairs) grid = pairs;
-    if (grid < 1) return;
-    ck(launch_spectral(a, dtype, mode, static_cast<int>(grid), c->stream), "spectral kernel");
-    c->launches++;
+    a.ready = &c->ready;
+    return a;
 }
 
-// Run the spectral stage of a batch into `out` (device) in the given mode.
-void run_spectral(octgb_ctx* c, const void* raw, int dtype, int loc, int B, int interf, int apod, int mode,
-                  float* out_dev, int z0, int nz, unsigned int* mm_dev, const double* hann = nullptr,
-                  const float2* hann2 = nullptr) {
+// A-scans of a pass of a call of `total`; the scratch grows to hold them.
+unsigned int pass_lines(octgb_ctx* c, unsigned int total) {
+    const unsigned int pass = std::min<unsigned int>(total, kMaxPass);
+    ck(c->lines.ensure(static_cast<size_t>(pass) * kN * sizeof(float)), "cudaMalloc(lines)");
+    return pass;
+}
+
+// Linearised lines of A-scans [l0, l1) into `scratch`, then their transform:
+// |X| or dB rows from `out` on.
+void transform_pass(octgb_ctx* c, LinesArgs a, float* scratch, int dtype, unsigned int l0, unsigned int l1, int mode, float* out,
+                    int z0, int nz, unsigned int* mm_dev) {
+    a.l0 = a.out_l0 = l0;
+    a.l1 = l1;
+    a.out = scratch;
+    ck(launch_lines(a, dtype, kModeReal, c->num_sms, c->stream), "lines kernel");
+    DispArgs d{};
+    d.X = a.out;
+    d.phase = a.g.win;
+    d.tw = a.g.tw;
+    d.A = out;
+    d.mode = mode;
+    d.z0 = z0;
+    d.nz = nz;
+    d.minmax = mm_dev;
+    d.n_beta = d.nb = d.rep = 1;
+    d.ready = &c->ready;
+    d.nx = static_cast<int>(l1 - l0);
+    ck(launch_disp_mag(d, c->num_sms, c->stream), "transform kernel");
+    c->launches += 2;
+}
+
+// |X| or dB of n_seg device batches, in passes through the lines' scratch.
+// With apod_mean (room for a row per B-scan) nothing is allocated: the passes
+// go through lines_fixed, which no other call uses or frees (a graph captured
+// by the caller may hold it).
+void launch_spectral_segs(octgb_ctx* c, const void* const* segs, int n_seg, int dtype, int B, int interf, int apod,
+                          int mode, float* out_dev, int z0, int nz, unsigned int* mm_dev, float* apod_mean = nullptr) {
+    if (B == 0 || n_seg == 0) return;
+    const int64_t n = static_cast<int64_t>(n_seg) * B * (interf - apod);
+    require(n < (int64_t(1) << 31), "batch too large");
+    const bool fixed = apod_mean != nullptr;         // no buffer may grow
+    if (!fixed) {
+        ck(c->apod.ensure(static_cast<size_t>(n_seg) * B * kN * sizeof(float) + 16), "cudaMalloc(apod)");
+        apod_mean = c->apod.as<float>();
+    }
+    const LinesArgs a = lines_args(c, segs, n_seg, B, interf, apod, apod_mean);
+    ck(launch_apod_mean(a, dtype, n_seg * B, apod_mean, c->stream), "apod kernel");
+    c->launches++;
+    const unsigned int total = static_cast<unsigned int>(n), pass = fixed ? kMinPass : pass_lines(c, total);
+    float* scratch = (fixed ? c->lines_fixed : c->lines).as<float>();
+    const int64_t row = mode == kModeDb ? nz : kHalf;
+    for (unsigned int l0 = 0, l1; l0 < total; l0 = l1) {
+        l1 = l0 + std::min(pass, total - l0);
+        transform_pass(c, a, scratch, dtype, l0, l1, mode, out_dev + l0 * row, z0, nz, mm_dev);
+    }
+}
+
+// What every entry point of the spectral stage checks first.
+void require_spectral(octgb_ctx* c) {
     if (!c->has_geom) throw Error(OCTGB_ERR_STATE, "octgb_set_geometry has not been called");
     if (c->cancel.load()) throw Error(OCTGB_ERR_CANCELLED, "cancelled");
+}
+
+// Run the spectral stage of a batch into `out` (device): |X| or dB.
+void run_spectral(octgb_ctx* c, const void* raw, int dtype, int loc, int B, int interf, int apod, int mode,
+                  float* out_dev, int z0, int nz, unsigned int* mm_dev) {
+    require_spectral(c);
     if (B == 0) return;  // empty batch: nothing to launch
     const size_t bytes = static_cast<size_t>(B) * interf * kN * raw_elem(dtype);
     const void* rd = stage_raw(c, raw, dtype, loc, bytes);
-    launch_spectral_segs(c, &rd, 1, dtype, B, interf, apod, mode, out_dev, z0, nz, mm_dev, hann, hann2);
+    launch_spectral_segs(c, &rd, 1, dtype, B, interf, apod, mode, out_dev, z0, nz, mm_dev);
+}
+
+// The lines of a batch (kModeSpec or kModeLinHann) into `out` (device, 16-byte aligned).
+void run_lines(octgb_ctx* c, const void* raw, int dtype, int loc, int B, int interf, int apod, int mode, float* out_dev,
+               const double* hann = nullptr, const float2* hann2 = nullptr) {
+    require_spectral(c);
+    if (B == 0) return;
+    const int64_t n = static_cast<int64_t>(B) * (interf - apod);
+    require(n < (int64_t(1) << 31), "batch too large");
+    const size_t bytes = static_cast<size_t>(B) * interf * kN * raw_elem(dtype);
+    const void* rd = stage_raw(c, raw, dtype, loc, bytes);
+    ck(c->apod.ensure(static_cast<size_t>(B) * kN * sizeof(float) + 16), "cudaMalloc(apod)");
+    LinesArgs a = lines_args(c, &rd, 1, B, interf, apod, c->apod.as<float>());
+    ck(launch_apod_mean(a, dtype, B, c->apod.as<float>(), c->stream), "apod kernel");
+    a.l1 = static_cast<unsigned int>(n);
+    a.out = out_dev;
+    a.hann = hann;
+    a.hann2 = hann2;
+    ck(launch_lines(a, dtype, mode, c->num_sms, c->stream), "lines kernel");
+    c->launches += 2;
 }
 
 void copy_out(octgb_ctx* c, void* dst, int loc, const void* src_dev, size_t bytes) {
@@ -313,6 +376,11 @@ void copy_out(octgb_ctx* c, void* dst, int loc, const void* src_dev, size_t byte
     ck(cudaMemcpyAsync(dst, src_dev, bytes, loc == OCTGB_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                        c->stream),
        "copy out");
+}
+
+void reset_minmax(octgb_ctx* c, unsigned int* mm_dev) {
+    ck(cudaMemcpyAsync(mm_dev, c->mm_empty.p, 2 * sizeof(unsigned int), cudaMemcpyDeviceToDevice, c->stream),
+       "reset range");
 }
 
 void read_minmax(octgb_ctx* c, const unsigned int* mm_dev, double* out2) {
@@ -474,6 +542,9 @@ int octgb_create(int device, octgb_ctx** out) {
         ck(cudaHostGetDevicePointer(reinterpret_cast<void**>(&c->status_dev), c->status_host, 0),
            "cudaHostGetDevicePointer");
         ck(c->mm.ensure(4096), "cudaMalloc(minmax)");
+        const unsigned int empty[2] = {0xffffffffu, 0u};
+        ck(c->mm_empty.ensure(sizeof(empty)), "cudaMalloc(empty range)");
+        ck(cudaMemcpy(c->mm_empty.p, empty, sizeof(empty), cudaMemcpyHostToDevice), "H2D empty range");
         *out = c;
         g_create_error.clear();
         return OCTGB_OK;
@@ -498,9 +569,9 @@ int octgb_destroy(octgb_ctx* c) {
             delete p;
         }
     }
-    for (DevBuf* b : {&c->w, &c->start, &c->win, &c->tw, &c->wsh, &c->s0, &c->raw, &c->apod, &c->out, &c->mm, &c->frames, &c->num,
+    for (DevBuf* b : {&c->start, &c->win, &c->tw, &c->wsh, &c->s0, &c->lines, &c->lines_fixed, &c->raw, &c->apod, &c->out, &c->mm, &c->mm_empty, &c->frames, &c->num,
                       &c->den, &c->plan_table, &c->run_mm, &c->magbuf, &c->dbbuf, &c->planemm, &c->segs, &c->qtable,
-                      &c->qcounter, &c->disp_x, &c->disp_hann, &c->disp_dk2, &c->disp_betas, &c->disp_phase, &c->disp_a, &c->disp_score, &c->xmed,
+                      &c->disp_x, &c->disp_hann, &c->disp_dk2, &c->disp_betas, &c->disp_phase, &c->disp_a, &c->disp_score, &c->xmed,
                       &c->prec_w, &c->prec_kb, &c->prec_hi, &c->prec_lo, &c->prec_m, &c->prec_x, &c->ex_w, &c->ex_win, &c->ex_tw, &c->bias_part, &c->wgrad_part, &c->prep,
                       &c->prep_apod, &c->magrep, &c->srr, &c->gemm_part, &c->enc_bits, &c->enc_lut, &c->enc_slots, &c->enc_sizes, &c->enc_offsets, &c->enc_packed})
         b->release();
@@ -576,10 +647,11 @@ int octgb_set_geometry(octgb_ctx* c, int n, int taps, const int64_t* idx, const 
             }
             st[i] = s;
         }
-        // shifted dense weights of the spectral kernel: thread t owns outputs
+        // shifted dense weights of the lines kernel: thread t owns outputs
         // 4t..4t+3 and reads the U source samples s0_t .. s0_t + U - 1; at step u
-        // it reads the one congruent to u (mod U), so wsh[t][r][u] = weight of
-        // source s0_t + v, (s0_t + v) = u (mod U), for output 4t + r.  With
+        // it reads the one congruent to u (mod U): the weight of source
+        // s0_t + v, (s0_t + v) = u (mod U), for output 4t + 2 h + e is the
+        // e-th of the pair wsh[h][u][t] (a warp reads consecutive pairs).  With
         // gcd(U, 32) = 2 the samples a warp reads at one step are U apart (or
         // the same sample): distinct banks of a linear line.
         std::vector<int> len(kN, 0);
@@ -588,7 +660,7 @@ int octgb_set_geometry(octgb_ctx* c, int n, int taps, const int64_t* idx, const 
                 if (!(t > 0 && idx[static_cast<size_t>(i) * taps + t] == 0)) len[i] = t + 1;
         }
         int U_need = 0;
-        for (int t = 0; t < kThreads; ++t) {
+        for (int t = 0; t < kSincThreads; ++t) {
             const int base = st[4 * t];
             for (int r = 0; r < 4; ++r) {
                 const int i = 4 * t + r;
@@ -598,36 +670,40 @@ int octgb_set_geometry(octgb_ctx* c, int n, int taps, const int64_t* idx, const 
             }
         }
         int U = U_need <= 14 ? 14 : (U_need <= 18 ? 18 : (U_need <= 22 ? 22 : (U_need <= 26 ? 26 : 0)));
-        require(U > 0, "sinc band too wide for the spectral kernel (4 outputs need > 26 source samples)");
-        std::vector<float> wsh(static_cast<size_t>(kThreads) * 4 * U, 0.f);
-        std::vector<int> s0v(kThreads);
-        for (int t = 0; t < kThreads; ++t) {
+        require(U > 0, "sinc band too wide for the lines kernel (4 outputs need > 26 source samples)");
+        std::vector<float> wsh(static_cast<size_t>(kSincThreads) * 4 * U, 0.f);
+        std::vector<int> s0v(kSincThreads);
+        for (int t = 0; t < kSincThreads; ++t) {
             const int base = st[4 * t];
             s0v[t] = base;
             for (int r = 0; r < 4; ++r) {
                 const int i = 4 * t + r;
                 for (int k = 0; k < len[i]; ++k) {
                     const int u = (st[i] + k) % U;         // step that reads source st[i] + k
-                    wsh[(static_cast<size_t>(t) * 4 + r) * U + u] = wt[static_cast<size_t>(k) * kN + i];
+                    wsh[((static_cast<size_t>(r / 2) * U + u) * kSincThreads + t) * 2 + r % 2] =
+                        wt[static_cast<size_t>(k) * kN + i];
                 }
             }
         }
-        std::vector<float2> win(kN), tw(kN);
+        std::vector<float2> win(kN), root(kN), tw(kTwTable);
         for (int i = 0; i < kN; ++i) {
             // complex64 window (core/spectral.py:219) times 1/N: exact power-of-two scaling
             win[i] = make_float2(static_cast<float>(window[2 * i]) * (1.0f / kN),
                                  static_cast<float>(window[2 * i + 1]) * (1.0f / kN));
             const double ang = 2.0 * 3.14159265358979323846 * i / kN;
-            tw[i] = make_float2(static_cast<float>(cos(ang)), static_cast<float>(sin(ang)));
+            root[i] = make_float2(static_cast<float>(cos(ang)), static_cast<float>(sin(ang)));
         }
-        ck(c->w.ensure(wt.size() * sizeof(float)), "cudaMalloc(w)");
+        // tw2[16 r + j] = w^(r j N/256), tw3[256 (r - 1) + j] = w^(r j), w = e^(2 pi i / N)
+        for (int k = 0; k < 256; ++k) tw[k] = root[(k >> 4) * (k & 15) * (kN / 256) % kN];
+        for (int k = 0; k < 7 * 256; ++k) tw[256 + k] = root[((k >> 8) + 1) * (k & 255) % kN];
+        ck(c->lines.ensure(static_cast<size_t>(kFirstPass) * kN * sizeof(float)), "cudaMalloc(lines)");
+        ck(c->lines_fixed.ensure(static_cast<size_t>(kMinPass) * kN * sizeof(float)), "cudaMalloc(lines)");
         ck(c->start.ensure(kN * sizeof(int)), "cudaMalloc(start)");
         ck(c->win.ensure(kN * sizeof(float2)), "cudaMalloc(win)");
-        ck(c->tw.ensure(kN * sizeof(float2)), "cudaMalloc(tw)");
-        ck(cudaMemcpyAsync(c->w.p, wt.data(), wt.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream), "H2D w");
+        ck(c->tw.ensure(kTwTable * sizeof(float2)), "cudaMalloc(tw)");
         ck(cudaMemcpyAsync(c->start.p, st.data(), kN * sizeof(int), cudaMemcpyHostToDevice, c->stream), "H2D start");
         ck(cudaMemcpyAsync(c->win.p, win.data(), kN * sizeof(float2), cudaMemcpyHostToDevice, c->stream), "H2D win");
-        ck(cudaMemcpyAsync(c->tw.p, tw.data(), kN * sizeof(float2), cudaMemcpyHostToDevice, c->stream), "H2D tw");
+        ck(cudaMemcpyAsync(c->tw.p, tw.data(), kTwTable * sizeof(float2), cudaMemcpyHostToDevice, c->stream), "H2D tw");
         ck(c->wsh.ensure(wsh.size() * sizeof(float)), "cudaMalloc(wsh)");
         ck(c->s0.ensure(s0v.size() * sizeof(int)), "cudaMalloc(s0)");
         ck(cudaMemcpyAsync(c->wsh.p, wsh.data(), wsh.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream),
@@ -685,12 +761,14 @@ int octgb_fused_pre_fft(octgb_ctx* c, const void* raw, int dtype, int loc, int B
         require(spec != nullptr, "spec is NULL");
         const size_t ob = static_cast<size_t>(B) * (interf - apod) * kN * 2 * sizeof(float);
         float* dst = spec;
-        if (spec_loc != OCTGB_DEVICE) {
+        // the kernel stores 16 bytes at a time
+        const bool direct = spec_loc == OCTGB_DEVICE && (reinterpret_cast<uintptr_t>(spec) & 15u) == 0;
+        if (!direct) {
             ck(c->out.ensure(ob), "cudaMalloc(out)");
             dst = c->out.as<float>();
         }
-        run_spectral(c, raw, dtype, loc, B, interf, apod, kModeSpec, dst, 0, 0, nullptr);
-        if (spec_loc != OCTGB_DEVICE) copy_out(c, spec, OCTGB_HOST, dst, ob);
+        run_lines(c, raw, dtype, loc, B, interf, apod, kModeSpec, dst);
+        if (!direct) copy_out(c, spec, spec_loc, dst, ob);
         check_status(c);
     });
 }
@@ -725,10 +803,7 @@ int octgb_db(octgb_ctx* c, const void* raw, int dtype, int loc, int B, int inter
             dst = c->out.as<float>();
         }
         unsigned int* mm = c->mm.as<unsigned int>();
-        if (minmax) {
-            ck(launch_minmax_init(mm, 2, c->stream), "minmax init");
-            c->launches++;
-        }
+        if (minmax) reset_minmax(c, mm);
         run_spectral(c, raw, dtype, loc, B, interf, apod, kModeDb, dst, z0, nz, minmax ? mm : nullptr);
         if (db_loc != OCTGB_DEVICE) copy_out(c, db, OCTGB_HOST, dst, ob);
         if (minmax)
@@ -873,16 +948,16 @@ int octgb_stitch_plan(octgb_ctx* c, int n_rows, int r0, int r1, int c0, int c1, 
                 "stitch patch too large (output pixel much coarser than the tile sampling)");
         Plan* p = new Plan();
         p->lateral_identity = c0 == 0 && C == n_tile_x;
-        // batched form: every quad holding output column cc must also hold the
-        // A-scans it reads (xr with weight wx0, xr + 1 with wx1); quads start
+        // batched form: every group of four holding output column cc must also hold the
+        // A-scans it reads (xr with weight wx0, xr + 1 with wx1); groups start
         // at multiples of 4, the last one of a B-scan at C - 4
         p->lateral_quad_local = c0 == 0 && C == n_tile_x;
-        const int qpb = (C + kPerCta - 1) / kPerCta;
+        const int qpb = (C + kLateral - 1) / kLateral;
         for (int qb = 0; qb < qpb && p->lateral_quad_local; ++qb) {
-            const int q0 = (qb == qpb - 1 && C >= kPerCta) ? C - kPerCta : qb * kPerCta;
-            for (int cc = q0; cc < q0 + kPerCta && cc < C; ++cc) {
-                const bool ok0 = wx0[cc] == 0.f || (xr[cc] >= q0 && xr[cc] < q0 + kPerCta && xr[cc] < C);
-                const bool ok1 = wx1[cc] == 0.f || (xr[cc] + 1 >= q0 && xr[cc] + 1 < q0 + kPerCta && xr[cc] + 1 < C);
+            const int q0 = (qb == qpb - 1 && C >= kLateral) ? C - kLateral : qb * kLateral;
+            for (int cc = q0; cc < q0 + kLateral && cc < C; ++cc) {
+                const bool ok0 = wx0[cc] == 0.f || (xr[cc] >= q0 && xr[cc] < q0 + kLateral && xr[cc] < C);
+                const bool ok1 = wx1[cc] == 0.f || (xr[cc] + 1 >= q0 && xr[cc] + 1 < q0 + kLateral && xr[cc] + 1 < C);
                 if (xr[cc] < 0 || !ok0 || !ok1) p->lateral_quad_local = false;
             }
         }
@@ -1161,7 +1236,7 @@ int octgb_frames_process(octgb_ctx* c, int n_tiles, const int* plan_ids, const v
             slot = c->ring_next;
             c->ring_next = (slot + 1) % octgb_ctx::kRing;
             ck(c->ring[slot].ensure(tile_bytes * n_tiles), "cudaMalloc(raw ring)");
-            // the slot's previous batch must have left the spectral kernel
+            // the slot's previous batch must have left the lines kernel
             ck(cudaStreamWaitEvent(c->copy, c->ring_free[slot], 0), "cudaStreamWaitEvent");
             for (int t = 0; t < n_tiles; ++t) {
                 void* dst = static_cast<char*>(c->ring[slot].p) + t * tile_bytes;
@@ -1219,8 +1294,7 @@ int octgb_frames_process(octgb_ctx* c, int n_tiles, const int* plan_ids, const v
 int octgb_clim_reset(octgb_ctx* c) {
     return guarded(c, [&] {
         ck(c->run_mm.ensure(2 * sizeof(unsigned int)), "cudaMalloc(run mm)");
-        ck(launch_minmax_init(c->run_mm.as<unsigned int>(), 2, c->stream), "minmax init");
-        c->launches++;
+        reset_minmax(c, c->run_mm.as<unsigned int>());
     });
 }
 
@@ -1268,8 +1342,8 @@ int octgb_graph_end(octgb_ctx* c, int* graph_id) {
         c->graph_kernels.push_back(c->launches.load() - c->capture_launch0);
         // the graph holds the addresses of the context's buffers: from now on
         // a buffer that grows keeps its old allocation until octgb_destroy
-        for (DevBuf* b : {&c->raw, &c->apod, &c->out, &c->mm, &c->frames, &c->num, &c->den, &c->plan_table,
-                          &c->run_mm, &c->magbuf, &c->dbbuf, &c->planemm, &c->segs, &c->qtable, &c->qcounter,
+        for (DevBuf* b : {&c->lines, &c->raw, &c->apod, &c->out, &c->mm, &c->frames, &c->num, &c->den, &c->plan_table,
+                          &c->run_mm, &c->magbuf, &c->dbbuf, &c->planemm, &c->segs, &c->qtable,
                           &c->disp_x, &c->disp_hann, &c->disp_dk2, &c->disp_betas, &c->disp_phase, &c->disp_a, &c->disp_score, &c->xmed,
                           &c->prec_hi, &c->prec_lo, &c->prec_m, &c->prec_x, &c->prep, &c->prep_apod,
                           &c->magrep, &c->srr, &c->gemm_part, &c->enc_bits, &c->enc_lut, &c->enc_slots, &c->enc_sizes, &c->enc_offsets, &c->enc_packed})
@@ -1319,7 +1393,7 @@ int octgb_batch_process(octgb_ctx* c, int n_tiles, const octgb_tile* tiles, int 
         require(tiles != nullptr, "tiles is NULL");
         require(grab >= 1 && grab <= 4096, "grab must be in [1, 4096]");
         std::vector<QueueTile> qt(n_tiles);
-        unsigned int quads = 0;
+        unsigned int lines = 0;
         int rows = 0;
         for (int t = 0; t < n_tiles; ++t) {
             const octgb_tile& d = tiles[t];
@@ -1332,9 +1406,8 @@ int octgb_batch_process(octgb_ctx* c, int n_tiles, const octgb_tile* tiles, int 
                     "a batched tile's plan must be a single-tile plan (output columns = the tile's A-scans)");
             require(!p.opc, "the batched form does not take optical-path correction");
             require(p.n_out_z <= 1600, "the batched form resamples to at most 1600 output rows per A-scan");
-            const int qpb = (d.interf - d.apod_size + kPerCta - 1) / kPerCta;
-            const unsigned int nq = static_cast<unsigned int>(static_cast<int64_t>(d.B) * qpb);
-            require(static_cast<uint64_t>(quads) + nq < (1ull << 31), "batch too large");
+            const int64_t n = static_cast<int64_t>(d.B) * (d.interf - d.apod_size);
+            require(lines + n < (int64_t(1) << 31), "batch too large");
             QueueTile& q = qt[t];
             q.raw = d.raw;
             q.out = d.db;
@@ -1345,46 +1418,44 @@ int octgb_batch_process(octgb_ctx* c, int n_tiles, const octgb_tile* tiles, int 
             q.nx = d.interf - d.apod_size;
             q.nz = p.n_out_z;
             q.apod_row0 = rows;
-            q.quad0 = quads;
-            q.nquads = nq;
-            q.qpb = qpb;
-            quads += nq;
+            q.line0 = lines;
+            lines += static_cast<unsigned int>(n);
             rows += d.B;
         }
-        if (quads == 0) return;
+        if (lines == 0) return;
         const QueueTile* qdev = tile_table(c, qt);
         ck(c->apod.ensure(static_cast<size_t>(rows) * kN * sizeof(float) + 16), "cudaMalloc(apod)");
-        ck(c->qcounter.ensure(sizeof(unsigned int)), "cudaMalloc(queue head)");
         ck(c->run_mm.ensure(2 * sizeof(unsigned int)), "cudaMalloc(run mm)");
-        ck(cudaMemsetAsync(c->qcounter.p, 0, sizeof(unsigned int), c->stream), "memset queue head");
-        ck(launch_apod_mean_tiles(qdev, n_tiles, rows, dtype, c->apod.as<float>(), c->stream),
-           "apod kernel");
-        c->launches++;
-        SpectralArgs a{};
-        a.n_seg = 1;
-        a.B = 1;
-        a.nx = 1;
-        a.apod_mean = c->apod.as<float>();
-        a.g.w = c->w.as<float>();
-        a.g.start = c->start.as<int>();
-        a.g.taps = c->taps;
-        a.g.win = c->win.as<float2>();
-        a.g.tw = c->tw.as<float2>();
-        a.g.wsh = c->wsh.as<float>();
-        a.g.s0 = c->s0.as<int>();
-        a.g.U = c->U;
-        a.minmax = c->run_mm.as<unsigned int>();
-        a.status = c->status_dev;
+        LinesArgs a = lines_args(c, nullptr, 0, 0, 0, 0, c->apod.as<float>());
         a.qt = qdev;
         a.n_qt = n_tiles;
-        a.counter = c->qcounter.as<unsigned int>();
-        a.total_quads = quads;
-        a.grab = grab;
-        a.thr = thr;
-        int64_t grid = static_cast<int64_t>(c->num_sms) * spectral_max_ctas_per_sm(dtype, kModeResample);
-        if (grid > quads) grid = quads;
-        ck(launch_spectral(a, dtype, kModeResample, static_cast<int>(grid), c->stream), "spectral kernel");
+        ck(launch_apod_mean(a, dtype, rows, c->apod.as<float>(), c->stream), "apod kernel");
         c->launches++;
+        const unsigned int pass = pass_lines(c, lines);
+        ck(c->magbuf.ensure(static_cast<size_t>(pass) * kHalf * sizeof(float)), "cudaMalloc(mag)");
+        // passes of whole B-scans (the lateral blend reads neighbours of the same
+        // B-scan); one longer than a pass is cut between groups of four
+        int t = 0;
+        for (unsigned int l0 = 0, l1; l0 < lines; l0 = l1) {
+            l1 = l0 + std::min(pass, lines - l0);
+            if (l1 < lines) {
+                while (t + 1 < n_tiles && qt[t + 1].line0 <= l1) ++t;
+                const unsigned int nx = static_cast<unsigned int>(qt[t].nx);
+                const unsigned int b0 = l1 - (l1 - qt[t].line0) % nx;     // the B-scan l1 lies in
+                if (b0 > l0) {
+                    l1 = b0;
+                } else {
+                    unsigned int x = (l1 - b0) / kLateral * kLateral;
+                    if (nx - x < 2 * kLateral) x -= kLateral;             // the last group may start off the grid of four
+                    l1 = b0 + x;
+                }
+            }
+            transform_pass(c, a, c->lines.as<float>(), dtype, l0, l1, kModeMag, c->magbuf.as<float>(), 0, 0, nullptr);
+            ck(launch_resample(qdev, n_tiles, l0, l1, c->magbuf.as<float>(), thr, c->run_mm.as<unsigned int>(),
+                               c->stream),
+               "resample kernel");
+            c->launches++;
+        }
     });
 }
 
@@ -1404,7 +1475,7 @@ int octgb_disp_load(octgb_ctx* c, const void* raw, int dtype, int loc, int n_bsc
         const size_t lines = static_cast<size_t>(B) * nx;
         // linearised interferogram (window 1: the kernel's output is sum + m)
         // windowed in float64 and rounded once, as (eq * hann).astype(complex64)
-        // (dispersion.py:84), written by the spectral kernel itself
+        // (dispersion.py:84), written by the lines kernel itself
         ck(c->disp_x.ensure(lines * kN * sizeof(float)), "cudaMalloc(X)");
         // the window in float64, and split hi + lo in float32 for the kernel's
         // float32 form of the float64 product
@@ -1418,8 +1489,8 @@ int octgb_disp_load(octgb_ctx* c, const void* raw, int dtype, int loc, int n_bsc
         ck(c->disp_hann.ensure(kN * 2 * sizeof(double)), "cudaMalloc(hann)");
         ck(cudaMemcpyAsync(c->disp_hann.p, hw.data(), hw.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream),
            "H2D hann");
-        run_spectral(c, raw, dtype, loc, B, interf, apod, kModeLinHann, c->disp_x.as<float>(), 0, 0, nullptr,
-                     c->disp_hann.as<double>(), reinterpret_cast<const float2*>(c->disp_hann.as<double>() + kN));
+        run_lines(c, raw, dtype, loc, B, interf, apod, kModeLinHann, c->disp_x.as<float>(), c->disp_hann.as<double>(),
+                  reinterpret_cast<const float2*>(c->disp_hann.as<double>() + kN));
         check_status(c);
         c->disp_b = n_bscans;
         c->disp_rep = rep;
@@ -1502,6 +1573,7 @@ int octgb_disp_eval(octgb_ctx* c, int n_beta, const double* betas, int b0, int n
             a.b0 = b0;
             a.nx = nx;
             a.rep = c->disp_rep;
+            a.ready = &c->ready;
             ck(launch_disp_mag(a, c->num_sms, c->stream), "dispersion magnitude kernel");
             c->launches++;
             if (metric != 0) {
@@ -1794,8 +1866,6 @@ float* precision_linearise(octgb_ctx* c, const void* raw, int dtype, int loc, in
     ck(c->apod.ensure(static_cast<size_t>(B) * kN * sizeof(double) + kPKW * sizeof(int) + 16), "cudaMalloc(apod)");
     SpectralArgs a{};
     a.raw = rd;
-    a.seg[0] = rd;
-    a.n_seg = 1;
     a.B = B;
     a.interf = interf;
     a.apod = apod;
@@ -1837,7 +1907,7 @@ float* precision_linearise(octgb_ctx* c, const void* raw, int dtype, int loc, in
 
 int octgb_selftest_wait_expiry(octgb_ctx* c, int which, int wait_limit_us) {
     return guarded(c, [&] {
-        require(which == 0 || which == 1, "which must be 0 (spectral kernel) or 1 (precision form)");
+        require(which == 0 || which == 1, "which must be 0 (lines kernel) or 1 (precision form)");
         require(wait_limit_us >= 100 && wait_limit_us <= 2000000, "wait_limit_us must be in [100, 2000000]");
         if (!c->has_geom) throw Error(OCTGB_ERR_STATE, "octgb_set_geometry has not been called");
         if (which == 1) require(c->prec_ok, "the geometry has no precision-form (tensor-core) tiles");
@@ -1951,6 +2021,7 @@ int octgb_magnitude_precision(octgb_ctx* c, const void* raw, int dtype, int loc,
         a.b0 = 0;
         a.nx = interf - apod;
         a.rep = 1;
+        a.ready = &c->ready;
         ck(launch_disp_mag(a, c->num_sms, c->stream), "FFT kernel");
         c->launches++;
         if (mag_loc != OCTGB_DEVICE) copy_out(c, mag, OCTGB_HOST, dst, ob);
@@ -1988,6 +2059,7 @@ int octgb_disp_images(octgb_ctx* c, int n_beta, const double* betas, int b0, int
         a.b0 = b0;
         a.nx = nx;
         a.rep = c->disp_rep;
+        a.ready = &c->ready;
         ck(launch_disp_mag(a, c->num_sms, c->stream), "dispersion magnitude kernel");
         ck(launch_image_cols(a.zcol, n_beta, nb, nx, z_keep, img, c->stream), "image column kernel");
         c->launches += 2;
@@ -2177,10 +2249,10 @@ int octgb_cnn_adam(octgb_ctx* c, float* p, const float* g, float* m, float* v, i
 // can synchronise the device and stall the camera stream), or a host process
 // whose GPU memory is owned by another framework's pooling allocator under a
 // fixed budget.  For them octgb_magnitude_noalloc does the work of
-// octgb_magnitude on device buffers the caller already owns, and keeps its one
-// piece of scratch (the per-B-scan apodisation mean) in the fixed array below
-// instead of a context buffer.  The array is part of the loaded library image:
-// every GPU that loads the library holds it until the process exits.
+// octgb_magnitude on device buffers the caller already owns.  Its scratch is
+// the per-B-scan apodisation mean, in the fixed array below (part of the loaded
+// library image: every GPU that loads the library holds it until the process
+// exits), and the context's own lines_fixed, allocated with the geometry.
 namespace {
 
 constexpr int kNoAllocMaxBscans = 64;   // B-scans per call: 64 x 2048 floats = 512 KiB
@@ -2222,34 +2294,9 @@ extern "C" int octgb_magnitude_noalloc(octgb_ctx* c, const void* raw, int dtype,
         if (B == 0) return;
         float* scratch = noalloc_scratch(c->device);
         // the same launches as octgb_magnitude, with the apodisation mean in
-        // the fixed array; k_apod_mean writes every element the spectral
-        // kernel then reads, so nothing in the array needs clearing
-        SpectralArgs a{};
-        a.raw = raw;
-        a.seg[0] = raw;
-        a.n_seg = 1;
-        a.B = B;
-        a.interf = interf;
-        a.apod = apod;
-        a.nx = interf - apod;
-        a.n_ascans = static_cast<int64_t>(B) * (interf - apod);
-        a.apod_mean = scratch;
-        a.g.w = c->w.as<float>();
-        a.g.start = c->start.as<int>();
-        a.g.taps = c->taps;
-        a.g.win = c->win.as<float2>();
-        a.g.tw = c->tw.as<float2>();
-        a.g.wsh = c->wsh.as<float>();
-        a.g.s0 = c->s0.as<int>();
-        a.g.U = c->U;
-        a.out = mag;
-        a.status = c->status_dev;
-        ck(launch_apod_mean(a, dtype, c->stream), "apod kernel");
-        c->launches++;
-        const int64_t quads = (a.n_ascans + kPerCta - 1) / kPerCta;
-        int64_t grid = static_cast<int64_t>(c->num_sms) * spectral_max_ctas_per_sm(dtype, kModeMag);
-        if (grid > quads) grid = quads;
-        ck(launch_spectral(a, dtype, kModeMag, static_cast<int>(grid), c->stream), "spectral kernel");
-        c->launches++;
+        // the fixed array (the lines' scratch came with the geometry);
+        // k_apod_mean writes every element the lines kernel then reads, so
+        // nothing in the array needs clearing
+        launch_spectral_segs(c, &raw, 1, dtype, B, interf, apod, kModeMag, mag, 0, 0, nullptr, scratch);
     });
 }

@@ -44,8 +44,7 @@ namespace {
 constexpr int kDispWarps = 4;
 
 struct DispSmem {
-    alignas(16) float2 tw2[256];
-    alignas(16) float2 tw3[kTw3];
+    alignas(16) float2 tw[kTwTable];                     // tw2, tw3
     alignas(16) float2 ex[kDispWarps][kWarpExchange];
     // followed by [kDispWarps][kHalf] floats (a line's magnitudes) with pooling or repeats
 };
@@ -57,15 +56,19 @@ __device__ __forceinline__ float ld_stream(const float* p) {
     return v;
 }
 
-// Rep: several B-scan repeats (a.rep > 1)
-template <bool Pool, bool Rep>
+// Pool: probe images; Db: dB of a depth crop; Rep: several B-scan repeats (a.rep > 1)
+template <bool Pool, bool Db, bool Rep>
 __global__ void __launch_bounds__(kDispWarps * 32, 3) k_disp_mag(const DispArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     DispSmem& S = *reinterpret_cast<DispSmem*>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int k = tid; k < 256; k += kDispWarps * 32) S.tw2[k] = __ldg(a.tw + ((k >> 4) * (k & 15) * (kN / 256)) % kN);   // symmetric in its indices
-    for (int k = tid; k < kTw3; k += kDispWarps * 32) S.tw3[k] = __ldg(a.tw + (((k >> 8) + 1) * (k & 255)) % kN);
+    for (int k = tid; k < kTwTable / 2; k += kDispWarps * 32)
+        reinterpret_cast<float4*>(S.tw)[k] = __ldg(reinterpret_cast<const float4*>(a.tw) + k);
+    const float2 *tw2 = S.tw, *tw3 = S.tw + 256;
     __syncthreads();
+    pdl_wait();                                          // the lines and phase rows
+    pdl_launch();
+    float run_min = __int_as_float(0x7f800000), run_max = -__int_as_float(0x7f800000);
     float2* ex = S.ex[warp];
     float* sums = reinterpret_cast<float*>(&S + 1) + warp * kHalf;
     // items < 2^32 - the grid's warps (the launcher checks): 32-bit item arithmetic
@@ -81,7 +84,7 @@ __global__ void __launch_bounds__(kDispWarps * 32, 3) k_disp_mag(const DispArgs 
     for (unsigned int item = blockIdx.x * kDispWarps + warp; item < n_items; item += step) {
         const float2* ph = a.phase + static_cast<int64_t>(item / nbx) * kN + lane;
         const float* line = line_of(item) + lane;
-        float* out = Pool ? sums : a.A + static_cast<int64_t>(item) * kHalf;
+        float* out = Pool ? sums : a.A + static_cast<int64_t>(item) * (Db ? a.nz : kHalf);
         // the warp's next line into L2 behind this one's transform
         if (!Rep && lane == 0 && item + step < n_items) bulk_prefetch_l2(line_of(item + step), kN * sizeof(float));
         for (int rp = 0; rp < (Rep ? a.rep : 1); ++rp, line += static_cast<int64_t>(a.nx) * kN) {
@@ -94,7 +97,18 @@ __global__ void __launch_bounds__(kDispWarps * 32, 3) k_disp_mag(const DispArgs 
                 // complex64 (xv + 0i) * p, as numpy multiplies (dispersion.py:94)
                 v[r] = make_float2(v[r].x * p.x, v[r].x * p.y);
             }
-            ifft2048_low_mag_warp(v, ex, S.tw2, S.tw3, lane, [&](int k, float m) {
+            ifft2048_low_mag_warp(v, ex, tw2, tw3, lane, [&](int k, float m) {
+                if (Db) {
+                    // (no branch around the few depths cropped)
+                    const int z = k - a.z0;
+                    const bool in = static_cast<unsigned int>(z) < static_cast<unsigned int>(a.nz);
+                    const float db = 20.0f * log10f(m);
+                    if (in) out[z] = db;
+                    const bool use = in && isfinite(db);
+                    run_min = fminf(run_min, use ? db : __int_as_float(0x7f800000));
+                    run_max = fmaxf(run_max, use ? db : -__int_as_float(0x7f800000));
+                    return;
+                }
                 if (!Rep) {
                     out[k] = m;
                     return;
@@ -118,6 +132,17 @@ __global__ void __launch_bounds__(kDispWarps * 32, 3) k_disp_mag(const DispArgs 
                 a.zcol[static_cast<int64_t>(item) * 256 + zi] = sum;
             }
             __syncwarp();
+        }
+    }
+    if (Db && a.minmax != nullptr) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            run_min = fminf(run_min, __shfl_xor_sync(0xffffffffu, run_min, o));
+            run_max = fmaxf(run_max, __shfl_xor_sync(0xffffffffu, run_max, o));
+        }
+        if (lane == 0 && run_min <= run_max) {
+            atomicMin(&a.minmax[0], f2ord(run_min));
+            atomicMax(&a.minmax[1], f2ord(run_max));
         }
     }
 }
@@ -517,16 +542,19 @@ cudaError_t launch_xmedian_t(const float* mag, int n_frames, int nx, int nz, int
 
 cudaError_t launch_disp_mag(const DispArgs& a, int num_sms, cudaStream_t st) {
     const size_t smem = sizeof(DispSmem) + (a.zcol != nullptr || a.rep > 1 ? kDispWarps * kHalf * sizeof(float) : 0);
-    const auto kernel = a.zcol != nullptr ? (a.rep > 1 ? k_disp_mag<true, true> : k_disp_mag<true, false>)
-                                          : (a.rep > 1 ? k_disp_mag<false, true> : k_disp_mag<false, false>);
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (a.mode == kModeDb && (a.rep > 1 || a.zcol != nullptr)) return cudaErrorInvalidValue;
+    const auto kernel = a.mode == kModeDb   ? k_disp_mag<false, true, false>
+                        : a.zcol != nullptr ? (a.rep > 1 ? k_disp_mag<true, false, true> : k_disp_mag<true, false, false>)
+                        : a.rep > 1         ? k_disp_mag<false, false, true>
+                                            : k_disp_mag<false, false, false>;
+    const int bit = a.mode == kModeDb ? 4 : (a.zcol != nullptr ? 2 : 0) + (a.rep > 1 ? 1 : 0);
+    const cudaError_t e = kernel_ready(a.ready, kReadyDisp + bit, kernel, smem);
     if (e != cudaSuccess) return e;
     const int64_t items = static_cast<int64_t>(a.n_beta) * a.nb * a.nx;
     if (items >= (int64_t(1) << 32) - 3 * kDispWarps * num_sms) return cudaErrorInvalidValue;   // 32-bit item index
     int64_t grid = (items + kDispWarps - 1) / kDispWarps;
     if (grid > 3 * num_sms) grid = 3 * num_sms;
-    kernel<<<static_cast<int>(grid), kDispWarps * 32, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(kernel, dim3(static_cast<unsigned int>(grid)), dim3(kDispWarps * 32), smem, st, a);
 }
 
 cudaError_t launch_phase(const double* betas, const double* dk2, int n, float2* phase, cudaStream_t st) {

@@ -1,0 +1,512 @@
+// Spectral stage up to the transform for sm_103a: raw camera counts ->
+// background-free, k-linearised lines.
+//
+// Per A-scan (2048 samples):
+//   d[j] = float(raw[j]) - apod[j] (float32 apodisation mean of the B-scan,
+//     rounded from an exact sum as core/cpu_kernels.py:20-25 does), line mean
+//     m removed (cpu_kernels.py:26-36);
+//   v[i] = sum_t w[t,i] (d - m)[start_i + t] + m (banded sinc, cpu_kernels.py:
+//     37-40, float32 accumulation), written as the real line that the
+//     transform (estimate.cu) takes, times the complex window (the fused
+//     pre-FFT operator's output, cpu_kernels.py:41) or times a float64 window
+//     rounded once (the scorer's lines).
+//
+// k_lines is one persistent CTA an SM with two kinds of warps, joined by a
+// ring of background-free lines in shared memory:
+//   sinc warps (16)        thread t owns outputs 4t .. 4t + 3; its band weights
+//                          stay in registers for the whole launch, in a dense
+//                          form over its window of U source samples.  Step u
+//                          reads the sample congruent to u (mod U): at one
+//                          step a warp's threads read the same samples or
+//                          samples U apart, which with gcd(U, 32) = 2 lie in
+//                          distinct banks;
+//   background warps       one A-scan each: the raw row arrives by a bulk copy
+//                          two A-scans ahead, the apodisation-mean row when the
+//                          B-scan changes; 64 samples a lane stay in registers
+//                          until the line mean is known, so no two warps wait
+//                          for one another except through the ring.
+// A CTA takes a contiguous range of A-scans, so the apodisation row changes
+// once a B-scan.
+// Bound by the shared-memory path: 471 wavefronts an A-scan, 67 % of its
+// cycles, with 1718 warp instructions (issue active 52 %); 25 000 A-scans in
+// 65 us (382 M/s, 12.4 kB read and written an A-scan = 4.7 TB/s).  With the
+// transform after it (estimate.cu) they take 260 us to dB rows; one kernel for
+// both, 512 threads in lock step through two block barriers per four A-scans
+// (1619 wavefronts, 5880 instructions an A-scan), took 314 us, and 324 000
+// A-scans stitched 3888 us against 3295 now.
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "octgb_device.cuh"
+#include "octgb_internal.h"
+
+namespace octgb {
+namespace {
+
+constexpr int kSincWarps = 16;                   // 512 threads x 4 outputs
+constexpr int kBgWarps = 4;
+constexpr int kThr = (kSincWarps + kBgWarps) * 32;
+constexpr int kRing = 8;                         // background-free lines in shared memory
+constexpr int kDLine = kN + kTail;               // line incl. zero tail (16-byte rows)
+
+// float32 values of four raw samples
+template <typename RawT>
+__device__ __forceinline__ void raw4(const RawT* p, float2& a, float2& b);
+// 2^23 + u is exact in float32 with u in its low bits, so subtracting 2^23
+// gives the 16-bit integer u exactly, two at a time (int16: u offset by 2^15)
+__device__ __forceinline__ void raw4_u16(uint2 q, uint32_t flip, float2 off, float2& a, float2& b) {
+    q.x ^= flip;
+    q.y ^= flip;
+    a = sub2(make_float2(__uint_as_float(__byte_perm(q.x, 0x4b000000u, 0x7610)),
+                         __uint_as_float(__byte_perm(q.x, 0x4b000000u, 0x7632))),
+             off);
+    b = sub2(make_float2(__uint_as_float(__byte_perm(q.y, 0x4b000000u, 0x7610)),
+                         __uint_as_float(__byte_perm(q.y, 0x4b000000u, 0x7632))),
+             off);
+}
+template <>
+__device__ __forceinline__ void raw4<uint16_t>(const uint16_t* p, float2& a, float2& b) {
+    raw4_u16(*reinterpret_cast<const uint2*>(p), 0u, make_float2(8388608.f, 8388608.f), a, b);
+}
+template <>
+__device__ __forceinline__ void raw4<int16_t>(const int16_t* p, float2& a, float2& b) {
+    raw4_u16(*reinterpret_cast<const uint2*>(p), 0x80008000u, make_float2(8421376.f, 8421376.f), a, b);
+}
+template <>
+__device__ __forceinline__ void raw4<float>(const float* p, float2& a, float2& b) {
+    const float4 u = *reinterpret_cast<const float4*>(p);
+    a = make_float2(u.x, u.y);
+    b = make_float2(u.z, u.w);
+}
+
+// float32(float64(x) * h) for a float64 h given as float32 hi + lo (h2.x +
+// h2.y, the rest below 2^-48 |h|) without the FP64 pipe: p + e1 = x * hi
+// exactly (fma), q = x lo + e1 (one rounding), o = p + q rounded once.  The
+// exact product differs from p + q by < 2^-46 |o|; when p + q lies more than
+// 2^-40 |o| from a float32 rounding boundary (r = (p + q) - o exactly, by
+// Fast2Sum), both the product and its float64 rounding round to o.  Otherwise
+// (about one sample in 65 000), and for powers of two (asymmetric boundaries)
+// and tiny values, the float64 product is formed as the reference does.  A
+// window value of exactly zero (the Hann window's end points) gives the exact
+// product x * 0 (signed zero, or NaN) in both forms and needs no float64 step:
+// without this case the two warps holding the end points took the float64 path
+// for every A-scan.
+// The caller forms the float64 product for the lanes whose `safe` is false,
+// behind a warp vote, so the FP64 pipe only runs in the rare warps that need it.
+__device__ __forceinline__ float mul_window(float x, float2 h2, bool& safe) {
+    const float p = x * h2.x;
+    const float e1 = fmaf(x, h2.x, -p);
+    const float q = fmaf(x, h2.y, e1);
+    const float o = p + q;
+    const float r = q - (o - p);
+    const float ao = fabsf(o);
+    const int bits = __float_as_int(ao);
+    const float half_ulp = __int_as_float((bits & 0x7f800000) - (24 << 23));
+    const bool zero_h = h2.x == 0.f && h2.y == 0.f;
+    safe = zero_h || (ao > 1e-30f && (bits & 0x007fffff) != 0 && fabsf(fabsf(r) - half_ulp) > ao * 9.094947e-13f);
+    // x * 0 keeps x's sign, as the float64 product does (p + q would give +0)
+    return zero_h ? p : o;
+}
+
+template <typename RawT>
+struct LinesSmem {
+    uint64_t raw_full[kBgWarps][2], full[kRing], empty[kRing];
+    int abort;
+    float mval[kRing];
+    alignas(16) RawT raw[kBgWarps][2][kN];
+    alignas(16) float apod[kBgWarps][2][kN];
+    alignas(16) float d[kRing][kDLine];
+};
+static_assert(sizeof(LinesSmem<float>) <= 232448, "k_lines shared memory exceeds 227 KB");
+
+// the place of one A-scan: segment (or tile), B-scan, column
+struct LinePos {
+    unsigned int sg, b, x;
+};
+
+template <typename RawT, int Mode, int U, bool Tiles>
+__global__ void __launch_bounds__(kThr, 1) k_lines(const LinesArgs a) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    using Smem = LinesSmem<RawT>;
+    Smem& S = *reinterpret_cast<Smem*>(smem_raw);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // this CTA's A-scans
+    const unsigned int n_all = a.l1 - a.l0;
+    const unsigned int first = a.l0 + static_cast<unsigned int>(static_cast<uint64_t>(n_all) * blockIdx.x / gridDim.x);
+    const int n = static_cast<int>(
+        a.l0 + static_cast<unsigned int>(static_cast<uint64_t>(n_all) * (blockIdx.x + 1) / gridDim.x) - first);
+
+    if (tid == 0) {
+        for (int w = 0; w < kBgWarps; ++w)
+            for (int s = 0; s < 2; ++s) mbar_init(&S.raw_full[w][s], 1);
+        for (int s = 0; s < kRing; ++s) {
+            mbar_init(&S.full[s], 1);
+            mbar_init(&S.empty[s], kSincWarps);
+        }
+        S.abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int k = tid; k < kRing * kTail; k += kThr) S.d[k / kTail][kN + k % kTail] = 0.f;
+    // a wait that runs out ends every role of the CTA
+    auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+        if (*reinterpret_cast<volatile int*>(&S.abort)) return false;
+        if (mbar_wait_bounded(bar, parity, a.status)) return true;
+        atomicExch(&S.abort, 1);
+        return false;
+    };
+
+    if (warp >= kSincWarps) {
+        // ------------------------------------------------ background
+        const int w = warp - kSincWarps;
+        __syncthreads();
+        pdl_wait();                                          // the lines' readers, the apodisation means
+        pdl_launch();
+        if (w >= n) return;
+        LinePos pos;
+        auto dims = [&](unsigned int sg, unsigned int& B, unsigned int& nx) {
+            if (Tiles) {
+                B = static_cast<unsigned int>(a.qt[sg].B);
+                nx = static_cast<unsigned int>(a.qt[sg].nx);
+            } else {
+                B = static_cast<unsigned int>(a.B);
+                nx = static_cast<unsigned int>(a.nx);
+            }
+        };
+        {
+            unsigned int l = first + static_cast<unsigned int>(w);
+            if (Tiles) {
+                int lo = 0, hi = a.n_qt - 1;                 // last tile with line0 <= l
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (a.qt[mid].line0 <= l) lo = mid; else hi = mid - 1;
+                }
+                pos.sg = static_cast<unsigned int>(lo);
+                l -= a.qt[lo].line0;
+            } else {
+                pos.sg = l / (static_cast<unsigned int>(a.B) * static_cast<unsigned int>(a.nx));
+                l -= pos.sg * (static_cast<unsigned int>(a.B) * static_cast<unsigned int>(a.nx));
+            }
+            unsigned int B, nx;
+            dims(pos.sg, B, nx);
+            pos.b = l / nx;
+            pos.x = l - pos.b * nx;
+        }
+        auto row_of = [&](const LinePos& p, unsigned int& apod_row) -> const RawT* {
+            if (Tiles) {
+                const QueueTile& t = a.qt[p.sg];
+                apod_row = static_cast<unsigned int>(t.apod_row0) + p.b;
+                return static_cast<const RawT*>(t.raw) +
+                       (static_cast<int64_t>(p.b) * t.interf + t.apod + p.x) * kN;
+            }
+            apod_row = p.sg * static_cast<unsigned int>(a.B) + p.b;
+            return static_cast<const RawT*>(a.seg[p.sg]) +
+                   (static_cast<int64_t>(p.b) * a.interf + a.apod + p.x) * kN;
+        };
+        auto advance = [&](LinePos& p) {                     // kBgWarps A-scans on (tiles without A-scans are skipped)
+            unsigned int B, nx;
+            dims(p.sg, B, nx);
+            p.x += kBgWarps;
+            while (p.x >= nx) {
+                p.x -= nx;
+                if (++p.b == B) {
+                    p.b = 0;
+                    do {
+                        ++p.sg;
+                        dims(p.sg, B, nx);
+                    } while (B == 0);
+                }
+            }
+        };
+        // A-scan k of this warp: raw row into stage k & 1, its apodisation row
+        // into the other slot when it differs from the previous A-scan's
+        unsigned int have_row = 0xffffffffu;
+        int slot = 0;
+        auto issue = [&](int k, const LinePos& p) {
+            unsigned int ar;
+            const RawT* row = row_of(p, ar);
+            const bool load = ar != have_row;
+            if (load) {
+                have_row = ar;
+                slot ^= 1;
+            }
+            if (lane == 0) {
+                uint64_t* bar = &S.raw_full[w][k & 1];
+                mbar_expect_tx(bar, kN * sizeof(RawT) + (load ? kN * sizeof(float) : 0) +
+                                        starved_bytes(w == 0 && k == 0));
+                tma_bulk_g2s(S.raw[w][k & 1], row, kN * sizeof(RawT), bar);
+                if (load)
+                    tma_bulk_g2s(S.apod[w][slot], a.apod_mean + static_cast<int64_t>(ar) * kN, kN * sizeof(float), bar);
+            }
+        };
+        const int mine = (n - w + kBgWarps - 1) / kBgWarps;    // A-scans of this warp
+        issue(0, pos);
+        int issued = 1;
+        bool ok = true;
+        for (int k = 0; k < mine; ++k) {
+            const int cur = slot;                            // the current A-scan's apodisation row
+            if (k + 1 < mine) {
+                advance(pos);
+                __syncwarp();                                // stage (k + 1) & 1 was read by every lane
+                issue(k + 1, pos);
+                ++issued;
+            }
+            ok = wait(&S.raw_full[w][k & 1], static_cast<uint32_t>(k >> 1) & 1u);
+            if (__any_sync(0xffffffffu, !ok)) break;
+            // lane holds samples 4 lane + 128 i .. + 3, i = 0 .. 15 (i = p + 4 q).
+            // The sum keeps the order of the four partial sums of 128 threads
+            // with 16 samples each: p = lt / 32 of thread lt's, q within it.
+            float2 d[32];
+            float part[4];
+            const RawT* rw = S.raw[w][k & 1] + 4 * lane;
+            const float* ap = S.apod[w][cur] + 4 * lane;
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                float sum = 0.f;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int i = p + 4 * q;
+                    float2 r01, r23;
+                    raw4<RawT>(rw + 128 * i, r01, r23);
+                    const float4 m = *reinterpret_cast<const float4*>(ap + 128 * i);
+                    d[2 * i] = sub2(r01, make_float2(m.x, m.y));
+                    d[2 * i + 1] = sub2(r23, make_float2(m.z, m.w));
+                    sum += (d[2 * i].x + d[2 * i].y) + (d[2 * i + 1].x + d[2 * i + 1].y);
+                }
+                part[p] = sum;
+            }
+            // the four trees over 32 lanes (o = 16, 8, 4, 2, 1), two at a time
+            // after the first two steps: lane bit 4 selects the pair, bit 3 the sum
+            float s0, s1;
+            {
+                const bool up = (lane & 16) != 0;
+                s0 = (up ? part[2] : part[0]) + __shfl_xor_sync(0xffffffffu, up ? part[0] : part[2], 16);
+                s1 = (up ? part[3] : part[1]) + __shfl_xor_sync(0xffffffffu, up ? part[1] : part[3], 16);
+                const bool up2 = (lane & 8) != 0;
+                s0 = (up2 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, up2 ? s0 : s1, 8);
+            }
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+            s0 += __shfl_xor_sync(0xffffffffu, s0, 8);       // part 0 + part 1, part 2 + part 3
+            s0 += __shfl_xor_sync(0xffffffffu, s0, 16);
+            const float m = s0 * (1.0f / kN);
+            const int i_line = w + kBgWarps * k, st = i_line % kRing;
+            ok = wait(&S.empty[st], (static_cast<uint32_t>(i_line / kRing) & 1u) ^ 1u);
+            if (__any_sync(0xffffffffu, !ok)) break;
+            const float2 m2 = make_float2(m, m);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const float2 e01 = sub2(d[2 * i], m2), e23 = sub2(d[2 * i + 1], m2);
+                *reinterpret_cast<float4*>(&S.d[st][4 * lane + 128 * i]) = make_float4(e01.x, e01.y, e23.x, e23.y);
+            }
+            if (lane == 0) S.mval[st] = m;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&S.full[st]);
+        }
+        // copies still in flight land before the CTA's memory is released
+        if (!ok || issued < mine)
+            for (int k = issued - 2 < 0 ? 0 : issued - 2; k < issued; ++k)
+                mbar_wait_bounded(&S.raw_full[w][k & 1], static_cast<uint32_t>(k >> 1) & 1u, a.status);
+        return;
+    }
+
+    // ---------------------------------------------------- sinc
+    // the weights of outputs 4t, 4t + 1 (4t + 2, 4t + 3) at window step u form
+    // one packed pair wp[0][u] (wp[1][u]): two outputs per f32x2 fma
+    float2 wp[2][U];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int u = 0; u < U; ++u) wp[h][u] = __ldg(a.g.wsh + (h * U + u) * (kSincWarps * 32) + tid);
+    const int s0 = __ldg(a.g.s0 + tid);
+    const int wrot = s0 % U;                                 // window samples before s0 wrap to the next period
+    const int wbase = s0 - wrot;
+    float4 wa{}, wb{};                                       // window of outputs 4t .. 4t + 3
+    if (Mode == kModeSpec) {
+        wa = __ldg(reinterpret_cast<const float4*>(a.g.win + 4 * tid));
+        wb = __ldg(reinterpret_cast<const float4*>(a.g.win + 4 * tid + 2));
+    }
+    __syncthreads();
+    pdl_wait();                                              // the previous lines have been read
+    pdl_launch();
+    const int64_t out0 = static_cast<int64_t>(first - a.out_l0);
+    // two A-scans an iteration (their ring stages are adjacent, so the window
+    // addresses are formed once for both)
+    for (int i = 0; i < n; i += 2) {
+        const int st = i % kRing;
+        const uint32_t ph = static_cast<uint32_t>(i / kRing) & 1u;
+        const bool two = i + 1 < n;
+        bool ok = wait(&S.full[st], ph);
+        if (ok && two) ok = wait(&S.full[st + 1], ph);
+        if (__any_sync(0xffffffffu, !ok)) return;
+        const float* dk = S.d[st] + wbase;
+        float2 acc[2][2] = {};
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const float* p = dk + (u < wrot ? u + U : u);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float x = p[h * kDLine];
+                acc[h][0] = fma2(wp[0][u], make_float2(x, x), acc[h][0]);
+                acc[h][1] = fma2(wp[1][u], make_float2(x, x), acc[h][1]);
+            }
+        }
+        const float mk[2] = {S.mval[st], S.mval[st + 1]};
+        __syncwarp();
+        if (lane == 0) {
+            mbar_arrive(&S.empty[st]);
+            if (two) mbar_arrive(&S.empty[st + 1]);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (h == 1 && !two) break;
+            const float2 m2 = make_float2(mk[h], mk[h]);
+            const float2 v01 = add2(acc[h][0], m2), v23 = add2(acc[h][1], m2);
+            if (Mode == kModeReal) {
+                *reinterpret_cast<float4*>(a.out + (out0 + i + h) * kN + 4 * tid) = make_float4(v01.x, v01.y, v23.x, v23.y);
+            } else if (Mode == kModeSpec) {
+                // spec output undoes the 1/N ifft scaling folded into the window
+                float4* o = reinterpret_cast<float4*>(a.out + ((out0 + i + h) * kN + 4 * tid) * 2);
+                o[0] = make_float4(v01.x * wa.x * kN, v01.x * wa.y * kN, v01.y * wa.z * kN, v01.y * wa.w * kN);
+                o[1] = make_float4(v23.x * wb.x * kN, v23.x * wb.y * kN, v23.y * wb.z * kN, v23.y * wb.w * kN);
+            } else {
+                // the plain line (its window is one) times the float64 window, one rounding to float32
+                const float lx[4] = {v01.x, v01.y, v23.x, v23.y};
+                float lh[4];
+                bool lsafe[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) lh[r] = mul_window(lx[r], __ldg(a.hann2 + 4 * tid + r), lsafe[r]);
+                const bool all_safe = lsafe[0] && lsafe[1] && lsafe[2] && lsafe[3];
+                if (__any_sync(0xffffffffu, !all_safe)) {
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        if (!lsafe[r])
+                            lh[r] = static_cast<float>(static_cast<double>(lx[r]) * __ldg(a.hann + 4 * tid + r));
+                }
+                *reinterpret_cast<float4*>(a.out + (out0 + i + h) * kN + 4 * tid) = make_float4(lh[0], lh[1], lh[2], lh[3]);
+            }
+        }
+    }
+}
+
+// apodisation mean (cpu_kernels.py:20-25): exact sum, divided in float64,
+// stored float32.  Four samples a thread, five lines in flight.
+constexpr int kApodThreads = 128;                // x 4 samples = a quarter of a row
+template <typename RawT, bool Tiles>
+__global__ void __launch_bounds__(kApodThreads) k_apod_mean(const LinesArgs a, float* __restrict__ out) {
+    pdl_launch();                                // the lines kernel loads its weights meanwhile
+    const int row = blockIdx.x >> 2;             // segment * B + b, or the tiles' apod_row0 + b
+    const int j = ((blockIdx.x & 3) * kApodThreads + threadIdx.x) * 4;
+    const RawT* p;
+    int apod;
+    if (Tiles) {
+        int lo = 0, hi = a.n_qt - 1;             // last tile with apod_row0 <= row
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (a.qt[mid].apod_row0 <= row) lo = mid; else hi = mid - 1;
+        }
+        const QueueTile& t = a.qt[lo];
+        apod = t.apod;
+        p = static_cast<const RawT*>(t.raw) + static_cast<int64_t>(row - t.apod_row0) * t.interf * kN + j;
+    } else {
+        const int sg = row / a.B;
+        apod = a.apod;
+        p = static_cast<const RawT*>(a.seg[sg]) + static_cast<int64_t>(row - sg * a.B) * a.interf * kN + j;
+    }
+    double s[4];
+    if (sizeof(RawT) == 2) {
+        int acc[4] = {0, 0, 0, 0};
+#pragma unroll 5
+        for (int k = 0; k < apod; ++k) {
+            const uint2 q = __ldg(reinterpret_cast<const uint2*>(p + static_cast<int64_t>(k) * kN));
+            acc[0] += static_cast<int>(static_cast<RawT>(q.x & 0xffffu));
+            acc[1] += static_cast<int>(static_cast<RawT>(q.x >> 16));
+            acc[2] += static_cast<int>(static_cast<RawT>(q.y & 0xffffu));
+            acc[3] += static_cast<int>(static_cast<RawT>(q.y >> 16));
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[e] = static_cast<double>(acc[e]);
+    } else {
+        s[0] = s[1] = s[2] = s[3] = 0.0;
+#pragma unroll 5
+        for (int k = 0; k < apod; ++k) {
+            const float4 q = __ldg(reinterpret_cast<const float4*>(p + static_cast<int64_t>(k) * kN));
+            s[0] += static_cast<double>(q.x);
+            s[1] += static_cast<double>(q.y);
+            s[2] += static_cast<double>(q.z);
+            s[3] += static_cast<double>(q.w);
+        }
+    }
+    *reinterpret_cast<float4*>(out + static_cast<int64_t>(row) * kN + j) =
+        make_float4(static_cast<float>(s[0] / apod), static_cast<float>(s[1] / apod), static_cast<float>(s[2] / apod),
+                    static_cast<float>(s[3] / apod));
+}
+
+template <typename RawT, int Mode, int U, bool Tiles>
+cudaError_t launch_t(const LinesArgs& a, int num_sms, cudaStream_t st) {
+    const size_t smem = sizeof(LinesSmem<RawT>);
+    const auto kernel = k_lines<RawT, Mode, U, Tiles>;
+    constexpr int kType = sizeof(RawT) == 4 ? 2 : static_cast<RawT>(-1) < 0 ? 1 : 0;
+    constexpr int kBit = (kType * 4 + (Tiles ? 3 : Mode)) * 4 + (U - 14) / 4;
+    static_assert(kBit < kReadyDisp, "the bits of the kernels overlap");
+    const cudaError_t e = kernel_ready(a.ready, kBit, kernel, smem);
+    if (e != cudaSuccess) return e;
+    const unsigned int n = a.l1 - a.l0;
+    const unsigned int grid = n < static_cast<unsigned int>(num_sms) ? n : static_cast<unsigned int>(num_sms);
+    return launch_dependent(kernel, dim3(grid), dim3(kThr), smem, st, a);
+}
+
+// (wider windows than 14 spill a few weights: five warps a scheduler have 96 registers a thread)
+template <typename RawT, int Mode, bool Tiles>
+cudaError_t launch_u(const LinesArgs& a, int num_sms, cudaStream_t st) {
+    switch (a.g.U) {
+        case 14: return launch_t<RawT, Mode, 14, Tiles>(a, num_sms, st);
+        case 18: return launch_t<RawT, Mode, 18, Tiles>(a, num_sms, st);
+        case 22: return launch_t<RawT, Mode, 22, Tiles>(a, num_sms, st);
+        case 26: return launch_t<RawT, Mode, 26, Tiles>(a, num_sms, st);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+template <typename RawT>
+cudaError_t launch_mode(const LinesArgs& a, int mode, int num_sms, cudaStream_t st) {
+    if (a.qt != nullptr) return launch_u<RawT, kModeReal, true>(a, num_sms, st);
+    switch (mode) {
+        case kModeSpec: return launch_u<RawT, kModeSpec, false>(a, num_sms, st);
+        case kModeLinHann: return launch_u<RawT, kModeLinHann, false>(a, num_sms, st);
+        default: return launch_u<RawT, kModeReal, false>(a, num_sms, st);
+    }
+}
+
+template <typename RawT>
+void launch_apod_t(const LinesArgs& a, int rows, float* out, cudaStream_t st) {
+    if (a.qt != nullptr)
+        k_apod_mean<RawT, true><<<4 * rows, kApodThreads, 0, st>>>(a, out);
+    else
+        k_apod_mean<RawT, false><<<4 * rows, kApodThreads, 0, st>>>(a, out);
+}
+
+}  // namespace
+
+cudaError_t launch_apod_mean(const LinesArgs& a, int dtype, int rows, float* out, cudaStream_t st) {
+    if (rows == 0) return cudaSuccess;
+    if (dtype == 0)
+        launch_apod_t<uint16_t>(a, rows, out, st);
+    else if (dtype == 1)
+        launch_apod_t<int16_t>(a, rows, out, st);
+    else
+        launch_apod_t<float>(a, rows, out, st);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_lines(const LinesArgs& a, int dtype, int mode, int num_sms, cudaStream_t st) {
+    if (a.l1 == a.l0) return cudaSuccess;
+    if (dtype == 0) return launch_mode<uint16_t>(a, mode, num_sms, st);
+    if (dtype == 1) return launch_mode<int16_t>(a, mode, num_sms, st);
+    return launch_mode<float>(a, mode, num_sms, st);
+}
+
+cudaError_t set_wait_test_spectral(unsigned long long limit_ns, int starve, cudaStream_t st) {
+    return set_wait_test_here(limit_ns, starve, st);
+}
+
+}  // namespace octgb

@@ -10,11 +10,6 @@
 namespace octgb {
 namespace {
 
-constexpr int kPadShift = 4;                              // one pad slot per 16 complex
-constexpr int kSpecStride = kN + (kN >> kPadShift);       // padded complex line length
-
-__device__ __forceinline__ int pad(int e) { return e + (e >> kPadShift); }
-
 // Packed float32 pairs (sm_100 family f32x2 instructions): one instruction
 // for both lanes, each lane rounded to nearest exactly as the scalar operation,
 // so results are bit-identical to two scalar ops.  The explicit rounding mode
@@ -133,38 +128,6 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 
-// one arrival on the mbarrier once every cp.async this thread issued so far
-// has landed (counted against the barrier's expected arrivals)
-// asynchronous global -> shared copy of 16 bytes (both addresses 16-byte
-// aligned) through L2 only, no L1 line allocated; tracked per thread
-__device__ __forceinline__ void cp_async_cg16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-// raise the barrier's pending transaction count without arriving
-__device__ __forceinline__ void mbar_expect_tx_only(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-
-// shared -> global bulk copy (both addresses 16-byte aligned, bytes a multiple
-// of 16) in this thread's bulk group; the shared source must stay unchanged
-// until bulk_wait_read().  Generic-proxy writes of the source need
-// fence_proxy_async() by their writers (and a barrier) before the copy.
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tma_bulk_s2g(void* dst, const void* src, uint32_t bytes) {
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)),
-                 "r"(bytes)
-                 : "memory");
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-}
-// this thread's bulk copies have read their sources / are complete
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
     uint32_t done;
     asm volatile(
@@ -204,6 +167,30 @@ __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
 // (octgb_selftest_wait_expiry); the product never changes them.
 __device__ unsigned long long g_wait_limit_ns = 2000000000ull;
 __device__ int g_starve_first_copy = 0;
+
+// Programmatic dependent launch: a kernel started by launch_dependent() may
+// begin while the one before it in the stream drains; pdl_wait() returns when
+// that one has completed and its writes are visible, so a kernel calls it
+// before it touches anything an earlier one wrote or reads.  pdl_launch() lets
+// the next such kernel's blocks take the places of blocks that exit.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... Params, typename... Args>
+inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                    Args&&... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
 
 // bytes a CTA's first bulk-copy barrier expects beyond its copies (0 outside the self-test)
 __device__ __forceinline__ uint32_t starved_bytes(bool first) { return first && g_starve_first_copy ? 16u : 0u; }
@@ -289,109 +276,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ void group_sync(int g) {
-    asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(kGroup) : "memory");
-}
-
-// Inverse FFT of one 2048-point line X (padded, see pad()) by the 128 threads
-// of group g (thread lt of the group), Stockham radix 16, 16, 8 with the last
-// stage pruned to the low half: on return mag[h][r] = |X[k]| for
-// k = lt + 128 h + 256 r (k < N/2), the square root correctly rounded.  The
-// transform is unnormalised (any 1/N is folded into the input).  X is
-// overwritten.  tw2[r][j] = w^(r j N/256), tw3[r][j] = w^(r j), w = e^(2 pi i/N).
-// ifft2048_low_mag_regs is the same transform with the first stage's inputs
-// v[r] = x[lt + 128 r] already in registers (X is then only work space).
-__device__ __forceinline__ void ifft2048_low_mag_regs(float2 (&v0)[16], float2* X, const float2 (*tw2)[16],
-                                                      const float2 (*tw3)[256], int g, int lt,
-                                                      float (&mag)[2][4]) {
-    {
-        float2 (&v)[16] = v0;
-        dft16(v);
-        group_sync(g);
-#pragma unroll
-        for (int r = 0; r < 16; ++r) X[pad(16 * lt + r)] = v[r];
-        group_sync(g);
-    }
-    {
-        float2 v[16];
-        const int jm = lt & 15;
-#pragma unroll
-        for (int r = 0; r < 16; ++r) v[r] = X[pad(lt + 128 * r)];
-#pragma unroll
-        for (int r = 1; r < 16; ++r) v[r] = cmul(v[r], tw2[r][jm]);
-        dft16(v);
-        group_sync(g);
-        const int idxD = (lt >> 4) * 256 + jm;
-#pragma unroll
-        for (int r = 0; r < 16; ++r) X[pad(idxD + 16 * r)] = v[r];
-        group_sync(g);
-    }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int j = lt + 128 * h;
-        float2 v[8];
-#pragma unroll
-        for (int r = 0; r < 8; ++r) v[r] = X[pad(j + 256 * r)];
-#pragma unroll
-        for (int r = 1; r < 8; ++r) v[r] = cmul(v[r], tw3[r][j]);
-        float2 Xk[4];
-        dft8_low(v, Xk);
-#pragma unroll
-        for (int r = 0; r < 4; ++r) mag[h][r] = __fsqrt_rn(fmaf(Xk[r].x, Xk[r].x, Xk[r].y * Xk[r].y));
-    }
-}
-
-// The same transform with a second padded line Y: the first stage writes Y
-// and the second writes X back, so a stage never overwrites the line it reads
-// and only the barrier after its stores is needed (two group barriers per
-// line instead of four).  X holds the input; both lines are work space.
-__device__ __forceinline__ void ifft2048_low_mag_pp(float2* X, float2* Y, const float2 (*tw2)[16],
-                                                    const float2 (*tw3)[256], int g, int lt, float (&mag)[2][4]) {
-    {
-        float2 v[16];
-#pragma unroll
-        for (int r = 0; r < 16; ++r) v[r] = X[pad(lt + 128 * r)];
-        dft16(v);
-#pragma unroll
-        for (int r = 0; r < 16; ++r) Y[pad(16 * lt + r)] = v[r];
-        group_sync(g);
-    }
-    {
-        float2 v[16];
-        const int jm = lt & 15;
-#pragma unroll
-        for (int r = 0; r < 16; ++r) v[r] = Y[pad(lt + 128 * r)];
-#pragma unroll
-        for (int r = 1; r < 16; ++r) v[r] = cmul(v[r], tw2[r][jm]);
-        dft16(v);
-        const int idxD = (lt >> 4) * 256 + jm;
-#pragma unroll
-        for (int r = 0; r < 16; ++r) X[pad(idxD + 16 * r)] = v[r];
-        group_sync(g);
-    }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int j = lt + 128 * h;
-        float2 v[8];
-#pragma unroll
-        for (int r = 0; r < 8; ++r) v[r] = X[pad(j + 256 * r)];
-#pragma unroll
-        for (int r = 1; r < 8; ++r) v[r] = cmul(v[r], tw3[r][j]);
-        float2 Xk[4];
-        dft8_low(v, Xk);
-#pragma unroll
-        for (int r = 0; r < 4; ++r) mag[h][r] = __fsqrt_rn(fmaf(Xk[r].x, Xk[r].x, Xk[r].y * Xk[r].y));
-    }
-}
-
-__device__ __forceinline__ void ifft2048_low_mag(float2* X, const float2 (*tw2)[16], const float2 (*tw3)[256],
-                                                 int g, int lt, float (&mag)[2][4]) {
-    float2 v[16];
-#pragma unroll
-    for (int r = 0; r < 16; ++r) v[r] = X[pad(lt + 128 * r)];
-    ifft2048_low_mag_regs(v, X, tw2, tw3, g, lt, mag);
-}
-
 // Inverse FFT of one 2048-point line by one warp, 64 points a lane, with one
 // exchange through the warp's own shared memory and no block barrier.  The
 // arithmetic is that of the radix 16, 16, 8 transform above, operation for
@@ -409,7 +293,6 @@ __device__ __forceinline__ void ifft2048_low_mag(float2* X, const float2 (*tw2)[
 // tw2[16 j + r] = w^(r j N/256), tw3[256 (r - 1) + j] = w^(r j) for r >= 1.
 constexpr int kWarpPitch = 33;
 constexpr int kWarpExchange = 32 * kWarpPitch;            // float2 of a warp's exchange buffer
-constexpr int kTw3 = 7 * 256;
 
 template <typename Emit>
 __device__ __forceinline__ void ifft2048_low_mag_warp(float2 (&v)[64], float2* ex, const float2* tw2,

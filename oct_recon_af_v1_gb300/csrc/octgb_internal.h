@@ -10,30 +10,39 @@ constexpr int kN = 2048;          // spectral samples per A-scan (FFT length)
 constexpr int kHalf = kN / 2;     // depth bins kept (core/spectral.py:153, nz = N/2)
 constexpr int kMaxTaps = 32;      // sinc taps supported
 constexpr int kTail = 32;         // zero tail after each line so padded taps stay in bounds
-constexpr int kGroup = 128;       // threads per A-scan in the FFT (16 points each)
-constexpr int kPerCta = 4;        // A-scans per CTA iteration
-constexpr int kThreads = kGroup * kPerCta;
+constexpr int kSincThreads = 512; // threads of the banded sinc, four outputs each
+// A-scans of one pass (lines kernel, transform) through the linearised lines'
+// scratch: at most 600 per SM (712 MiB).  A pass costs its two kernels' ramps
+// and tails (~12 us) and longer ones win although their lines go through DRAM:
+// 324 000 A-scans stitched took 4043, 3685, 3479, 3356 and 3290 us with 24,
+// 48, 96, 192 and 600 per SM.  set_geometry makes room for kFirstPass (228
+// MiB: a first call of up to 29 184 A-scans allocates nothing), longer calls
+// grow it; the allocation-free entry point has its own of kMinPass.
+constexpr int kMaxPass = 152 * 600, kFirstPass = 152 * 192, kMinPass = 152 * 24;
+constexpr int kTwTable = 256 + 7 * 256;   // the transform's twiddles tw2, tw3
 
 // device-side status word values
 constexpr int kStatusOk = 0;
 constexpr int kStatusTimeout = 1;
 
-// kModeLinHann: the real linearised line times a float64 window, rounded once
-// to float32 (the scorer's input, (eq * hann).astype(complex64) with a window of ones)
-enum OutMode : int { kModeSpec = 0, kModeMag = 1, kModeDb = 2, kModeResample = 3, kModeLinHann = 4 };
+// What k_lines writes per A-scan: the real linearised line; that times the
+// complex window (the fused pre-FFT operator); or that times a float64 window,
+// rounded once to float32 (the scorer's input, (eq * hann).astype(complex64)
+// with a window of ones).
+enum LineMode : int { kModeReal = 0, kModeSpec = 1, kModeLinHann = 2 };
+// What follows the transform: |X|, dB of a depth crop with its range
+enum OutMode : int { kModeMag = 0, kModeDb = 1 };
 
 constexpr int kBlk = 32;          // output rows / columns per stitch block
 constexpr int kMaxSeg = 32;       // tiles per multi-tile launch
 
 struct DevGeometry {
-    const float* w;       // [taps][kN] sinc weights, tap-major, float32
-    const int* start;     // [kN] first source sample of each output sample
-    int taps;
-    const float* wsh;     // [kThreads][4][U] shifted weights of outputs 4t..4t+3
-    const int* s0;        // [kThreads] source window base of thread t
-    int U;                // window width (16, 20 or 24)
+    // [2][U][kSincThreads] shifted weights of outputs 4t, 4t + 1 (4t + 2, 4t + 3) at window step u
+    const float2* wsh;
+    const int* s0;        // [kSincThreads] source window base of thread t
+    int U;                // window width (14, 18, 22 or 26)
     const float2* win;    // [kN] complex64 window scaled by 1/kN (ifft normalisation)
-    const float2* tw;     // [kN] exp(+2*pi*i*k/kN), rounded from float64
+    const float2* tw;     // [kTwTable] twiddles of the transform, rounded from float64
 };
 
 struct StitchDev;
@@ -46,12 +55,13 @@ struct QueueTile {
     const StitchDev* plan;    // device pointer into the context's plan table
     int B, interf, apod, nx, nz;
     int apod_row0;            // first row of the tile in the apodisation-mean buffer
-    unsigned int quad0;       // first global quad (4 A-scans) of the tile
-    unsigned int nquads;      // B * qpb
-    int qpb;                  // quads per B-scan (quads never span two B-scans)
+    unsigned int line0;       // first global A-scan of the tile
     int pad_;
 };
 constexpr int kMaxQueueTiles = 256;
+// a batched tile's lateral weights stay inside groups of this many A-scans (the
+// last group of a B-scan ends on its last A-scan)
+constexpr int kLateral = 4;
 
 // float64 form of the spectral stage (exact.cu)
 struct ExactArgs {
@@ -68,40 +78,47 @@ struct ExactArgs {
 };
 cudaError_t launch_exact(const ExactArgs& a, int dtype, int* sums, int num_sms, cudaStream_t st);
 
+// the raw batches of the precision form's kernels
 struct SpectralArgs {
-    const void* raw;          // (B, interf, kN), segment 0
-    const void* seg[kMaxSeg]; // raw batches of n_seg tiles, each (B, interf, kN); seg[0] == raw
-    int n_seg;
+    const void* raw;          // (B, interf, kN)
     int B, interf, apod, nx;  // nx = interf - apod
-    int64_t n_ascans;         // n_seg * B * nx
-    const float* apod_mean;   // (n_seg * B, kN) float32 apodisation mean
-    DevGeometry g;
-    float* out;               // spec (M, kN, 2) | mag (M, kHalf) | db (M, nz) | windowed line (M, kN)
-    const double* hann;       // kModeLinHann: the float64 window (kN)
-    const float2* hann2;      // kModeLinHann: the window split hi + lo in float32 (kN)
-    int z0, nz;               // depth crop (db mode)
-    unsigned int* minmax;     // [2] ordered-uint min / max (db / resample modes), may be null
-    int* status;              // device status word
-    // work-queue mode (resample): tiles of uneven size, quads taken from a counter
-    const QueueTile* qt;
-    int n_qt;
-    unsigned int* counter;    // queue head in quads, zero before the launch
-    unsigned int total_quads;
-    int grab;                 // quads taken per atomic grab
-    float thr;                // weight threshold (pipeline.py:296-297)
-    // static mode, set by the launcher: a CTA's grid stride (gridDim.x quads)
-    // as whole B-scans plus A-scans, step_x < nx
-    unsigned int step_bt, step_x;
+    int64_t n_ascans;         // B * nx
 };
 
-// spectral.cu
-cudaError_t launch_apod_mean(const SpectralArgs& a, int dtype, cudaStream_t st);
-// apodisation mean of every B-scan of the queue tiles (rows by tile.apod_row0)
-cudaError_t launch_apod_mean_tiles(const QueueTile* tiles_dev, int n_tiles, int total_rows, int dtype,
-                                   float* apod_mean, cudaStream_t st);
-cudaError_t launch_spectral(const SpectralArgs& a, int dtype, int mode, int grid, cudaStream_t st);
-int spectral_max_ctas_per_sm(int dtype, int mode);
-size_t spectral_smem_bytes(int dtype);
+// The context's device allows `kernel` its shared memory; the attribute is set
+// on the kernel's first launch through a context (bit `bit` of its `ready`), not
+// on every one (~1 us of host time each).
+template <typename Kernel>
+inline cudaError_t kernel_ready(uint64_t* ready, int bit, Kernel kernel, size_t smem) {
+    if (*ready >> bit & 1u) return cudaSuccess;
+    const cudaError_t e =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e == cudaSuccess) *ready |= uint64_t(1) << bit;
+    return e;
+}
+constexpr int kReadyDisp = 48;            // bits 0 .. 47: k_lines, 48 .. 52: k_disp_mag
+
+// lines.cu: A-scans [l0, l1) of n_seg raw batches of one shape, or of tiles of
+// uneven size (qt), numbered segment by segment, B-scan by B-scan
+struct LinesArgs {
+    const void* seg[kMaxSeg]; // raw batches, each (B, interf, kN)
+    int B, interf, apod, nx;  // nx = interf - apod
+    const QueueTile* qt;      // null: the batches above
+    int n_qt;
+    unsigned int l0, l1;
+    const float* apod_mean;   // float32 apodisation mean, a row per B-scan
+    DevGeometry g;
+    float* out;               // line l at (l - out_l0) kN (kModeSpec: complex)
+    unsigned int out_l0;
+    const double* hann;       // kModeLinHann: the float64 window (kN)
+    const float2* hann2;      // kModeLinHann: the window split hi + lo in float32 (kN)
+    int* status;              // device status word
+    uint64_t* ready;          // host: bits of the caller's context, see kernel_ready
+};
+// apodisation mean of every B-scan (`rows` of them) into out
+cudaError_t launch_apod_mean(const LinesArgs& a, int dtype, int rows, float* out, cudaStream_t st);
+// launched dependent on the kernel before it in the stream (as launch_disp_mag's)
+cudaError_t launch_lines(const LinesArgs& a, int dtype, int mode, int num_sms, cudaStream_t st);
 
 // stitch.cu
 struct StitchDev {
@@ -154,6 +171,10 @@ cudaError_t launch_stitch_frames(const StitchDev* plans_dev, const TileList& til
                                  int64_t mag_tile_stride, int B, int n_tile_x, int f0, int n_out_z, int n_out_x,
                                  float thr, float* db, unsigned int* plane_mm, unsigned int* run_mm, int rows,
                                  cudaStream_t st);
+// batched form: dB rows of the A-scans [l0, l1) of tiles of uneven size from
+// their magnitudes (A-scan l at (l - l0) kHalf), with the running range
+cudaError_t launch_resample(const QueueTile* qt, int n_qt, unsigned int l0, unsigned int l1, const float* mag,
+                            float thr, unsigned int* run_mm, cudaStream_t st);
 cudaError_t launch_finalise(const float* num, const float* den, int64_t n_per_plane, int n_planes, float thr,
                             float* db, unsigned int* plane_minmax, cudaStream_t st);
 // quantisation: `table` is scratch of kQuantTable floats (the code thresholds of the clim)
@@ -170,11 +191,15 @@ cudaError_t launch_minmax_init(unsigned int* minmax, int count, cudaStream_t st)
 struct DispArgs {
     const float* X;        // (B, rep, nx, kN) linearised, windowed, real
     const float2* phase;   // (n_beta, kN) exp(-i beta dk^2) / N
-    const float2* tw;      // (kN) e^(2 pi i k / N)
-    float* A;              // (n_beta, nb, nx, kHalf), or null with zcol
+    const float2* tw;      // kTwTable twiddles
+    float* A;              // (n_beta, nb, nx, kHalf), or null with zcol; dB rows of nz with mode kModeDb
+    int mode;              // kModeMag, or kModeDb: 20 log10 |X| of depths [z0, z0 + nz) (rep = 1)
+    int z0, nz;
+    unsigned int* minmax;  // kModeDb: [2] ordered-uint range of the finite dB, may be null
     float* zcol;           // (n_beta, nb, nx, 256) depth-pooled sums of |X| (probe images), or null
     int z_keep;            // depths pooled into the 256 image rows
     int n_beta, nb, b0, nx, rep;
+    uint64_t* ready;       // host: bits of the caller's context, see kernel_ready
 };
 cudaError_t launch_disp_mag(const DispArgs& a, int num_sms, cudaStream_t st);
 // per segment (n_seg rows of nx x kHalf magnitudes): metric 1 top_percentile

@@ -42,8 +42,7 @@ class SpectralProcessor:
         if isinstance(raw, np.ndarray):
             return np.empty(shape, dtype)
         import torch
-        tdt = {np.dtype(np.float32): torch.float32, np.dtype(np.complex64): torch.complex64}[np.dtype(dtype)]
-        return torch.empty(shape, dtype=tdt, device=raw.device)
+        return torch.empty(shape, dtype=torch.float32 if dtype is np.float32 else torch.complex64, device=raw.device)
 
     def prepare(self, raw):
         """(prepared raw, its apodisation line count): `raw` itself for the

@@ -103,3 +103,69 @@ def test_x_profiles_equal_numpy(gpu_ctx, nx, nz):
         np.testing.assert_array_equal(gpu_ctx.xmedian(mag), np.median(mag.astype(np.float64), axis=1))
         np.testing.assert_array_equal(gpu_ctx.xmedian(mag, ignore_nan=True),
                                       np.nanmedian(mag.astype(np.float64), axis=1))
+
+
+@pytest.mark.parametrize("dtype", [np.uint16, np.int16, np.float32])
+@pytest.mark.parametrize("bscans,nx", [(1, 1), (1, 2), (3, 1), (2, 7), (1, 305), (5, 123)])
+def test_lines_and_magnitudes_of_ragged_batches(gpu_ctx, dtype, bscans, nx):
+    """Fewer A-scans than blocks, odd counts, B-scans of one A-scan, signed and
+    negative counts: the linearised spectra and magnitudes against the oracle's
+    float32 restatement.  Tolerance 2e-6 of the largest value: about ten
+    float32 roundings in the band sum, eleven layers of the transform."""
+    from oracle import numerics as O
+    from oct_recon_af_v1_gb300 import geometry as G
+    from oct_recon_af_v1_gb300 import synthetic
+    lam, beta = synthetic.lambda_nm(), synthetic.beta_ref_from_px(1e-5)
+    sg = G.build_spectral_geometry(lam, beta, 1.33)
+    gpu_ctx.set_geometry(sg.sinc_idx, sg.sinc_w, sg.window)
+    raw = synthetic.generate_numpy(bscans, nx, 25, seed=bscans * 1000 + nx)
+    if dtype == np.int16:
+        raw = (raw.astype(np.int32) - 9000).astype(np.int16)
+    raw = raw.astype(dtype)
+    og = O.spectral_geometry(lam, beta, 1.33)
+    ref = O.magnitude_numba(raw, og, 25)
+    assert np.abs(gpu_ctx.magnitude(raw, 25) - ref).max() < 2e-6 * np.abs(ref).max()
+    spec = O.fused_pre_fft_numba(raw, 25, og.sinc_idx.T, og.sinc_w.T.astype(np.float32),
+                                 og.window.astype(np.complex64))
+    assert np.abs(gpu_ctx.fused_pre_fft(raw, 25) - spec).max() < 2e-6 * np.abs(spec).max()
+
+
+def test_batched_tiles_equal_single_tiles_across_passes(gpu_ctx):
+    """Tiles of uneven size (an empty one, B-scans shorter than a group of
+    four, one B-scan longer than the smallest pass) in one call against one
+    call a tile: the same bits and the same running range."""
+    torch = pytest.importorskip("torch")
+    from oct_recon_af_v1_gb300 import _lib
+    from oct_recon_af_v1_gb300 import geometry as G
+    from oct_recon_af_v1_gb300 import stitching as S
+    from oct_recon_af_v1_gb300 import synthetic
+    ctx = _lib.Context(0)
+    try:
+        sg = G.build_spectral_geometry(synthetic.lambda_nm(), 0.0, 1.33)
+        ctx.set_geometry(sg.sinc_idx, sg.sinc_w, sg.window)
+        tiles = []
+        for k, (b, nx, rows) in enumerate(((2, 3, 50), (0, 9, 40), (1, 3801, 33), (3, 130, 257), (1, 5, 700))):
+            lay = S.ScanLayout(np.array([0.0]), np.array([0.0]), np.array([0.0]), nx, max(b, 1), nx * 1e-3,
+                                max(b, 1) * 1e-3)
+            z = S.tiled_geometry(lay, sg.z_um, [np.nan], 1.0).out_z_mm
+            tg = S.tiled_geometry(lay, sg.z_um, [np.nan], 1.0, (z[10] - 1e-9, z[9 + rows] + 1e-9))
+            plan = S.TileStitcher.build(tg, 0.0, 0.0, np.nan, 80.0).upload(ctx)
+            raw = torch.from_numpy(synthetic.generate_numpy(max(b, 1), nx, 25, seed=k).view(np.int16)).cuda()[:b]
+            tiles.append((raw.contiguous(), 25, plan, torch.empty((b, nx, len(tg.out_z_mm)), device="cuda")))
+        if tiles[1][3].data_ptr() == 0:                     # an empty tile still has a place in memory
+            tiles[1] = (tiles[0][0][:0], 25, tiles[1][2], torch.empty(16, device="cuda")[:0].view(0, 9, 0))
+        args = [t for t in tiles if t[0].data_ptr() and t[3].data_ptr()]
+        thr = S.min_weight_threshold(np.float32)
+        ctx.clim_reset()
+        ctx.batch_process(args, thr)
+        together, clim = [t[3].clone() for t in args], ctx.clim_get()
+        ctx.clim_reset()
+        for t in args:
+            t[3].fill_(0)
+            ctx.batch_process([t], thr)
+        assert ctx.clim_get() == clim
+        for t, ref in zip(args, together):
+            assert torch.isfinite(ref).all()
+            assert torch.equal(t[3], ref)
+    finally:
+        ctx.close()
