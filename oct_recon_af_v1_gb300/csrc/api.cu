@@ -55,14 +55,36 @@ struct DevBuf {
     }
 };
 
+// Which tiles touch each output block of the stitch kernel, with
+// their patch extents and shared-memory offsets; built once per tile list.
+struct SlotTable {
+    std::vector<int> key;        // plan ids, n_out_z, n_out_x, rows per block
+    DevBuf slots, counts, tslots;
+    // tensor copies (no optical-path correction, patches of one shape that fit):
+    bool tma = false;
+    int pitch = 0, box_lines = 0, tma_round = 1;
+    uint32_t patch_bytes = 0, slot_bytes = 0;
+    size_t smem = 0;             // largest patch footprint of a round (bytes)
+    int ns_round = 1;            // most slots of a round
+    void release() {
+        slots.release();
+        counts.release();
+        tslots.release();
+    }
+};
+
 struct Plan {
     int n_rows, r0, R, c0, C, n_out_z, n_tile_x, n_y;
-    int cblk_first = 0, n_cblk = 0, xs_max = 1, rs_max = 1;
-    std::vector<int2> zblk_h, cblk_h;   // host copies of the block tables
+    int cblk_first = 0, n_cblk = 0;
+    std::vector<int2> zblk_h;           // per 32 output rows: input rows [x, y] they read; x = -1: none
+    std::vector<int2> cblk_h;           // per 32 output columns from block cblk_first: A-scans [x, y]; x = -1: none
+    std::vector<int2> cblk1_h;          // the same where each column takes one A-scan; x = -1: not all do
     bool lateral_identity = false;      // WxT is the identity (single-tile output grid)
     bool lateral_quad_local = false;    // every non-zero lateral weight stays inside the column's group of four
-    DevBuf zr, wz0, wz1, xr, wx0, wx1, fz, shift, lo, hi, zblk, cblk, zrow, zf, xcol;
+    DevBuf zr, wz0, wz1, xr, wx0, wx1, fz, shift, lo, hi, zrow, zf, xcol;
     bool opc = false;
+    SlotTable row_table;                // blocks of this tile alone, from column block cblk_first (row interface)
+    int row_rows = kStitchRows;         // their height
     StitchDev dev() const {
         StitchDev d;
         d.zr = zr.as<int>();
@@ -75,13 +97,9 @@ struct Plan {
         d.shift = opc ? shift.as<int>() : nullptr;
         d.lo = opc ? lo.as<int>() : nullptr;
         d.hi = opc ? hi.as<int>() : nullptr;
-        d.zblk = zblk.as<int2>();
-        d.cblk = cblk.as<int2>();
         d.zrow = zrow.as<float4>();
         d.zf = zf.as<float2>();
-        d.xcol = xcol.as<float4>();
-        d.cblk_first = cblk_first;
-        d.n_cblk = n_cblk;
+        d.xcol = xcol.as<float4>() + kBlk;
         d.r0 = r0;
         d.R = R;
         d.c0 = c0;
@@ -92,21 +110,9 @@ struct Plan {
         return d;
     }
     void release() {
-        for (DevBuf* b : {&zr, &wz0, &wz1, &xr, &wx0, &wx1, &fz, &shift, &lo, &hi, &zblk, &cblk, &zrow, &zf, &xcol})
+        for (DevBuf* b : {&zr, &wz0, &wz1, &xr, &wx0, &wx1, &fz, &shift, &lo, &hi, &zrow, &zf, &xcol})
             b->release();
-    }
-};
-
-// Which tiles touch each output block of the frame-batch stitch kernel, with
-// their patch extents and shared-memory offsets; built once per tile list.
-struct SlotTable {
-    std::vector<int> key;        // plan ids, n_out_z, n_out_x, rows per block
-    DevBuf slots, counts;
-    size_t smem = 0;             // largest patch footprint of a block (bytes)
-    int ns_max = 1;              // most tiles touching one block
-    void release() {
-        slots.release();
-        counts.release();
+        row_table.release();
     }
 };
 
@@ -156,7 +162,6 @@ struct octgb_ctx {
     // plans and row state
     std::vector<Plan*> plans;
     DevBuf plan_table;           // device array of StitchDev, one per plan
-    int xs_max = 1, rs_max = 1;  // largest stitch patch over all plans
     DevBuf run_mm;               // running [min, max] (ordered uint) of finite dB
     std::vector<cudaGraphExec_t> graphs;
     std::vector<int64_t> graph_kernels;
@@ -395,6 +400,134 @@ void read_minmax(octgb_ctx* c, const unsigned int* mm_dev, double* out2) {
     }
 }
 
+// Shared memory of a stitch block that leaves six blocks an SM, and the floats
+// of a slot's row and column parameters in it.
+constexpr size_t kStitchSmem = 36 * 1024;
+constexpr int kStitchRowFloats(int rows) { return 6 * rows + 4 * kBlk; }
+
+// Fills `t` with the slots of the plans over column blocks [cb0, cb0 + nxb)
+// and uploads them.
+void build_slots(octgb_ctx* c, SlotTable& t, const std::vector<const Plan*>& plans, int n_out_z, int cb0, int nxb,
+                 int rows) {
+    const int nzb = (n_out_z + rows - 1) / rows, n_tiles = static_cast<int>(plans.size());
+    std::vector<StitchSlot> slots(static_cast<size_t>(nxb) * nzb * n_tiles);
+    std::vector<int> counts(static_cast<size_t>(nxb) * nzb, 0);
+    for (int bz = 0; bz < nzb; ++bz) {
+        for (int bx = 0; bx < nxb; ++bx) {
+            const int blk = bz * nxb + bx;
+            int n = 0, n0 = 0, off = 0;                      // n0: the round's first slot
+            for (int k = 0; k < n_tiles; ++k) {
+                const Plan& p = *plans[k];
+                const int cbi = cb0 + bx - p.cblk_first;
+                if (cbi < 0 || cbi >= p.n_cblk || p.cblk_h[cbi].x < 0) continue;
+                int lo = 1 << 30, hi = -1;
+                for (int z = bz * (rows / kBlk); z < (bz + 1) * (rows / kBlk); ++z) {
+                    if (z >= static_cast<int>(p.zblk_h.size()) || p.zblk_h[z].x < 0) continue;
+                    lo = lo < p.zblk_h[z].x ? lo : p.zblk_h[z].x;
+                    hi = hi > p.zblk_h[z].y ? hi : p.zblk_h[z].y;
+                }
+                if (hi < 0) continue;
+                const bool single = p.cblk1_h[cbi].x >= 0;
+                const int2 xs = single ? p.cblk1_h[cbi] : p.cblk_h[cbi];
+                StitchSlot s{};
+                s.t = k;
+                s.x_lo = xs.x;
+                s.xs = xs.y - xs.x + 1;
+                s.r_lo = lo;
+                s.rs = hi - lo + 1;
+                s.kind = (p.opc ? kSlotOpc : 0) | (single ? kSlotSingle : 0);
+                // one zero row after each A-scan's rows and (two A-scans a column) one
+                // zero A-scan after the last, so the kernel's reads need no bounds
+                // tests; an odd stride puts neighbouring A-scans in different banks
+                s.rst = (s.rs + 1) | 1;
+                const int need = (single ? s.xs : s.xs + 1) * s.rst * (p.opc ? 2 : 1);
+                if (n > n0 && (off + need + kStitchRowFloats(rows) * (n - n0 + 1)) * sizeof(float) > kStitchSmem) {
+                    slots[static_cast<size_t>(blk) * n_tiles + n - 1].last = 1;
+                    n0 = n;
+                    off = 0;
+                }
+                s.off = off;
+                off += need;
+                slots[static_cast<size_t>(blk) * n_tiles + n++] = s;
+                t.ns_round = std::max(t.ns_round, n - n0);
+                t.smem = std::max(t.smem, static_cast<size_t>(off) * sizeof(float));
+            }
+            if (n > 0) slots[static_cast<size_t>(blk) * n_tiles + n - 1].last = 1;
+            counts[blk] = n;
+        }
+    }
+    // the same slots for tensor copies: patches of one shape, rows from a
+    // multiple of 4 (a copy's 16-byte rule) at a pitch of 4 x an odd number
+    // (distinct banks); without them where the optical-path correction gathers,
+    // or one patch does not fit
+    std::vector<StitchTmaSlot> tslots;
+    bool tma = true;
+    for (const Plan* p : plans) tma = tma && !p->opc;
+    if (tma) {
+        int pitch = 4, lines = 1, most = 1;
+        tslots.resize(slots.size());
+        for (size_t blk = 0; blk < counts.size(); ++blk) {
+            most = std::max(most, counts[blk]);
+            for (int k = 0; k < counts[blk]; ++k) {
+                const StitchSlot& s = slots[blk * n_tiles + k];
+                const Plan& p = *plans[s.t];
+                StitchTmaSlot& q = tslots[blk * n_tiles + k];
+                const int zb = static_cast<int>(blk) / nxb * rows, cb = (cb0 + static_cast<int>(blk) % nxb) * kBlk;
+                q.t = s.t;
+                q.row0 = (p.r0 + s.r_lo) & ~3;
+                q.r_lo = q.row0 - p.r0;
+                q.x_lo = s.x_lo;
+                q.single = (s.kind & kSlotSingle) ? 1 : 0;
+                q.zrow = p.zrow.as<float4>() + zb;
+                q.zf = p.zf.as<float2>() + zb;
+                q.xcol = p.xcol.as<float4>() + kBlk + cb - p.c0;
+                pitch = std::max(pitch, s.r_lo + s.rs + 1 - q.r_lo);     // and the row after the last
+                lines = std::max(lines, s.xs);
+            }
+        }
+        pitch = (pitch + 3) / 4;
+        pitch = 4 * (pitch | 1);
+        t.pitch = pitch;
+        t.box_lines = lines;
+        t.patch_bytes = (static_cast<uint32_t>(pitch) * lines * 4 + 127) / 128 * 128;
+        t.slot_bytes = (t.patch_bytes + static_cast<uint32_t>(rows * 24 + kBlk * 16) + 127) / 128 * 128;
+        t.tma_round = std::max(1, std::min<int>(most, static_cast<int>(kStitchSmem / t.slot_bytes)));
+        tma = pitch <= 256 && lines <= 256 && t.slot_bytes <= 96 * 1024;
+    }
+    t.tma = tma;
+    if (tma) {
+        ck(t.tslots.ensure(tslots.size() * sizeof(StitchTmaSlot) + 16), "cudaMalloc(slots)");
+        ck(cudaMemcpyAsync(t.tslots.p, tslots.data(), tslots.size() * sizeof(StitchTmaSlot), cudaMemcpyHostToDevice,
+                           c->stream),
+           "H2D slots");
+    }
+    ck(t.slots.ensure(slots.size() * sizeof(StitchSlot) + 16), "cudaMalloc(slots)");
+    ck(t.counts.ensure(counts.size() * sizeof(int) + 16), "cudaMalloc(slot counts)");
+    ck(cudaMemcpyAsync(t.slots.p, slots.data(), slots.size() * sizeof(StitchSlot), cudaMemcpyHostToDevice, c->stream),
+       "H2D slots");
+    ck(cudaMemcpyAsync(t.counts.p, counts.data(), counts.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream),
+       "H2D slot counts");
+    ck(cudaStreamSynchronize(c->stream), "sync slot table");
+}
+
+// The table's part of a stitch launch over n_lines lines of magnitudes.
+void stitch_table_args(octgb_ctx* c, StitchArgs& a, const SlotTable& t, int64_t n_lines) {
+    a.slots = t.slots.as<StitchSlot>();
+    a.slot_count = t.counts.as<int>();
+    a.ns_round = t.ns_round;
+    a.status = c->status_dev;
+    if (t.tma && n_lines < (int64_t(1) << 31)) {
+        a.tslots = t.tslots.as<StitchTmaSlot>();
+        a.ns_round = t.tma_round;
+        a.pitch = t.pitch;
+        a.box_lines = t.box_lines;
+        a.patch_bytes = t.patch_bytes;
+        a.slot_bytes = t.slot_bytes;
+        a.n_lines = n_lines;
+        a.tile_lines = static_cast<int>(a.mag_tile_stride / kHalf);
+    }
+}
+
 const SlotTable& slot_table(octgb_ctx* c, int n_tiles, const int* plan_ids, int n_out_z, int n_out_x, int rows) {
     std::vector<int> key(plan_ids, plan_ids + n_tiles);
     key.push_back(n_out_z);
@@ -403,61 +536,13 @@ const SlotTable& slot_table(octgb_ctx* c, int n_tiles, const int* plan_ids, int 
     for (SlotTable* t : c->slot_tables)
         if (t->key == key) return *t;
     require(!c->capturing, "first use of a tile list during graph capture: run the sequence once before capturing");
-    const int nxb = (n_out_x + kBlk - 1) / kBlk, nzb = (n_out_z + rows - 1) / rows;
-    std::vector<StitchSlot> slots(static_cast<size_t>(nxb) * nzb * n_tiles);
-    std::vector<int> counts(static_cast<size_t>(nxb) * nzb, 0);
-    size_t smem = 0;
-    int ns_max = 1;
-    for (int bz = 0; bz < nzb; ++bz) {
-        for (int bx = 0; bx < nxb; ++bx) {
-            const int blk = bz * nxb + bx;
-            int n = 0, off = 0;
-            for (int t = 0; t < n_tiles; ++t) {
-                const Plan& p = *c->plans[plan_ids[t]];
-                const int cbi = bx - p.cblk_first;
-                if (cbi < 0 || cbi >= p.n_cblk || p.cblk_h[cbi].x < 0) continue;
-                int lo = 1 << 30, hi = -1;
-                for (int k = bz * (rows / kBlk); k < (bz + 1) * (rows / kBlk); ++k) {
-                    if (k >= static_cast<int>(p.zblk_h.size()) || p.zblk_h[k].x < 0) continue;
-                    lo = lo < p.zblk_h[k].x ? lo : p.zblk_h[k].x;
-                    hi = hi > p.zblk_h[k].y ? hi : p.zblk_h[k].y;
-                }
-                if (hi < 0) continue;
-                StitchSlot s{};
-                s.t = t;
-                s.x_lo = p.cblk_h[cbi].x;
-                s.xs = p.cblk_h[cbi].y - p.cblk_h[cbi].x + 1;
-                s.r_lo = lo;
-                s.rs = hi - lo + 1;
-                s.off = off;
-                s.opc = p.opc ? 1 : 0;
-                // one zero row after each A-scan's rows and one zero A-scan after the
-                // last, so the kernel's 2 x 2 reads need no bounds tests; an odd
-                // stride puts neighbouring A-scans in different banks
-                s.rst = (s.rs + 1) | 1;
-                off += (s.xs + 1) * s.rst * (p.opc ? 2 : 1);
-                slots[static_cast<size_t>(blk) * n_tiles + n++] = s;
-            }
-            counts[blk] = n;
-            ns_max = ns_max > n ? ns_max : n;
-            smem = smem > static_cast<size_t>(off) * sizeof(float) ? smem : static_cast<size_t>(off) * sizeof(float);
-        }
-    }
-    require(smem <= 160 * 1024, "stitch patches of one output block exceed shared memory");
+    std::vector<const Plan*> plans(n_tiles);
+    for (int t = 0; t < n_tiles; ++t) plans[t] = c->plans[plan_ids[t]];
     SlotTable* t = new SlotTable();
     t->key = key;
-    t->smem = smem;
-    t->ns_max = ns_max;
     try {
-        ck(t->slots.ensure(slots.size() * sizeof(StitchSlot) + 16), "cudaMalloc(slots)");
-        ck(t->counts.ensure(counts.size() * sizeof(int) + 16), "cudaMalloc(slot counts)");
-        ck(cudaMemcpyAsync(t->slots.p, slots.data(), slots.size() * sizeof(StitchSlot), cudaMemcpyHostToDevice,
-                           c->stream),
-           "H2D slots");
-        ck(cudaMemcpyAsync(t->counts.p, counts.data(), counts.size() * sizeof(int), cudaMemcpyHostToDevice,
-                           c->stream),
-           "H2D slot counts");
-        ck(cudaStreamSynchronize(c->stream), "sync slot table");
+        build_slots(c, *t, plans, n_out_z, 0, (n_out_x + kBlk - 1) / kBlk, rows);
+        require(t->smem <= 160 * 1024, "stitch patches of one output block exceed shared memory");
     } catch (...) {
         t->release();
         delete t;
@@ -930,17 +1015,27 @@ int octgb_stitch_plan(octgb_ctx* c, int n_rows, int r0, int r1, int c0, int c1, 
             }
         }
         const int cbf = c0 / kBlk, cbl = (c0 + C - 1) / kBlk;
-        std::vector<int2> cbt(cbl - cbf + 1, make_int2(-1, -1));
+        // the one A-scan of a column that takes one (its other weight is zero)
+        auto single = [&](int cc) {
+            return xr[cc] < 0 || (wx0[cc] != 0.f) == (wx1[cc] != 0.f) ? -1 : wx0[cc] != 0.f ? xr[cc] : xr[cc] + 1;
+        };
+        std::vector<int2> cbt(cbl - cbf + 1, make_int2(-1, -1)), cb1(cbl - cbf + 1, make_int2(-1, -1));
         for (int b = cbf; b <= cbl; ++b) {
-            int lo = 1 << 30, hi = -1;
+            int lo = 1 << 30, hi = -1, lo1 = 1 << 30, hi1 = -1;
+            bool all_single = true;
             for (int cabs = b * kBlk; cabs < (b + 1) * kBlk; ++cabs) {
                 const int cc = cabs - c0;
                 if (cc < 0 || cc >= C || xr[cc] < 0) continue;
                 lo = lo < xr[cc] ? lo : xr[cc];
                 hi = hi > xr[cc] + 1 ? hi : xr[cc] + 1;
+                const int x1 = single(cc);
+                all_single = all_single && x1 >= 0;
+                lo1 = std::min(lo1, x1);
+                hi1 = std::max(hi1, x1);
             }
             if (hi >= 0) {
                 cbt[b - cbf] = make_int2(lo, hi);
+                if (all_single) cb1[b - cbf] = make_int2(lo1, hi1);
                 xs_max = xs_max > hi - lo + 1 ? xs_max : hi - lo + 1;
             }
         }
@@ -963,10 +1058,9 @@ int octgb_stitch_plan(octgb_ctx* c, int n_rows, int r0, int r1, int c0, int c1, 
         }
         p->zblk_h = zb;
         p->cblk_h = cbt;
+        p->cblk1_h = cb1;
         p->cblk_first = cbf;
         p->n_cblk = cbl - cbf + 1;
-        p->xs_max = xs_max;
-        p->rs_max = rs_max;
         p->n_rows = n_rows;
         p->r0 = r0;
         p->R = R;
@@ -987,13 +1081,16 @@ int octgb_stitch_plan(octgb_ctx* c, int n_rows, int r0, int r1, int c0, int c1, 
             up(p->wx0, wx0.data(), wx0.size() * sizeof(float));
             up(p->wx1, wx1.data(), wx1.size() * sizeof(float));
             up(p->fz, fzf.data(), fzf.size() * sizeof(float));
-            up(p->zblk, zb.data(), zb.size() * sizeof(int2));
-            up(p->cblk, cbt.data(), cbt.size() * sizeof(int2));
             // per output row, for the batched form's depth resampling: {zr, w0,
             // w1, d} and the focus weights {F[zr], F[zr + 1] (0 past the window)},
             // d = fma(F1, w1, F0 w0) as the kernel forms it
-            std::vector<float4> zrow(n_out_z);
-            std::vector<float2> zfv(n_out_z);
+            // (padded with rows without a contribution to whole blocks of 128)
+            float none;
+            const int minus1 = -1;
+            memcpy(&none, &minus1, sizeof(float));
+            const int n_pad = (n_out_z + 127) / 128 * 128;
+            std::vector<float4> zrow(n_pad, make_float4(none, 0.f, 0.f, 0.f));
+            std::vector<float2> zfv(n_pad, make_float2(0.f, 0.f));
             for (int zo = 0; zo < n_out_z; ++zo) {
                 const int z = zr[zo];
                 const float f0 = z >= 0 ? fzf[z] : 0.f;
@@ -1006,12 +1103,15 @@ int octgb_stitch_plan(octgb_ctx* c, int n_rows, int r0, int r1, int c0, int c1, 
             }
             up(p->zrow, zrow.data(), zrow.size() * sizeof(float4));
             up(p->zf, zfv.data(), zfv.size() * sizeof(float2));
-            // per output column: {xr (int bits), wx0, wx1, 0}
-            std::vector<float4> xcol(C);
+            // per output column: {xr (int bits), wx0, wx1, the single A-scan (int bits)},
+            // a block of columns without a contribution on either side
+            std::vector<float4> xcol(C + 2 * kBlk, make_float4(none, 0.f, 0.f, none));
             for (int cc = 0; cc < C; ++cc) {
-                float xrf;
+                const int x1 = single(cc);
+                float xrf, x1f;
                 memcpy(&xrf, &xr[cc], sizeof(float));
-                xcol[cc] = make_float4(xrf, wx0[cc], wx1[cc], 0.f);
+                memcpy(&x1f, &x1, sizeof(float));
+                xcol[kBlk + cc] = make_float4(xrf, wx0[cc], wx1[cc], x1f);
             }
             up(p->xcol, xcol.data(), xcol.size() * sizeof(float4));
             if (shift != nullptr) {
@@ -1030,6 +1130,14 @@ int octgb_stitch_plan(octgb_ctx* c, int n_rows, int r0, int r1, int c0, int c1, 
                 p->opc = true;
             }
             ck(cudaStreamSynchronize(c->stream), "sync plan");
+            // the row interface's blocks: 64 rows where four blocks an SM hold their patches
+            build_slots(c, p->row_table, {p}, n_out_z, cbf, p->n_cblk, 64);
+            if (p->row_table.smem > 48 * 1024) {
+                p->row_rows = 32;
+                p->row_table.ns_round = 1;
+                p->row_table.smem = 0;
+                build_slots(c, p->row_table, {p}, n_out_z, cbf, p->n_cblk, 32);
+            }
         } catch (...) {
             p->release();
             delete p;
@@ -1045,8 +1153,6 @@ int octgb_stitch_plan(octgb_ctx* c, int n_rows, int r0, int r1, int c0, int c1, 
                            c->stream),
            "H2D plan table");
         ck(cudaStreamSynchronize(c->stream), "sync plan table");
-        c->xs_max = c->xs_max > xs_max ? c->xs_max : xs_max;
-        c->rs_max = c->rs_max > rs_max ? c->rs_max : rs_max;
     });
 }
 
@@ -1070,8 +1176,9 @@ int octgb_row_begin(octgb_ctx* c, int n_frames, int n_out_z, int n_out_x) {
 namespace {
 // TileStitcher.contribute of B frames of magnitudes (device, (B, n_tile_x,
 // N/2)) into the row accumulators (pipeline.py:283-285)
-void stitch_row(octgb_ctx* c, const Plan& p, const float* mag, const std::vector<int>& fy, bool contiguous, int B,
+void stitch_row(octgb_ctx* c, int plan_id, const float* mag, const std::vector<int>& fy, bool contiguous, int B,
                 int frame_offset) {
+    const Plan& p = *c->plans[plan_id];
     const int* fdev = nullptr;
     if (!contiguous) {
         // pageable copy: returns once staged, so `fy` may go out of scope
@@ -1080,8 +1187,21 @@ void stitch_row(octgb_ctx* c, const Plan& p, const float* mag, const std::vector
            "H2D frames");
         fdev = c->frames.as<int>();
     }
-    ck(launch_stitch(p.dev(), mag, fdev, fy[0], B, c->num.as<float>(), c->den.as<float>(), frame_offset, c->row_nx,
-                     p.xs_max, p.rs_max, c->stream),
+    StitchArgs a{};
+    a.tiles.n = 1;
+    a.tiles.id[0] = plan_id;
+    a.mag = mag;
+    stitch_table_args(c, a, p.row_table, static_cast<int64_t>(B) * p.n_tile_x);
+    a.n_tile_x = p.n_tile_x;
+    a.f0 = fy[0];
+    a.frame_y = fdev;
+    a.n_out_z = c->row_nz;
+    a.n_out_x = c->row_nx;
+    a.cblk0 = p.cblk_first;
+    a.num = c->num.as<float>();
+    a.den = c->den.as<float>();
+    a.frame_offset = frame_offset;
+    ck(launch_stitch(c->plan_table.as<StitchDev>(), a, p.row_table.smem, p.n_cblk, B, p.row_rows, c->stream),
        "stitch kernel");
     c->launches++;
 }
@@ -1151,7 +1271,7 @@ int octgb_row_add_batch(octgb_ctx* c, int plan_id, const void* raw, int dtype, i
         const size_t mb = static_cast<size_t>(B) * p.n_tile_x * kHalf * sizeof(float);
         ck(c->magbuf.ensure(mb), "cudaMalloc(mag)");
         run_spectral(c, raw, dtype, loc, B, interf, apod, kModeMag, c->magbuf.as<float>(), 0, 0, nullptr);
-        stitch_row(c, p, c->magbuf.as<float>(), fy, contiguous, B, frame_offset);
+        stitch_row(c, plan_id, c->magbuf.as<float>(), fy, contiguous, B, frame_offset);
     });
 }
 
@@ -1269,9 +1389,21 @@ int octgb_frames_process(octgb_ctx* c, int n_tiles, const int* plan_ids, const v
         }
         ck(c->run_mm.ensure(2 * sizeof(unsigned int)), "cudaMalloc(run mm)");
         const SlotTable& stab = slot_table(c, n_tiles, plan_ids, n_out_z, n_out_x, c->stitch_rows);
-        ck(launch_stitch_frames(c->plan_table.as<StitchDev>(), tl, stab.slots.as<StitchSlot>(), stab.counts.as<int>(),
-                                stab.ns_max, stab.smem, c->magbuf.as<float>(), tile_stride, B, nx, f0, n_out_z, n_out_x, thr, dst,
-                                pmm, c->run_mm.as<unsigned int>(), c->stitch_rows, c->stream),
+        StitchArgs a{};
+        a.tiles = tl;
+        a.mag = c->magbuf.as<float>();
+        a.mag_tile_stride = tile_stride;
+        stitch_table_args(c, a, stab, static_cast<int64_t>(n_tiles) * B * nx);
+        a.n_tile_x = nx;
+        a.f0 = f0;
+        a.n_out_z = n_out_z;
+        a.n_out_x = n_out_x;
+        a.thr = thr;
+        a.db = dst;
+        a.plane_mm = pmm;
+        a.run_mm = c->run_mm.as<unsigned int>();
+        ck(launch_stitch(c->plan_table.as<StitchDev>(), a, stab.smem, (n_out_x + kBlk - 1) / kBlk, B, c->stitch_rows,
+                         c->stream),
            "stitch frames kernel");
         c->launches++;
         if (db_loc != OCTGB_DEVICE) copy_out(c, db, OCTGB_HOST, dst, db_bytes);
@@ -1843,7 +1975,7 @@ int octgb_row_add_batch_ex(octgb_ctx* c, int plan_id, const void* raw, int dtype
                "repeat kernel");
             c->launches++;
         }
-        stitch_row(c, p, c->magbuf.as<float>(), fy, contiguous, n_frames, frame_offset);
+        stitch_row(c, plan_id, c->magbuf.as<float>(), fy, contiguous, n_frames, frame_offset);
     });
 }
 

@@ -197,9 +197,12 @@ __device__ __forceinline__ uint32_t starved_bytes(bool first) { return first && 
 
 // Bounded wait on an mbarrier phase: gives up after g_wait_limit_ns of wall
 // time and reports it through the status word (the copies and MMAs waited
-// for normally complete within microseconds).
+// for normally complete within microseconds).  The first try (it suspends the
+// thread for up to 100 us) comes before the timer and the limit are read: those
+// reads cost more than most waits.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, int* status) {
     if (mbar_test(bar, parity)) return true;
+    if (mbar_try(bar, parity)) return true;
     const uint64_t t0 = globaltimer_ns();
     const uint64_t limit = g_wait_limit_ns;
     for (uint32_t it = 0; it < (1u << 30); ++it) {

@@ -134,17 +134,13 @@ struct StitchDev {
     const int* shift;         // [n_y, n_tile_x] optical-path row shift, or null
     const int* lo;            // [n_y, n_tile_x] smallest valid r (incl.), or null
     const int* hi;            // [n_y, n_tile_x] largest valid r (incl.), or null
-    // per 32-row output block zb: input rows [x, y] (relative to r0) it reads; x = -1: none
-    const int2* zblk;
-    // per absolute 32-column output block cblk_first + i: A-scans [x, y] it reads; x = -1: none
-    const int2* cblk;
     // per output row: {zr (int bits), wz0, wz1, d = fma(F1, wz1, F0 wz0)} and
     // {F0 = fz[zr], F1 = fz[zr + 1] or 0 past the window} (batched form)
     const float4* zrow;
     const float2* zf;
-    // per output column c0 + cc: {xr (int bits), wx0, wx1, 0} (frame-batch form)
+    // per output column c0 + cc: {xr (int bits), wx0, wx1, the one A-scan with a
+    // weight (int bits; -1: two or none)}
     const float4* xcol;
-    int cblk_first, n_cblk;
     int r0, R, c0, C, n_out_z, n_tile_x, n_rows;
 };
 
@@ -153,24 +149,55 @@ struct TileList {
     int id[kMaxSeg];
 };
 
-// row API: one tile, accumulate into num/den (n_frames, n_out_z, n_out_x)
-cudaError_t launch_stitch(const StitchDev& p, const float* mag, const int* frame_y, int f0, int B, float* num,
-                          float* den, int frame_offset, int n_out_x, int xs_max, int rs_max, cudaStream_t st);
-// frames API: all tiles of a frame batch, num/den kept on chip, dB + clim written
-constexpr int kStitchRows = 64;   // default output rows per frame-batch stitch block (x 32 columns; 32, 64 or 128)
+constexpr int kStitchRows = 64;   // default output rows per stitch block (x 32 columns; 32, 64 or 128)
+constexpr int kSlotOpc = 1;       // optical-path correction on (patch of F follows the magnitudes')
+constexpr int kSlotSingle = 2;    // every column of the block takes one A-scan of the tile
 struct StitchSlot {               // one tile touching one output block
     int t;                        // index into the TileList
     int x_lo, xs;                 // A-scans read
     int r_lo, rs;                 // rows (relative to r0) read
     int off;                      // float offset of the patch in shared memory
-    int opc;                      // optical-path correction on (patch of F follows)
+    int kind;                     // kSlotOpc | kSlotSingle
     int rst;                      // patch stride per A-scan: rs + a zero row, made odd (distinct banks)
+    int last;                     // last slot of a round (the patches of a round are staged together)
 };
-cudaError_t launch_stitch_frames(const StitchDev* plans_dev, const TileList& tiles, const StitchSlot* slots,
-                                 const int* slot_count, int ns_max, size_t patch_smem_bytes, const float* mag,
-                                 int64_t mag_tile_stride, int B, int n_tile_x, int f0, int n_out_z, int n_out_x,
-                                 float thr, float* db, unsigned int* plane_mm, unsigned int* run_mm, int rows,
-                                 cudaStream_t st);
+struct StitchTmaSlot {            // one tile touching one output block, staged by tensor copies
+    const float4* zrow;           // the block's row parameters in the plan's tables
+    const float2* zf;
+    const float4* xcol;           // the block's column parameters
+    int t;                        // index into the TileList
+    int row0;                     // first magnitude row copied (a multiple of 4)
+    int x_lo, r_lo;               // A-scan and row (relative to r0; row0 is r0 + r_lo) at the patch's origin
+    int single;                   // every column of the block takes one A-scan of the tile
+    int pad_;
+};
+struct StitchArgs {
+    TileList tiles;
+    const StitchSlot* slots;      // [blocks][tiles.n], the first slot_count[block] used
+    const int* slot_count;
+    int ns_round;                 // most slots of a round
+    const StitchTmaSlot* tslots;  // null: slots; else the same blocks' slots for tensor copies,
+    uint32_t patch_bytes, slot_bytes;   // each with slot_bytes of shared memory, the patch (padded) first:
+    int pitch, box_lines;         // box_lines lines of `pitch` floats
+    int tile_lines;               // lines of `mag` per tile,
+    int64_t n_lines;              // and in all
+    int* status;                  // device status word (bounded waits)
+    const float* mag;             // tile t, frame f, A-scan x at t mag_tile_stride + (f n_tile_x + x) kHalf
+    int64_t mag_tile_stride;
+    int n_tile_x, f0, n_out_z, n_out_x;
+    int cblk0;                    // first 32-column block
+    // frame batch: all tiles, dB and clim
+    float thr;
+    float* db;                    // (B, n_out_z, n_out_x)
+    unsigned int* plane_mm;       // [B][2] or null
+    unsigned int* run_mm;         // [2] or null
+    // row interface: one tile added to num / den (frames, n_out_z, n_out_x); null otherwise
+    float *num, *den;
+    const int* frame_y;           // frame of the optical-path correction, null: f0 + f
+    int frame_offset;
+};
+cudaError_t launch_stitch(const StitchDev* plans_dev, const StitchArgs& a, size_t patch_smem_bytes, int n_cblk, int B,
+                          int rows, cudaStream_t st);
 // batched form: dB rows of the A-scans [l0, l1) of tiles of uneven size from
 // their magnitudes (A-scan l at (l - l0) kHalf), with the running range
 cudaError_t launch_resample(const QueueTile* qt, int n_qt, unsigned int l0, unsigned int l1, const float* mag,

@@ -10,166 +10,31 @@
 // Wz / WxT are linear-interpolation operators with at most two adjacent
 // non-zeros per output row / column, stored compactly.
 //
-// The work unit is a 32 x 32 block of output voxels (rows zo, columns c) of
-// one frame.  The block reads a small patch of the tile's magnitudes (the
+// The work unit (k_stitch) is a block of 32 to 128 rows zo x 32 columns c of
+// one frame.  The block reads a small patch of each tile's magnitudes (the
 // A-scans feeding its columns x the depth rows feeding its rows) into shared
-// memory with reads along depth (the magnitude layout), applies the depth
-// interpolation per A-scan, then the lateral interpolation, and writes along
-// x (the output layout): a transpose through shared memory, so both global
-// sides are coalesced.
-//
-// Two kernels use it:
-//   k_stitch_tile    one tile, num/den += contribution (per-tile row API);
-//   k_stitch_frames  every tile of a frame batch in tile order, num/den kept in
-//                    registers, then finalise (threshold -> NaN, 20 log10) and
-//                    the plane / running clim: num/den never reach memory.
-// In both the per-voxel floating-point operations and their order are those of
-// the reference loop (tile contributions added one after the other).
+// memory with reads along depth (the magnitude layout) and writes along x (the
+// output layout): a transpose through shared memory, so both global sides are
+// coalesced.  For a frame batch every tile is summed in tile order with
+// num/den in registers, then finalised (threshold -> NaN, 20 log10) with the
+// plane / running clim: num/den never reach memory.  For the row interface one
+// tile's contribution is added to num/den in memory.  In both the per-voxel
+// floating-point operations and their order are those of the reference loop
+// (tile contributions added one after the other); an A-scan whose lateral
+// weight is zero is not read.
+#include <cuda.h>
+#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
 
+#include "octgb_device.cuh"
 #include "octgb_internal.h"
 
 namespace octgb {
 namespace {
 
 constexpr int kStThreads = 256;          // 32 columns x 8 row groups
-constexpr int kRowsPerThread = kBlk / 8; // 4 output rows per thread
-
-struct PatchSmem {
-    float* pa;   // [xs_max][rs_max] a * F
-    float* pf;   // [xs_max][rs_max] F
-    float* un;   // [xs_max][kBlk]   depth-interpolated a F
-    float* ud;   // [xs_max][kBlk]   depth-interpolated F
-};
-
-__device__ __forceinline__ PatchSmem carve(float* sm, int xs_max, int rs_max) {
-    PatchSmem s;
-    s.pa = sm;
-    s.pf = s.pa + xs_max * rs_max;
-    s.un = s.pf + xs_max * rs_max;
-    s.ud = s.un + xs_max * kBlk;
-    return s;
-}
-
-// Contribution of one tile to the block (zb, cb) of frame f; adds it to
-// an/ad (4 voxels per thread: rows zb + ty + 8q, column cb + tx).  Uniform
-// control flow across the CTA; returns false when the tile misses the block.
-__device__ bool block_contrib(const StitchDev& p, const float* __restrict__ mag_f, int fy, int zb, int cb,
-                              const PatchSmem& s, int rs_max, float (&an)[kRowsPerThread],
-                              float (&ad)[kRowsPerThread]) {
-    const int cbi = cb / kBlk - p.cblk_first;
-    if (cbi < 0 || cbi >= p.n_cblk) return false;
-    const int2 xb = p.cblk[cbi];
-    const int2 zr_b = p.zblk[zb / kBlk];
-    if (xb.x < 0 || zr_b.x < 0) return false;
-    const int x_lo = xb.x, xs = xb.y - xb.x + 1;
-    const int r_lo = zr_b.x, rs = zr_b.y - zr_b.x + 1;
-    const int tid = threadIdx.x;
-
-    // 1. gather the patch: rows fastest (contiguous in the magnitude layout);
-    //    magnitudes by asynchronous 4-byte copies (all in flight at once), the
-    //    focus weight F beside them (a = magnitude * F is formed on read)
-    for (int i = tid; i < xs * rs; i += kStThreads) {
-        const int xx = i / rs, rr = i - xx * rs;
-        const int x = x_lo + xx;
-        const int r = r_lo + rr;
-        const int ra = p.r0 + r;
-        int src = ra;
-        float F = p.fz[r];
-        if (p.shift != nullptr) {
-            const int64_t o = static_cast<int64_t>(fy) * p.n_tile_x + x;
-            if (ra < p.lo[o] || ra > p.hi[o]) F = 0.f;
-            src = ra + p.shift[o];
-            src = src < 0 ? 0 : (src > p.n_rows - 1 ? p.n_rows - 1 : src);
-        }
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
-                         static_cast<uint32_t>(__cvta_generic_to_shared(s.pa + xx * rs_max + rr))),
-                     "l"(mag_f + static_cast<int64_t>(x) * kHalf + src)
-                     : "memory");
-        s.pf[xx * rs_max + rr] = F;
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
-
-    // 2. depth interpolation (Wz) for every A-scan of the patch and row of the block
-    for (int i = tid; i < xs * kBlk; i += kStThreads) {
-        const int xx = i / kBlk, z = i - xx * kBlk;
-        const int zo = zb + z;
-        float un = 0.f, ud = 0.f;
-        if (zo < p.n_out_z) {
-            const int zr = p.zr[zo];
-            if (zr >= 0) {
-                const int rr = zr - r_lo;
-                const float w0 = p.wz0[zo], w1 = p.wz1[zo];
-                const float f0 = s.pf[xx * rs_max + rr], a0 = s.pa[xx * rs_max + rr] * f0;
-                float a1 = 0.f, f1 = 0.f;
-                if (rr + 1 < rs) {
-                    f1 = s.pf[xx * rs_max + rr + 1];
-                    a1 = s.pa[xx * rs_max + rr + 1] * f1;
-                }
-                un = fmaf(a1, w1, a0 * w0);
-                ud = fmaf(f1, w1, f0 * w0);
-            }
-        }
-        s.un[xx * kBlk + z] = un;
-        s.ud[xx * kBlk + z] = ud;
-    }
-    __syncthreads();
-
-    // 3. lateral interpolation (WxT) and accumulation
-    const int tx = tid & (kBlk - 1), ty = tid / kBlk;
-    const int cc = cb + tx - p.c0;
-    if (cc >= 0 && cc < p.C) {
-        const int xr = p.xr[cc];
-        if (xr >= 0) {
-            const int xx = xr - x_lo;
-            const float w0 = p.wx0[cc], w1 = p.wx1[cc];
-#pragma unroll
-            for (int q = 0; q < kRowsPerThread; ++q) {
-                const int z = ty + 8 * q;
-                const int zo = zb + z;
-                if (zo < p.n_out_z && p.zr[zo] >= 0) {
-                    const float u0 = s.un[xx * kBlk + z], d0 = s.ud[xx * kBlk + z];
-                    const float u1 = xx + 1 < xs ? s.un[(xx + 1) * kBlk + z] : 0.f;
-                    const float d1 = xx + 1 < xs ? s.ud[(xx + 1) * kBlk + z] : 0.f;
-                    an[q] += fmaf(u1, w1, u0 * w0);
-                    ad[q] += fmaf(d1, w1, d0 * w0);
-                }
-            }
-        }
-    }
-    __syncthreads();
-    return true;
-}
-
-__global__ void __launch_bounds__(kStThreads) k_stitch_tile(const StitchDev p, const float* __restrict__ mag,
-                                                            const int* __restrict__ frame_y, int f0,
-                                                            float* __restrict__ num, float* __restrict__ den,
-                                                            int frame_offset, int n_out_x, int xs_max, int rs_max) {
-    extern __shared__ __align__(16) float sm[];
-    const PatchSmem s = carve(sm, xs_max, rs_max);
-    const int f = blockIdx.z;
-    const int zb = blockIdx.y * kBlk;
-    const int cb = (p.cblk_first + blockIdx.x) * kBlk;
-    const int fy = frame_y ? frame_y[f] : f0 + f;
-    float an[kRowsPerThread] = {0.f, 0.f, 0.f, 0.f}, ad[kRowsPerThread] = {0.f, 0.f, 0.f, 0.f};
-    const float* mag_f = mag + static_cast<int64_t>(f) * p.n_tile_x * kHalf;
-    if (!block_contrib(p, mag_f, fy, zb, cb, s, rs_max, an, ad)) return;
-    const int tx = threadIdx.x & (kBlk - 1), ty = threadIdx.x / kBlk;
-    const int c = cb + tx;
-    const int cc = c - p.c0;
-    if (cc < 0 || cc >= p.C || p.xr[cc] < 0) return;
-#pragma unroll
-    for (int q = 0; q < kRowsPerThread; ++q) {
-        const int zo = zb + ty + 8 * q;
-        if (zo >= p.n_out_z || p.zr[zo] < 0) continue;
-        const int64_t o = (static_cast<int64_t>(frame_offset + f) * p.n_out_z + zo) * n_out_x + c;
-        num[o] += an[q];
-        den[o] += ad[q];
-    }
-}
 
 __device__ __forceinline__ void warp_minmax(float& mn, float& mx) {
 #pragma unroll
@@ -179,20 +44,17 @@ __device__ __forceinline__ void warp_minmax(float& mn, float& mx) {
     }
 }
 
-// The fields of a tile's stitch plan that the frame-batch kernel reads,
-// copied to shared memory once per CTA (one load round for all slots).
-struct SlotPlan {
-    const float4* zrow;       // per output row {zr, wz0, wz1, d}
-    const float2* zf;         // per output row {F[zr], F[zr + 1]}
-    const float4* xcol;       // per output column {xr, wx0, wx1, 0}
-    const float* fz;
-    const int* shift;         // null without the optical-path correction
-    const int* lo;
-    const int* hi;
-    int r0, c0, C, n_out_z, n_tile_x, n_rows;
-};
-
-static_assert(sizeof(SlotPlan) % 16 == 0, "the row parameters after the slot plans need 16-byte alignment");
+// Folds [mn, mx] into an ordered-uint range in memory.  Most ranges add
+// nothing: the current one is read first (an older, wider value only costs an
+// atomic), since atomics of every warp on one address serialise in L2: 726 000 warps of a
+// frame batch took ~1 ms, whatever else they did.
+__device__ __forceinline__ void fold_range(unsigned int* mm, float mn, float mx) {
+    if (!(mn <= mx)) return;
+    const unsigned int lo = f2ord(mn), hi = f2ord(mx);
+    const uint2 cur = __ldcg(reinterpret_cast<const uint2*>(mm));
+    if (lo < cur.x) atomicMin(&mm[0], lo);
+    if (hi > cur.y) atomicMax(&mm[1], hi);
+}
 
 // asynchronous global -> shared copy of one 8- or 16-byte element (both addresses aligned to its size)
 template <int kBytes>
@@ -204,143 +66,143 @@ __device__ __forceinline__ void cp_async(void* dst, const void* src) {
                  : "memory");
 }
 
-// Frame-batch kernel: one CTA = one frame x kFZ output rows x 32 output
-// columns.  The tiles touching each block and their patch extents come from a
-// table built once per tile list on the host (StitchSlot); the CTA reads the
-// table and each tile's plan fields in one round of loads, then stages every
-// contributing patch and the tiles' per-row / per-column interpolation
-// parameters (precomputed per plan) in shared memory by asynchronous copies:
-// no load waits on another before the one barrier.  Then every voxel sums
-// the tiles in order.
-// kFZ output rows per CTA (the tile shape the autotuner picks: 32, 64 or 128)
-template <int kFZ>
-__global__ void __launch_bounds__(kStThreads) k_stitch_frames(const StitchDev* __restrict__ plans, const TileList tl,
-                                                              const StitchSlot* __restrict__ slots,
-                                                              const int* __restrict__ slot_count,
-                                                              const float* __restrict__ mag, int64_t mag_tile_stride,
-                                                              int n_tile_x, int f0, int n_out_z, int n_out_x,
-                                                              float thr, float* __restrict__ db,
-                                                              unsigned int* __restrict__ plane_mm,
-                                                              unsigned int* __restrict__ run_mm, int ns_max) {
+// One CTA = one frame x kFZ output rows x 32 output columns.  The tiles
+// touching each block and their patch extents come from a table built once per
+// tile list on the host (StitchSlot); the CTA reads the table and each tile's
+// plan fields in one round of loads, then stages every contributing patch and
+// the tiles' per-row / per-column interpolation parameters (precomputed per
+// plan) in shared memory by asynchronous copies: no load waits on another
+// before the one barrier.  Then every voxel sums the tiles in order.
+// kFZ output rows per CTA (the tile shape the autotuner picks: 32, 64 or 128).
+// Where every column of a block takes one A-scan of a tile (kSlotSingle: the
+// output grid and the tile's share their pixels, as a scan's do except in the
+// first columns of a tile and between tiles at a fraction of a pixel) the
+// second A-scan, its weight of zero and half of the reads fall away.
+// kRow: one tile, its contribution added to num / den (the row interface);
+// otherwise all tiles, finalised to dB with the plane and running range.
+// Issue-bound (1776 warp instructions a warp of 256 voxels, a third of them
+// staging): 183 M voxels of 6 tiles in ~1180 us; k_stitch_tma takes what it can.
+template <int kFZ, bool kRow>
+__global__ void __launch_bounds__(kStThreads) k_stitch(const StitchDev* __restrict__ plans, const StitchArgs a) {
     constexpr int kFRows = kFZ / 8;          // rows per thread
-    // dynamic shared memory: per-slot plan fields, row / column parameters, then the patches
+    // dynamic shared memory: row / column parameters of a round's slots, then the patches
     extern __shared__ __align__(16) float smem_all[];
     __shared__ StitchSlot slot[kMaxSeg];
-    SlotPlan* spl = reinterpret_cast<SlotPlan*>(smem_all);              // [ns_max]
-    float4* rowp = reinterpret_cast<float4*>(spl + ns_max);             // [ns_max][kFZ] {zr, w0, w1, F interpolated}
-    float2* rowf = reinterpret_cast<float2*>(rowp + ns_max * kFZ);      // [ns_max][kFZ] {F of the row's two taps}
-    float4* colp = reinterpret_cast<float4*>(rowf + ns_max * kFZ);      // [ns_max][kBlk] {xr, wx0, wx1, 0}
-    float* sm = reinterpret_cast<float*>(colp + ns_max * kBlk);
+    float4* rowp = reinterpret_cast<float4*>(smem_all);                 // [ns_round][kFZ] {zr, w0, w1, F interpolated}
+    float2* rowf = reinterpret_cast<float2*>(rowp + a.ns_round * kFZ);  // [ns_round][kFZ] {F of the row's two taps}
+    float4* colp = reinterpret_cast<float4*>(rowf + a.ns_round * kFZ);  // [ns_round][kBlk] {xr, wx0, wx1, single A-scan}
+    float* sm = reinterpret_cast<float*>(colp + a.ns_round * kBlk);
     const int f = blockIdx.z;
     const int zb = blockIdx.y * kFZ;
-    const int cb = blockIdx.x * kBlk;
-    const int tid = threadIdx.x;
+    const int cb = (a.cblk0 + blockIdx.x) * kBlk;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int blk = blockIdx.y * gridDim.x + blockIdx.x;
-    const int ns = slot_count[blk];
-    if (tid < ns) {
-        const StitchSlot s = slots[static_cast<int64_t>(blk) * tl.n + tid];
-        const StitchDev& p = plans[tl.id[s.t]];
-        SlotPlan q;
-        q.zrow = p.zrow;
-        q.zf = p.zf;
-        q.xcol = p.xcol;
-        q.fz = p.fz;
-        q.shift = p.shift;
-        q.lo = p.lo;
-        q.hi = p.hi;
-        q.r0 = p.r0;
-        q.c0 = p.c0;
-        q.C = p.C;
-        q.n_out_z = p.n_out_z;
-        q.n_tile_x = p.n_tile_x;
-        q.n_rows = p.n_rows;
-        slot[tid] = s;
-        spl[tid] = q;
-    }
+    const int ns = a.slot_count[blk];
+    if (kRow && ns == 0) return;
+    if (tid < ns) slot[tid] = a.slots[static_cast<int64_t>(blk) * a.tiles.n + tid];
     __syncthreads();
 
     // 1. stage each contributing tile's interpolation parameters and its
-    //    magnitude patch (a * F, and F when the optical-path correction makes
-    //    it depend on the A-scan); depth fastest in the patch, one zero row
-    //    after each A-scan's rows and one zero A-scan after the last (stride
-    //    s.rst), so every 2 x 2 read below is in the patch
-    for (int k = 0; k < ns; ++k) {
+    //    magnitude patch (F beside it when the optical-path correction makes it
+    //    depend on the A-scan); depth fastest in the patch, one zero row after
+    //    each A-scan's rows and (unless single) one zero A-scan after the last
+    //    (stride s.rst), so every read below is in the patch.  Slots k0 .. k1 - 1
+    //    of a round are spread over the warps (a warp deals with one slot, not
+    //    each with all of them); the patch is copied as is (asynchronous 4-byte
+    //    copies, 32 rows of an A-scan a warp); the focus weight multiplies it
+    //    when it is read, the same single product a * F.
+    auto stage = [&](int k, int kr, int part, int parts) {
         const StitchSlot s = slot[k];
-        const SlotPlan& p = spl[k];
-        if (tid < kFZ) {
-            // without the optical-path correction F depends on the row only:
-            // its two taps and the depth-interpolated F (the den term) per row.
-            // The slot's rows reach zr + 1 of every row, so the per-plan F[zr + 1]
-            // (0 past the window) is the one the patch holds.
-            const int zo = zb + tid;
-            if (zo < p.n_out_z) {
-                cp_async<16>(rowp + k * kFZ + tid, p.zrow + zo);
-                cp_async<8>(rowf + k * kFZ + tid, p.zf + zo);
-            } else {
-                rowp[k * kFZ + tid] = make_float4(__int_as_float(-1), 0.f, 0.f, 0.f);
-                rowf[k * kFZ + tid] = make_float2(0.f, 0.f);
-            }
-        } else if (tid < kFZ + kBlk) {
-            // the slot's A-scans reach xr + 1 of every column of the block
-            const int cc = cb + tid - kFZ - p.c0;
-            if (cc >= 0 && cc < p.C)
-                cp_async<16>(colp + k * kBlk + tid - kFZ, p.xcol + cc);
-            else
-                colp[k * kBlk + tid - kFZ] = make_float4(__int_as_float(-1), 0.f, 0.f, 0.f);
-        }
-        const float* mag_f = mag + s.t * mag_tile_stride + static_cast<int64_t>(f) * n_tile_x * kHalf;
+        const StitchDev& p = plans[a.tiles.id[s.t]];
+        const bool opc = (s.kind & kSlotOpc) != 0;
+        const int na = (s.kind & kSlotSingle) ? s.xs : s.xs + 1;
         float* pa = sm + s.off;
-        float* pf = pa + (s.xs + 1) * s.rst;
-        const int fy = f0 + f;
-        // zero rows (rst - rs of them after each A-scan's rows) and the zero
-        // A-scan after the last (plain stores, before the barrier)
-        {
-            const int zr = s.rst - s.rs;                     // 1 or 2
-            const int nz = s.xs * zr;
-            for (int i = tid; i < nz + s.rst; i += kStThreads) {
-                int o;
-                if (i < nz) {
-                    const int xx = zr == 1 ? i : i >> 1;
-                    o = xx * s.rst + s.rs + (i - xx * zr);
-                } else {
-                    o = s.xs * s.rst + (i - nz);
-                }
-                pa[o] = 0.f;
-                if (s.opc) pf[o] = 0.f;
-            }
-        }
-        // the patch is copied as is (asynchronous 4-byte copies, every slot's
-        // in flight at once); the focus weight multiplies it when it is read,
-        // the same single product a * F.  64 consecutive threads copy 64
-        // consecutive rows of one A-scan, four A-scans per pass
-        if (p.shift == nullptr) {
-            // source and destination advance by four A-scans a pass
-            for (int rr = tid & 63; rr < s.rs; rr += 64) {
-                const int xx0 = tid >> 6;
-                const float* src = mag_f + static_cast<int64_t>(s.x_lo + xx0) * kHalf + p.r0 + s.r_lo + rr;
-                uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(pa + xx0 * s.rst + rr));
-                const uint32_t dstep = static_cast<uint32_t>(kStThreads / 64 * s.rst) * 4u;
-                for (int xx = xx0; xx < s.xs; xx += kStThreads / 64) {
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-                    src += kStThreads / 64 * kHalf;
-                    dst += dstep;
-                }
+        float* pf = pa + na * s.rst;
+        const int r0 = p.r0 + s.r_lo;
+        const float* mag_f = a.mag + s.t * a.mag_tile_stride + static_cast<int64_t>(f) * a.n_tile_x * kHalf;
+        if (!opc) {
+            const float* src = mag_f + static_cast<int64_t>(s.x_lo + part) * kHalf + r0 + lane;
+            uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(pa + part * s.rst + lane));
+            for (int xx = part; xx < s.xs; xx += parts) {
+                for (int rr = 0; rr < s.rs; rr += 32)
+                    if (rr + lane < s.rs)
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 4 * rr), "l"(src + rr)
+                                     : "memory");
+                src += static_cast<int64_t>(parts) * kHalf;
+                dst += static_cast<uint32_t>(parts * s.rst) * 4u;
             }
         } else {
-            for (int rr = tid & 63; rr < s.rs; rr += 64)
-                for (int xx = tid >> 6; xx < s.xs; xx += kStThreads / 64) {
+            const int fy = kRow && a.frame_y != nullptr ? a.frame_y[f] : a.f0 + f;
+            for (int xx = part; xx < s.xs; xx += parts) {
+                const int x = s.x_lo + xx;
+                const int64_t o = static_cast<int64_t>(fy) * p.n_tile_x + x;
+                const int lo = p.lo[o], hi = p.hi[o], shift = p.shift[o];
+                for (int rr = lane; rr < s.rs; rr += 32) {
                     const int i = xx * s.rst + rr;
-                    const int x = s.x_lo + xx;
-                    const int ra = p.r0 + s.r_lo + rr;
-                    const int64_t o = static_cast<int64_t>(fy) * p.n_tile_x + x;
-                    pf[i] = (ra < p.lo[o] || ra > p.hi[o]) ? 0.f : p.fz[s.r_lo + rr];
-                    int src = ra + p.shift[o];
+                    const int ra = r0 + rr;
+                    pf[i] = (ra < lo || ra > hi) ? 0.f : p.fz[s.r_lo + rr];
+                    int src = ra + shift;
                     src = src < 0 ? 0 : (src > p.n_rows - 1 ? p.n_rows - 1 : src);
                     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
                                      static_cast<uint32_t>(__cvta_generic_to_shared(pa + i))),
                                  "l"(mag_f + static_cast<int64_t>(x) * kHalf + src)
                                  : "memory");
                 }
+            }
+        }
+        if (part != 0) return;
+        // without the optical-path correction F depends on the row only: its two
+        // taps and the depth-interpolated F (the den term) per row.  The slot's
+        // rows reach zr + 1 of every row, so the per-plan F[zr + 1] (0 past the
+        // window) is the one the patch holds.
+        for (int z = lane; z < kFZ; z += 32) {
+            const int zo = zb + z;
+            if (zo < p.n_out_z) {
+                cp_async<16>(rowp + kr * kFZ + z, p.zrow + zo);
+                cp_async<8>(rowf + kr * kFZ + z, p.zf + zo);
+            } else {
+                rowp[kr * kFZ + z] = make_float4(__int_as_float(-1), 0.f, 0.f, 0.f);
+                rowf[kr * kFZ + z] = make_float2(0.f, 0.f);
+            }
+        }
+        // the slot's A-scans reach every one a column of the block reads
+        const int cc = cb + lane - p.c0;
+        if (cc >= 0 && cc < p.C)
+            cp_async<16>(colp + kr * kBlk + lane, p.xcol + cc);
+        else
+            colp[kr * kBlk + lane] = make_float4(__int_as_float(-1), 0.f, 0.f, __int_as_float(-1));
+        // zero rows (rst - rs of them, 1 or 2) and the zero A-scan (plain stores, before the barrier)
+        for (int xx = lane; xx < s.xs; xx += 32)
+            for (int r = s.rs; r < s.rst; ++r) {
+                pa[xx * s.rst + r] = 0.f;
+                if (opc) pf[xx * s.rst + r] = 0.f;
+            }
+        if (na > s.xs)
+            for (int r = lane; r < s.rst; r += 32) {
+                pa[s.xs * s.rst + r] = 0.f;
+                if (opc) pf[s.xs * s.rst + r] = 0.f;
+            }
+    };
+    float an[kFRows], ad[kFRows];
+#pragma unroll
+    for (int q = 0; q < kFRows; ++q) an[q] = ad[q] = 0.f;
+    const int tx = lane, ty = warp;
+    const int c = cb + tx;
+    // (most blocks take one round; those where many tiles meet take several, so
+    // that they do not set the shared memory of all)
+    for (int k0 = 0, k1; k0 < ns; k0 = k1) {
+    k1 = k0;
+    while (!slot[k1++].last) {
+    }
+    if (k0 > 0) __syncthreads();                             // the previous round's patches have been read
+    {
+        const int n = k1 - k0;
+        constexpr int kWarps = kStThreads / 32;
+        if (n <= kWarps) {
+            const int kr = warp % n;
+            stage(k0 + kr, kr, warp / n, (kWarps - 1 - kr) / n + 1);
+        } else {
+            for (int kr = warp; kr < n; kr += kWarps) stage(k0 + kr, kr, 0, 1);
         }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -349,22 +211,32 @@ __global__ void __launch_bounds__(kStThreads) k_stitch_frames(const StitchDev* _
     // 2. per voxel: tiles in order, depth (Wz) then lateral (WxT) interpolation.
     //    A tap outside the patch reads a zero, so a * F and F of it are the
     //    zeros the reference's operators give there.
-    const int tx = tid & (kBlk - 1), ty = tid / kBlk;
-    const int c = cb + tx;
-    float an[kFRows], ad[kFRows];
-#pragma unroll
-    for (int q = 0; q < kFRows; ++q) an[q] = ad[q] = 0.f;
-    for (int k = 0; k < ns; ++k) {
-        const float4 cp = colp[k * kBlk + tx];
-        const int xr = __float_as_int(cp.x);
+    for (int k = k0; k < k1; ++k) {
+        const float4 cp = colp[(k - k0) * kBlk + tx];
+        const int kind = slot[k].kind;
+        const int xr = __float_as_int((kind & kSlotSingle) ? cp.w : cp.x);
         if (xr < 0) continue;
         const int rst = slot[k].rst;
         // this thread's first A-scan of the patch, rows indexed by zr directly
         const float* pa = sm + slot[k].off + (xr - slot[k].x_lo) * rst - slot[k].r_lo;
         const float wx0 = cp.y, wx1 = cp.z;
-        const float4* rpk = rowp + k * kFZ + ty;
-        const float2* rfk = rowf + k * kFZ + ty;
-        if (slot[k].opc == 0) {
+        const float4* rpk = rowp + (k - k0) * kFZ + ty;
+        const float2* rfk = rowf + (k - k0) * kFZ + ty;
+        if (kind == kSlotSingle) {
+            const float w = wx0 != 0.f ? wx0 : wx1;          // the other is zero
+#pragma unroll
+            for (int q = 0; q < kFRows; ++q) {
+                const float4 rp = rpk[8 * q];
+                const int zr = __float_as_int(rp.x);
+                if (zr < 0) continue;
+                const float2 ff = rfk[8 * q];
+                // a = magnitude * F (TileStitcher.contribute, stitching.py:136)
+                const float a0 = pa[zr] * ff.x, a1 = pa[zr + 1] * ff.y;
+                const float u = fmaf(a1, rp.z, a0 * rp.y);
+                an[q] += __fmul_rn(u, w);
+                ad[q] += __fmul_rn(rp.w, w);
+            }
+        } else if (kind == 0) {
             // F depends on the row only: its two taps and the den term per row
 #pragma unroll
             for (int q = 0; q < kFRows; ++q) {
@@ -375,15 +247,28 @@ __global__ void __launch_bounds__(kStThreads) k_stitch_frames(const StitchDev* _
                 const float* p1 = p0 + rst;
                 const float w0 = rp.y, w1 = rp.z, d = rp.w;
                 const float2 ff = rfk[8 * q];
-                // a = magnitude * F (TileStitcher.contribute, stitching.py:136)
                 const float a00 = p0[0] * ff.x, a01 = p0[1] * ff.y;
                 const float a10 = p1[0] * ff.x, a11 = p1[1] * ff.y;
                 const float u0 = fmaf(a01, w1, a00 * w0), u1 = fmaf(a11, w1, a10 * w0);
                 an[q] += fmaf(u1, wx1, u0 * wx0);
                 ad[q] += fmaf(d, wx1, d * wx0);
             }
-        } else {
+        } else if (kind & kSlotSingle) {
             // optical-path correction: F per A-scan and row, its patch after the magnitudes
+            const float w = wx0 != 0.f ? wx0 : wx1;
+            const float* pf = pa + slot[k].xs * rst;
+#pragma unroll
+            for (int q = 0; q < kFRows; ++q) {
+                const float4 rp = rpk[8 * q];
+                const int zr = __float_as_int(rp.x);
+                if (zr < 0) continue;
+                const float f0 = pf[zr], f1 = pf[zr + 1];
+                const float a0 = pa[zr] * f0, a1 = pa[zr + 1] * f1;
+                const float u = fmaf(a1, rp.z, a0 * rp.y), d = fmaf(f1, rp.z, f0 * rp.y);
+                an[q] += __fmul_rn(u, w);
+                ad[q] += __fmul_rn(d, w);
+            }
+        } else {
             const float* pf = pa + (slot[k].xs + 1) * rst;
 #pragma unroll
             for (int q = 0; q < kFRows; ++q) {
@@ -401,35 +286,185 @@ __global__ void __launch_bounds__(kStThreads) k_stitch_frames(const StitchDev* _
             }
         }
     }
+    }
 
+    if (kRow) {
+        if (c >= a.n_out_x) return;
+#pragma unroll
+        for (int q = 0; q < kFRows; ++q) {
+            const int zo = zb + ty + 8 * q;
+            if (zo >= a.n_out_z || (an[q] == 0.f && ad[q] == 0.f)) continue;
+            const int64_t o = (static_cast<int64_t>(a.frame_offset + f) * a.n_out_z + zo) * a.n_out_x + c;
+            a.num[o] += an[q];
+            a.den[o] += ad[q];
+        }
+        return;
+    }
     // 3. finalise (pipeline.py:296-300) and clim (io/tiff_writer.py:48-50)
     float mn = __int_as_float(0x7f800000), mx = -__int_as_float(0x7f800000);
 #pragma unroll
     for (int q = 0; q < kFRows; ++q) {
         const int zo = zb + ty + 8 * q;
-        if (zo >= n_out_z || c >= n_out_x) continue;
+        if (zo >= a.n_out_z || c >= a.n_out_x) continue;
         float v;
-        if (ad[q] < thr || isnan(ad[q])) {
+        if (ad[q] < a.thr || isnan(ad[q])) {
             v = __int_as_float(0x7fc00000);
         } else {
             v = 20.0f * log10f(__fdiv_rn(an[q], ad[q]));
         }
-        db[(static_cast<int64_t>(f) * n_out_z + zo) * n_out_x + c] = v;
+        a.db[(static_cast<int64_t>(f) * a.n_out_z + zo) * a.n_out_x + c] = v;
         if (isfinite(v)) {
             mn = fminf(mn, v);
             mx = fmaxf(mx, v);
         }
     }
     warp_minmax(mn, mx);
-    if ((tid & 31) == 0 && mn <= mx) {
-        if (plane_mm) {
-            atomicMin(&plane_mm[2 * f], f2ord(mn));
-            atomicMax(&plane_mm[2 * f + 1], f2ord(mx));
+    if (lane == 0) {
+        if (a.plane_mm) fold_range(a.plane_mm + 2 * f, mn, mx);
+        if (a.run_mm) fold_range(a.run_mm, mn, mx);
+    }
+}
+
+// k_stitch without the optical-path correction, its staging by tensor copies:
+// per slot one thread issues a two-dimensional copy of the patch (an aligned
+// window of pitch rows of xs A-scans) and bulk copies of the block's row and
+// column parameters from the plan's tables (padded, so that a block never
+// leaves them); the other threads only wait.  Rows past a tile's window carry
+// weights of zero.  A copy starts at a row that is a multiple of four and its
+// pitch is 4 x an odd number: a warp takes 8 columns x 4 rows, whose reads then
+// fall in distinct banks (8 A-scans a pitch apart x 4 neighbouring rows), and
+// writes whole 32-byte sectors.  Five blocks an SM (48 registers): 183 M voxels
+// of 6 tiles in ~720 us, ~1180 with the copies spread over the threads
+// (k_stitch); four blocks ~840, six (spills) ~815.
+template <int kFZ, bool kRow>
+__global__ void __launch_bounds__(kStThreads, kFZ == 128 ? 3 : 5) k_stitch_tma(const __grid_constant__ CUtensorMap map,
+                                                           const StitchArgs a) {
+    constexpr int kFRows = kFZ / 8;          // rows per thread
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ uint64_t bar;
+    __shared__ StitchTmaSlot slot[kMaxSeg];
+    unsigned char* sm = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);   // tensor copies: 128-byte aligned
+    const int f = blockIdx.z;
+    const int zb = blockIdx.y * kFZ;
+    const int cb = (a.cblk0 + blockIdx.x) * kBlk;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int blk = blockIdx.y * gridDim.x + blockIdx.x;
+    const int ns = a.slot_count[blk];
+    if (kRow && ns == 0) return;
+    if (tid < ns) slot[tid] = a.tslots[static_cast<int64_t>(blk) * a.tiles.n + tid];
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    const int cl = 8 * (warp & 3) + (lane & 7);                      // column of the block
+    const int zl = (warp >> 2) * (kFZ / 2) + (lane >> 3);            // first row; then every fourth
+    const int c = cb + cl;
+    const uint32_t row_off = a.patch_bytes, rowf_off = row_off + kFZ * 16, col_off = rowf_off + kFZ * 8;
+    float an[kFRows], ad[kFRows];
+#pragma unroll
+    for (int q = 0; q < kFRows; ++q) an[q] = ad[q] = 0.f;
+    for (int k0 = 0, round = 0; k0 < ns; k0 += a.ns_round, ++round) {
+        const int n = min(a.ns_round, ns - k0);
+        if (round > 0) __syncthreads();                              // the previous round has been read
+        if (warp == 0) {
+            if (lane == 0)
+                mbar_expect_tx(&bar, static_cast<uint32_t>(n) * (a.pitch * a.box_lines * 4 + kFZ * 24 + kBlk * 16));
+            __syncwarp();
+            if (lane < n) {
+                const StitchTmaSlot& s = slot[k0 + lane];
+                unsigned char* d = sm + lane * a.slot_bytes;
+                asm volatile(
+                    "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], "
+                    "[%1, {%2, %3}], [%4];" ::"r"(smem_u32(d)),
+                    "l"(reinterpret_cast<uint64_t>(&map)), "r"(s.row0), "r"(s.t * a.tile_lines + f * a.n_tile_x + s.x_lo),
+                    "r"(smem_u32(&bar))
+                    : "memory");
+                tma_bulk_g2s(d + row_off, s.zrow, kFZ * 16, &bar);
+                tma_bulk_g2s(d + rowf_off, s.zf, kFZ * 8, &bar);
+                tma_bulk_g2s(d + col_off, s.xcol, kBlk * 16, &bar);
+            }
         }
-        if (run_mm) {
-            atomicMin(&run_mm[0], f2ord(mn));
-            atomicMax(&run_mm[1], f2ord(mx));
+        if (!mbar_wait_bounded(&bar, round & 1, a.status)) return;
+        for (int kr = 0; kr < n; ++kr) {
+            const StitchTmaSlot& s = slot[k0 + kr];
+            const unsigned char* d = sm + kr * a.slot_bytes;
+            const float4 cp = reinterpret_cast<const float4*>(d + col_off)[cl];
+            const int x = __float_as_int(s.single ? cp.w : cp.x);
+            if (x < 0) continue;
+            const int P = a.pitch;
+            // this thread's first A-scan of the patch, rows indexed by zr directly
+            const float* pa = reinterpret_cast<const float*>(d) + (x - s.x_lo) * P - s.r_lo;
+            const float4* rpk = reinterpret_cast<const float4*>(d + row_off) + zl;
+            const float2* rfk = reinterpret_cast<const float2*>(d + rowf_off) + zl;
+            if (s.single) {
+                const float w = cp.y != 0.f ? cp.y : cp.z;           // the other is zero
+#pragma unroll
+                for (int q = 0; q < kFRows; ++q) {
+                    const float4 rp = rpk[4 * q];
+                    const int zr = __float_as_int(rp.x);
+                    if (zr < 0) continue;
+                    const float2 ff = rfk[4 * q];
+                    // a = magnitude * F (TileStitcher.contribute, stitching.py:136)
+                    const float a0 = pa[zr] * ff.x, a1 = pa[zr + 1] * ff.y;
+                    const float u = fmaf(a1, rp.z, a0 * rp.y);
+                    an[q] += __fmul_rn(u, w);
+                    ad[q] += __fmul_rn(rp.w, w);
+                }
+            } else {
+                const float wx0 = cp.y, wx1 = cp.z;
+#pragma unroll
+                for (int q = 0; q < kFRows; ++q) {
+                    const float4 rp = rpk[4 * q];
+                    const int zr = __float_as_int(rp.x);
+                    if (zr < 0) continue;
+                    const float* p0 = pa + zr;
+                    const float* p1 = p0 + P;
+                    const float w0 = rp.y, w1 = rp.z, dd = rp.w;
+                    const float2 ff = rfk[4 * q];
+                    const float a00 = p0[0] * ff.x, a01 = p0[1] * ff.y;
+                    const float a10 = p1[0] * ff.x, a11 = p1[1] * ff.y;
+                    const float u0 = fmaf(a01, w1, a00 * w0), u1 = fmaf(a11, w1, a10 * w0);
+                    an[q] += fmaf(u1, wx1, u0 * wx0);
+                    ad[q] += fmaf(dd, wx1, dd * wx0);
+                }
+            }
         }
+    }
+    if (kRow) {
+        if (c >= a.n_out_x) return;
+#pragma unroll
+        for (int q = 0; q < kFRows; ++q) {
+            const int zo = zb + zl + 4 * q;
+            if (zo >= a.n_out_z || (an[q] == 0.f && ad[q] == 0.f)) continue;
+            const int64_t o = (static_cast<int64_t>(a.frame_offset + f) * a.n_out_z + zo) * a.n_out_x + c;
+            a.num[o] += an[q];
+            a.den[o] += ad[q];
+        }
+        return;
+    }
+    // finalise (pipeline.py:296-300) and clim (io/tiff_writer.py:48-50)
+    float mn = __int_as_float(0x7f800000), mx = -__int_as_float(0x7f800000);
+    float* out = a.db + (static_cast<int64_t>(f) * a.n_out_z + zb + zl) * a.n_out_x + c;
+#pragma unroll
+    for (int q = 0; q < kFRows; ++q) {
+        if (zb + zl + 4 * q >= a.n_out_z || c >= a.n_out_x) continue;
+        float v;
+        if (ad[q] < a.thr || isnan(ad[q])) {
+            v = __int_as_float(0x7fc00000);
+        } else {
+            v = 20.0f * log10f(__fdiv_rn(an[q], ad[q]));
+        }
+        out[static_cast<int64_t>(4 * q) * a.n_out_x] = v;
+        if (isfinite(v)) {
+            mn = fminf(mn, v);
+            mx = fmaxf(mx, v);
+        }
+    }
+    warp_minmax(mn, mx);
+    if (lane == 0) {
+        if (a.plane_mm) fold_range(a.plane_mm + 2 * f, mn, mx);
+        if (a.run_mm) fold_range(a.run_mm, mn, mx);
     }
 }
 
@@ -534,10 +569,7 @@ __global__ void __launch_bounds__(kResThreads) k_resample(const QueueTile* __res
         atomicMax(&mm[1], f2ord(mx));
     }
     __syncthreads();
-    if (tid == 0 && mm[0] != 0xffffffffu) {
-        atomicMin(&run_mm[0], mm[0]);
-        atomicMax(&run_mm[1], mm[1]);
-    }
+    if (tid == 0 && mm[0] != 0xffffffffu) fold_range(run_mm, ord2f(mm[0]), ord2f(mm[1]));
 }
 
 // pipeline.py:296-300 plus plane_clim (io/tiff_writer.py:48-50)
@@ -721,10 +753,7 @@ __global__ void k_minmax(const float* __restrict__ x, int64_t n, unsigned int* _
         }
     }
     warp_minmax(mn, mx);
-    if ((threadIdx.x & 31) == 0 && mn <= mx) {
-        atomicMin(&mm[0], f2ord(mn));
-        atomicMax(&mm[1], f2ord(mx));
-    }
+    if ((threadIdx.x & 31) == 0) fold_range(mm, mn, mx);
 }
 
 __global__ void k_minmax_init(unsigned int* mm, int count) {
@@ -738,49 +767,67 @@ int grid_for(int64_t n, int threads) {
     return static_cast<int>(b < 1 ? 1 : b);
 }
 
-size_t patch_smem(int xs_max, int rs_max) {
-    return sizeof(float) * (2 * static_cast<size_t>(xs_max) * rs_max + 2 * static_cast<size_t>(xs_max) * kBlk);
-}
-
 }  // namespace
 
-cudaError_t launch_stitch(const StitchDev& p, const float* mag, const int* frame_y, int f0, int B, float* num,
-                          float* den, int frame_offset, int n_out_x, int xs_max, int rs_max, cudaStream_t st) {
-    if (B == 0 || p.n_cblk == 0) return cudaSuccess;
-    const size_t smem = patch_smem(xs_max, rs_max);
-    cudaError_t e = cudaFuncSetAttribute(k_stitch_tile, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
-    const dim3 grid(p.n_cblk, (p.n_out_z + kBlk - 1) / kBlk, B);
-    k_stitch_tile<<<grid, kStThreads, smem, st>>>(p, mag, frame_y, f0, num, den, frame_offset, n_out_x, xs_max,
-                                                   rs_max);
-    return cudaGetLastError();
+namespace {
+// the magnitudes as lines of kHalf floats, boxes of `pitch` floats x `lines`
+bool encode_mag_map(CUtensorMap* map, const float* mag, int64_t n_lines, int pitch, int lines) {
+    static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
+    if (encode == nullptr) {
+        cudaDriverEntryPointQueryResult q;
+        void* fn = nullptr;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) !=
+                cudaSuccess ||
+            q != cudaDriverEntryPointSuccess || fn == nullptr)
+            return false;
+        encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+    }
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(kHalf), static_cast<cuuint64_t>(n_lines)};
+    const cuuint64_t strides[1] = {kHalf * sizeof(float)};
+    const cuuint32_t box[2] = {static_cast<cuuint32_t>(pitch), static_cast<cuuint32_t>(lines)};
+    const cuuint32_t estr[2] = {1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(mag), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+}  // namespace
 
-cudaError_t launch_stitch_frames(const StitchDev* plans_dev, const TileList& tiles, const StitchSlot* slots,
-                                 const int* slot_count, int ns_max, size_t patch_smem_bytes, const float* mag,
-                                 int64_t mag_tile_stride, int B, int n_tile_x, int f0, int n_out_z, int n_out_x,
-                                 float thr, float* db, unsigned int* plane_mm, unsigned int* run_mm, int rows,
-                                 cudaStream_t st) {
-    if (B == 0) return cudaSuccess;
-    if (rows != 32 && rows != 64 && rows != 128) return cudaErrorInvalidValue;
+cudaError_t launch_stitch(const StitchDev* plans_dev, const StitchArgs& a, size_t patch_smem_bytes, int n_cblk, int B,
+                          int rows, cudaStream_t st) {
+    if (B == 0 || n_cblk == 0) return cudaSuccess;
+    const bool row = a.num != nullptr;
+    if (a.tslots != nullptr) {
+        const auto kern = rows == 32   ? (row ? k_stitch_tma<32, true> : k_stitch_tma<32, false>)
+                          : rows == 64 ? (row ? k_stitch_tma<64, true> : k_stitch_tma<64, false>)
+                                       : (row ? k_stitch_tma<128, true> : k_stitch_tma<128, false>);
+        const size_t smem = static_cast<size_t>(a.ns_round) * a.slot_bytes + 128;
+        CUtensorMap map;
+        if (!encode_mag_map(&map, a.mag, a.n_lines, a.pitch, a.box_lines)) return cudaErrorInvalidValue;
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (e != cudaSuccess) return e;
+        kern<<<dim3(n_cblk, (a.n_out_z + rows - 1) / rows, B), kStThreads, smem, st>>>(map, a);
+        return cudaGetLastError();
+    }
+    const auto kern = rows == 32   ? (row ? k_stitch<32, true> : k_stitch<32, false>)
+                      : rows == 64 ? (row ? k_stitch<64, true> : k_stitch<64, false>)
+                                   : k_stitch<128, false>;
+    if ((rows != 32 && rows != 64 && rows != 128) || (row && rows == 128)) return cudaErrorInvalidValue;
     const size_t smem = patch_smem_bytes +
-                        static_cast<size_t>(ns_max) * (sizeof(SlotPlan) + sizeof(float) * (6 * rows + 4 * kBlk)) + 16;
-    if (smem > 160 * 1024) return cudaErrorInvalidValue;
-    auto kern = rows == 32 ? k_stitch_frames<32> : (rows == 64 ? k_stitch_frames<64> : k_stitch_frames<128>);
+                        static_cast<size_t>(a.ns_round) * sizeof(float) * (6 * rows + 4 * kBlk) + 16;
+    if (smem > 200 * 1024) return cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
-    const dim3 grid((n_out_x + kBlk - 1) / kBlk, (n_out_z + rows - 1) / rows, B);
-    kern<<<grid, kStThreads, smem, st>>>(plans_dev, tiles, slots, slot_count, mag, mag_tile_stride, n_tile_x, f0,
-                                         n_out_z, n_out_x, thr, db, plane_mm, run_mm, ns_max);
+    kern<<<dim3(n_cblk, (a.n_out_z + rows - 1) / rows, B), kStThreads, smem, st>>>(plans_dev, a);
     return cudaGetLastError();
 }
 
 cudaError_t launch_finalise(const float* num, const float* den, int64_t n_per_plane, int n_planes, float thr,
                             float* db, unsigned int* plane_minmax, cudaStream_t st) {
     if (n_planes == 0 || n_per_plane == 0) return cudaSuccess;
-    int gx = grid_for(n_per_plane, 256);
-    if (gx > 64) gx = 64;
+    // enough blocks for every SM whatever the number of planes, eight values a thread at least
+    int gx = grid_for((n_per_plane + 7) / 8, 256);
+    const int most = n_planes < 16 ? 1024 / n_planes : 64;
+    if (gx > most) gx = most;
     k_finalise<<<dim3(gx, n_planes), 256, 0, st>>>(num, den, n_per_plane, thr, db, plane_minmax);
     return cudaGetLastError();
 }

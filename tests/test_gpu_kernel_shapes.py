@@ -169,3 +169,70 @@ def test_batched_tiles_equal_single_tiles_across_passes(gpu_ctx):
             assert torch.equal(t[3], ref)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("nx,frames,tiles_x,depths,fraction", [(7, 1, 1, 1, 0.0), (33, 2, 2, 3, 0.0), (64, 3, 2, 2, 0.5),
+                                                               (301, 2, 2, 3, 0.3), (1000, 1, 2, 3, 0.0)])
+def test_stitched_frames_against_oracle_and_row_interface(gpu_ctx, nx, frames, tiles_x, depths, fraction):
+    """Blocks where columns take one A-scan of a tile, two (tiles a fraction of
+    a pixel apart, the widened end columns), tiles that miss a block, ragged
+    last blocks, every block height: the oracle's planes from the same
+    magnitudes, the row interface bit for bit, and the range of the planes.
+    Tolerance: a ratio of sums of at most 12 products, each rounded a few
+    times (2e-6 relative, 2e-5 dB), and dB values up to 100 to an ulp."""
+    torch = pytest.importorskip("torch")
+    from oracle import numerics as O
+    from oct_recon_af_v1_gb300 import geometry as G
+    from oct_recon_af_v1_gb300 import reconstruct as R
+    from oct_recon_af_v1_gb300 import stitching as S
+    from oct_recon_af_v1_gb300 import synthetic
+    sg = G.build_spectral_geometry(synthetic.lambda_nm(), 0.0, 1.33)
+    gpu_ctx.set_geometry(sg.sinc_idx, sg.sinc_w, sg.window)
+    xc = np.array([0.0, (nx - max(1, nx // 10) + fraction) * 1e-3])[:tiles_x]
+    zd = np.array([0.0, 0.15, 0.3])[:depths]
+    focus = np.array([411.0, 392.5, 422.25])[:depths]
+    lay = S.ScanLayout(xc, np.array([0.0]), zd, nx, frames, nx * 1e-3, frames * 1e-3)
+    tg = S.tiled_geometry(lay, sg.z_um, focus, 1.0)
+    desc = O.ScanDesc(xc, np.array([0.0]), zd, nx, frames, nx * 1e-3, frames * 1e-3)
+    og = O.tiled_geometry(desc, sg.z_um, focus, 1.0)
+    nz, nxo = len(tg.out_z_mm), len(tg.out_x_mm)
+    num, den = np.zeros((frames, nz, nxo), np.float32), np.zeros((frames, nz, nxo), np.float32)
+    ids, raws, stitchers = [], [], []
+    for xi in range(tiles_x):
+        for zi in range(depths):
+            st = S.TileStitcher.build(tg, xc[xi], zd[zi], focus[zi], 80.0)
+            ids.append(st.upload(gpu_ctx))
+            stitchers.append(st)
+            raw = torch.from_numpy(synthetic.generate_numpy(frames, nx, 25, seed=9 * xi + zi).view(np.int16)).cuda()
+            raws.append(raw)
+            mag = torch.empty((frames, nx, 1024), device="cuda")
+            gpu_ctx.magnitude(raw, 25, mag, raw_dtype=0)
+            gpu_ctx.synchronize()
+            o = O.Stitcher(og, xc[xi], zd[zi], focus[zi], 80.0)
+            a, b = o.contribute(mag.cpu().numpy())
+            num[:, :, o.c0:o.c1] += a
+            den[:, :, o.c0:o.c1] += b
+    ref = O.finalise(num, den)
+    thr = S.min_weight_threshold(np.float32)
+    row = R.RowReconstructor(gpu_ctx, 25, nz, nxo, 2)
+    out = torch.empty((frames, nz, nxo), device="cuda")
+    row.process_row([R.RowTile(t, lambda fr, r=r: r[int(fr[0]):int(fr[-1]) + 1].view(torch.uint16))
+                     for t, r in zip(stitchers, raws)], np.arange(frames), out)
+    gpu_ctx.synchronize()
+    rows_db = out.cpu().numpy()
+    try:
+        for height in (32, 64, 128):
+            gpu_ctx.set_stitch_rows(height)
+            gpu_ctx.clim_reset()
+            planes = torch.full((frames, nz, nxo), 7.0, device="cuda")
+            _, mm = gpu_ctx.frames_process(ids, raws, 25, 0, nz, nxo, thr, out=planes, plane_minmax=True, raw_dtype=0)
+            db = planes.cpu().numpy()
+            np.testing.assert_array_equal(db, rows_db)
+            assert np.array_equal(np.isnan(db), np.isnan(ref))
+            fin = np.isfinite(ref)
+            assert np.abs(db[fin] - ref[fin]).max() < 4e-5
+            for f in range(frames):
+                assert (mm[f] == [db[f][np.isfinite(db[f])].min(), db[f][np.isfinite(db[f])].max()]).all()
+            assert gpu_ctx.clim_get() == (db[fin].min(), db[fin].max())
+    finally:
+        gpu_ctx.set_stitch_rows(64)
