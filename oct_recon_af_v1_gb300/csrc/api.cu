@@ -319,7 +319,8 @@ void transform_pass(octgb_ctx* c, LinesArgs a, float* scratch, int dtype, unsign
 // go through lines_fixed, which no other call uses or frees (a graph captured
 // by the caller may hold it).
 void launch_spectral_segs(octgb_ctx* c, const void* const* segs, int n_seg, int dtype, int B, int interf, int apod,
-                          int mode, float* out_dev, int z0, int nz, unsigned int* mm_dev, float* apod_mean = nullptr) {
+                          int mode, float* out_dev, int z0, int nz, unsigned int* mm_dev, float* apod_mean = nullptr,
+                          bool exact = false) {
     if (B == 0 || n_seg == 0) return;
     const int64_t n = static_cast<int64_t>(n_seg) * B * (interf - apod);
     require(n < (int64_t(1) << 31), "batch too large");
@@ -328,7 +329,8 @@ void launch_spectral_segs(octgb_ctx* c, const void* const* segs, int n_seg, int 
         ck(c->apod.ensure(static_cast<size_t>(n_seg) * B * kN * sizeof(float) + 16), "cudaMalloc(apod)");
         apod_mean = c->apod.as<float>();
     }
-    const LinesArgs a = lines_args(c, segs, n_seg, B, interf, apod, apod_mean);
+    LinesArgs a = lines_args(c, segs, n_seg, B, interf, apod, apod_mean);
+    a.exact = exact;
     ck(launch_apod_mean(a, dtype, n_seg * B, apod_mean, c->stream), "apod kernel");
     c->launches++;
     const unsigned int total = static_cast<unsigned int>(n), pass = fixed ? kMinPass : pass_lines(c, total);
@@ -346,19 +348,20 @@ void require_spectral(octgb_ctx* c) {
     if (c->cancel.load()) throw Error(OCTGB_ERR_CANCELLED, "cancelled");
 }
 
-// Run the spectral stage of a batch into `out` (device): |X| or dB.
+// Run the spectral stage of a batch into `out` (device): |X| or dB (exact: with the exact background).
 void run_spectral(octgb_ctx* c, const void* raw, int dtype, int loc, int B, int interf, int apod, int mode,
-                  float* out_dev, int z0, int nz, unsigned int* mm_dev) {
+                  float* out_dev, int z0, int nz, unsigned int* mm_dev, bool exact = false) {
     require_spectral(c);
     if (B == 0) return;  // empty batch: nothing to launch
     const size_t bytes = static_cast<size_t>(B) * interf * kN * raw_elem(dtype);
     const void* rd = stage_raw(c, raw, dtype, loc, bytes);
-    launch_spectral_segs(c, &rd, 1, dtype, B, interf, apod, mode, out_dev, z0, nz, mm_dev);
+    launch_spectral_segs(c, &rd, 1, dtype, B, interf, apod, mode, out_dev, z0, nz, mm_dev, nullptr, exact);
 }
 
-// The lines of a batch (kModeSpec or kModeLinHann) into `out` (device, 16-byte aligned).
+// The lines of a batch (any LineMode; exact: kModeReal with the exact
+// background) into `out` (device, 16-byte aligned).
 void run_lines(octgb_ctx* c, const void* raw, int dtype, int loc, int B, int interf, int apod, int mode, float* out_dev,
-               const double* hann = nullptr, const float2* hann2 = nullptr) {
+               const double* hann = nullptr, const float2* hann2 = nullptr, bool exact = false) {
     require_spectral(c);
     if (B == 0) return;
     const int64_t n = static_cast<int64_t>(B) * (interf - apod);
@@ -367,6 +370,7 @@ void run_lines(octgb_ctx* c, const void* raw, int dtype, int loc, int B, int int
     const void* rd = stage_raw(c, raw, dtype, loc, bytes);
     ck(c->apod.ensure(static_cast<size_t>(B) * kN * sizeof(float) + 16), "cudaMalloc(apod)");
     LinesArgs a = lines_args(c, &rd, 1, B, interf, apod, c->apod.as<float>());
+    a.exact = exact;
     ck(launch_apod_mean(a, dtype, B, c->apod.as<float>(), c->stream), "apod kernel");
     a.l1 = static_cast<unsigned int>(n);
     a.out = out_dev;
@@ -1980,50 +1984,47 @@ int octgb_row_add_batch_ex(octgb_ctx* c, int plan_id, const void* raw, int dtype
 }
 
 // ---------------------------------------------------------------------------
-// Precision form: the sinc on the tensor cores (split-FP16, three products).
+// Precision form: the float32 form's operations without its float32
+// apodisation mean.  Integer raws: k_lines with the exact background.  Float32
+// raws: the background in float64, the sinc on the tensor cores (split-FP16,
+// three products).
 
 namespace {
-// X (B * nx lines of kN float32, device) = linearised interferogram of a raw batch
-float* precision_linearise(octgb_ctx* c, const void* raw, int dtype, int loc, int B, int interf, int apod,
-                           float* x_dev = nullptr) {
+void require_precision(octgb_ctx* c) {
     if (!c->has_geom) throw Error(OCTGB_ERR_STATE, "octgb_set_geometry has not been called");
     if (!c->prec_ok)
         throw Error(OCTGB_ERR_STATE, "the precision form needs every 64-output block's sinc band within 96 samples");
     if (c->cancel.load()) throw Error(OCTGB_ERR_CANCELLED, "cancelled");
+}
+
+// X (B * nx lines of kN float32, device) = linearised interferogram of a raw batch
+float* precision_linearise(octgb_ctx* c, const void* raw, int dtype, int loc, int B, int interf, int apod,
+                           float* x_dev = nullptr) {
+    require_precision(c);
     const int nx = interf - apod;
     const int64_t n = static_cast<int64_t>(B) * nx;
-    const size_t bytes = static_cast<size_t>(B) * interf * kN * raw_elem(dtype);
-    const void* rd = stage_raw(c, raw, dtype, loc, bytes);
-    // (+ one window of padding: the sinc kernel copies whole 96-sample windows of the sums)
-    ck(c->apod.ensure(static_cast<size_t>(B) * kN * sizeof(double) + kPKW * sizeof(int) + 16), "cudaMalloc(apod)");
-    SpectralArgs a{};
-    a.raw = rd;
-    a.B = B;
-    a.interf = interf;
-    a.apod = apod;
-    a.nx = nx;
-    a.n_ascans = n;
     float* X = x_dev;
     if (X == nullptr) {
         ck(c->prec_x.ensure(static_cast<size_t>(n) * kN * sizeof(float)), "cudaMalloc(X)");
         X = c->prec_x.as<float>();
     }
-    ck(c->prec_m.ensure(static_cast<size_t>(n) * sizeof(float)), "cudaMalloc(line means)");
     if (dtype != OCTGB_F32) {
-        // integer raws: the sinc kernel reads the raw window itself (no d' in memory)
-        ck(c->prec_hi.ensure(static_cast<size_t>(n) * sizeof(long long)), "cudaMalloc(line sums)");
-        CUtensorMap mr;
-        if (!encode_raw_map(&mr, rd, B, interf, apod)) throw Error(OCTGB_ERR_CUDA, "cuTensorMapEncodeTiled failed");
-        ck(launch_prec_sinc_raw(a, dtype, mr, c->prec_w.as<uint8_t>(), c->prec_kb.as<int>(), c->apod.as<int>(),
-                                c->prec_hi.as<long long>(), c->prec_m.as<float>(), X, c->status_dev, c->num_sms,
-                                c->stream),
-           "tensor-core sinc kernels");
-        c->launches += 3;
+        run_lines(c, raw, dtype, loc, B, interf, apod, kModeReal, X, nullptr, nullptr, true);
         return X;
     }
+    const size_t bytes = static_cast<size_t>(B) * interf * kN * raw_elem(dtype);
+    SpectralArgs a{};
+    a.raw = stage_raw(c, raw, dtype, loc, bytes);
+    a.B = B;
+    a.interf = interf;
+    a.apod = apod;
+    a.nx = nx;
+    a.n_ascans = n;
+    ck(c->apod.ensure(static_cast<size_t>(B) * kN * sizeof(double)), "cudaMalloc(apod)");
+    ck(c->prec_m.ensure(static_cast<size_t>(n) * sizeof(float)), "cudaMalloc(line means)");
     ck(c->prec_hi.ensure(static_cast<size_t>(n) * kN * sizeof(__half)), "cudaMalloc(d hi)");
     ck(c->prec_lo.ensure(static_cast<size_t>(n) * kN * sizeof(__half)), "cudaMalloc(d lo)");
-    ck(launch_prec_split(a, dtype, c->apod.p, c->prec_hi.as<__half>(), c->prec_lo.as<__half>(),
+    ck(launch_prec_split(a, c->apod.as<double>(), c->prec_hi.as<__half>(), c->prec_lo.as<__half>(),
                          c->prec_m.as<float>(), c->num_sms, c->stream),
        "background / split kernels");
     CUtensorMap mh, ml;
@@ -2046,9 +2047,10 @@ int octgb_selftest_wait_expiry(octgb_ctx* c, int which, int wait_limit_us) {
         if (c->capturing) throw Error(OCTGB_ERR_STATE, "self-test during graph capture");
         auto set = which == 0 ? set_wait_test_spectral : set_wait_test_precision;
         constexpr unsigned long long kDefaultLimit = 2000000000ull;
-        // zero raws, 2 B-scans x (1 apodisation + 256) lines, already on the device
+        // zero raws (float32 for the tensor-core sinc), 2 B-scans x (1 apodisation
+        // + 256) lines, already on the device
         const int B = 2, interf = 257, apod = 1;
-        const size_t bytes = static_cast<size_t>(B) * interf * kN * sizeof(uint16_t);
+        const size_t bytes = static_cast<size_t>(B) * interf * kN * sizeof(float);
         ck(c->raw.ensure(bytes), "cudaMalloc(raw)");
         ck(cudaMemsetAsync(c->raw.p, 0, bytes, c->stream), "memset raw");
         ck(set(static_cast<unsigned long long>(wait_limit_us) * 1000ull, 1, c->stream), "set wait limit");
@@ -2059,7 +2061,7 @@ int octgb_selftest_wait_expiry(octgb_ctx* c, int which, int wait_limit_us) {
                 run_spectral(c, c->raw.p, OCTGB_U16, OCTGB_DEVICE, B, interf, apod, kModeMag, c->magbuf.as<float>(), 0,
                              0, nullptr);
             } else {
-                precision_linearise(c, c->raw.p, OCTGB_U16, OCTGB_DEVICE, B, interf, apod);
+                precision_linearise(c, c->raw.p, OCTGB_F32, OCTGB_DEVICE, B, interf, apod);
             }
             check_status(c);                    // a wait that expired throws OCTGB_ERR_TIMEOUT here
         } catch (...) {
@@ -2135,13 +2137,20 @@ int octgb_magnitude_precision(octgb_ctx* c, const void* raw, int dtype, int loc,
         validate_raw(raw, dtype, loc, B, interf, apod);
         require(mag != nullptr, "mag is NULL");
         if (B == 0) return;
-        const float* X = precision_linearise(c, raw, dtype, loc, B, interf, apod);
+        require_precision(c);
         const size_t ob = static_cast<size_t>(B) * (interf - apod) * kHalf * sizeof(float);
         float* dst = mag;
         if (mag_loc != OCTGB_DEVICE) {
             ck(c->out.ensure(ob), "cudaMalloc(out)");
             dst = c->out.as<float>();
         }
+        if (dtype != OCTGB_F32) {
+            run_spectral(c, raw, dtype, loc, B, interf, apod, kModeMag, dst, 0, 0, nullptr, true);
+            if (mag_loc != OCTGB_DEVICE) copy_out(c, mag, OCTGB_HOST, dst, ob);
+            if (mag_loc != OCTGB_DEVICE || loc != OCTGB_DEVICE) check_status(c);
+            return;
+        }
+        const float* X = precision_linearise(c, raw, dtype, loc, B, interf, apod);
         // window (Hann/rms x dispersion phase / N), inverse FFT, |.|: the scorer's FFT kernel
         DispArgs a{};
         a.X = X;

@@ -27,6 +27,15 @@
 //                          for one another except through the ring.
 // A CTA takes a contiguous range of A-scans, so the apodisation row changes
 // once a B-scan.
+//
+// Exact (integer raws; the precision form): the background without the float32
+// form's rounding of the apodisation mean.  With S the integer sum of the
+// apodisation lines and A their count, n = A raw - S is an exact integer, the
+// line mean m = sum(n) / (2048 A) comes from integer sums, and
+// d - m = fma(n, 1/A, -m) takes one rounding; then the same band.  30 000
+// A-scans to magnitudes in 217 us, 1.2e-7 off float64 (2-norm); with a
+// split-FP16 tensor-core product over 96-sample windows (1.5 x the outputs,
+// three products, copies of 16-byte rows: 248 us of its 351) 2.2e-7.
 // Bound by the shared-memory path: 471 wavefronts an A-scan, 67 % of its
 // cycles, with 1718 warp instructions (issue active 52 %); 25 000 A-scans in
 // 65 us (382 M/s, 12.4 kB read and written an A-scan = 4.7 TB/s).  With the
@@ -124,7 +133,18 @@ struct LinePos {
     unsigned int sg, b, x;
 };
 
-template <typename RawT, int Mode, int U, bool Tiles>
+// sum of the two 16-bit integers of a word, added to c
+template <typename RawT>
+__device__ __forceinline__ int add_pair(uint32_t w, int c) {
+    return static_cast<RawT>(-1) < 0 ? __dp2a_lo(static_cast<int>(w), 0x0101, c)
+                                     : static_cast<int>(__dp2a_lo(w, 0x0101u, static_cast<uint32_t>(c)));
+}
+
+// With more apodisation lines than this A raw - S may not be exact in float32,
+// and the sums are kept as integers.
+constexpr int kExactFloat = 255;
+
+template <typename RawT, int Mode, int U, bool Tiles, bool Exact>
 __global__ void __launch_bounds__(kThr, 1) k_lines(const LinesArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     using Smem = LinesSmem<RawT>;
@@ -221,7 +241,7 @@ __global__ void __launch_bounds__(kThr, 1) k_lines(const LinesArgs a) {
         // into the other slot when it differs from the previous A-scan's
         unsigned int have_row = 0xffffffffu;
         int slot = 0;
-        auto issue = [&](int k, const LinePos& p) {
+        auto issue = [&](int k, const LinePos& p) -> bool {
             unsigned int ar;
             const RawT* row = row_of(p, ar);
             const bool load = ar != have_row;
@@ -237,70 +257,116 @@ __global__ void __launch_bounds__(kThr, 1) k_lines(const LinesArgs a) {
                 if (load)
                     tma_bulk_g2s(S.apod[w][slot], a.apod_mean + static_cast<int64_t>(ar) * kN, kN * sizeof(float), bar);
             }
+            return load;
         };
         const int mine = (n - w + kBgWarps - 1) / kBgWarps;    // A-scans of this warp
         issue(0, pos);
         int issued = 1;
-        bool ok = true;
+        bool ok = true, fresh = true, fresh_next = false;    // the A-scan's apodisation row is new
+        long long row_sum = 0;                               // Exact: sum of S over the row
+        const bool exact_float = Exact && a.apod <= kExactFloat;
+        const float apod_f = static_cast<float>(a.apod), inv_apod = 1.0f / apod_f;
         for (int k = 0; k < mine; ++k) {
             const int cur = slot;                            // the current A-scan's apodisation row
             if (k + 1 < mine) {
                 advance(pos);
                 __syncwarp();                                // stage (k + 1) & 1 was read by every lane
-                issue(k + 1, pos);
+                fresh_next = issue(k + 1, pos);
                 ++issued;
             }
             ok = wait(&S.raw_full[w][k & 1], static_cast<uint32_t>(k >> 1) & 1u);
             if (__any_sync(0xffffffffu, !ok)) break;
-            // lane holds samples 4 lane + 128 i .. + 3, i = 0 .. 15 (i = p + 4 q).
-            // The sum keeps the order of the four partial sums of 128 threads
-            // with 16 samples each: p = lt / 32 of thread lt's, q within it.
             float2 d[32];
-            float part[4];
+            float m;
             const RawT* rw = S.raw[w][k & 1] + 4 * lane;
             const float* ap = S.apod[w][cur] + 4 * lane;
+            if constexpr (Exact) {
+                int tot = 0;
+                if (fresh) {
+                    row_sum = 0;
 #pragma unroll
-            for (int p = 0; p < 4; ++p) {
-                float sum = 0.f;
+                    for (int i = 0; i < 16; ++i) {
+                        const int4 q = *reinterpret_cast<const int4*>(ap + 128 * i);
+                        row_sum += exact_float
+                                       ? -static_cast<long long>(__int_as_float(q.x)) - static_cast<long long>(__int_as_float(q.y)) -
+                                             static_cast<long long>(__int_as_float(q.z)) - static_cast<long long>(__int_as_float(q.w))
+                                       : static_cast<long long>(q.x) + q.y + q.z + q.w;
+                    }
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int i = p + 4 * q;
-                    float2 r01, r23;
-                    raw4<RawT>(rw + 128 * i, r01, r23);
-                    const float4 m = *reinterpret_cast<const float4*>(ap + 128 * i);
-                    d[2 * i] = sub2(r01, make_float2(m.x, m.y));
-                    d[2 * i + 1] = sub2(r23, make_float2(m.z, m.w));
-                    sum += (d[2 * i].x + d[2 * i].y) + (d[2 * i + 1].x + d[2 * i + 1].y);
+                    for (int o = 16; o > 0; o >>= 1) row_sum += __shfl_xor_sync(0xffffffffu, row_sum, o);
                 }
-                part[p] = sum;
-            }
-            // the four trees over 32 lanes (o = 16, 8, 4, 2, 1), two at a time
-            // after the first two steps: lane bit 4 selects the pair, bit 3 the sum
-            float s0, s1;
-            {
-                const bool up = (lane & 16) != 0;
-                s0 = (up ? part[2] : part[0]) + __shfl_xor_sync(0xffffffffu, up ? part[0] : part[2], 16);
-                s1 = (up ? part[3] : part[1]) + __shfl_xor_sync(0xffffffffu, up ? part[1] : part[3], 16);
-                const bool up2 = (lane & 8) != 0;
-                s0 = (up2 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, up2 ? s0 : s1, 8);
-            }
 #pragma unroll
-            for (int o = 4; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-            s0 += __shfl_xor_sync(0xffffffffu, s0, 8);       // part 0 + part 1, part 2 + part 3
-            s0 += __shfl_xor_sync(0xffffffffu, s0, 16);
-            const float m = s0 * (1.0f / kN);
+                for (int i = 0; i < 16; ++i) {
+                    const uint2 q = *reinterpret_cast<const uint2*>(rw + 128 * i);
+                    tot = add_pair<RawT>(q.y, add_pair<RawT>(q.x, tot));
+                    if (exact_float) {
+                        // the row holds -S; A raw - S exactly
+                        float2 r01, r23;
+                        raw4<RawT>(rw + 128 * i, r01, r23);
+                        const float4 ns = *reinterpret_cast<const float4*>(ap + 128 * i);
+                        const float2 a2 = make_float2(apod_f, apod_f);
+                        d[2 * i] = fma2(r01, a2, make_float2(ns.x, ns.y));
+                        d[2 * i + 1] = fma2(r23, a2, make_float2(ns.z, ns.w));
+                    } else {
+                        const int4 sv = *reinterpret_cast<const int4*>(ap + 128 * i);
+                        d[2 * i].x = static_cast<float>(a.apod * static_cast<int>(static_cast<RawT>(q.x & 0xffffu)) - sv.x);
+                        d[2 * i].y = static_cast<float>(a.apod * static_cast<int>(static_cast<RawT>(q.x >> 16)) - sv.y);
+                        d[2 * i + 1].x = static_cast<float>(a.apod * static_cast<int>(static_cast<RawT>(q.y & 0xffffu)) - sv.z);
+                        d[2 * i + 1].y = static_cast<float>(a.apod * static_cast<int>(static_cast<RawT>(q.y >> 16)) - sv.w);
+                    }
+                }
+                const long long sum_n = static_cast<long long>(a.apod) * __reduce_add_sync(0xffffffffu, tot) - row_sum;
+                m = static_cast<float>(sum_n) / (static_cast<float>(kN) * apod_f);
+            } else {
+                // lane holds samples 4 lane + 128 i .. + 3, i = 0 .. 15 (i = p + 4 q).
+                // The sum keeps the order of the four partial sums of 128 threads
+                // with 16 samples each: p = lt / 32 of thread lt's, q within it.
+                float part[4];
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {
+                    float sum = 0.f;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int i = p + 4 * q;
+                        float2 r01, r23;
+                        raw4<RawT>(rw + 128 * i, r01, r23);
+                        const float4 m = *reinterpret_cast<const float4*>(ap + 128 * i);
+                        d[2 * i] = sub2(r01, make_float2(m.x, m.y));
+                        d[2 * i + 1] = sub2(r23, make_float2(m.z, m.w));
+                        sum += (d[2 * i].x + d[2 * i].y) + (d[2 * i + 1].x + d[2 * i + 1].y);
+                    }
+                    part[p] = sum;
+                }
+                // the four trees over 32 lanes (o = 16, 8, 4, 2, 1), two at a time
+                // after the first two steps: lane bit 4 selects the pair, bit 3 the sum
+                float s0, s1;
+                {
+                    const bool up = (lane & 16) != 0;
+                    s0 = (up ? part[2] : part[0]) + __shfl_xor_sync(0xffffffffu, up ? part[0] : part[2], 16);
+                    s1 = (up ? part[3] : part[1]) + __shfl_xor_sync(0xffffffffu, up ? part[1] : part[3], 16);
+                    const bool up2 = (lane & 8) != 0;
+                    s0 = (up2 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, up2 ? s0 : s1, 8);
+                }
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+                s0 += __shfl_xor_sync(0xffffffffu, s0, 8);       // part 0 + part 1, part 2 + part 3
+                s0 += __shfl_xor_sync(0xffffffffu, s0, 16);
+                m = s0 * (1.0f / kN);
+            }
             const int i_line = w + kBgWarps * k, st = i_line % kRing;
             ok = wait(&S.empty[st], (static_cast<uint32_t>(i_line / kRing) & 1u) ^ 1u);
             if (__any_sync(0xffffffffu, !ok)) break;
-            const float2 m2 = make_float2(m, m);
+            const float2 m2 = make_float2(m, m), nm2 = make_float2(-m, -m), ia2 = make_float2(inv_apod, inv_apod);
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
-                const float2 e01 = sub2(d[2 * i], m2), e23 = sub2(d[2 * i + 1], m2);
+                const float2 e01 = Exact ? fma2(d[2 * i], ia2, nm2) : sub2(d[2 * i], m2);
+                const float2 e23 = Exact ? fma2(d[2 * i + 1], ia2, nm2) : sub2(d[2 * i + 1], m2);
                 *reinterpret_cast<float4*>(&S.d[st][4 * lane + 128 * i]) = make_float4(e01.x, e01.y, e23.x, e23.y);
             }
             if (lane == 0) S.mval[st] = m;
             __syncwarp();
             if (lane == 0) mbar_arrive(&S.full[st]);
+            fresh = fresh_next;
         }
         // copies still in flight land before the CTA's memory is released
         if (!ok || issued < mine)
@@ -340,15 +406,34 @@ __global__ void __launch_bounds__(kThr, 1) k_lines(const LinesArgs a) {
         if (__any_sync(0xffffffffu, !ok)) return;
         const float* dk = S.d[st] + wbase;
         float2 acc[2][2] = {};
+        // Exact: the window in two halves, their sums added last (each rounds
+        // at about half the magnitude)
+        constexpr int kHalfU = Exact ? (U / 2 + 1) / 2 * 2 : U;
+        float2 first_half[2][2] = {};
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const float* p = dk + (u < wrot ? u + U : u);
+            if (Exact && u == kHalfU) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        first_half[h][e] = acc[h][e];
+                        acc[h][e] = make_float2(0.f, 0.f);
+                    }
+            }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const float x = p[h * kDLine];
                 acc[h][0] = fma2(wp[0][u], make_float2(x, x), acc[h][0]);
                 acc[h][1] = fma2(wp[1][u], make_float2(x, x), acc[h][1]);
             }
+        }
+        if (Exact) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) acc[h][e] = add2(first_half[h][e], acc[h][e]);
         }
         const float mk[2] = {S.mval[st], S.mval[st + 1]};
         __syncwarp();
@@ -391,7 +476,8 @@ __global__ void __launch_bounds__(kThr, 1) k_lines(const LinesArgs a) {
 // apodisation mean (cpu_kernels.py:20-25): exact sum, divided in float64,
 // stored float32.  Four samples a thread, five lines in flight.
 constexpr int kApodThreads = 128;                // x 4 samples = a quarter of a row
-template <typename RawT, bool Tiles>
+// Exact: the sums instead, as -S in float32 while that is exact, else as int32.
+template <typename RawT, bool Tiles, bool Exact>
 __global__ void __launch_bounds__(kApodThreads) k_apod_mean(const LinesArgs a, float* __restrict__ out) {
     pdl_launch();                                // the lines kernel loads its weights meanwhile
     const int row = blockIdx.x >> 2;             // segment * B + b, or the tiles' apod_row0 + b
@@ -423,6 +509,14 @@ __global__ void __launch_bounds__(kApodThreads) k_apod_mean(const LinesArgs a, f
             acc[2] += static_cast<int>(static_cast<RawT>(q.y & 0xffffu));
             acc[3] += static_cast<int>(static_cast<RawT>(q.y >> 16));
         }
+        if (Exact) {
+            *reinterpret_cast<float4*>(out + static_cast<int64_t>(row) * kN + j) =
+                apod <= kExactFloat ? make_float4(-static_cast<float>(acc[0]), -static_cast<float>(acc[1]),
+                                                  -static_cast<float>(acc[2]), -static_cast<float>(acc[3]))
+                                    : make_float4(__int_as_float(acc[0]), __int_as_float(acc[1]),
+                                                  __int_as_float(acc[2]), __int_as_float(acc[3]));
+            return;
+        }
 #pragma unroll
         for (int e = 0; e < 4; ++e) s[e] = static_cast<double>(acc[e]);
     } else {
@@ -441,13 +535,14 @@ __global__ void __launch_bounds__(kApodThreads) k_apod_mean(const LinesArgs a, f
                     static_cast<float>(s[3] / apod));
 }
 
-template <typename RawT, int Mode, int U, bool Tiles>
+template <typename RawT, int Mode, int U, bool Tiles, bool Exact>
 cudaError_t launch_t(const LinesArgs& a, int num_sms, cudaStream_t st) {
     const size_t smem = sizeof(LinesSmem<RawT>);
-    const auto kernel = k_lines<RawT, Mode, U, Tiles>;
+    const auto kernel = k_lines<RawT, Mode, U, Tiles, Exact>;
     constexpr int kType = sizeof(RawT) == 4 ? 2 : static_cast<RawT>(-1) < 0 ? 1 : 0;
-    constexpr int kBit = (kType * 4 + (Tiles ? 3 : Mode)) * 4 + (U - 14) / 4;
-    static_assert(kBit < kReadyDisp, "the bits of the kernels overlap");
+    constexpr int kBit = Exact ? kReadyExact + kType * 4 + (U - 14) / 4
+                               : (kType * 4 + (Tiles ? 3 : Mode)) * 4 + (U - 14) / 4;
+    static_assert(Exact ? kBit < 64 : kBit < kReadyDisp, "the bits of the kernels overlap");
     const cudaError_t e = kernel_ready(a.ready, kBit, kernel, smem);
     if (e != cudaSuccess) return e;
     const unsigned int n = a.l1 - a.l0;
@@ -456,33 +551,38 @@ cudaError_t launch_t(const LinesArgs& a, int num_sms, cudaStream_t st) {
 }
 
 // (wider windows than 14 spill a few weights: five warps a scheduler have 96 registers a thread)
-template <typename RawT, int Mode, bool Tiles>
+template <typename RawT, int Mode, bool Tiles, bool Exact>
 cudaError_t launch_u(const LinesArgs& a, int num_sms, cudaStream_t st) {
     switch (a.g.U) {
-        case 14: return launch_t<RawT, Mode, 14, Tiles>(a, num_sms, st);
-        case 18: return launch_t<RawT, Mode, 18, Tiles>(a, num_sms, st);
-        case 22: return launch_t<RawT, Mode, 22, Tiles>(a, num_sms, st);
-        case 26: return launch_t<RawT, Mode, 26, Tiles>(a, num_sms, st);
+        case 14: return launch_t<RawT, Mode, 14, Tiles, Exact>(a, num_sms, st);
+        case 18: return launch_t<RawT, Mode, 18, Tiles, Exact>(a, num_sms, st);
+        case 22: return launch_t<RawT, Mode, 22, Tiles, Exact>(a, num_sms, st);
+        case 26: return launch_t<RawT, Mode, 26, Tiles, Exact>(a, num_sms, st);
         default: return cudaErrorInvalidValue;
     }
 }
 
 template <typename RawT>
 cudaError_t launch_mode(const LinesArgs& a, int mode, int num_sms, cudaStream_t st) {
-    if (a.qt != nullptr) return launch_u<RawT, kModeReal, true>(a, num_sms, st);
+    if constexpr (sizeof(RawT) == 2)
+        if (a.exact) return launch_u<RawT, kModeReal, false, true>(a, num_sms, st);
+    if (a.exact) return cudaErrorInvalidValue;
+    if (a.qt != nullptr) return launch_u<RawT, kModeReal, true, false>(a, num_sms, st);
     switch (mode) {
-        case kModeSpec: return launch_u<RawT, kModeSpec, false>(a, num_sms, st);
-        case kModeLinHann: return launch_u<RawT, kModeLinHann, false>(a, num_sms, st);
-        default: return launch_u<RawT, kModeReal, false>(a, num_sms, st);
+        case kModeSpec: return launch_u<RawT, kModeSpec, false, false>(a, num_sms, st);
+        case kModeLinHann: return launch_u<RawT, kModeLinHann, false, false>(a, num_sms, st);
+        default: return launch_u<RawT, kModeReal, false, false>(a, num_sms, st);
     }
 }
 
 template <typename RawT>
 void launch_apod_t(const LinesArgs& a, int rows, float* out, cudaStream_t st) {
-    if (a.qt != nullptr)
-        k_apod_mean<RawT, true><<<4 * rows, kApodThreads, 0, st>>>(a, out);
+    if (a.exact)
+        k_apod_mean<RawT, false, true><<<4 * rows, kApodThreads, 0, st>>>(a, out);
+    else if (a.qt != nullptr)
+        k_apod_mean<RawT, true, false><<<4 * rows, kApodThreads, 0, st>>>(a, out);
     else
-        k_apod_mean<RawT, false><<<4 * rows, kApodThreads, 0, st>>>(a, out);
+        k_apod_mean<RawT, false, false><<<4 * rows, kApodThreads, 0, st>>>(a, out);
 }
 
 }  // namespace

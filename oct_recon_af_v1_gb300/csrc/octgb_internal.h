@@ -96,7 +96,8 @@ inline cudaError_t kernel_ready(uint64_t* ready, int bit, Kernel kernel, size_t 
     if (e == cudaSuccess) *ready |= uint64_t(1) << bit;
     return e;
 }
-constexpr int kReadyDisp = 48;            // bits 0 .. 47: k_lines, 48 .. 52: k_disp_mag
+// bits 0 .. 47: k_lines, 48 .. 52: k_disp_mag, 53 .. 60: k_lines with the exact background
+constexpr int kReadyDisp = 48, kReadyExact = 53;
 
 // lines.cu: A-scans [l0, l1) of n_seg raw batches of one shape, or of tiles of
 // uneven size (qt), numbered segment by segment, B-scan by B-scan
@@ -106,7 +107,8 @@ struct LinesArgs {
     const QueueTile* qt;      // null: the batches above
     int n_qt;
     unsigned int l0, l1;
-    const float* apod_mean;   // float32 apodisation mean, a row per B-scan
+    const float* apod_mean;   // float32 apodisation mean (exact: sums), a row per B-scan
+    bool exact;               // integer raws: the exact background (kModeReal, no tiles)
     DevGeometry g;
     float* out;               // line l at (l - out_l0) kN (kModeSpec: complex)
     unsigned int out_l0;
@@ -115,7 +117,7 @@ struct LinesArgs {
     int* status;              // device status word
     uint64_t* ready;          // host: bits of the caller's context, see kernel_ready
 };
-// apodisation mean of every B-scan (`rows` of them) into out
+// apodisation mean (exact: sums) of every B-scan (`rows` of them) into out
 cudaError_t launch_apod_mean(const LinesArgs& a, int dtype, int rows, float* out, cudaStream_t st);
 // launched dependent on the kernel before it in the stream (as launch_disp_mag's)
 cudaError_t launch_lines(const LinesArgs& a, int dtype, int mode, int num_sms, cudaStream_t st);
@@ -263,7 +265,7 @@ int packbits_slot(int cols);
 cudaError_t launch_packbits(const uint16_t* img, int rows, int cols, uint8_t* slots, int* sizes, long long* offsets,
                             uint8_t* out, cudaStream_t st);
 
-// precision form (precision.cu): tensor-core sinc
+// precision form of float32 raws (precision.cu): tensor-core sinc
 constexpr int kPM = 128;                 // A-scans per tile (MMA M)
 constexpr int kPN = 64;                  // output samples per block (MMA N)
 constexpr int kPKW = 96;                 // source window per block (6 K-steps of 16)
@@ -274,24 +276,17 @@ constexpr int kPBlocks = kN / kPN;       // output blocks per A-scan
 #include <cuda_fp16.h>
 #include <vector>
 namespace octgb {
-// apod_scratch: B x kN int32 (integer raws) or float64 (float32 raws)
-cudaError_t launch_prec_split(const SpectralArgs& a, int dtype, void* apod_scratch, __half* hi, __half* lo,
-                              float* mline, int num_sms, cudaStream_t st);
+// apod64: B x kN of scratch
+cudaError_t launch_prec_split(const SpectralArgs& a, double* apod64, __half* hi, __half* lo, float* mline,
+                              int num_sms, cudaStream_t st);
 cudaError_t launch_prec_sinc(const CUtensorMap& tm_hi, const CUtensorMap& tm_lo, const uint8_t* wtiles,
                              const int* kb, const float* mline, float* X, int64_t n_ascans, int* status, int num_sms,
                              cudaStream_t st);
 bool encode_prec_map(CUtensorMap* map, const void* base, int64_t n_ascans);
-// integer raws, fused: apodisation sums, line sums, then the tensor-core sinc
-// reading the raw window directly (apod_sum: B x kN ints; sum_n, mline: per A-scan)
-cudaError_t launch_prec_sinc_raw(const SpectralArgs& a, int dtype, const CUtensorMap& tm_raw, const uint8_t* wtiles,
-                                 const int* kb, int* apod_sum, long long* sum_n, float* mline, float* X, int* status,
-                                 int num_sms, cudaStream_t st);
-bool encode_raw_map(CUtensorMap* map, const void* raw, int B, int interf, int apod);
 // W tiles (per output block: hi then lo, canonical K-major no-swizzle, W x 64)
 // and window starts kb; false when a block's band exceeds the window
 bool build_prec_tiles(const int* start, const int* len, const float* wt, std::vector<uint16_t>& tiles,
                       std::vector<int>& kb);
-size_t prec_smem_bytes();
 
 // learned beta/focus estimator (cnn.cu)
 cudaError_t launch_image_pool(const float* A, int n_probe, int nb, int nx, int z_keep, float* img, cudaStream_t st);

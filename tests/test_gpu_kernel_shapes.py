@@ -236,3 +236,25 @@ def test_stitched_frames_against_oracle_and_row_interface(gpu_ctx, nx, frames, t
             assert gpu_ctx.clim_get() == (db[fin].min(), db[fin].max())
     finally:
         gpu_ctx.set_stitch_rows(64)
+
+
+@pytest.mark.parametrize("dtype", [np.uint16, np.int16])
+@pytest.mark.parametrize("bscans,nx,apod", [(1, 1, 1), (3, 5, 25), (1, 200, 255), (2, 130, 256), (1, 40, 700)])
+def test_precision_lines_of_integer_raws(gpu_ctx, dtype, bscans, nx, apod):
+    """The exact background on either side of the count up to which its sums
+    are float32 integers, full-range counts included: the linearised lines
+    against float64.  Tolerance: one rounding of d - m and about eleven of the
+    band (2^-24 each of sums up to ~3 times the largest value): 2e-6."""
+    from oracle import numerics as O
+    from oct_recon_af_v1_gb300 import geometry as G
+    from oct_recon_af_v1_gb300 import synthetic
+    lam = synthetic.lambda_nm()
+    sg = G.build_spectral_geometry(lam, 0.0, 1.33)
+    gpu_ctx.set_geometry(sg.sinc_idx, sg.sinc_w, np.ones(2048, np.complex128))
+    raw = synthetic.generate_numpy(bscans, nx, apod, seed=nx)
+    raw[0, -1, ::3] = 65535                                   # the ends of the range beside ordinary counts
+    raw[0, 0, ::5] = 65535
+    raw = (raw.astype(np.int64) - (32768 if dtype == np.int16 else 0)).astype(dtype)
+    x64 = O.linearise_numpy(raw, O.spectral_geometry(lam, 0.0, 1.33), apod, np.float64)
+    got = gpu_ctx.linearise_precision(raw, apod)
+    assert np.abs(got - x64).max() < 2e-6 * np.abs(x64).max()
