@@ -258,3 +258,28 @@ def test_precision_lines_of_integer_raws(gpu_ctx, dtype, bscans, nx, apod):
     x64 = O.linearise_numpy(raw, O.spectral_geometry(lam, 0.0, 1.33), apod, np.float64)
     got = gpu_ctx.linearise_precision(raw, apod)
     assert np.abs(got - x64).max() < 2e-6 * np.abs(x64).max()
+
+
+@pytest.mark.parametrize("dtype", [np.uint16, np.int16])
+@pytest.mark.parametrize("bscans,nx,apod", [(1, 1, 1), (1, 6, 700), (2, 3, 255), (1, 9, 3)])
+def test_float64_form_at_the_ends_of_the_range(gpu_ctx, dtype, bscans, nx, apod):
+    """Full-range counts, many apodisation lines, a constant spectrum (all its
+    magnitudes zero): the float32 rounding of float64's magnitudes but for the
+    pairs' ~1e-12 of the line's largest."""
+    from oracle import numerics as O
+    from oct_recon_af_v1_gb300 import geometry as G
+    from oct_recon_af_v1_gb300 import synthetic
+    lam, beta = synthetic.lambda_nm(), synthetic.beta_ref_from_px(1e-5)
+    sg = G.build_spectral_geometry(lam, beta, 1.33)
+    gpu_ctx.set_geometry(sg.sinc_idx, sg.sinc_w, sg.window)
+    raw = synthetic.generate_numpy(bscans, nx, apod, seed=nx + apod)
+    raw[0, apod, ::3] = 65535
+    raw = (raw.astype(np.int64) - (32768 if dtype == np.int16 else 0)).astype(dtype)
+    if nx == 9:
+        raw[:, :apod] = raw[:, apod:apod + 1]
+        raw[:, -2:] = raw[:, apod:apod + 1]               # equal to the apodisation lines
+    ref = O.magnitude_numpy(raw, O.spectral_geometry(lam, beta, 1.33), apod, np.float64)
+    got = gpu_ctx.magnitude_exact(raw, apod).astype(np.float64)
+    assert (np.abs(got - ref) <= 2.0 ** -24 * np.abs(ref) + 1e-12 * np.abs(ref).max(-1, keepdims=True)).all()
+    if nx == 9:
+        assert (got[:, -2:] == 0).all()
