@@ -2254,7 +2254,8 @@ int octgb_cnn_conv3x3_tc(octgb_ctx* c, const float* x, const float* w, const flo
         require(conv3x3_tc_supported(cin, cout, h, wd),
                 "tensor-core convolution: 1 <= cin <= 32, cout a multiple of 32 up to 128, and the width a "
                 "multiple of 128 or a divisor of 128 whose row count divides the height");
-        ck(launch_conv3x3_tc(x, w, b, y, n, cin, cout, h, wd, 0, c->status_dev, c->stream), "tensor-core conv kernel");
+        ck(launch_conv3x3_tc(x, w, b, y, n, cin, cout, h, wd, 0, c->num_sms, c->status_dev, c->stream),
+           "tensor-core conv kernel");
         c->launches++;
     });
 }
@@ -2267,7 +2268,7 @@ int octgb_cnn_conv3x3_relu_pool_tc(octgb_ctx* c, const float* x, const float* w,
         require(conv3x3_tc_pool_supported(cin, cout, h, wd),
                 "fused tensor-core convolution + pool: 1 <= cin <= 32, cout a multiple of 32 up to 128, the width "
                 "a multiple of 128 and the height even");
-        ck(launch_conv3x3_tc(x, w, b, p, n, cin, cout, h, wd, 1, c->status_dev, c->stream),
+        ck(launch_conv3x3_tc(x, w, b, p, n, cin, cout, h, wd, 1, c->num_sms, c->status_dev, c->stream),
            "tensor-core conv + pool kernel");
         c->launches++;
     });
@@ -2301,21 +2302,18 @@ int octgb_cnn_conv3x3_bwd_tc(octgb_ctx* c, const float* x, const float* w, const
         require(parts > 0, "tensor-core weight gradient: 1 <= cin <= 48, 1 <= cout <= 128 and a band of rows "
                            "dividing the height whose staged input fits in shared memory");
         ck(c->wgrad_part.ensure(parts * sizeof(float)), "cudaMalloc(weight-gradient partial sums)");
-        ck(launch_conv3x3_wgrad_tc(x, dy, dw, n, cin, cout, h, wd, c->wgrad_part.as<float>(), c->num_sms,
+        ck(launch_conv3x3_wgrad_tc(x, dy, dw, db, n, cin, cout, h, wd, c->wgrad_part.as<float>(), c->num_sms,
                                    c->status_dev, c->stream),
            "tensor-core weight-gradient kernel");
-        ck(c->bias_part.ensure(static_cast<size_t>(n) * cout * sizeof(float)), "cudaMalloc(bias partial sums)");
-        ck(launch_bias_grad(dy, n, cout, static_cast<int64_t>(h) * wd, db, c->bias_part.as<float>(), c->stream),
-           "bias-gradient kernel");
-        c->launches += 2 + ((static_cast<int64_t>(h) * wd) % 4 == 0 ? 2 : 1);
+        c->launches += 2;
         if (dx != nullptr) {
             require(w_scratch != nullptr, "w_scratch is NULL");
             ck(launch_flip_weights(w, cout, cin, w_scratch, c->stream), "weight flip kernel");
             // the data gradient is the convolution of dy with the flipped kernel
             // (cout -> cin channels): BF16 tensor cores where the shape allows
             if (conv3x3_tc_supported(cout, cin, h, wd))
-                ck(launch_conv3x3_tc(dy, w_scratch, nullptr, dx, n, cout, cin, h, wd, 0, c->status_dev, c->stream,
-                                     true),
+                ck(launch_conv3x3_tc(dy, w_scratch, nullptr, dx, n, cout, cin, h, wd, 0, c->num_sms, c->status_dev,
+                                     c->stream, true),
                    "tensor-core conv kernel");
             else
                 ck(launch_conv3x3(dy, w_scratch, nullptr, dx, n, cout, cin, h, wd, c->stream), "conv kernel");

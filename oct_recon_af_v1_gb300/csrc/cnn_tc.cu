@@ -5,33 +5,41 @@
 // (BF16 for the data gradient) and float32 accumulation on the 5th-generation
 // tensor cores (tcgen05.mma kind::f16, accumulator in TMEM).  Forward pass of
 // training and inference, and the data gradient (the convolution of dy with
-// the flipped kernel).  k_conv3x3_wgrad_tc (further down): the weight
-// gradient.
+// the flipped kernel).  k_conv3x3_wgrad_tc (further down): the weight and
+// bias gradients.
 //
-// Implicit GEMM without an im2col copy: M = 128 output pixels of one image (a
-// row segment when the width W >= 128, else 128 / W whole rows), N = the
-// output channels, K = 3 x 3 taps x the input channels (chunks of 8, an even
-// number of chunks).  The tile's input rows are staged once in shared memory
-// as fp16, eight channels per 16 bytes, pixel rows contiguous per chunk, so
-// the A operand of tap (dy, dx) is the staged block itself seen through a
-// shifted matrix descriptor (canonical no-swizzle K-major layout, rows 16
-// bytes apart):
-//   W >= 128  rows y0 - 1 .. y0 + 1 with a one-pixel halo (columns x0 - 1 ..
-//             x0 + 128, zero outside the image); tap (dy, dx) starts at pixel
-//             dy * 130 + dx;
-//   W < 128   rows y0 - 1 .. y0 + R without halo, in three copies shifted by
-//             dx - 1 columns with the wrapped column zeroed; tap (dy, dx)
-//             starts at pixel dy * W of copy dx.
-// Per tile one thread issues 9 taps x (chunks / 2) K16 MMAs; the staged block
-// and the accumulator (2 x N TMEM columns) are double-buffered, so tile j's
-// MMAs run while the CTA writes tile j - 1's pre-activations (every warp its
-// 32 TMEM lanes = pixels, + bias, coalesced along x) and stages tile j + 1.
-// With ReLU + 2x2 mean fused (W >= 128) a unit is a vertical pair of tiles;
-// where the CTAs per SM allow, the pair's four input rows are staged as one
-// block (its halo rows read once) and the second tile's MMAs read it one row
-// down.  Persistent over units.  Every mbarrier wait is bounded; on expiry the CTA
-// records the status, waits (bounded) for its MMAs, frees its TMEM and
-// returns.
+// Both are bound by the float32 planes they read and write, so both are built
+// around that stream.  The unit of work is a band: R rows (of one column
+// segment where whole rows would not fit) of one image.  Specialised warps
+// hand a band on through mbarriers:
+//   producer   copies the band's rows, eight channels at a time, into a ring of
+//              raw slots (one tensor copy a slot; 4-byte cp.async where the rows
+//              are not on 16-byte boundaries);
+//   converters pack a slot's rows to 16-bit operands in one of two staged blocks;
+//   MMA        one warp issues the band's tcgen05.mma;
+//   epilogue   (convolution) drains the accumulators to global memory.
+// Copies of later bands are in flight throughout, so no phase waits for the
+// memory latency.  Measured at 128 images, against kernels that staged each tile
+// with plain loads between two block barriers (and summed the bias gradient in a
+// pass of its own):
+//   convolution       3 x 256 x 256: 516 -> 270 us (4.3 TB/s), 32 x 128 x 128: 370 -> 108 us (5.0 TB/s)
+//     + ReLU + mean   280 -> 217 us, 265 -> 96 us
+//   gradients of w, b 1100 -> 311 us (3.8 TB/s), 470 -> 233 us (2.3 TB/s)
+// What bounds them now: the 1.1 GB stream of the first convolution and its nine
+// MMAs a tile about equally; the MMAs of the gradients at 32 channels (167 us
+// without them), whose M = 128 rows hold 32 output channels.
+//
+// A staged block holds the band's input rows y0 - 1 .. y0 + R with a zero
+// column before each row and zeros after it up to the row pitch Wp (W + 2
+// rounded up to 4), as [channel group of 8][pixel][8 channels x 2 B].  Output
+// pixel q = r * Wp + ox then meets input pixel q + ty * Wp + tx, so tap
+// (ty, tx) is the staged block itself seen from that pixel on: a matrix
+// descriptor offset of 16 bytes a pixel, no im2col copy.
+//
+// Every mbarrier wait is bounded; on expiry the CTA records the status, waits
+// (bounded) for its copies and MMAs, frees its TMEM and returns.
+#include <cuda.h>
+#include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -43,34 +51,45 @@
 namespace octgb {
 namespace {
 
-constexpr int kCM = 128;                    // output pixels per tile (MMA M)
-constexpr int kCThreads = 128;              // four warps = the 128 TMEM lanes
-constexpr int kCSlots = 5;                  // staged pixels per thread (a staged block holds <= 640)
+constexpr int kCM = 128;                    // MMA M: output pixels per tile (convolution), output channels (gradient)
+constexpr int kMaxSlots = 8;                // raw slots (3 at least: a copy in flight while two are converted)
+constexpr int kMaxBox = 256;                // elements per dimension of a tensor copy
+constexpr uint32_t kSmemBudget = 226u * 1024u;
 
-struct ConvGeom {
-    int n, cin, cout, H, W;
-    int cin8;          // channel chunks of 8, even (chunks past cin8r are zero)
-    int cin8r;         // chunks holding channels
-    int wseg, rows;    // tile: rows x wseg pixels
-    int halo;          // 1: one staged copy with halo columns (W >= 128); 0: three shifted copies
-    int cols_s;        // staged pixels per row
-    int pix_c;         // staged pixels per chunk (one copy)
-    int nbuf;          // staged buffers (2: the next block stages while the MMAs read the other)
-    int sh;            // tiles per staged block: 2 = a pooled pair's rows and halo read once, else 1
-    int pool;          // 1: ReLU + 2x2 mean fused into the epilogue (units = vertical tile pairs)
-    int tiles_img;     // tiles per image
-    int64_t n_units;   // tiles, or tile pairs with pool
-    uint32_t xbytes;   // one staged buffer
-    uint32_t off_b, smem;
-    int tmem_cols;
+// the bands of an image and the shape of a raw slot
+struct Band {
+    int C, H, W;
+    int R;               // rows per band
+    int Ws, Wp;          // columns per segment, staged row pitch
+    int nseg, nband;     // per image
+    int rp, rawp;        // raw slot of x: floats per row (W, or Ws + 8: from column x0 - 4), per channel (R + 2 rows)
+    int vec;             // rows on 16-byte boundaries: tensor copies
+    uint32_t wp_inv;     // ceil(2^32 / Wp)
+    int64_t n_units;
 };
 
-struct ConvBars {
-    uint64_t x[2], d[2], drain;
-    uint32_t tmem;
-    int abort;
-    float bias[128];
+struct BandAt {
+    int img, y0, x0, rows;                  // rows: R, fewer in an image's last band
 };
+
+__device__ __forceinline__ int div_wp(const Band& g, int q) {
+    return static_cast<int>(__umulhi(static_cast<uint32_t>(q), g.wp_inv));      // exact: q * Wp < 2^32
+}
+
+__device__ __forceinline__ BandAt band_at(const Band& g, int64_t u) {
+    BandAt o;
+    const int per_img = g.nband * g.nseg;
+    o.img = static_cast<int>(u / per_img);
+    const int i = static_cast<int>(u - static_cast<int64_t>(o.img) * per_img);
+    const int band = i / g.nseg;
+    o.y0 = band * g.R;
+    o.x0 = (i - band * g.nseg) * g.Ws;
+    o.rows = min(g.R, g.H - o.y0);
+    return o;
+}
+
+// first column in a raw slot of x (4 before a segment: its halo column, on a 16-byte boundary)
+__device__ __forceinline__ int slot_x0(const Band& g, const BandAt& o) { return g.nseg == 1 ? 0 : o.x0 - 4; }
 
 __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
     const __half2 h = __floats2half2_rn(a, b);
@@ -91,58 +110,193 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 // kind::f16 A and B formats: 0 = FP16, 1 = BF16 (both operands the same type)
 constexpr uint32_t kIdescBf16 = (1u << 7) | (1u << 10);
 
-__device__ __forceinline__ bool conv_wait(uint64_t* bar, uint32_t parity, ConvBars& S, int* status) {
-    bool ok = true;
-    if (*reinterpret_cast<volatile int*>(&S.abort) == 0) {
+// a bounded wait of a warp (all lanes go on, or none); false ends its role's loop
+__device__ __forceinline__ bool role_wait(uint64_t* bar, uint32_t parity, int* abort, int* status) {
+    bool ok = false;
+    if (*reinterpret_cast<volatile int*>(abort) == 0) {
         ok = mbar_wait_bounded(bar, parity, status);
-        if (!ok) atomicExch(&S.abort, 1);
-    } else {
-        ok = false;
+        if (!ok) atomicExch(abort, 1);
     }
-    return __syncthreads_and(ok ? 1 : 0) != 0;
+    return __all_sync(0xffffffffu, ok);
 }
 
-// image and origin of tile h (0, or 1 = the row below with pool) of unit u
-__device__ __forceinline__ void unit_tile(const ConvGeom& g, int64_t u, int h, int& img, int& y0, int& x0) {
-    if (g.pool) {                                 // W >= 128: pairs of row segments
-        const int per_row = g.W / kCM;
-        const int64_t pairs = static_cast<int64_t>(g.H / 2) * per_row;
-        img = static_cast<int>(u / pairs);
-        const int pi = static_cast<int>(u - static_cast<int64_t>(img) * pairs);
-        y0 = 2 * (pi / per_row) + h;
-        x0 = (pi % per_row) * kCM;
-        return;
-    }
-    img = static_cast<int>(u / g.tiles_img);
-    const int ti = static_cast<int>(u - static_cast<int64_t>(img) * g.tiles_img);
-    if (g.W >= kCM) {
-        const int per_row = g.W / kCM;
-        y0 = ti / per_row;
-        x0 = (ti - y0 * per_row) * kCM;
+// Producer warp: nch channels from plane `plane` on, rows y0 .. y0 + rows - 1 and
+// columns x0 .. x0 + cols - 1, into a raw slot.  One tensor copy (box: the whole
+// slot, zeros outside the planes), or 4-byte copies of the part inside the image
+// where the rows are not on 16-byte boundaries.  (One bulk copy per channel and
+// row of 512 bytes measured 100 cycles a copy: 751 us for 1.1 GB, copies alone.)
+__device__ __forceinline__ void load_slot(const CUtensorMap& map, const float* src, int H, int W, int vec, int plane,
+                                          int nch, int y0, int rows, int x0, int cols, int box_floats, float* slot,
+                                          uint64_t* bar) {
+    const int lane = threadIdx.x & 31;
+    if (vec) {
+        if (lane == 0) {
+            mbar_expect_tx(bar, static_cast<uint32_t>(box_floats) * 4u);
+            asm volatile(
+                "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], "
+                "[%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(slot)),
+                "l"(reinterpret_cast<uint64_t>(&map)), "r"(x0), "r"(y0), "r"(plane), "r"(smem_u32(bar))
+                : "memory");
+        }
+        __syncwarp();
     } else {
-        y0 = ti * g.rows;
-        x0 = 0;
+        const int r0 = max(0, -y0), r1 = min(rows, H - y0), c0 = max(0, -x0), c1 = min(cols, W - x0);
+        for (int c = 0; c < nch; ++c)
+            for (int r = r0; r < r1; ++r) {
+                const float* p = src + (static_cast<int64_t>(plane + c) * H + y0 + r) * W + x0;
+                for (int i = c0 + lane; i < c1; i += 32)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(slot + (c * rows + r) * cols + i)),
+                                 "l"(p + i)
+                                 : "memory");
+            }
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
     }
+}
+
+// converter thread t of nt: a raw slot's pixels as 16-byte groups of 8
+// channels, zero outside the image
+template <bool kBf16>
+__device__ __forceinline__ void stage_slot(const Band& g, const BandAt& o, const float* raw, int nch, uint4* dst,
+                                           int npix, int t, int nt) {
+    const int sx = o.x0 - 1 - slot_x0(g, o);               // slot column of staged column 0
+#pragma unroll 2
+    for (int i = t; i < npix; i += nt) {
+        const int r = div_wp(g, i), cc = i - r * g.Wp;
+        const int iy = o.y0 - 1 + r, ix = o.x0 - 1 + cc;
+        const bool in = r < o.rows + 2 && cc < g.Ws + 2 && iy >= 0 && iy < g.H && ix >= 0 && ix < g.W;
+        const float* p = raw + (in ? r * g.rp + sx + cc : 0);
+        float v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = in && e < nch ? p[e * g.rawp] : 0.f;
+        dst[i] = make_uint4(pack2<kBf16>(v[0], v[1]), pack2<kBf16>(v[2], v[3]), pack2<kBf16>(v[4], v[5]),
+                            pack2<kBf16>(v[6], v[7]));
+    }
+}
+
+// The same from a tensor copy's slot, whose rows and columns outside the image
+// are zeros already: what is left of the bounds (the pitch's padding, and column
+// -1 of a slot that holds whole rows) is the same in every band, so the slot
+// offset of each of the thread's pixels is kept in registers (-1: zero).
+template <int kIt>
+struct Pixels {
+    int off[kIt];
+    __device__ __forceinline__ Pixels(const Band& g, int npix, int t, int nt) {
+        const int sx = g.nseg == 1 ? -1 : 3;               // slot column of staged column 0
+#pragma unroll
+        for (int k = 0; k < kIt; ++k) {
+            const int i = t + k * nt;
+            const int r = div_wp(g, i), cc = i - r * g.Wp;
+            const bool in = i < npix && r < g.R + 2 && cc < g.Ws + 2 && cc + sx >= 0 && cc + sx < g.rp;
+            off[k] = in ? r * g.rp + sx + cc : -1;
+        }
+    }
+    template <bool kBf16, bool kAll>
+    __device__ __forceinline__ void stage(const float* raw, int rawp, int nch, uint4* dst, int npix, int t, int nt) const {
+#pragma unroll
+        for (int k = 0; k < kIt; ++k) {
+            const int i = t + k * nt;
+            if (i >= npix) break;
+            float v[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = off[k] >= 0 && (kAll || e < nch) ? raw[off[k] + e * rawp] : 0.f;
+            dst[i] = make_uint4(pack2<kBf16>(v[0], v[1]), pack2<kBf16>(v[2], v[3]), pack2<kBf16>(v[4], v[5]),
+                                pack2<kBf16>(v[6], v[7]));
+        }
+    }
+};
+
+// the raw ring's place in the sequence of slots
+struct Ring {
+    int slot = 0;
+    uint32_t use = 0;
+    __device__ __forceinline__ void next(int slots) {
+        if (++slot == slots) {
+            slot = 0;
+            ++use;
+        }
+    }
+};
+
+// ---------------------------------------------------------------- convolution
+// Implicit GEMM: M = 128 staged pixels, N = the output channels, K = 3 x 3 taps
+// x the input channels (chunks of 8, an even number of chunks).  W >= 128: a
+// tile is 128 columns of a row (with ReLU + 2x2 mean fused a vertical pair of
+// them, two accumulators); W < 128: 128 consecutive pixels of the staged pitch,
+// whose padding columns are computed and not written.  Tile t's accumulator is
+// drained by one of two sets of four warps (each warp its 32 TMEM lanes =
+// pixels, + bias, coalesced along x) while the next tiles' MMAs run.
+constexpr int kCEpi = 8, kCConv = 8;                       // epilogue and converter warps
+constexpr int kCThreads = 32 * (kCEpi + kCConv + 2);
+constexpr int kBandPix = 1024;                             // most pixels of a band (of more than two rows)
+constexpr int kCPix = 7;                                   // staged pixels a converter thread: 1024 + 2 (256 + 4) of them
+
+struct ConvGeom {
+    Band b;
+    int cout;
+    int cin8, cin8r;   // channel chunks of 8, even (chunks past cin8r are zero)
+    int xpix;          // pixels per chunk of a staged block
+    int pool, wide;    // wide: W >= 128
+    int slots, nd;     // raw slots, accumulators
+    uint32_t slotb, xbytes, off_x, off_b, smem;
+    int tmem_cols;
+};
+
+struct ConvBars {
+    uint64_t full[kMaxSlots], empty[kMaxSlots], sfull[2], sempty[2], dfull[4], dempty[4], drain;
+    uint32_t tmem;
+    int abort;
+    float bias[128];
+};
+
+__device__ __forceinline__ int conv_tiles(const ConvGeom& g, const BandAt& o) {
+    if (g.wide) return (g.pool ? o.rows / 2 : o.rows) * (g.b.Ws / kCM);
+    return (o.rows * g.b.Wp + kCM - 1) / kCM;
+}
+
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ uint64_t uniform64(uint64_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+
+// a tile's MMAs: nine taps x kKs steps of 16 channels
+template <int kKs>
+__device__ __forceinline__ void conv_mmas(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, int Wp, int xpix,
+                                          int cout) {
+    d = uniform(d);
+    a = uniform64(a);
+#pragma unroll
+    for (int tap = 0; tap < 9; ++tap)
+#pragma unroll
+        for (int ks = 0; ks < kKs; ++ks)
+            mma_f16_warp(d, a + static_cast<uint64_t>(tap / 3 * Wp + tap % 3 + 2 * ks * xpix),
+                         b + static_cast<uint64_t>((2 * kKs * tap + 2 * ks) * cout), idesc, tap > 0 || ks > 0 ? 1u : 0u);
 }
 
 template <bool kBf16>
-__global__ void __launch_bounds__(kCThreads, 4)
-    k_conv3x3_tc(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
+__global__ void __launch_bounds__(kCThreads, 1)
+    k_conv3x3_tc(const __grid_constant__ CUtensorMap xmap, const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
                  float* __restrict__ y, const ConvGeom g, int* status) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ ConvBars S;
-    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* base = smem_raw + align_up_smem(smem_raw, 1024);
+    uint8_t* X = base + g.off_x;                         // two blocks [cin8][xpix][16 B]
     uint8_t* B = base + g.off_b;                         // [9 taps][cin8][cout][16 B]
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);          // uniform: the roles are warps
     const uint32_t b_chunk = static_cast<uint32_t>(g.cout) * 16;
-    const int64_t hw = static_cast<int64_t>(g.H) * g.W;
-    const int copies = g.halo ? 1 : 3;
-    const int U = g.pool ? 2 : 1;                        // tiles per unit
+    const int64_t hw = static_cast<int64_t>(g.b.H) * g.b.W;
+    const int U = g.pool ? 2 : 1;                        // accumulators per tile
 
     if (tid == 0) {
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(&S.x[b], 1);
-            mbar_init(&S.d[b], 1);
+        for (int i = 0; i < g.slots; ++i) {
+            mbar_init(&S.full[i], g.b.vec ? 1 : 32);
+            mbar_init(&S.empty[i], kCConv);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&S.sfull[i], kCConv);
+            mbar_init(&S.sempty[i], 1);
+        }
+        for (int i = 0; i < g.nd; ++i) {
+            mbar_init(&S.dfull[i], 1);
+            mbar_init(&S.dempty[i], 4);
         }
         mbar_init(&S.drain, 1);
         S.abort = 0;
@@ -155,207 +309,193 @@ __global__ void __launch_bounds__(kCThreads, 4)
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     for (int co = tid; co < g.cout; co += kCThreads) S.bias[co] = bias != nullptr ? bias[co] : 0.f;
-    // weights: B[tap][c8][co] = 8 fp16 of channels 8 c8 .. 8 c8 + 7 (zero past cin)
+    // weights: B[tap][c8][co] = 8 values of channels 8 c8 .. 8 c8 + 7 (zero past cin)
     for (int i = tid; i < 9 * g.cin8 * g.cout; i += kCThreads) {
         const int kb = i / g.cout, co = i - kb * g.cout;
         const int tap = kb / g.cin8, c8 = kb - tap * g.cin8;
-        const int dy = tap / 3, dx = tap - 3 * dy;
         float v[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             const int c = 8 * c8 + e;
-            v[e] = c < g.cin ? w[((static_cast<int64_t>(co) * g.cin + c) * 3 + dy) * 3 + dx] : 0.f;
+            v[e] = c < g.b.C ? w[(static_cast<int64_t>(co) * g.b.C + c) * 9 + tap] : 0.f;
         }
         *reinterpret_cast<uint4*>(B + static_cast<uint32_t>(kb) * b_chunk + co * 16) =
             make_uint4(pack2<kBf16>(v[0], v[1]), pack2<kBf16>(v[2], v[3]), pack2<kBf16>(v[4], v[5]),
                        pack2<kBf16>(v[6], v[7]));
     }
-    // the padding chunks of every staged buffer (never rewritten)
-    {
-        const int npad = (g.cin8 - g.cin8r) * g.pix_c;
-        for (int i = tid; i < g.nbuf * copies * npad; i += kCThreads) {
-            const int bc = i / npad, r = i - bc * npad;                 // bc = buffer * copies + copy
-            uint4* X = reinterpret_cast<uint4*>(base + (bc / copies) * g.xbytes);
-            X[((bc % copies) * g.cin8 + g.cin8r) * g.pix_c + r] = make_uint4(0, 0, 0, 0);
+    // the padding chunk of both staged blocks (never rewritten)
+    if (g.cin8 > g.cin8r)
+        for (int i = tid; i < 2 * g.xpix; i += kCThreads) {
+            const int bb = i / g.xpix;
+            reinterpret_cast<uint4*>(X + bb * g.xbytes)[g.cin8r * g.xpix + i - bb * g.xpix] = make_uint4(0, 0, 0, 0);
         }
-    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = S.tmem;
-    const uint32_t idesc = mma_idesc_f16(kCM, g.cout) | (kBf16 ? kIdescBf16 : 0u);
-    // the staged source pixels this thread loads: p = tid + 128 k (row, column), -1 past the block
-    int prs[kCSlots], pcs[kCSlots];
-#pragma unroll
-    for (int k = 0; k < kCSlots; ++k) {
-        const int p = tid + kCThreads * k;
-        prs[k] = p < g.pix_c ? p / g.cols_s : -1;
-        pcs[k] = p < g.pix_c ? p - prs[k] * g.cols_s : 0;
-    }
+    const uint32_t tmem = __shfl_sync(0xffffffffu, S.tmem, 0);
 
-    // the tile origin (img, y0, x0) of the unit (its first tile with pool)
-    auto epilogue = [&](int ab, int img, int y0, int x0) {
-        const int m = 32 * warp + lane;
-        const uint32_t taddr = tmem + (static_cast<uint32_t>(32 * warp) << 16) + static_cast<uint32_t>(ab * U * g.cout);
-        if (!g.pool) {
-            const int oy = y0 + m / g.wseg, ox = x0 + m % g.wseg;
-            float* yo = y + static_cast<int64_t>(img) * g.cout * hw + static_cast<int64_t>(oy) * g.W + ox;
-            for (int c0 = 0; c0 < g.cout; c0 += 32) {
-                float v[32];
-                tmem_ld32(taddr + static_cast<uint32_t>(c0), v);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    *yo = v[i] + S.bias[c0 + i];
-                    yo += hw;
-                }
-            }
-        } else {
-            // rows y0 (accumulator 0) and y0 + 1 (accumulator 1); lanes m, m + 1
-            // are the two columns.  Per pair of channels each lane sums its
-            // column's two ReLUs for both, swaps one with its neighbour and
-            // writes one: the even lane the first channel, the odd lane the
-            // second (0.25 x the 2x2 sum; the summation order is not
-            // k_relu_pool's, the operands being FP16-rounded already)
-            const int Ho = g.H / 2, Wo = g.W / 2;
-            const int64_t pw = static_cast<int64_t>(Ho) * Wo;
-            const int odd = lane & 1;
-            float* po = y + static_cast<int64_t>(img) * g.cout * pw + static_cast<int64_t>(y0 / 2) * Wo + (x0 + m) / 2 +
-                        odd * pw;
-            for (int c0 = 0; c0 < g.cout; c0 += 32) {
-                float v0[32], v1[32];
-                tmem_ld32(taddr + static_cast<uint32_t>(c0), v0);
-                tmem_ld32(taddr + static_cast<uint32_t>(g.cout + c0), v1);
-#pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    const float b0 = S.bias[c0 + i], b1 = S.bias[c0 + i + 1];
-                    const float t0 = fmaxf(v0[i] + b0, 0.f) + fmaxf(v1[i] + b0, 0.f);
-                    const float t1 = fmaxf(v0[i + 1] + b1, 0.f) + fmaxf(v1[i + 1] + b1, 0.f);
-                    const float other = __shfl_xor_sync(0xffffffffu, odd ? t0 : t1, 1);
-                    *po = 0.25f * ((odd ? t1 : t0) + other);
-                    po += 2 * pw;
-                }
+    if (warp == kCEpi + kCConv) {
+        // ---- producer
+        Ring k;
+        bool ok = true;
+        for (int64_t u = blockIdx.x; u < g.b.n_units && ok; u += gridDim.x) {
+            const BandAt o = band_at(g.b, u);
+            for (int c8 = 0; c8 < g.cin8r; ++c8, k.next(g.slots)) {
+                if (k.use > 0 && !(ok = role_wait(&S.empty[k.slot], (k.use - 1) & 1u, &S.abort, status))) break;
+                load_slot(xmap, x, g.b.H, g.b.W, g.b.vec, o.img * g.b.C + 8 * c8, min(8, g.b.C - 8 * c8), o.y0 - 1,
+                          g.b.R + 2, slot_x0(g.b, o), g.b.rp, min(8, g.b.C) * g.b.rawp,
+                          reinterpret_cast<float*>(base + k.slot * g.slotb), &S.full[k.slot]);
             }
         }
-        tc_fence_before();
-    };
-
-    uint32_t j = 0;            // blocks staged by this CTA so far
-    uint32_t ju = 0;           // units so far (accumulator set ju & 1)
-    bool have_prev = false;
-    int prev_img = 0, prev_y0 = 0, prev_x0 = 0;  // origin of the previous unit
-    bool ok = true;
-    for (int64_t u = blockIdx.x; u < g.n_units && ok; u += gridDim.x, ++ju) {
-        const int ab = static_cast<int>(ju & 1);
-        int img, y0u, x0;
-        unit_tile(g, u, 0, img, y0u, x0);
-        for (int h0 = 0; h0 < U && ok; h0 += g.sh, ++j) {
-            // one staged block per sh tiles (sh = 2: a pooled pair's rows and
-            // their halo read once); nbuf is 1 or 2: the buffer and the parity
-            // of its previous use
-            const int b = g.nbuf == 2 ? static_cast<int>(j & 1u) : 0;
-            if (j >= static_cast<uint32_t>(g.nbuf)) {
-                // the MMAs of the block staged nbuf blocks ago have read X[b]
-                const uint32_t use = g.nbuf == 2 ? (j - 2) >> 1 : j - 1;
-                ok = conv_wait(&S.x[b], use & 1u, S, status);
-                if (!ok) break;
-            }
-            const int y0 = y0u + h0;
-            uint4* X = reinterpret_cast<uint4*>(base + b * g.xbytes);
-            const float* xi = x + static_cast<int64_t>(img) * g.cin * hw;
-            int off[kCSlots];
-#pragma unroll
-            for (int k = 0; k < kCSlots; ++k) {
-                const int iy = y0 - 1 + prs[k];
-                const int ix = g.halo ? x0 - 1 + pcs[k] : pcs[k];
-                off[k] = (prs[k] >= 0 && iy >= 0 && iy < g.H && ix >= 0 && ix < g.W) ? iy * g.W + ix : -1;
-            }
-            // each source pixel is loaded once (eight channels in flight) and
-            // stored into every copy that holds it: the halo block, or the
-            // three shifted copies (copy dx holds column c + dx - 1; the
-            // wrapped column is zero)
-            for (int c8 = 0; c8 < g.cin8r; ++c8) {
-                const float* xc = xi + static_cast<int64_t>(8 * c8) * hw;
-                const int ne = g.cin - 8 * c8;
-#pragma unroll
-                for (int k = 0; k < kCSlots; ++k) {
-                    if (prs[k] < 0) continue;
-                    float v[8];
-                    const float* pe = xc + (off[k] >= 0 ? off[k] : 0);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        v[e] = (off[k] >= 0 && e < ne) ? __ldg(pe) : 0.f;
-                        pe += hw;
-                    }
-                    const uint4 q = make_uint4(pack2<kBf16>(v[0], v[1]), pack2<kBf16>(v[2], v[3]),
-                                               pack2<kBf16>(v[4], v[5]), pack2<kBf16>(v[6], v[7]));
-                    const int p = tid + kCThreads * k;
-                    if (g.halo) {
-                        X[c8 * g.pix_c + p] = q;
-                    } else {
-                        const uint4 z = make_uint4(0, 0, 0, 0);
-                        X[(1 * g.cin8 + c8) * g.pix_c + p] = q;
-                        uint4* X0 = X + c8 * g.pix_c;
-                        uint4* X2 = X + (2 * g.cin8 + c8) * g.pix_c;
-                        if (pcs[k] + 1 < g.W) X0[p + 1] = q;
-                        if (pcs[k] == 0) X0[p] = z;
-                        if (pcs[k] >= 1) X2[p - 1] = q;
-                        if (pcs[k] == g.W - 1) X2[p] = z;
-                    }
+        // no copy may be in flight when the block ends
+        for (int i = 0; i < g.slots; ++i) {
+            const uint32_t n = k.use + (i < k.slot ? 1u : 0u);            // copies into slot i
+            if (n > 0) mbar_wait_bounded(&S.full[i], (n - 1) & 1u, status);
+        }
+    } else if (warp == kCEpi + kCConv + 1) {
+        // ---- MMA issue
+        const uint32_t idesc = mma_idesc_f16(kCM, g.cout) | (kBf16 ? kIdescBf16 : 0u);
+        const uint32_t lbo = static_cast<uint32_t>(g.xpix) * 16;
+        const int spr = g.b.Ws / kCM;                                     // tiles a row (wide)
+        const uint64_t db0 = smem_desc(B, b_chunk, 128);
+        uint32_t j = 0, d = 0, use = 0;
+        bool ok = true;
+        for (int64_t u = blockIdx.x; u < g.b.n_units && ok; u += gridDim.x, ++j) {
+            const BandAt o = band_at(g.b, u);
+            const int nt = conv_tiles(g, o);
+            const uint32_t b = j & 1u;
+            ok = role_wait(&S.sfull[b], (j >> 1) & 1u, &S.abort, status);
+            if (!ok) break;
+            const uint64_t da0 = uniform64(smem_desc(X + b * g.xbytes, lbo, 128));
+            for (int t = 0; t < nt; ++t) {
+                if (use > 0 && !(ok = role_wait(&S.dempty[d], (use - 1) & 1u, &S.abort, status))) break;
+                tc_fence_after();
+                const int pix = g.wide ? U * (t / spr) * g.b.Wp + kCM * (t % spr) : kCM * t;
+                for (int h = 0; h < U; ++h) {
+                    const uint64_t dah = da0 + static_cast<uint64_t>(pix + h * g.b.Wp);       // 16-byte units: pixels
+                    if (g.cin8 == 2)
+                        conv_mmas<1>(tmem + (d * U + h) * g.cout, dah, db0, idesc, g.b.Wp, g.xpix, g.cout);
+                    else
+                        conv_mmas<2>(tmem + (d * U + h) * g.cout, dah, db0, idesc, g.b.Wp, g.xpix, g.cout);
+                }
+                mma_commit_warp(&S.dfull[d]);
+                if (++d == static_cast<uint32_t>(g.nd)) {
+                    d = 0;
+                    ++use;
                 }
             }
+            mma_commit_warp(&S.sempty[b]);
+        }
+        // every MMA this CTA issued has completed before its TMEM is released
+        mma_commit_warp(&S.drain);
+        mbar_wait_bounded(&S.drain, 0, status);
+        __syncwarp();
+    } else if (warp >= kCEpi) {
+        // ---- converters
+        const int t = tid - 32 * kCEpi;
+        const Pixels<kCPix> px(g.b, (g.b.R + 2) * g.b.Wp, t, 32 * kCConv);
+        Ring k;
+        uint32_t j = 0;
+        bool ok = true;
+        for (int64_t u = blockIdx.x; u < g.b.n_units && ok; u += gridDim.x, ++j) {
+            const BandAt o = band_at(g.b, u);
+            const uint32_t b = j & 1u;
+            // the MMAs of the band two before have read block b
+            if (j >= 2 && !(ok = role_wait(&S.sempty[b], ((j >> 1) - 1) & 1u, &S.abort, status))) break;
+            for (int c8 = 0; c8 < g.cin8r; ++c8, k.next(g.slots)) {
+                ok = role_wait(&S.full[k.slot], k.use & 1u, &S.abort, status);
+                if (!ok) break;
+                const float* raw = reinterpret_cast<const float*>(base + k.slot * g.slotb);
+                uint4* dst = reinterpret_cast<uint4*>(X + b * g.xbytes) + c8 * g.xpix;
+                const int nch = min(8, g.b.C - 8 * c8), npix = (o.rows + 2) * g.b.Wp;
+                if (!g.b.vec)
+                    stage_slot<kBf16>(g.b, o, raw, nch, dst, npix, t, 32 * kCConv);
+                else if (nch == 8)
+                    px.template stage<kBf16, true>(raw, g.b.rawp, 8, dst, npix, t, 32 * kCConv);
+                else
+                    px.template stage<kBf16, false>(raw, g.b.rawp, nch, dst, npix, t, 32 * kCConv);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&S.empty[k.slot]);
+            }
+            if (!ok) break;
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            tc_fence_before();
-            __syncthreads();
-            if (tid == 0) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&S.sfull[b]);
+        }
+    } else {
+        // ---- epilogue: set e drains tiles e, e + 2, ...
+        const uint32_t e = static_cast<uint32_t>(warp) >> 2;
+        const int quarter = warp & 3;
+        const int m = 32 * quarter + lane;
+        const int spr = g.b.Ws / kCM;
+        uint32_t T = 0;
+        bool ok = true;
+        for (int64_t u = blockIdx.x; u < g.b.n_units && ok; u += gridDim.x) {
+            const BandAt o = band_at(g.b, u);
+            const int nt = conv_tiles(g, o);
+            for (int t = 0; t < nt; ++t, ++T) {
+                if ((T & 1u) != e) continue;
+                const uint32_t d = T % static_cast<uint32_t>(g.nd), use = T / static_cast<uint32_t>(g.nd);
+                ok = role_wait(&S.dfull[d], use & 1u, &S.abort, status);
+                if (!ok) break;
                 tc_fence_after();
-                const uint8_t* Xb = base + b * g.xbytes;
-                const uint32_t lbo = static_cast<uint32_t>(g.pix_c) * 16;
-                for (int h = h0; h < h0 + g.sh; ++h) {
-                    // tile h of the unit: its rows start (h - h0) tile heights down the staged block
-                    const uint32_t d_tmem = tmem + static_cast<uint32_t>((ab * U + h) * g.cout);
-                    const uint8_t* Xh = Xb + static_cast<uint32_t>((h - h0) * g.rows * g.cols_s) * 16u;
-                    for (int tap = 0; tap < 9; ++tap) {
-                        const int dy = tap / 3, dx = tap - 3 * dy;
-                        const uint8_t* a0 = g.halo ? Xh + (dy * g.cols_s + dx) * 16
-                                                   : Xh + static_cast<uint32_t>(dx * g.cin8) * lbo + dy * g.W * 16;
-                        for (int ks = 0; ks < g.cin8 / 2; ++ks) {
-                            const uint64_t da = smem_desc(a0 + 2 * ks * lbo, lbo, 128);
-                            const uint64_t db = smem_desc(B + static_cast<uint32_t>(tap * g.cin8 + 2 * ks) * b_chunk,
-                                                          b_chunk, 128);
-                            mma_f16_id(d_tmem, da, db, idesc, (tap > 0 || ks > 0) ? 1u : 0u);
+                const uint32_t taddr =
+                    tmem + (static_cast<uint32_t>(32 * quarter) << 16) + d * static_cast<uint32_t>(U * g.cout);
+                int r, ox;
+                if (g.wide) {
+                    r = U * (t / spr);
+                    ox = o.x0 + kCM * (t % spr) + m;
+                } else {
+                    r = div_wp(g.b, kCM * t + m);
+                    ox = kCM * t + m - r * g.b.Wp;
+                }
+                if (!g.pool) {
+                    const bool in = r < o.rows && ox < g.b.W;
+                    float* yo = y + static_cast<int64_t>(o.img) * g.cout * hw + static_cast<int64_t>(o.y0 + r) * g.b.W + ox;
+                    for (int c0 = 0; c0 < g.cout; c0 += 32) {
+                        float v[32];
+                        tmem_ld32(taddr + static_cast<uint32_t>(c0), v);
+                        if (in) {
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) {
+                                *yo = v[i] + S.bias[c0 + i];
+                                yo += hw;
+                            }
+                        }
+                    }
+                } else {
+                    // rows r (accumulator 0) and r + 1 (accumulator 1); lanes m, m + 1
+                    // are the two columns.  Per pair of channels each lane sums its
+                    // column's two ReLUs for both, swaps one with its neighbour and
+                    // writes one: the even lane the first channel, the odd lane the
+                    // second (0.25 x the 2x2 sum; the summation order is not
+                    // k_relu_pool's, the operands being FP16-rounded already)
+                    const int Ho = g.b.H / 2, Wo = g.b.W / 2;
+                    const int64_t pw = static_cast<int64_t>(Ho) * Wo;
+                    const int odd = lane & 1;
+                    float* po = y + static_cast<int64_t>(o.img) * g.cout * pw +
+                                static_cast<int64_t>((o.y0 + r) / 2) * Wo + ox / 2 + odd * pw;
+                    for (int c0 = 0; c0 < g.cout; c0 += 32) {
+                        float v0[32], v1[32];
+                        tmem_ld32(taddr + static_cast<uint32_t>(c0), v0);
+                        tmem_ld32(taddr + static_cast<uint32_t>(g.cout + c0), v1);
+#pragma unroll
+                        for (int i = 0; i < 32; i += 2) {
+                            const float b0 = S.bias[c0 + i], b1 = S.bias[c0 + i + 1];
+                            const float t0 = fmaxf(v0[i] + b0, 0.f) + fmaxf(v1[i] + b0, 0.f);
+                            const float t1 = fmaxf(v0[i + 1] + b1, 0.f) + fmaxf(v1[i + 1] + b1, 0.f);
+                            const float other = __shfl_xor_sync(0xffffffffu, odd ? t0 : t1, 1);
+                            *po = 0.25f * ((odd ? t1 : t0) + other);
+                            po += 2 * pw;
                         }
                     }
                 }
-                mma_commit(&S.x[b]);
-                if (h0 + g.sh == U) mma_commit(&S.d[ab]);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&S.dempty[d]);
             }
         }
-        if (!ok) break;
-        if (have_prev) {
-            const int pab = static_cast<int>((ju - 1) & 1);
-            ok = conv_wait(&S.d[pab], ((ju - 1) >> 1) & 1u, S, status);
-            if (!ok) break;
-            tc_fence_after();
-            epilogue(pab, prev_img, prev_y0, prev_x0);
-        }
-        have_prev = true;
-        prev_img = img;
-        prev_y0 = y0u;
-        prev_x0 = x0;
-    }
-    if (ok && have_prev) {
-        const int pab = static_cast<int>((ju - 1) & 1);
-        ok = conv_wait(&S.d[pab], ((ju - 1) >> 1) & 1u, S, status);
-        if (ok) {
-            tc_fence_after();
-            epilogue(pab, prev_img, prev_y0, prev_x0);
-        }
-    }
-    // every MMA this CTA issued has completed before its TMEM is released
-    __syncthreads();
-    if (tid == 0) {
-        mma_commit(&S.drain);
-        mbar_wait_bounded(&S.drain, 0, status);
     }
     tc_fence_before();
     __syncthreads();
@@ -365,7 +505,6 @@ __global__ void __launch_bounds__(kCThreads, 4)
                      : "memory");
 }
 
-
 // ---------------------------------------------------------------- weight gradient
 // dw[k][c][ty][tx] = sum over the images and output pixels (oy, ox) of
 //   dy[k](oy, ox) * x[c](oy + ty - 1, ox + tx - 1)          (x zero outside the image)
@@ -373,73 +512,61 @@ __global__ void __launch_bounds__(kCThreads, 4)
 // (rows past cout read in-bounds data of the following chunks into
 // accumulator rows that are never read), N = the input channels rounded up to
 // 16, K = 16 pixels per MMA; BF16 operands (gradients span float32's exponent
-// range), float32 accumulation.  A tile is R image rows.  Its input rows
-// y0 - 1 .. y0 + R are staged with a zero column before each row and zeros
-// after it up to the row pitch Wp (W + 2 rounded up to 4), channel-contiguous
-// ([channel group][pixel][8 channels x 2 B], the MN-major B operand), and dy
-// on the same pitch pixel-contiguous ([8-pixel chunk][output channel][8 pixels
-// x 2 B], the K-major A operand) with zeros past each row's W pixels: output
-// pixel q = r * Wp + ox meets input pixel q + ty * Wp + tx, so tap (ty, tx) is
-// the staged input block seen from that pixel on (a descriptor offset of 16
-// bytes a pixel, no shifted copies).  The pitch being a multiple of 4, dy's
-// rows arrive as 16-byte loads, four pixels per half chunk.  The nine
-// accumulators (9 x N TMEM columns) stay in TMEM over all the CTA's tiles; the
-// staged blocks are double-buffered.  Warp 0 only issues the MMAs (one
-// thread), so tile j's MMAs are issued while warps 1.. stage tile j + 1.  Each
-// CTA then writes its partial sums and k_sum_partials adds them in CTA order
-// (the result does not depend on timing).
-constexpr int kWThreads = 512;
-constexpr int kWStage = kWThreads - 32;       // staging threads (warps 1..)
+// range), float32 accumulation.  x is staged as above (the MN-major B operand);
+// dy on the same pitch pixel-contiguous ([8-pixel chunk][output channel][8
+// pixels x 2 B], the K-major A operand) with zeros past each row's pixels.  The
+// nine accumulators (9 x N TMEM columns) stay in TMEM over all the CTA's bands.
+// The converters also sum each channel of dy (float32, before its rounding) for
+// the bias gradient.  Each CTA then writes its partial sums, which
+// k_sum_partials adds in an order that does not depend on timing.
+constexpr int kWConv = 14;                                 // converter warps (2 ..)
+constexpr int kWThreads = 32 * (kWConv + 2);
+constexpr int kWPix = 4, kWDy = 5;                         // per converter thread: staged pixels, 32-pixel steps of dy
 
 struct WgradGeom {
-    int n, C, K, H, W;
-    int R, Wp, Q;        // rows per tile, staged row pitch (W + 2 rounded up to 4), pixels per tile (R Wp rounded up to 32)
+    Band b;
+    int K;
+    int Q;               // pixels per band (R Wp rounded up to 32)
     int N;               // MMA N: C rounded up to 16
-    int cg, kg;          // channel groups of 8 staged (x: N / 8; dy: ceil(K / 8))
-    int xpix;            // staged input pixels per channel group (Q + 2 Wp + 2, rounded up to 8)
-    int nbuf;            // staged blocks: 2 (tile j + 1 stages while tile j's MMAs run), or 1 for wide rows
-    int vec4;            // dy rows load as float4 (W a multiple of 4)
-    int fold;            // C <= 8: the three column taps are one MMA (N = 32: copies of the block shifted by
-                         // tx = 0, 1, 2 pixels as channel groups 0-2, group 3 zero): 3 MMAs a K step, not 9
+    int cgr, kg;         // channel groups of 8: of x (loaded), of dy
+    int xpix;            // staged input pixels per channel group (Q + 2 Wp + 3, rounded up to 8)
+    int rpd, rawd;       // raw slot of dy: floats per row, per channel
+    int apitch;          // bytes from a staged 8-pixel chunk of dy to the next
+    int fold;            // C <= 8: the column taps are one MMA (N = 32, its groups of 8 columns the one channel
+                         // group seen 0 .. 3 pixels on, the last not read): 3 MMAs a K step, not 9
     int acc_cols;        // TMEM columns of the accumulators (9 N, or 3 x 32 folded)
-    int tiles_img;
-    int64_t n_units;
-    uint32_t xbytes, stage, smem;
+    int slots;           // raw slots
+    uint32_t slotb, xbytes, stage, smem;
     int tmem_cols;
 };
 
 struct WgradBars {
-    uint64_t x[2], drain;
+    uint64_t full[kMaxSlots], empty[kMaxSlots], sfull[2], sempty[2], drain;
     uint32_t tmem;
-    int abort;
-    int drained;
+    int abort, drained;
+    float bias[kWConv][128];
 };
 
-__device__ __forceinline__ bool wg_wait(uint64_t* bar, uint32_t parity, WgradBars& S, int* status) {
-    bool ok = true;
-    if (*reinterpret_cast<volatile int*>(&S.abort) == 0) {
-        ok = mbar_wait_bounded(bar, parity, status);
-        if (!ok) atomicExch(&S.abort, 1);
-    } else {
-        ok = false;
-    }
-    return __syncthreads_and(ok ? 1 : 0) != 0;
-}
-
 __global__ void __launch_bounds__(kWThreads, 1)
-    k_conv3x3_wgrad_tc(const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ part,
+    k_conv3x3_wgrad_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap dmap,
+                       const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ part,
                        const WgradGeom g, int* status) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ WgradBars S;
-    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int st = tid - 32;                       // staging thread index (warps 1..)
-    const int64_t hw = static_cast<int64_t>(g.H) * g.W;
-    const int kp = 8 * g.kg;
+    uint8_t* base = smem_raw + align_up_smem(smem_raw, 1024);    // raw slots, then the staged blocks
+    uint8_t* stages = base + g.slots * g.slotb;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);          // uniform: the roles are warps
 
     if (tid == 0) {
-        mbar_init(&S.x[0], 1);
-        mbar_init(&S.x[1], 1);
+        for (int i = 0; i < g.slots; ++i) {
+            mbar_init(&S.full[i], g.b.vec ? 1 : 32);
+            mbar_init(&S.empty[i], kWConv);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&S.sfull[i], kWConv);
+            mbar_init(&S.sempty[i], 1);
+        }
         mbar_init(&S.drain, 1);
         S.abort = 0;
         S.drained = 0;
@@ -451,202 +578,188 @@ __global__ void __launch_bounds__(kWThreads, 1)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    for (int i = tid; i < kWConv * 128; i += kWThreads) (&S.bias[0][0])[i] = 0.f;
+    {   // a channel group that no slot fills stays zero (the last one of an odd count)
+        const int zg = g.cgr, ng = g.fold ? 0 : g.N / 8 - zg;
+        for (int i = tid; i < 2 * ng * g.xpix; i += kWThreads) {
+            const int bb = i / (ng * g.xpix), p = i - bb * ng * g.xpix;
+            *reinterpret_cast<uint4*>(stages + bb * g.stage + (static_cast<uint32_t>(zg) * g.xpix + p) * 16u) =
+                make_uint4(0, 0, 0, 0);
+        }
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = S.tmem;
-    // BF16 A (K-major) and B (MN-major: bit 16)
-    const uint32_t idesc = mma_idesc_f16(128, g.fold ? 32 : g.N) | kIdescBf16 | (1u << 16);
-    const uint32_t lbo_a = static_cast<uint32_t>(kp) * 16;      // next 8-pixel chunk of dy
-    // B is MN-major without swizzle: there the descriptor's leading offset is
-    // the step along K (the next 8 pixels, 128 bytes on) and the stride offset
-    // the step along N (the next channel group)
-    const uint32_t sbo_b = static_cast<uint32_t>(g.xpix) * 16;
-    const int ksteps = g.Q / 16;
-    const int qw = g.Wp / 4;                       // half chunks (4 pixels) a staged row
-    if (g.fold && warp > 0)                        // channel group 3 of every stage stays zero
-        for (int i = st; i < g.nbuf * g.xpix; i += kWStage) {
-            const int bb = i / g.xpix, p = i - bb * g.xpix;
-            *reinterpret_cast<uint4*>(base + bb * g.stage + (3u * g.xpix + p) * 16u) = make_uint4(0, 0, 0, 0);
-        }
-    const int dtasks = g.Q / 4 * kp;               // (output channel, half chunk) pairs
+    const uint32_t tmem = __shfl_sync(0xffffffffu, S.tmem, 0);
 
-    uint32_t j = 0;
-    bool ok = true;
-    for (int64_t u = blockIdx.x; u < g.n_units; u += gridDim.x, ++j) {
-        const int b = g.nbuf == 2 ? static_cast<int>(j & 1u) : 0;
-        if (j >= static_cast<uint32_t>(g.nbuf)) {
-            // the MMAs of the tile staged nbuf tiles ago have read buffer b
-            const uint32_t use = g.nbuf == 2 ? (j - 2) >> 1 : j - 1;
-            ok = wg_wait(&S.x[b], use & 1u, S, status);
+    if (warp == 0) {
+        // ---- producer: per band the channel groups of x, then of dy
+        Ring k;
+        bool ok = true;
+        for (int64_t u = blockIdx.x; u < g.b.n_units && ok; u += gridDim.x) {
+            const BandAt o = band_at(g.b, u);
+            for (int p = 0; p < g.cgr + g.kg; ++p, k.next(g.slots)) {
+                if (k.use > 0 && !(ok = role_wait(&S.empty[k.slot], (k.use - 1) & 1u, &S.abort, status))) break;
+                float* slot = reinterpret_cast<float*>(base + k.slot * g.slotb);
+                if (p < g.cgr)
+                    load_slot(xmap, x, g.b.H, g.b.W, g.b.vec, o.img * g.b.C + 8 * p, min(8, g.b.C - 8 * p), o.y0 - 1,
+                              g.b.R + 2, slot_x0(g.b, o), g.b.rp, min(8, g.b.C) * g.b.rawp, slot, &S.full[k.slot]);
+                else
+                    load_slot(dmap, dy, g.b.H, g.b.W, g.b.vec, o.img * g.K + 8 * (p - g.cgr),
+                              min(8, g.K - 8 * (p - g.cgr)), o.y0, g.b.R, o.x0, g.rpd, min(8, g.K) * g.rawd, slot,
+                              &S.full[k.slot]);
+            }
+        }
+        // no copy may be in flight when the block ends
+        for (int i = 0; i < g.slots; ++i) {
+            const uint32_t n = k.use + (i < k.slot ? 1u : 0u);            // copies into slot i
+            if (n > 0) mbar_wait_bounded(&S.full[i], (n - 1) & 1u, status);
+        }
+    } else if (warp == 1) {
+        // ---- MMA issue: BF16 A (K-major) and B (MN-major: bit 16)
+        const uint32_t idesc = mma_idesc_f16(kCM, g.fold ? 32 : g.N) | kIdescBf16 | (1u << 16);
+        const uint32_t lbo_a = static_cast<uint32_t>(g.apitch);         // next 8-pixel chunk of dy
+        // B is MN-major without swizzle: there the descriptor's leading offset is
+        // the step along K (the next 8 pixels, 128 bytes on) and the stride offset
+        // the step along N (the next channel group; folded the next pixel)
+        const uint32_t sbo_b = g.fold ? 16u : static_cast<uint32_t>(g.xpix) * 16;
+        const int ksteps = g.Q / 16;
+        uint32_t j = 0;
+        bool ok = true;
+        for (int64_t u = blockIdx.x; u < g.b.n_units; u += gridDim.x, ++j) {
+            const uint32_t b = j & 1u, use = j >> 1;
+            ok = role_wait(&S.sfull[b], use & 1u, &S.abort, status);
             if (!ok) break;
-        }
-        const int img = static_cast<int>(u / g.tiles_img);
-        const int y0 = static_cast<int>(u - static_cast<int64_t>(img) * g.tiles_img) * g.R;
-        uint8_t* Xs = base + b * g.stage;
-        uint8_t* Ds = Xs + g.xbytes;
-        if (warp > 0) {
-            // input block: pixel i = r * Wp + cc is x(y0 - 1 + r, cc - 1); zero
-            // outside the image, past each row's W + 1 columns and past the R + 2
-            // staged rows.  Two channel groups (16 loads) in flight per pass.
-            const float* xi = x + static_cast<int64_t>(img) * g.C * hw;
-            if (g.fold) {
-                // C <= 8: pixel i of the block goes to copy tx at pixel i - tx
-                for (int i0 = st; i0 < g.xpix; i0 += 2 * kWStage) {
-                    float v[2][8];
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int i = i0 + h * kWStage;
-                        const int r = i / g.Wp, cc = i - r * g.Wp;
-                        const int iy = y0 - 1 + r, ix = cc - 1;
-                        const bool in = i < g.xpix && r < g.R + 2 && iy >= 0 && iy < g.H && ix >= 0 && ix < g.W;
-                        const float* px = xi + (in ? static_cast<int64_t>(iy) * g.W + ix : 0);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) v[h][e] = (in && e < g.C) ? __ldg(px + static_cast<int64_t>(e) * hw) : 0.f;
-                    }
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int i = i0 + h * kWStage;
-                        if (i >= g.xpix) continue;
-                        const uint4 q = make_uint4(pack_bf2(v[h][0], v[h][1]), pack_bf2(v[h][2], v[h][3]),
-                                                   pack_bf2(v[h][4], v[h][5]), pack_bf2(v[h][6], v[h][7]));
-#pragma unroll
-                        for (int tx = 0; tx < 3; ++tx)
-                            if (i - tx >= 0)
-                                *reinterpret_cast<uint4*>(Xs + (static_cast<uint32_t>(tx) * g.xpix + i - tx) * 16u) = q;
-                    }
-                }
-            } else
-            for (int i0 = st; i0 < g.xpix; i0 += 2 * kWStage) {
-                // two pixels a pass, each with two channel groups: 32 loads in flight
-                const float* px[2];
-                bool in[2];
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int i = i0 + h * kWStage;
-                    const int r = i / g.Wp, cc = i - r * g.Wp;
-                    const int iy = y0 - 1 + r, ix = cc - 1;
-                    in[h] = i < g.xpix && r < g.R + 2 && iy >= 0 && iy < g.H && ix >= 0 && ix < g.W;
-                    px[h] = xi + (in[h] ? static_cast<int64_t>(iy) * g.W + ix : 0);
-                }
-                for (int c8 = 0; c8 < g.cg; c8 += 2) {
-                    float v[2][16];
-#pragma unroll
-                    for (int h = 0; h < 2; ++h)
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) {
-                            const int c = 8 * c8 + e;
-                            v[h][e] = (in[h] && c < g.C) ? __ldg(px[h] + static_cast<int64_t>(c) * hw) : 0.f;
-                        }
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int i = i0 + h * kWStage;
-                        if (i >= g.xpix) continue;
-#pragma unroll
-                        for (int q = 0; q < 2; ++q)
-                            *reinterpret_cast<uint4*>(Xs + (static_cast<uint32_t>(c8 + q) * g.xpix + i) * 16u) =
-                                make_uint4(pack_bf2(v[h][8 * q], v[h][8 * q + 1]), pack_bf2(v[h][8 * q + 2], v[h][8 * q + 3]),
-                                           pack_bf2(v[h][8 * q + 4], v[h][8 * q + 5]),
-                                           pack_bf2(v[h][8 * q + 6], v[h][8 * q + 7]));
-                    }
-                }
-            }
-            // dy block: half chunk h4 (q = 4 h4 .. 4 h4 + 3, one row: the pitch is a
-            // multiple of 4) of channel k.  A warp takes 8 channels x 4 half
-            // chunks: each channel's 16 pixels are one 64-byte read, and the
-            // 8-byte stores of two chunks fill two 128-byte rows of banks.
-            const float* di = dy + static_cast<int64_t>(img) * g.K * hw + static_cast<int64_t>(y0) * g.W;
-            constexpr int kDU = 4;                 // tasks a pass: four 16-byte loads in flight
-            for (int i0 = st; i0 < dtasks; i0 += kDU * kWStage) {
-                float v[kDU][4];
-                uint32_t so[kDU];
-#pragma unroll
-                for (int t = 0; t < kDU; ++t) {
-                    const int i = i0 + t * kWStage;
-                    const int l = i & 31, w = i >> 5;
-                    const int hb = w / g.kg, kgi = w - hb * g.kg;
-                    const int k = 8 * kgi + (l >> 2);
-                    const int h4 = 4 * hb + (l & 3);
-                    const int r = h4 / qw;
-                    const int ox = 4 * (h4 - r * qw);
-                    so[t] = i < dtasks ? (static_cast<uint32_t>(h4 >> 1) * kp + k) * 16u + (h4 & 1) * 8u : ~0u;
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) v[t][e] = 0.f;
-                    if (i < dtasks && k < g.K && r < g.R && ox < g.W) {
-                        const float* pr = di + static_cast<int64_t>(k) * hw + r * g.W + ox;
-                        if (g.vec4) {
-                            const float4 f = __ldg(reinterpret_cast<const float4*>(pr));
-                            v[t][0] = f.x;
-                            v[t][1] = f.y;
-                            v[t][2] = f.z;
-                            v[t][3] = f.w;
-                        } else {
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) v[t][e] = ox + e < g.W ? __ldg(pr + e) : 0.f;
-                        }
-                    }
-                }
-#pragma unroll
-                for (int t = 0; t < kDU; ++t)
-                    if (so[t] != ~0u)
-                        *reinterpret_cast<uint2*>(Ds + so[t]) =
-                            make_uint2(pack_bf2(v[t][0], v[t][1]), pack_bf2(v[t][2], v[t][3]));
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        }
-        tc_fence_before();
-        __syncthreads();
-        if (tid == 0) {
             tc_fence_after();
-            const uint64_t da0 = smem_desc(Ds, lbo_a, 128);
-            const uint64_t db0 = smem_desc(Xs, 128, sbo_b);
+            const uint8_t* Xs = stages + b * g.stage;
+            uint64_t da = uniform64(smem_desc(Xs + g.xbytes, lbo_a, 128));
+            // descriptor addresses are in 16-byte units: one unit per staged pixel of x
+            uint64_t db = uniform64(smem_desc(Xs, 128, sbo_b));
             // K steps outer, taps inner: consecutive MMAs go to different
             // accumulators, so no MMA waits for the previous one's sum
-            for (int ks = 0; ks < ksteps; ++ks) {
-                const uint64_t da = da0 + static_cast<uint64_t>(ks) * (2u * lbo_a >> 4);
-                // descriptor addresses are in 16-byte units: one unit per staged pixel of x
-                const uint64_t dbk = db0 + static_cast<uint64_t>(16 * ks);
+            for (int ks = 0; ks < ksteps; ++ks, da += 2u * lbo_a >> 4, db += 16) {
                 const uint32_t acc = (j > 0 || ks > 0) ? 1u : 0u;
                 if (g.fold) {
-                    // one MMA per row tap: N = the three column taps x 8 channels (+ the zero group)
+                    // one MMA per row tap: N = the column taps x 8 channels
 #pragma unroll
                     for (int ty = 0; ty < 3; ++ty)
-                        mma_f16_id(tmem + static_cast<uint32_t>(32 * ty), da, dbk + static_cast<uint64_t>(ty * g.Wp),
-                                   idesc, acc);
+                        mma_f16_warp(tmem + static_cast<uint32_t>(32 * ty), da,
+                                     db + static_cast<uint64_t>(ty * g.b.Wp), idesc, acc);
                 } else {
 #pragma unroll
                     for (int tap = 0; tap < 9; ++tap) {
                         const int ty = tap / 3, tx = tap - 3 * ty;
-                        mma_f16_id(tmem + static_cast<uint32_t>(tap * g.N), da,
-                                   dbk + static_cast<uint64_t>(ty * g.Wp + tx), idesc, acc);
+                        mma_f16_warp(tmem + static_cast<uint32_t>(tap * g.N), da,
+                                     db + static_cast<uint64_t>(ty * g.b.Wp + tx), idesc, acc);
                     }
                 }
             }
-            mma_commit(&S.x[b]);
+            mma_commit_warp(&S.sempty[b]);
         }
-    }
-    // every MMA this CTA issued has completed before the accumulators are read
-    __syncthreads();
-    if (tid == 0) {
-        mma_commit(&S.drain);
-        S.drained = mbar_wait_bounded(&S.drain, 0, status) ? 1 : 0;
+        // every MMA this CTA issued has completed before the accumulators are read
+        mma_commit_warp(&S.drain);
+        const bool drained = mbar_wait_bounded(&S.drain, 0, status) && ok;
+        if (lane == 0) S.drained = drained ? 1 : 0;
+        __syncwarp();
+    } else {
+        // ---- converters
+        const int cw = warp - 2;
+        const Pixels<kWPix> px(g.b, g.xpix, tid - 64, 32 * kWConv);
+        // dy: a warp takes four channels of a group x 8 half chunks (of 4 pixels, one
+        // row: the pitch is a multiple of 4) at a time, so that the eight lanes of a
+        // 16-byte load phase read one channel's 128 bytes; the staged chunks lie 32
+        // bytes off a multiple of 128, so that the stores of a phase (two channels x
+        // four chunks) fall on different banks
+        const int kk = 4 * (cw & 1) + (lane >> 3);             // this lane's channel of the group
+        int doff[kWDy];
+#pragma unroll
+        for (int i = 0; i < kWDy; ++i) {
+            const int q = 32 * ((cw >> 1) + kWConv / 2 * i) + 4 * (lane & 7);
+            const int r = div_wp(g.b, q), ox = q - r * g.b.Wp;
+            doff[i] = r < g.b.R && ox < g.rpd ? kk * g.rawd + r * g.rpd + ox : -1;
+        }
+        const uint32_t d0 = static_cast<uint32_t>((4 * (cw >> 1) + ((lane & 7) >> 1)) * g.apitch + kk * 16 + (lane & 1) * 8);
+        Ring k;
+        uint32_t j = 0;
+        bool ok = true;
+        for (int64_t u = blockIdx.x; u < g.b.n_units && ok; u += gridDim.x, ++j) {
+            const BandAt o = band_at(g.b, u);
+            const uint32_t b = j & 1u, use = j >> 1;
+            uint8_t* Xs = stages + b * g.stage;
+            uint8_t* Ds = Xs + g.xbytes;
+            // the MMAs of the band staged in block b before have read it
+            if (use > 0 && !(ok = role_wait(&S.sempty[b], (use - 1) & 1u, &S.abort, status))) break;
+            for (int p = 0; p < g.cgr + g.kg; ++p, k.next(g.slots)) {
+                ok = role_wait(&S.full[k.slot], k.use & 1u, &S.abort, status);
+                if (!ok) break;
+                const float* raw = reinterpret_cast<const float*>(base + k.slot * g.slotb);
+                if (p < g.cgr) {
+                    uint4* dst = reinterpret_cast<uint4*>(Xs) + p * g.xpix;
+                    const int nch = min(8, g.b.C - 8 * p);
+                    const int t = tid - 64, nt = 32 * kWConv;
+                    if (!g.b.vec)
+                        stage_slot<true>(g.b, o, raw, nch, dst, g.xpix, t, nt);
+                    else if (nch == 8)
+                        px.template stage<true, true>(raw, g.b.rawp, 8, dst, g.xpix, t, nt);
+                    else
+                        px.template stage<true, false>(raw, g.b.rawp, nch, dst, g.xpix, t, nt);
+                } else {
+                    const int ch = 8 * (p - g.cgr) + kk;
+                    uint8_t* dd = Ds + d0 + (p - g.cgr) * 128;
+                    float sum = 0.f;
+#pragma unroll
+                    for (int i = 0; i < kWDy; ++i) {
+                        const int hb = (cw >> 1) + kWConv / 2 * i;
+                        if (hb >= g.Q / 32) break;
+                        float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (g.b.vec) {
+                            if (doff[i] >= 0 && ch < g.K) f = *reinterpret_cast<const float4*>(raw + doff[i]);
+                        } else {
+                            const int q = 32 * hb + 4 * (lane & 7);
+                            const int r = div_wp(g.b, q), ox = q - r * g.b.Wp;
+                            const int nx = ch < g.K && r < o.rows ? min(g.b.Ws - ox, g.b.W - o.x0 - ox) : 0;
+                            const float* pr = raw + kk * g.rawd + r * g.rpd + ox;
+                            if (nx > 0) f.x = pr[0];
+                            if (nx > 1) f.y = pr[1];
+                            if (nx > 2) f.z = pr[2];
+                            if (nx > 3) f.w = pr[3];
+                        }
+                        *reinterpret_cast<uint2*>(dd + i * (2 * kWConv * g.apitch)) =
+                            make_uint2(pack_bf2(f.x, f.y), pack_bf2(f.z, f.w));
+                        sum += (f.x + f.y) + (f.z + f.w);
+                    }
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+                    if ((lane & 7) == 0) S.bias[cw][ch] += sum;
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&S.empty[k.slot]);
+            }
+            if (!ok) break;
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&S.sfull[b]);
+        }
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (ok && S.drained) {
+    if (S.drained) {
         // warp w reads TMEM lanes 32 (w % 4) .. + 31 (output channels), 32-column
         // chunks w / 4, w / 4 + 4, ...; column t * N + c is tap t of channel c
         const int quarter = warp & 3;
         const int k = 32 * quarter + lane;
         const int cols = g.acc_cols;
-        const int64_t kc9 = static_cast<int64_t>(g.K) * g.C * 9;
+        const int64_t kc9 = static_cast<int64_t>(g.K) * g.b.C * 9;
+        float* mine = part + blockIdx.x * (kc9 + g.K);
         if (32 * quarter < g.K) {
             for (int ch = warp >> 2; 32 * ch < cols; ch += kWThreads / 128) {
                 float v[32];
                 tmem_ld32(tmem + (static_cast<uint32_t>(32 * quarter) << 16) + static_cast<uint32_t>(32 * ch), v);
                 if (k < g.K) {
-                    float* pk = part + blockIdx.x * kc9 + static_cast<int64_t>(k) * g.C * 9;
+                    float* pk = mine + static_cast<int64_t>(k) * g.b.C * 9;
 #pragma unroll
                     for (int i = 0; i < 32; ++i) {
                         const int col = 32 * ch + i;
@@ -659,10 +772,15 @@ __global__ void __launch_bounds__(kWThreads, 1)
                             t = col / g.N;
                             c = col - t * g.N;
                         }
-                        if (col < cols && t >= 0 && c < g.C) pk[c * 9 + t] = v[i];
+                        if (col < cols && t >= 0 && c < g.b.C) pk[c * 9 + t] = v[i];
                     }
                 }
             }
+        }
+        for (int c = tid; c < g.K; c += kWThreads) {
+            float s = 0.f;
+            for (int i = 0; i < kWConv; ++i) s += S.bias[i][c];
+            mine[kc9 + c] = s;
         }
     }
     tc_fence_before();
@@ -673,69 +791,177 @@ __global__ void __launch_bounds__(kWThreads, 1)
                      : "memory");
 }
 
-// out[i] = sum over b < nb (in order) of part[b * n + i]
-__global__ void k_sum_partials(const float* __restrict__ part, int nb, int64_t n, float* __restrict__ out) {
-    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        float s = 0.f;
-        for (int b = 0; b < nb; ++b) s += part[b * n + i];
-        out[i] = s;
+// sums over the nb partials (rows of n0 + n1 values) of each value, the first n0
+// into out0, the rest into out1: a CTA takes 32 values, its eight warps every
+// eighth partial each, then adds the warps' sums in order
+__global__ void __launch_bounds__(256) k_sum_partials(const float* __restrict__ part, int nb, int64_t n0, int n1,
+                                                      float* __restrict__ out0, float* __restrict__ out1) {
+    __shared__ float red[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t n = n0 + n1, i = blockIdx.x * 32ll + lane;
+    float s = 0.f;
+    if (i < n) {
+#pragma unroll 4
+        for (int b = warp; b < nb; b += 8) s += part[b * n + i];
+    }
+    red[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && i < n) {
+        for (int w = 1; w < 8; ++w) s += red[w][lane];
+        if (i < n0) out0[i] = s;
+        else out1[i - n0] = s;
     }
 }
 
-// tile geometry: the band of R rows (R dividing H) with at least 512 pixels,
-// or the tallest whose staged blocks fit (two, else one for wide rows)
-bool wgrad_geom(int n, int cin, int cout, int H, int W, WgradGeom& g) {
+// ---------------------------------------------------------------- geometries
+// bands of R rows and segments of Ws columns of n images (rows on 16-byte
+// boundaries where vec)
+void band_set(Band& b, int n, int R, int Ws) {
+    b.R = R;
+    b.Ws = Ws;
+    b.nseg = (b.W + Ws - 1) / Ws;
+    b.nband = (b.H + R - 1) / R;
+    b.Wp = (Ws + 2 + 3) / 4 * 4;
+    b.rp = b.nseg == 1 ? b.W : Ws + 8;
+    b.rawp = (R + 2) * b.rp;
+    b.wp_inv = static_cast<uint32_t>(((1ull << 32) + b.Wp - 1) / b.Wp);
+    b.n_units = static_cast<int64_t>(n) * b.nband * b.nseg;
+}
+
+// Rows per band: as many as leave three raw slots beside the staged blocks (the
+// halo rows are read and packed once per band), up to 1024 pixels (more brings
+// nothing), and few enough that every SM has two bands where the work allows.
+// Columns: whole rows where a band of two of them fits, else the longest
+// segment for which it does.  fits(R, Ws) lays the geometry out.
+template <class Fits>
+bool band_choose(Band& b, int n, int unit, int col_unit, int num_sms, Fits fits) {
+    for (int nseg = 1;; ++nseg) {
+        const int Ws = (b.W + nseg - 1) / nseg;
+        const int Wu = nseg == 1 ? b.W : (Ws + col_unit - 1) / col_unit * col_unit;
+        const int need = b.H < 2 ? 1 : 2;
+        if (fits(need, Wu)) {
+            int R = need;
+            for (int r = need + unit; r <= b.H && r * (Wu + 4) <= kBandPix; r += unit) {
+                if (static_cast<int64_t>(n) * ((b.H + r - 1) / r) * nseg < 2ll * num_sms || !fits(r, Wu)) break;
+                R = r;
+            }
+            const int nband = (b.H + R - 1) / R;
+            R = (b.H + nband - 1) / nband;         // bands of one height
+            R = (R + unit - 1) / unit * unit;
+            return fits(R < need ? need : R, Wu);
+        }
+        if (Wu <= col_unit) return fits(1, Wu);
+    }
+}
+
+int tmem_columns(int cols) { return cols <= 32 ? 32 : (cols <= 64 ? 64 : (cols <= 128 ? 128 : (cols <= 256 ? 256 : 512))); }
+
+bool conv_geom(int n, int cin, int cout, int H, int W, int pool, int num_sms, ConvGeom& g) {
+    g = ConvGeom{};
+    g.b.C = cin;
+    g.b.H = H;
+    g.b.W = W;
+    g.cout = cout;
+    g.pool = pool;
+    g.wide = W >= kCM ? 1 : 0;
+    g.cin8r = (cin + 7) / 8;
+    g.cin8 = (g.cin8r + 1) / 2 * 2;
+    const int cols = (pool ? 2 : 1) * cout;
+    g.nd = 512 / cols < 4 ? 512 / cols : 4;
+    g.tmem_cols = tmem_columns(g.nd * cols);
+    const uint32_t bbytes = 9u * static_cast<uint32_t>(g.cin8) * static_cast<uint32_t>(cout) * 16u;
+    return band_choose(g.b, n, pool ? 2 : 1, kCM, num_sms, [&](int R, int Ws) {
+        if (g.wide && (Ws % kCM != 0 || W % Ws != 0)) return false;
+        band_set(g.b, n, R, Ws);
+        if (g.b.rp > kMaxBox) return false;
+        // staged pixels; W < 128: the last tile reads on past them (rows that are not written)
+        const int last = (R * g.b.Wp + kCM - 1) / kCM * kCM + 2 * g.b.Wp + 2;
+        g.xpix = g.wide ? (R + 2) * g.b.Wp : (last > (R + 2) * g.b.Wp ? last : (R + 2) * g.b.Wp);
+        g.xbytes = static_cast<uint32_t>(g.cin8) * g.xpix * 16u;
+        g.slotb = (static_cast<uint32_t>(cin < 8 ? cin : 8) * g.b.rawp * 4u + 127u) & ~127u;
+        const uint32_t rest = 2u * g.xbytes + bbytes + 1024u;
+        if (rest + 3u * g.slotb + sizeof(ConvBars) > kSmemBudget) return false;
+        const uint32_t s = (kSmemBudget - static_cast<uint32_t>(sizeof(ConvBars)) - rest) / g.slotb;
+        g.slots = s < kMaxSlots ? static_cast<int>(s) : kMaxSlots;
+        g.off_x = g.slots * g.slotb;
+        g.off_b = g.off_x + 2u * g.xbytes;
+        g.smem = g.off_b + bbytes + 1024u;
+        return true;
+    });
+}
+
+bool wgrad_geom(int n, int cin, int cout, int H, int W, int num_sms, WgradGeom& g) {
     if (n < 1 || cin < 1 || cin > 48 || cout < 1 || cout > 128 || H < 1 || W < 1) return false;
     g = WgradGeom{};
-    g.n = n;
-    g.C = cin;
+    g.b.C = cin;
+    g.b.H = H;
+    g.b.W = W;
     g.K = cout;
-    g.H = H;
-    g.W = W;
     g.N = (cin + 15) / 16 * 16;
-    g.cg = g.N / 8;
+    g.cgr = (cin + 7) / 8;
     g.kg = (cout + 7) / 8;
-    g.Wp = (W + 2 + 3) / 4 * 4;
-    g.vec4 = W % 4 == 0 ? 1 : 0;
     g.fold = cin <= 8 ? 1 : 0;
-    const int xgroups = g.fold ? 4 : g.cg;          // staged channel groups of x
-    const uint32_t budget = 227u * 1024u;
-    g.R = 0;
-    for (int nbuf = 2; nbuf >= 1 && g.R == 0; --nbuf) {
-        for (int R = 1; R <= H; ++R) {
-            if (H % R != 0) continue;
-            const int Q = (R * g.Wp + 31) / 32 * 32;
-            const int xpix = (Q + 2 * g.Wp + 2 + 7) / 8 * 8;
-            const uint32_t xbytes = static_cast<uint32_t>(xgroups) * xpix * 16u;
-            const uint32_t dbytes = static_cast<uint32_t>(Q / 8) * 8u * g.kg * 16u;
-            const uint32_t stage = (xbytes + dbytes + 127u) & ~127u;
-            // the stages, 2 KB past the last one for the unused A rows, 1 KB alignment
-            const uint32_t smem = static_cast<uint32_t>(nbuf) * stage + 2048u + 1024u;
-            if (smem > budget) break;
-            g.R = R;
-            g.Q = Q;
-            g.xpix = xpix;
-            g.xbytes = xbytes;
-            g.stage = stage;
-            g.smem = smem;
-            g.nbuf = nbuf;
-            if (Q >= 512) break;         // 32+ K steps a tap: enough per tile
-        }
-    }
-    if (g.R == 0) return false;
-    g.tiles_img = H / g.R;
-    g.n_units = static_cast<int64_t>(n) * g.tiles_img;
+    g.apitch = 128 * g.kg + 32;
     g.acc_cols = g.fold ? 3 * 32 : 9 * g.N;
-    g.tmem_cols = g.acc_cols <= 128 ? 128 : (g.acc_cols <= 256 ? 256 : 512);
-    return g.acc_cols <= 512;
+    g.tmem_cols = tmem_columns(g.acc_cols < 128 ? 128 : g.acc_cols);
+    const uint32_t xgroups = g.fold ? 1 : g.N / 8;          // staged channel groups of x
+    auto stage_bytes = [&](int R, int Wp, int& Q, int& xpix, uint32_t& xbytes) {
+        Q = (R * Wp + 31) / 32 * 32;
+        xpix = (Q + 2 * Wp + 3 + 7) / 8 * 8;
+        xbytes = xgroups * static_cast<uint32_t>(xpix) * 16u;
+        return (xbytes + static_cast<uint32_t>(Q / 8 * g.apitch) + 127u) & ~127u;
+    };
+    {   // the widths taken: those of which one staged row of whole width fits (the rest go to the CUDA cores)
+        if (W > (1 << 16)) return false;
+        const uint32_t Wp = (W + 2 + 3) / 4 * 4, Q = (Wp + 31) / 32 * 32, xpix = (Q + 2 * Wp + 2 + 7) / 8 * 8;
+        if ((((g.fold ? 4 : xgroups) * xpix * 16u + Q * g.kg * 16u + 127u) & ~127u) + 3072u > 227u * 1024u) return false;
+    }
+    return band_choose(g.b, n, 1, 4, num_sms, [&](int R, int Ws) {
+        band_set(g.b, n, R, Ws);
+        if (g.b.rp > kMaxBox) return false;
+        g.stage = stage_bytes(R, g.b.Wp, g.Q, g.xpix, g.xbytes);
+        g.rpd = g.b.nseg == 1 ? W : Ws;
+        g.rawd = R * g.rpd;
+        const int xc = cin < 8 ? cin : 8, dc = cout < 8 ? cout : 8;
+        const int f = xc * g.b.rawp > dc * g.rawd ? xc * g.b.rawp : dc * g.rawd;
+        g.slotb = (static_cast<uint32_t>(f) * 4u + 127u) & ~127u;
+        // the blocks, 2 KB past the last one for the unused A rows, 1 KB alignment
+        const uint32_t rest = 2u * g.stage + 2048u + 1024u;
+        if (rest + 3u * g.slotb + sizeof(WgradBars) > kSmemBudget) return false;
+        const uint32_t s = (kSmemBudget - static_cast<uint32_t>(sizeof(WgradBars)) - rest) / g.slotb;
+        g.slots = s < kMaxSlots ? static_cast<int>(s) : kMaxSlots;
+        g.smem = rest + static_cast<uint32_t>(g.slots) * g.slotb;
+        return true;
+    });
 }
 
-int wgrad_grid(const WgradGeom& g, int num_sms) {
-    const int per_sm = g.tmem_cols == 512 || g.smem > 113u * 1024u ? 1 : 2;   // TMEM and shared memory allow
-    const int64_t slots = static_cast<int64_t>(per_sm) * num_sms;
-    return static_cast<int>(g.n_units < slots ? g.n_units : slots);
+int units_grid(const Band& b, int num_sms) {
+    return static_cast<int>(b.n_units < num_sms ? b.n_units : num_sms);
 }
+
+// n planes of H x W floats, boxes of bw x bh x bn
+bool encode_planes(CUtensorMap* map, const float* p, int64_t n, int H, int W, int bw, int bh, int bn) {
+    static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
+    if (encode == nullptr) {
+        cudaDriverEntryPointQueryResult q;
+        void* fn = nullptr;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) !=
+                cudaSuccess ||
+            q != cudaDriverEntryPointSuccess || fn == nullptr)
+            return false;
+        encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+    }
+    const cuuint64_t dims[3] = {static_cast<cuuint64_t>(W), static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(n)};
+    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(W) * 4, static_cast<cuuint64_t>(W) * H * 4};
+    const cuuint32_t box[3] = {static_cast<cuuint32_t>(bw), static_cast<cuuint32_t>(bh), static_cast<cuuint32_t>(bn)};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(p), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// rows that tensor copies can take
+int aligned_rows(const void* p, int W) { return W % 4 == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0 ? 1 : 0; }
 }  // namespace
 
 bool conv3x3_tc_supported(int cin, int cout, int H, int W) {
@@ -749,90 +975,45 @@ bool conv3x3_tc_pool_supported(int cin, int cout, int H, int W) {
 }
 
 cudaError_t launch_conv3x3_tc(const float* x, const float* w, const float* b, float* y, int n, int cin, int cout,
-                              int H, int W, int pool, int* status, cudaStream_t st, bool bf16) {
+                              int H, int W, int pool, int num_sms, int* status, cudaStream_t st, bool bf16) {
     if (!conv3x3_tc_supported(cin, cout, H, W)) return cudaErrorInvalidValue;
     if (pool && !conv3x3_tc_pool_supported(cin, cout, H, W)) return cudaErrorInvalidValue;
-    ConvGeom g{};
-    g.n = n;
-    g.cin = cin;
-    g.cout = cout;
-    g.H = H;
-    g.W = W;
-    g.cin8r = (cin + 7) / 8;
-    g.cin8 = (g.cin8r + 1) / 2 * 2;
-    g.halo = W >= kCM ? 1 : 0;
-    g.wseg = W >= kCM ? kCM : W;
-    g.rows = kCM / g.wseg;
-    g.cols_s = g.halo ? g.wseg + 2 : g.wseg;
-    g.nbuf = g.halo ? 2 : 1;
-    g.pool = pool ? 1 : 0;
-    g.tiles_img = static_cast<int>(static_cast<int64_t>(H) * W / kCM);
-    g.n_units = static_cast<int64_t>(n) * g.tiles_img / (pool ? 2 : 1);
-    const int cols = 2 * (pool ? 2 : 1) * cout;                   // two units of accumulators
-    g.tmem_cols = cols <= 32 ? 32 : (cols <= 64 ? 64 : (cols <= 128 ? 128 : (cols <= 256 ? 256 : 512)));
-    if (g.n_units == 0) return cudaSuccess;
+    ConvGeom g;
+    if (!conv_geom(n, cin, cout, H, W, pool ? 1 : 0, num_sms, g)) return cudaErrorInvalidValue;
+    if (g.b.n_units == 0) return cudaSuccess;
+    CUtensorMap xmap{};
+    g.b.vec = aligned_rows(x, W) &&
+              encode_planes(&xmap, x, static_cast<int64_t>(n) * cin, H, W, g.b.rp, g.b.R + 2, cin < 8 ? cin : 8);
     auto kern = bf16 ? k_conv3x3_tc<true> : k_conv3x3_tc<false>;
-    int dev = 0, sms = 0, smem_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-    cudaFuncAttributes fa{};
-    cudaError_t e = cudaFuncGetAttributes(&fa, kern);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(g.smem));
     if (e != cudaSuccess) return e;
-    // staged layout for sh tiles per block, and the CTAs per SM it allows
-    // (shared memory, registers, TMEM columns)
-    auto layout = [&](int sh) -> int {
-        g.sh = sh;
-        g.pix_c = (sh * g.rows + 2) * g.cols_s;
-        g.xbytes = static_cast<uint32_t>((g.halo ? 1 : 3) * g.cin8 * g.pix_c) * 16u;
-        g.xbytes = (g.xbytes + 127u) & ~127u;
-        g.off_b = static_cast<uint32_t>(g.nbuf) * g.xbytes;
-        g.smem = g.off_b + 9u * static_cast<uint32_t>(g.cin8) * static_cast<uint32_t>(cout) * 16u + 1024u;
-        if (g.smem > 227u * 1024u || g.pix_c > kCSlots * kCThreads) return 0;
-        const int by_smem = smem_sm / static_cast<int>(g.smem + fa.sharedSizeBytes + 1024);
-        const int regs = (fa.numRegs + 7) / 8 * 8;
-        const int by_regs = 65536 / (regs * kCThreads);
-        const int by_tmem = 512 / g.tmem_cols;
-        int ps = by_smem < by_regs ? by_smem : by_regs;
-        ps = ps < by_tmem ? ps : by_tmem;
-        return ps;
-    };
-    // a pooled pair staged once (its halo rows read once) unless that costs CTAs per SM
-    int per_sm = layout(1);
-    if (g.pool && g.halo) {
-        const int ps2 = layout(2);
-        if (ps2 < per_sm || ps2 == 0) per_sm = layout(1);
-        else per_sm = ps2;
-    }
-    if (per_sm == 0) return cudaErrorInvalidValue;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(g.smem));
-    if (e != cudaSuccess) return e;
-    const int64_t slots = static_cast<int64_t>(per_sm) * sms;
-    const int64_t grid = g.n_units < slots ? g.n_units : slots;
-    kern<<<static_cast<unsigned int>(grid), kCThreads, g.smem, st>>>(x, w, b, y, g, status);
+    kern<<<units_grid(g.b, num_sms), kCThreads, g.smem, st>>>(xmap, x, w, b, y, g, status);
     return cudaGetLastError();
 }
 
 size_t conv3x3_wgrad_tc_partials(int n, int cin, int cout, int H, int W, int num_sms) {
     WgradGeom g;
-    if (!wgrad_geom(n, cin, cout, H, W, g)) return 0;
-    return static_cast<size_t>(wgrad_grid(g, num_sms)) * cout * cin * 9;
+    if (!wgrad_geom(n, cin, cout, H, W, num_sms, g)) return 0;
+    return static_cast<size_t>(units_grid(g.b, num_sms)) * (static_cast<size_t>(cout) * cin * 9 + cout);
 }
 
-cudaError_t launch_conv3x3_wgrad_tc(const float* x, const float* dy, float* dw, int n, int cin, int cout, int H,
-                                    int W, float* partials, int num_sms, int* status, cudaStream_t st) {
+cudaError_t launch_conv3x3_wgrad_tc(const float* x, const float* dy, float* dw, float* db, int n, int cin, int cout,
+                                    int H, int W, float* partials, int num_sms, int* status, cudaStream_t st) {
     WgradGeom g;
-    if (!wgrad_geom(n, cin, cout, H, W, g) || partials == nullptr) return cudaErrorInvalidValue;
-    if (reinterpret_cast<uintptr_t>(dy) % 16 != 0) g.vec4 = 0;          // 16-byte loads need an aligned base
-    const int grid = wgrad_grid(g, num_sms);
+    if (!wgrad_geom(n, cin, cout, H, W, num_sms, g) || partials == nullptr) return cudaErrorInvalidValue;
+    CUtensorMap xmap{}, dmap{};
+    g.b.vec = aligned_rows(x, W) && aligned_rows(dy, W) &&
+              encode_planes(&xmap, x, static_cast<int64_t>(n) * cin, H, W, g.b.rp, g.b.R + 2, cin < 8 ? cin : 8) &&
+              encode_planes(&dmap, dy, static_cast<int64_t>(n) * cout, H, W, g.rpd, g.b.R, cout < 8 ? cout : 8);
+    const int grid = units_grid(g.b, num_sms);
     cudaError_t e = cudaFuncSetAttribute(k_conv3x3_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(g.smem));
     if (e != cudaSuccess) return e;
-    k_conv3x3_wgrad_tc<<<grid, kWThreads, g.smem, st>>>(x, dy, partials, g, status);
+    k_conv3x3_wgrad_tc<<<grid, kWThreads, g.smem, st>>>(xmap, dmap, x, dy, partials, g, status);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    const int64_t total = static_cast<int64_t>(cout) * cin * 9;
-    k_sum_partials<<<static_cast<unsigned int>((total + 255) / 256), 256, 0, st>>>(partials, grid, total, dw);
+    const int64_t kc9 = static_cast<int64_t>(cout) * cin * 9;
+    k_sum_partials<<<static_cast<unsigned int>((kc9 + cout + 31) / 32), 256, 0, st>>>(partials, grid, kc9, cout, dw, db);
     return cudaGetLastError();
 }
 

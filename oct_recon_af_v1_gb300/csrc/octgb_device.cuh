@@ -106,6 +106,12 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// bytes from p to the next multiple of `to` (added to a shared pointer it stays
+// one: through an integer cast the compiler would use generic accesses)
+__device__ __forceinline__ uint32_t align_up_smem(const void* p, uint32_t to) {
+    return (to - (smem_u32(p) & (to - 1u))) & (to - 1u);
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
@@ -254,6 +260,26 @@ __device__ __forceinline__ void mma_f16_id(uint32_t d_tmem, uint64_t a, uint64_t
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
+}
+
+// The same two issued by a converged warp (one elected lane, always the same):
+// control flow and operands stay uniform, so the compiler keeps the descriptors
+// in uniform registers.  Issued from a one-thread branch, every MMA first moves
+// its operands there: measured 160-235 cycles an MMA, more than a 128 x 32 x 16
+// one takes.
+__device__ __forceinline__ void mma_f16_warp(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc,
+                                             uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void mma_commit_warp(uint64_t* bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar))
+        : "memory");
 }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {

@@ -303,14 +303,14 @@ cudaError_t launch_image_norm(float* img, int n_images, int64_t per_image, cudaS
 bool conv3x3_tc_supported(int cin, int cout, int H, int W);
 bool conv3x3_tc_pool_supported(int cin, int cout, int H, int W);
 cudaError_t launch_conv3x3_tc(const float* x, const float* w, const float* b, float* y, int n, int cin, int cout,
-                              int H, int W, int pool, int* status, cudaStream_t st, bool bf16 = false);
-// weight gradient of the 3x3 convolution on the tensor cores (cnn_tc.cu; BF16
-// operands, float32 accumulation): dw (cout, cin, 3, 3) from x (n, cin, H, W)
-// and dy (n, cout, H, W).  conv3x3_wgrad_tc_partials: the float count of the
+                              int H, int W, int pool, int num_sms, int* status, cudaStream_t st, bool bf16 = false);
+// weight and bias gradients of the 3x3 convolution (cnn_tc.cu; dw on the tensor
+// cores with BF16 operands and float32 accumulation, db from dy in float32):
+// dw (cout, cin, 3, 3) and db (cout) from x (n, cin, H, W) and dy (n, cout, H, W).  conv3x3_wgrad_tc_partials: the float count of the
 // per-CTA partial sums the launch needs (0: shape not supported).
 size_t conv3x3_wgrad_tc_partials(int n, int cin, int cout, int H, int W, int num_sms);
-cudaError_t launch_conv3x3_wgrad_tc(const float* x, const float* dy, float* dw, int n, int cin, int cout, int H,
-                                    int W, float* partials, int num_sms, int* status, cudaStream_t st);
+cudaError_t launch_conv3x3_wgrad_tc(const float* x, const float* dy, float* dw, float* db, int n, int cin, int cout,
+                                    int H, int W, float* partials, int num_sms, int* status, cudaStream_t st);
 cudaError_t launch_conv3x3(const float* x, const float* w, const float* b, float* y, int Nn, int C, int K, int H,
                            int W, cudaStream_t st);
 cudaError_t launch_flip_weights(const float* w, int K, int C, float* wf, cudaStream_t st);

@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(kPThreads, 1)
                 float* __restrict__ X, int64_t n_ascans, int* status) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // tensor-copy destinations want 128-byte alignment: align the window by hand
-    PrecSmem& S = *reinterpret_cast<PrecSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    PrecSmem& S = *reinterpret_cast<PrecSmem*>(smem_raw + align_up_smem(smem_raw, 1024));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int64_t n_tiles = (n_ascans + kPM - 1) / kPM;
     const int64_t my_tiles = blockIdx.x < n_tiles ? (n_tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;

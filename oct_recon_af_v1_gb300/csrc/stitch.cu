@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kStThreads, kFZ == 128 ? 3 : 5) k_stitch_tma(c
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ uint64_t bar;
     __shared__ StitchTmaSlot slot[kMaxSeg];
-    unsigned char* sm = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);   // tensor copies: 128-byte aligned
+    unsigned char* sm = smem_raw + align_up_smem(smem_raw, 128);   // tensor copies: 128-byte aligned
     const int f = blockIdx.z;
     const int zb = blockIdx.y * kFZ;
     const int cb = (a.cblk0 + blockIdx.x) * kBlk;

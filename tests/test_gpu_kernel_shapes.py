@@ -283,3 +283,70 @@ def test_float64_form_at_the_ends_of_the_range(gpu_ctx, dtype, bscans, nx, apod)
     assert (np.abs(got - ref) <= 2.0 ** -24 * np.abs(ref) + 1e-12 * np.abs(ref).max(-1, keepdims=True)).all()
     if nx == 9:
         assert (got[:, -2:] == 0).all()
+
+
+def _offset(torch, a, shift):
+    """a on the device, its first element `shift` floats past a 16-byte boundary."""
+    buf = torch.empty(a.size + shift, device="cuda")
+    v = buf[shift:].reshape(a.shape)
+    v.copy_(torch.from_numpy(a))
+    return v
+
+
+@pytest.mark.parametrize("n,cin,cout,h,w,pool,shift", [
+    (1, 3, 32, 5, 640, 0, 0), (2, 9, 32, 7, 384, 0, 1), (1, 32, 128, 6, 1152, 1, 0), (1, 8, 32, 2, 256, 1, 3),
+    (1, 17, 32, 64, 2, 0, 0), (3, 16, 32, 33, 128, 0, 2), (1, 7, 96, 1, 256, 0, 0), (30, 24, 64, 32, 8, 0, 0),
+    (200, 3, 32, 10, 128, 1, 0)])
+def test_conv_bands(gpu_ctx, n, cin, cout, h, w, pool, shift):
+    """Bands at the ends of an image, column segments of wide rows, rows off
+    16-byte boundaries, one row or two columns: against the float64 convolution
+    of the FP16-rounded operands.  Tolerance: float32 accumulation of 9 cin
+    products, 1e-5 of the largest value per square root of their number."""
+    torch = pytest.importorskip("torch")
+    from oracle import cnn as C
+    from oct_recon_af_v1_gb300.learned import _p
+    rng = np.random.default_rng(h * w + cin)
+    x = rng.standard_normal((n, cin, h, w)).astype(np.float32)
+    wt = (rng.standard_normal((cout, cin, 3, 3)) * 0.3).astype(np.float32)
+    b = rng.standard_normal(cout).astype(np.float32)
+    keep = [0, n // 2, n - 1]                                  # images compared
+    r16 = lambda a: a.astype(np.float16).astype(np.float64)
+    ref = C.conv3x3(r16(x[keep]), r16(wt), b.astype(np.float64))
+    tol = 1e-5 * np.abs(ref).max() * np.sqrt(9 * cin)
+    if pool:
+        ref = np.maximum(ref, 0).reshape(3, cout, h // 2, 2, w // 2, 2).mean(axis=(3, 5))
+    xd, wd, bd = _offset(torch, x, shift), torch.tensor(wt, device="cuda"), torch.tensor(b, device="cuda")
+    y = torch.full((n,) + ref.shape[1:], float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    f = gpu_ctx.lib.octgb_cnn_conv3x3_relu_pool_tc if pool else gpu_ctx.lib.octgb_cnn_conv3x3_tc
+    gpu_ctx._check(f(gpu_ctx.h, _p(xd), _p(wd), _p(bd), _p(y), n, cin, cout, h, w))
+    gpu_ctx.synchronize()
+    assert torch.isfinite(y).all()
+    np.testing.assert_allclose(y[keep].cpu().numpy(), ref, rtol=0, atol=tol)
+
+
+@pytest.mark.parametrize("n,cin,cout,h,w,shift", [(1, 3, 32, 7, 640, 0), (2, 16, 40, 5, 701, 0), (1, 48, 128, 3, 130, 0),
+                                                  (2, 1, 9, 1, 260, 1), (3, 33, 8, 31, 128, 2), (200, 8, 16, 5, 4, 0),
+                                                  (1, 5, 1, 300, 1, 0), (90, 32, 32, 9, 64, 0)])
+def test_weight_gradient_bands(gpu_ctx, n, cin, cout, h, w, shift):
+    """The same for the weight and bias gradients: against the float64 sums of
+    the BF16-rounded operands' products (dw) and of dy (db).  Tolerance: float32
+    accumulation, 1e-4 of the sum of the terms' magnitudes."""
+    torch = pytest.importorskip("torch")
+    from oct_recon_af_v1_gb300.learned import _p
+    rng = np.random.default_rng(h * w + cin)
+    x = torch.tensor(rng.standard_normal((n, cin, h, w)), dtype=torch.float32)
+    dy = torch.tensor(rng.standard_normal((n, cout, h, w)), dtype=torch.float32)
+    xb, db16 = x.bfloat16().double(), dy.bfloat16().double()
+    grad = lambda a, g: torch.nn.grad.conv2d_weight(a, (cout, cin, 3, 3), g, padding=1).numpy()
+    ref, mag = grad(xb, db16), grad(xb.abs(), db16.abs())
+    xd, dyd = _offset(torch, x.numpy(), shift), _offset(torch, dy.numpy(), shift)
+    wd = torch.zeros((cout, cin, 3, 3), device="cuda")
+    dw, db = torch.full_like(wd, float("nan")), torch.full((cout,), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    gpu_ctx._check(gpu_ctx.lib.octgb_cnn_conv3x3_bwd_tc(gpu_ctx.h, _p(xd), _p(wd), _p(dyd), None, _p(dw), _p(db), None,
+                                                        n, cin, cout, h, w))
+    gpu_ctx.synchronize()
+    assert (np.abs(dw.cpu().numpy() - ref) <= 1e-4 * mag).all()
+    assert (np.abs(db.cpu().double().numpy() - dy.double().sum((0, 2, 3)).numpy())
+            <= 1e-4 * dy.double().abs().sum((0, 2, 3)).numpy()).all()
