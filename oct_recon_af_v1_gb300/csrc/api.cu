@@ -2298,12 +2298,12 @@ int octgb_cnn_conv3x3_bwd_tc(octgb_ctx* c, const float* x, const float* w, const
     return guarded(c, [&] {
         require(x && w && dy && dw && db, "NULL buffer");
         require(n >= 1 && cin >= 1 && cout >= 1 && h >= 1 && wd >= 1, "bad convolution shape");
-        const size_t parts = conv3x3_wgrad_tc_partials(n, cin, cout, h, wd, c->num_sms);
+        const size_t parts = conv3x3_wgrad_tc_partials(n, cin, cout, h, wd, false, c->num_sms);
         require(parts > 0, "tensor-core weight gradient: 1 <= cin <= 48, 1 <= cout <= 128 and a band of rows "
                            "dividing the height whose staged input fits in shared memory");
         ck(c->wgrad_part.ensure(parts * sizeof(float)), "cudaMalloc(weight-gradient partial sums)");
-        ck(launch_conv3x3_wgrad_tc(x, dy, dw, db, n, cin, cout, h, wd, c->wgrad_part.as<float>(), c->num_sms,
-                                   c->status_dev, c->stream),
+        ck(launch_conv3x3_wgrad_tc(x, dy, nullptr, dw, db, n, cin, cout, h, wd, c->wgrad_part.as<float>(),
+                                   c->num_sms, c->status_dev, c->stream),
            "tensor-core weight-gradient kernel");
         c->launches += 2;
         if (dx != nullptr) {
@@ -2319,6 +2319,23 @@ int octgb_cnn_conv3x3_bwd_tc(octgb_ctx* c, const float* x, const float* w, const
                 ck(launch_conv3x3(dy, w_scratch, nullptr, dx, n, cout, cin, h, wd, c->stream), "conv kernel");
             c->launches += 2;
         }
+    });
+}
+
+int octgb_cnn_conv3x3_pool_bwd_tc(octgb_ctx* c, const float* x, const float* y, const float* dp, float* dw, float* db,
+                                  int n, int cin, int cout, int h, int wd) {
+    return guarded(c, [&] {
+        require(x && y && dp && dw && db, "NULL buffer");
+        require(n >= 1 && cin >= 1 && cout >= 1 && h >= 1 && wd >= 1, "bad convolution shape");
+        const size_t parts = conv3x3_wgrad_tc_partials(n, cin, cout, h, wd, true, c->num_sms);
+        require(parts > 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0 && reinterpret_cast<uintptr_t>(dp) % 16 == 0,
+                "tensor-core weight gradient through ReLU + pool: as octgb_cnn_conv3x3_bwd_tc, and the height even, "
+                "the width a multiple of 8, y and dp on 16-byte boundaries");
+        ck(c->wgrad_part.ensure(parts * sizeof(float)), "cudaMalloc(weight-gradient partial sums)");
+        ck(launch_conv3x3_wgrad_tc(x, y, dp, dw, db, n, cin, cout, h, wd, c->wgrad_part.as<float>(), c->num_sms,
+                                   c->status_dev, c->stream),
+           "tensor-core weight-gradient kernel");
+        c->launches += 2;
     });
 }
 

@@ -120,10 +120,20 @@ __device__ __forceinline__ bool role_wait(uint64_t* bar, uint32_t parity, int* a
     return __all_sync(0xffffffffu, ok);
 }
 
+__device__ __forceinline__ void tensor_copy(const CUtensorMap& map, int x0, int y0, int plane, float* dst,
+                                            uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+            smem_u32(dst)),
+        "l"(reinterpret_cast<uint64_t>(&map)), "r"(x0), "r"(y0), "r"(plane), "r"(smem_u32(bar))
+        : "memory");
+}
+
 // Producer warp: nch channels from plane `plane` on, rows y0 .. y0 + rows - 1 and
 // columns x0 .. x0 + cols - 1, into a raw slot.  One tensor copy (box: the whole
 // slot, zeros outside the planes), or 4-byte copies of the part inside the image
-// where the rows are not on 16-byte boundaries.  (One bulk copy per channel and
+// where the rows are not on 16-byte boundaries; either way the slot's barrier
+// counts the 32 lanes.  (One bulk copy per channel and
 // row of 512 bytes measured 100 cycles a copy: 751 us for 1.1 GB, copies alone.)
 __device__ __forceinline__ void load_slot(const CUtensorMap& map, const float* src, int H, int W, int vec, int plane,
                                           int nch, int y0, int rows, int x0, int cols, int box_floats, float* slot,
@@ -132,11 +142,9 @@ __device__ __forceinline__ void load_slot(const CUtensorMap& map, const float* s
     if (vec) {
         if (lane == 0) {
             mbar_expect_tx(bar, static_cast<uint32_t>(box_floats) * 4u);
-            asm volatile(
-                "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], "
-                "[%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(slot)),
-                "l"(reinterpret_cast<uint64_t>(&map)), "r"(x0), "r"(y0), "r"(plane), "r"(smem_u32(bar))
-                : "memory");
+            tensor_copy(map, x0, y0, plane, slot, bar);
+        } else {
+            mbar_arrive(bar);
         }
         __syncwarp();
     } else {
@@ -287,7 +295,7 @@ __global__ void __launch_bounds__(kCThreads, 1)
 
     if (tid == 0) {
         for (int i = 0; i < g.slots; ++i) {
-            mbar_init(&S.full[i], g.b.vec ? 1 : 32);
+            mbar_init(&S.full[i], 32);
             mbar_init(&S.empty[i], kCConv);
         }
         for (int i = 0; i < 2; ++i) {
@@ -531,6 +539,8 @@ struct WgradGeom {
     int cgr, kg;         // channel groups of 8: of x (loaded), of dy
     int xpix;            // staged input pixels per channel group (Q + 2 Wp + 3, rounded up to 8)
     int rpd, rawd;       // raw slot of dy: floats per row, per channel
+    int dvec;            // dy's rows on 16-byte boundaries
+    int poff;            // floats from a slot of dy (pooled: of y) to dp
     int apitch;          // bytes from a staged 8-pixel chunk of dy to the next
     int fold;            // C <= 8: the column taps are one MMA (N = 32, its groups of 8 columns the one channel
                          // group seen 0 .. 3 pixels on, the last not read): 3 MMAs a K step, not 9
@@ -547,9 +557,14 @@ struct WgradBars {
     float bias[kWConv][128];
 };
 
+// kPool: dy is not in memory: dmap is then of the pre-activations y and pmap of the
+// gradient dp of their ReLU + 2x2 mean, and dy = y > 0 ? dp / 4 : 0 is formed while
+// it is packed (k_relu_pool_bwd's value).  That saves writing and reading dy, of
+// the first layer's 1.1 GB each at 128 images: 339 + 307 us -> 340 us.
+template <bool kPool>
 __global__ void __launch_bounds__(kWThreads, 1)
     k_conv3x3_wgrad_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap dmap,
-                       const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ part,
+                       const __grid_constant__ CUtensorMap pmap, const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ part,
                        const WgradGeom g, int* status) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ WgradBars S;
@@ -560,7 +575,7 @@ __global__ void __launch_bounds__(kWThreads, 1)
 
     if (tid == 0) {
         for (int i = 0; i < g.slots; ++i) {
-            mbar_init(&S.full[i], g.b.vec ? 1 : 32);
+            mbar_init(&S.full[i], 32);
             mbar_init(&S.empty[i], kWConv);
         }
         for (int i = 0; i < 2; ++i) {
@@ -605,8 +620,18 @@ __global__ void __launch_bounds__(kWThreads, 1)
                 if (p < g.cgr)
                     load_slot(xmap, x, g.b.H, g.b.W, g.b.vec, o.img * g.b.C + 8 * p, min(8, g.b.C - 8 * p), o.y0 - 1,
                               g.b.R + 2, slot_x0(g.b, o), g.b.rp, min(8, g.b.C) * g.b.rawp, slot, &S.full[k.slot]);
-                else
-                    load_slot(dmap, dy, g.b.H, g.b.W, g.b.vec, o.img * g.K + 8 * (p - g.cgr),
+                else if (kPool) {
+                    const int plane = o.img * g.K + 8 * (p - g.cgr), nd = min(8, g.K);
+                    if (lane == 0) {
+                        mbar_expect_tx(&S.full[k.slot], static_cast<uint32_t>(nd * (g.rawd + g.rawd / 4)) * 4u);
+                        tensor_copy(dmap, o.x0, o.y0, plane, slot, &S.full[k.slot]);
+                        tensor_copy(pmap, o.x0 / 2, o.y0 / 2, plane, slot + g.poff, &S.full[k.slot]);
+                    } else {
+                        mbar_arrive(&S.full[k.slot]);
+                    }
+                    __syncwarp();
+                } else
+                    load_slot(dmap, dy, g.b.H, g.b.W, g.dvec, o.img * g.K + 8 * (p - g.cgr),
                               min(8, g.K - 8 * (p - g.cgr)), o.y0, g.b.R, o.x0, g.rpd, min(8, g.K) * g.rawd, slot,
                               &S.full[k.slot]);
             }
@@ -672,12 +697,13 @@ __global__ void __launch_bounds__(kWThreads, 1)
         // bytes off a multiple of 128, so that the stores of a phase (two channels x
         // four chunks) fall on different banks
         const int kk = 4 * (cw & 1) + (lane >> 3);             // this lane's channel of the group
-        int doff[kWDy];
+        int doff[kWDy], poff[kWDy];
 #pragma unroll
         for (int i = 0; i < kWDy; ++i) {
             const int q = 32 * ((cw >> 1) + kWConv / 2 * i) + 4 * (lane & 7);
             const int r = div_wp(g.b, q), ox = q - r * g.b.Wp;
             doff[i] = r < g.b.R && ox < g.rpd ? kk * g.rawd + r * g.rpd + ox : -1;
+            poff[i] = g.poff + (kk * g.rawd / 2 + (r >> 1) * g.rpd + ox) / 2;
         }
         const uint32_t d0 = static_cast<uint32_t>((4 * (cw >> 1) + ((lane & 7) >> 1)) * g.apitch + kk * 16 + (lane & 1) * 8);
         Ring k;
@@ -713,8 +739,16 @@ __global__ void __launch_bounds__(kWThreads, 1)
                         const int hb = (cw >> 1) + kWConv / 2 * i;
                         if (hb >= g.Q / 32) break;
                         float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (g.b.vec) {
-                            if (doff[i] >= 0 && ch < g.K) f = *reinterpret_cast<const float4*>(raw + doff[i]);
+                        if (kPool || g.dvec) {
+                            if (doff[i] >= 0 && ch < g.K) {
+                                f = *reinterpret_cast<const float4*>(raw + doff[i]);
+                                if (kPool) {
+                                    const float2 d = *reinterpret_cast<const float2*>(raw + poff[i]);
+                                    const float g0 = 0.25f * d.x, g1 = 0.25f * d.y;
+                                    f = make_float4(f.x > 0.f ? g0 : 0.f, f.y > 0.f ? g0 : 0.f, f.z > 0.f ? g1 : 0.f,
+                                                    f.w > 0.f ? g1 : 0.f);
+                                }
+                            }
                         } else {
                             const int q = 32 * hb + 4 * (lane & 7);
                             const int r = div_wp(g.b, q), ox = q - r * g.b.Wp;
@@ -890,7 +924,8 @@ bool conv_geom(int n, int cin, int cout, int H, int W, int pool, int num_sms, Co
     });
 }
 
-bool wgrad_geom(int n, int cin, int cout, int H, int W, int num_sms, WgradGeom& g) {
+bool wgrad_geom(int n, int cin, int cout, int H, int W, bool pool, int num_sms, WgradGeom& g) {
+    if (pool && (H % 2 != 0 || W % 8 != 0)) return false;
     if (n < 1 || cin < 1 || cin > 48 || cout < 1 || cout > 128 || H < 1 || W < 1) return false;
     g = WgradGeom{};
     g.b.C = cin;
@@ -916,14 +951,17 @@ bool wgrad_geom(int n, int cin, int cout, int H, int W, int num_sms, WgradGeom& 
         const uint32_t Wp = (W + 2 + 3) / 4 * 4, Q = (Wp + 31) / 32 * 32, xpix = (Q + 2 * Wp + 2 + 7) / 8 * 8;
         if ((((g.fold ? 4 : xgroups) * xpix * 16u + Q * g.kg * 16u + 127u) & ~127u) + 3072u > 227u * 1024u) return false;
     }
-    return band_choose(g.b, n, 1, 4, num_sms, [&](int R, int Ws) {
+    return band_choose(g.b, n, pool ? 2 : 1, pool ? 8 : 4, num_sms, [&](int R, int Ws) {
+        if (pool && R % 2 != 0) return false;
         band_set(g.b, n, R, Ws);
         if (g.b.rp > kMaxBox) return false;
         g.stage = stage_bytes(R, g.b.Wp, g.Q, g.xpix, g.xbytes);
         g.rpd = g.b.nseg == 1 ? W : Ws;
         g.rawd = R * g.rpd;
         const int xc = cin < 8 ? cin : 8, dc = cout < 8 ? cout : 8;
-        const int f = xc * g.b.rawp > dc * g.rawd ? xc * g.b.rawp : dc * g.rawd;
+        g.poff = (dc * g.rawd + 31) / 32 * 32;
+        const int df = pool ? g.poff + dc * g.rawd / 4 : dc * g.rawd;
+        const int f = xc * g.b.rawp > df ? xc * g.b.rawp : df;
         g.slotb = (static_cast<uint32_t>(f) * 4u + 127u) & ~127u;
         // the blocks, 2 KB past the last one for the unused A rows, 1 KB alignment
         const uint32_t rest = 2u * g.stage + 2048u + 1024u;
@@ -991,25 +1029,32 @@ cudaError_t launch_conv3x3_tc(const float* x, const float* w, const float* b, fl
     return cudaGetLastError();
 }
 
-size_t conv3x3_wgrad_tc_partials(int n, int cin, int cout, int H, int W, int num_sms) {
+size_t conv3x3_wgrad_tc_partials(int n, int cin, int cout, int H, int W, bool pool, int num_sms) {
     WgradGeom g;
-    if (!wgrad_geom(n, cin, cout, H, W, num_sms, g)) return 0;
+    if (!wgrad_geom(n, cin, cout, H, W, pool, num_sms, g)) return 0;
     return static_cast<size_t>(units_grid(g.b, num_sms)) * (static_cast<size_t>(cout) * cin * 9 + cout);
 }
 
-cudaError_t launch_conv3x3_wgrad_tc(const float* x, const float* dy, float* dw, float* db, int n, int cin, int cout,
-                                    int H, int W, float* partials, int num_sms, int* status, cudaStream_t st) {
+cudaError_t launch_conv3x3_wgrad_tc(const float* x, const float* dy, const float* dp, float* dw, float* db, int n,
+                                    int cin, int cout, int H, int W, float* partials, int num_sms, int* status,
+                                    cudaStream_t st) {
     WgradGeom g;
-    if (!wgrad_geom(n, cin, cout, H, W, num_sms, g) || partials == nullptr) return cudaErrorInvalidValue;
-    CUtensorMap xmap{}, dmap{};
-    g.b.vec = aligned_rows(x, W) && aligned_rows(dy, W) &&
-              encode_planes(&xmap, x, static_cast<int64_t>(n) * cin, H, W, g.b.rp, g.b.R + 2, cin < 8 ? cin : 8) &&
-              encode_planes(&dmap, dy, static_cast<int64_t>(n) * cout, H, W, g.rpd, g.b.R, cout < 8 ? cout : 8);
+    const bool pool = dp != nullptr;
+    if (!wgrad_geom(n, cin, cout, H, W, pool, num_sms, g) || partials == nullptr) return cudaErrorInvalidValue;
+    const int dc = cout < 8 ? cout : 8;
+    const int64_t planes = static_cast<int64_t>(n) * cout;
+    CUtensorMap xmap{}, dmap{}, pmap{};
+    g.b.vec = aligned_rows(x, W) &&
+              encode_planes(&xmap, x, static_cast<int64_t>(n) * cin, H, W, g.b.rp, g.b.R + 2, cin < 8 ? cin : 8);
+    g.dvec = aligned_rows(dy, W) && encode_planes(&dmap, dy, planes, H, W, g.rpd, g.b.R, dc);
+    if (pool && !(g.dvec && aligned_rows(dp, W / 2) &&
+                  encode_planes(&pmap, dp, planes, H / 2, W / 2, g.rpd / 2, g.b.R / 2, dc)))
+        return cudaErrorInvalidValue;
+    const auto kern = pool ? k_conv3x3_wgrad_tc<true> : k_conv3x3_wgrad_tc<false>;
     const int grid = units_grid(g.b, num_sms);
-    cudaError_t e = cudaFuncSetAttribute(k_conv3x3_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(g.smem));
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(g.smem));
     if (e != cudaSuccess) return e;
-    k_conv3x3_wgrad_tc<<<grid, kWThreads, g.smem, st>>>(xmap, dmap, x, dy, partials, g, status);
+    kern<<<grid, kWThreads, g.smem, st>>>(xmap, dmap, pmap, x, dy, partials, g, status);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const int64_t kc9 = static_cast<int64_t>(cout) * cin * 9;

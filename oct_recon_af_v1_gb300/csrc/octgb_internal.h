@@ -306,11 +306,15 @@ cudaError_t launch_conv3x3_tc(const float* x, const float* w, const float* b, fl
                               int H, int W, int pool, int num_sms, int* status, cudaStream_t st, bool bf16 = false);
 // weight and bias gradients of the 3x3 convolution (cnn_tc.cu; dw on the tensor
 // cores with BF16 operands and float32 accumulation, db from dy in float32):
-// dw (cout, cin, 3, 3) and db (cout) from x (n, cin, H, W) and dy (n, cout, H, W).  conv3x3_wgrad_tc_partials: the float count of the
-// per-CTA partial sums the launch needs (0: shape not supported).
-size_t conv3x3_wgrad_tc_partials(int n, int cin, int cout, int H, int W, int num_sms);
-cudaError_t launch_conv3x3_wgrad_tc(const float* x, const float* dy, float* dw, float* db, int n, int cin, int cout,
-                                    int H, int W, float* partials, int num_sms, int* status, cudaStream_t st);
+// dw (cout, cin, 3, 3) and db (cout) from x (n, cin, H, W) and dy (n, cout, H, W).
+// With dp (n, cout, H/2, W/2; H even, W a multiple of 8, dy and dp 16-byte
+// aligned) dy is the pre-activation of a ReLU + 2x2 mean whose gradient is dp.
+// conv3x3_wgrad_tc_partials: the float count of the per-CTA partial sums the
+// launch needs (0: shape not supported).
+size_t conv3x3_wgrad_tc_partials(int n, int cin, int cout, int H, int W, bool pool, int num_sms);
+cudaError_t launch_conv3x3_wgrad_tc(const float* x, const float* dy, const float* dp, float* dw, float* db, int n,
+                                    int cin, int cout, int H, int W, float* partials, int num_sms, int* status,
+                                    cudaStream_t st);
 cudaError_t launch_conv3x3(const float* x, const float* w, const float* b, float* y, int Nn, int C, int K, int H,
                            int W, cudaStream_t st);
 cudaError_t launch_flip_weights(const float* w, int K, int C, float* wf, cudaStream_t st);

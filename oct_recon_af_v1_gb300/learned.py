@@ -153,7 +153,8 @@ class BetaFocusNet:
                  "dout": torch.empty((n, 2), dtype=torch.float32, device=dev),
                  "dh": torch.empty((n, self.hidden), dtype=torch.float32, device=dev),
                  "dflat": torch.empty((n, self.flat), dtype=torch.float32, device=dev),
-                 "dpre": [torch.empty_like(t) for t in pre],
+                 "dpre": [None if i == 0 and self._fused_first() else torch.empty_like(t)
+                          for i, t in enumerate(pre)],
                  "dpooled": [torch.empty_like(t) for t in pooled[:-1]]}
             self._acts[n] = b
         return b
@@ -164,6 +165,11 @@ class BetaFocusNet:
         if not (1 <= cin <= 32 and 32 <= cout <= 128 and cout % 32 == 0):
             return False
         return w % 128 == 0 if w >= 128 else (128 % w == 0 and h % (128 // w) == 0)
+
+    def _fused_first(self) -> bool:
+        """The first layer's gradient straight from its pre-activations
+        (octgb_cnn_conv3x3_pool_bwd_tc: rows of a multiple of 8)."""
+        return self.train_tensor_cores and self.img % 8 == 0
 
     def forward(self, x, tensor_cores: bool = False, fuse_pool=None):
         """x: (n, in_ch, img, img) float32 CUDA tensor -> (n, 2) predictions (a
@@ -224,9 +230,16 @@ class BetaFocusNet:
         h = self.img >> (len(self.chans) - 2)
         for i in reversed(range(len(self.chans) - 1)):
             cin, cout = self.chans[i], self.chans[i + 1]
+            xin = self._x if i == 0 else b["pooled"][i - 1]
+            if i == 0 and self._fused_first():
+                # no gradient of the input: ReLU, pooling and the sums in one kernel
+                self._check(self.lib.octgb_cnn_conv3x3_pool_bwd_tc(self.ctx.h, _p(xin), _p(b["pre"][0]), _p(dp),
+                                                                   _p(g[0]), _p(g[1]), n, cin, cout, h, h))
+                break
+            if b["dpre"][i] is None:                        # train_tensor_cores was switched off since
+                b["dpre"][i] = b["pre"][i].new_empty(b["pre"][i].shape)
             self._check(self.lib.octgb_cnn_relu_pool_bwd(self.ctx.h, _p(dp), _p(b["pre"][i]), _p(b["dpre"][i]),
                                                          n * cout, h, h))
-            xin = self._x if i == 0 else b["pooled"][i - 1]
             dx = None if i == 0 else b["dpooled"][i - 1]
             bwd = self.lib.octgb_cnn_conv3x3_bwd_tc if self.train_tensor_cores else self.lib.octgb_cnn_conv3x3_bwd
             self._check(bwd(self.ctx.h, _p(xin), _p(self.params[2 * i]), _p(b["dpre"][i]), _p(dx), _p(g[2 * i]),

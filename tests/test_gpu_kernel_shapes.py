@@ -350,3 +350,30 @@ def test_weight_gradient_bands(gpu_ctx, n, cin, cout, h, w, shift):
     assert (np.abs(dw.cpu().numpy() - ref) <= 1e-4 * mag).all()
     assert (np.abs(db.cpu().double().numpy() - dy.double().sum((0, 2, 3)).numpy())
             <= 1e-4 * dy.double().abs().sum((0, 2, 3)).numpy()).all()
+
+
+@pytest.mark.parametrize("n,cin,cout,h,w,shift", [(1, 3, 32, 6, 640, 0), (2, 16, 40, 2, 264, 1), (3, 33, 9, 10, 128, 0),
+                                                  (90, 5, 1, 8, 8, 0), (1, 48, 128, 4, 136, 0), (130, 3, 32, 14, 128, 2)])
+def test_weight_gradient_through_pool(gpu_ctx, n, cin, cout, h, w, shift):
+    """dy = y > 0 ? dp / 4 : 0 formed inside the kernel: the same comparison
+    and tolerance as test_weight_gradient_bands (x alone off 16-byte boundaries)."""
+    torch = pytest.importorskip("torch")
+    from oct_recon_af_v1_gb300.learned import _p
+    rng = np.random.default_rng(h * w + cin)
+    x = torch.tensor(rng.standard_normal((n, cin, h, w)), dtype=torch.float32)
+    y = torch.tensor(rng.standard_normal((n, cout, h, w)), dtype=torch.float32)
+    y[:, :, ::3, ::5] = 0.0
+    dp = torch.tensor(rng.standard_normal((n, cout, h // 2, w // 2)), dtype=torch.float32)
+    dy = torch.where(y > 0, 0.25 * dp.repeat_interleave(2, 2).repeat_interleave(2, 3), 0.0)
+    xb, dyb = x.bfloat16().double(), dy.bfloat16().double()
+    grad = lambda a, g: torch.nn.grad.conv2d_weight(a, (cout, cin, 3, 3), g, padding=1).numpy()
+    ref, mag = grad(xb, dyb), grad(xb.abs(), dyb.abs())
+    xd, yd, dpd = _offset(torch, x.numpy(), shift), y.cuda(), dp.cuda()
+    dw, db = torch.full((cout, cin, 3, 3), float("nan"), device="cuda"), torch.full((cout,), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    gpu_ctx._check(gpu_ctx.lib.octgb_cnn_conv3x3_pool_bwd_tc(gpu_ctx.h, _p(xd), _p(yd), _p(dpd), _p(dw), _p(db), n, cin,
+                                                             cout, h, w))
+    gpu_ctx.synchronize()
+    assert (np.abs(dw.cpu().numpy() - ref) <= 1e-4 * mag).all()
+    assert (np.abs(db.cpu().double().numpy() - dy.double().sum((0, 2, 3)).numpy())
+            <= 1e-4 * dy.double().abs().sum((0, 2, 3)).numpy()).all()
