@@ -413,6 +413,11 @@ int octgb_cnn_conv3x3_tc(octgb_ctx *ctx, const float *x, const float *w, const f
  * even. */
 int octgb_cnn_conv3x3_relu_pool_tc(octgb_ctx *ctx, const float *x, const float *w, const float *b, float *p, int n,
                                    int cin, int cout, int h, int wd);
+/* Both: octgb_cnn_conv3x3_tc into y and octgb_cnn_relu_pool of it into p, bit
+ * for bit, in one kernel (the forward pass of training).  Shapes as
+ * octgb_cnn_conv3x3_relu_pool_tc. */
+int octgb_cnn_conv3x3_keep_relu_pool_tc(octgb_ctx *ctx, const float *x, const float *w, const float *b, float *y,
+                                        float *p, int n, int cin, int cout, int h, int wd);
 /* Gradients of octgb_cnn_conv3x3: dw, db from dy and x; dx (optional) with
  * w_scratch (cout * cin * 9 floats) for the flipped kernel. */
 int octgb_cnn_conv3x3_bwd(octgb_ctx *ctx, const float *x, const float *w, const float *dy, float *dx, float *dw,

@@ -83,6 +83,8 @@ SIGNATURES = {
                                   c_int]),
     "octgb_cnn_conv3x3_relu_pool_tc": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                   c_int]),
+    "octgb_cnn_conv3x3_keep_relu_pool_tc": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
+                                                    c_int, c_int, c_int, c_int]),
     "octgb_cnn_conv3x3_bwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                       c_void_p, c_int, c_int, c_int, c_int, c_int]),
     "octgb_cnn_conv3x3_bwd_tc": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,

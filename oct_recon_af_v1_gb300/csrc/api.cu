@@ -2254,24 +2254,38 @@ int octgb_cnn_conv3x3_tc(octgb_ctx* c, const float* x, const float* w, const flo
         require(conv3x3_tc_supported(cin, cout, h, wd),
                 "tensor-core convolution: 1 <= cin <= 32, cout a multiple of 32 up to 128, and the width a "
                 "multiple of 128 or a divisor of 128 whose row count divides the height");
-        ck(launch_conv3x3_tc(x, w, b, y, n, cin, cout, h, wd, 0, c->num_sms, c->status_dev, c->stream),
+        ck(launch_conv3x3_tc(x, w, b, y, nullptr, n, cin, cout, h, wd, c->num_sms, c->status_dev, c->stream),
            "tensor-core conv kernel");
         c->launches++;
     });
 }
 
-int octgb_cnn_conv3x3_relu_pool_tc(octgb_ctx* c, const float* x, const float* w, const float* b, float* p, int n,
-                                   int cin, int cout, int h, int wd) {
+namespace {
+int conv_relu_pool_tc(octgb_ctx* c, const float* x, const float* w, const float* b, float* y, float* p, int n, int cin,
+                      int cout, int h, int wd) {
     return guarded(c, [&] {
-        require(x && w && p, "NULL buffer");
         require(n >= 1 && h >= 1 && wd >= 1, "bad convolution shape");
         require(conv3x3_tc_pool_supported(cin, cout, h, wd),
                 "fused tensor-core convolution + pool: 1 <= cin <= 32, cout a multiple of 32 up to 128, the width "
                 "a multiple of 128 and the height even");
-        ck(launch_conv3x3_tc(x, w, b, p, n, cin, cout, h, wd, 1, c->num_sms, c->status_dev, c->stream),
+        ck(launch_conv3x3_tc(x, w, b, y, p, n, cin, cout, h, wd, c->num_sms, c->status_dev, c->stream),
            "tensor-core conv + pool kernel");
         c->launches++;
     });
+}
+}  // namespace
+
+int octgb_cnn_conv3x3_relu_pool_tc(octgb_ctx* c, const float* x, const float* w, const float* b, float* p, int n,
+                                   int cin, int cout, int h, int wd) {
+    if (x == nullptr || w == nullptr || p == nullptr) return guarded(c, [] { require(false, "NULL buffer"); });
+    return conv_relu_pool_tc(c, x, w, b, nullptr, p, n, cin, cout, h, wd);
+}
+
+int octgb_cnn_conv3x3_keep_relu_pool_tc(octgb_ctx* c, const float* x, const float* w, const float* b, float* y,
+                                        float* p, int n, int cin, int cout, int h, int wd) {
+    if (x == nullptr || w == nullptr || y == nullptr || p == nullptr)
+        return guarded(c, [] { require(false, "NULL buffer"); });
+    return conv_relu_pool_tc(c, x, w, b, y, p, n, cin, cout, h, wd);
 }
 
 int octgb_cnn_conv3x3_bwd(octgb_ctx* c, const float* x, const float* w, const float* dy, float* dx, float* dw,
@@ -2312,8 +2326,8 @@ int octgb_cnn_conv3x3_bwd_tc(octgb_ctx* c, const float* x, const float* w, const
             // the data gradient is the convolution of dy with the flipped kernel
             // (cout -> cin channels): BF16 tensor cores where the shape allows
             if (conv3x3_tc_supported(cout, cin, h, wd))
-                ck(launch_conv3x3_tc(dy, w_scratch, nullptr, dx, n, cout, cin, h, wd, 0, c->num_sms, c->status_dev,
-                                     c->stream, true),
+                ck(launch_conv3x3_tc(dy, w_scratch, nullptr, dx, nullptr, n, cout, cin, h, wd, c->num_sms,
+                                     c->status_dev, c->stream, true),
                    "tensor-core conv kernel");
             else
                 ck(launch_conv3x3(dy, w_scratch, nullptr, dx, n, cout, cin, h, wd, c->stream), "conv kernel");

@@ -243,7 +243,7 @@ struct ConvGeom {
     int cout;
     int cin8, cin8r;   // channel chunks of 8, even (chunks past cin8r are zero)
     int xpix;          // pixels per chunk of a staged block
-    int pool, wide;    // wide: W >= 128
+    int pool, wide;    // wide: W >= 128; pool: 1 = ReLU + mean only, 2 = beside the pre-activations
     int slots, nd;     // raw slots, accumulators
     uint32_t slotb, xbytes, off_x, off_b, smem;
     int tmem_cols;
@@ -281,7 +281,7 @@ __device__ __forceinline__ void conv_mmas(uint32_t d, uint64_t a, uint64_t b, ui
 template <bool kBf16>
 __global__ void __launch_bounds__(kCThreads, 1)
     k_conv3x3_tc(const __grid_constant__ CUtensorMap xmap, const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
-                 float* __restrict__ y, const ConvGeom g, int* status) {
+                 float* __restrict__ y, float* __restrict__ pooled, const ConvGeom g, int* status) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ ConvBars S;
     uint8_t* base = smem_raw + align_up_smem(smem_raw, 1024);
@@ -474,28 +474,51 @@ __global__ void __launch_bounds__(kCThreads, 1)
                     }
                 } else {
                     // rows r (accumulator 0) and r + 1 (accumulator 1); lanes m, m + 1
-                    // are the two columns.  Per pair of channels each lane sums its
-                    // column's two ReLUs for both, swaps one with its neighbour and
-                    // writes one: the even lane the first channel, the odd lane the
-                    // second (0.25 x the 2x2 sum; the summation order is not
-                    // k_relu_pool's, the operands being FP16-rounded already)
+                    // are the two columns.  Per pair of channels a lane swaps values
+                    // with its neighbour and writes one mean: the even lane the first
+                    // channel's, the odd lane the second's.  Alone, the mean sums
+                    // columns first (one swap); beside the pre-activations it is
+                    // k_relu_pool's, rows first, bit for bit (a backward pass and
+                    // later layers see the same values as from the two kernels).
                     const int Ho = g.b.H / 2, Wo = g.b.W / 2;
                     const int64_t pw = static_cast<int64_t>(Ho) * Wo;
                     const int odd = lane & 1;
-                    float* po = y + static_cast<int64_t>(o.img) * g.cout * pw +
+                    float* po = pooled + static_cast<int64_t>(o.img) * g.cout * pw +
                                 static_cast<int64_t>((o.y0 + r) / 2) * Wo + ox / 2 + odd * pw;
+                    float* yo = y + static_cast<int64_t>(o.img) * g.cout * hw + static_cast<int64_t>(o.y0 + r) * g.b.W + ox;
                     for (int c0 = 0; c0 < g.cout; c0 += 32) {
                         float v0[32], v1[32];
                         tmem_ld32(taddr + static_cast<uint32_t>(c0), v0);
                         tmem_ld32(taddr + static_cast<uint32_t>(g.cout + c0), v1);
+                        if (g.pool == 1) {
 #pragma unroll
-                        for (int i = 0; i < 32; i += 2) {
-                            const float b0 = S.bias[c0 + i], b1 = S.bias[c0 + i + 1];
-                            const float t0 = fmaxf(v0[i] + b0, 0.f) + fmaxf(v1[i] + b0, 0.f);
-                            const float t1 = fmaxf(v0[i + 1] + b1, 0.f) + fmaxf(v1[i + 1] + b1, 0.f);
-                            const float other = __shfl_xor_sync(0xffffffffu, odd ? t0 : t1, 1);
-                            *po = 0.25f * ((odd ? t1 : t0) + other);
-                            po += 2 * pw;
+                            for (int i = 0; i < 32; i += 2) {
+                                const float b0 = S.bias[c0 + i], b1 = S.bias[c0 + i + 1];
+                                const float t0 = fmaxf(v0[i] + b0, 0.f) + fmaxf(v1[i] + b0, 0.f);
+                                const float t1 = fmaxf(v0[i + 1] + b1, 0.f) + fmaxf(v1[i + 1] + b1, 0.f);
+                                const float other = __shfl_xor_sync(0xffffffffu, odd ? t0 : t1, 1);
+                                *po = 0.25f * ((odd ? t1 : t0) + other);
+                                po += 2 * pw;
+                            }
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 32; i += 2) {
+                                float a[2][2];                         // [channel][row]
+#pragma unroll
+                                for (int e = 0; e < 2; ++e) {
+                                    const float bb = S.bias[c0 + i + e];
+                                    const float p0 = v0[i + e] + bb, p1 = v1[i + e] + bb;
+                                    yo[0] = p0;
+                                    yo[g.b.W] = p1;
+                                    yo += hw;
+                                    a[e][0] = fmaxf(p0, 0.f);
+                                    a[e][1] = fmaxf(p1, 0.f);
+                                }
+                                const float s0 = __shfl_xor_sync(0xffffffffu, odd ? a[0][0] : a[1][0], 1);
+                                const float s1 = __shfl_xor_sync(0xffffffffu, odd ? a[0][1] : a[1][1], 1);
+                                *po = 0.25f * (((odd ? a[1][0] : a[0][0]) + s0) + ((odd ? a[1][1] : a[0][1]) + s1));
+                                po += 2 * pw;
+                            }
                         }
                     }
                 }
@@ -1012,12 +1035,13 @@ bool conv3x3_tc_pool_supported(int cin, int cout, int H, int W) {
     return conv3x3_tc_supported(cin, cout, H, W) && W >= kCM && H % 2 == 0;
 }
 
-cudaError_t launch_conv3x3_tc(const float* x, const float* w, const float* b, float* y, int n, int cin, int cout,
-                              int H, int W, int pool, int num_sms, int* status, cudaStream_t st, bool bf16) {
+cudaError_t launch_conv3x3_tc(const float* x, const float* w, const float* b, float* y, float* pooled, int n, int cin,
+                              int cout, int H, int W, int num_sms, int* status, cudaStream_t st, bool bf16) {
     if (!conv3x3_tc_supported(cin, cout, H, W)) return cudaErrorInvalidValue;
+    const int pool = pooled == nullptr ? 0 : (y == nullptr ? 1 : 2);
     if (pool && !conv3x3_tc_pool_supported(cin, cout, H, W)) return cudaErrorInvalidValue;
     ConvGeom g;
-    if (!conv_geom(n, cin, cout, H, W, pool ? 1 : 0, num_sms, g)) return cudaErrorInvalidValue;
+    if (!conv_geom(n, cin, cout, H, W, pool, num_sms, g)) return cudaErrorInvalidValue;
     if (g.b.n_units == 0) return cudaSuccess;
     CUtensorMap xmap{};
     g.b.vec = aligned_rows(x, W) &&
@@ -1025,7 +1049,7 @@ cudaError_t launch_conv3x3_tc(const float* x, const float* w, const float* b, fl
     auto kern = bf16 ? k_conv3x3_tc<true> : k_conv3x3_tc<false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(g.smem));
     if (e != cudaSuccess) return e;
-    kern<<<units_grid(g.b, num_sms), kCThreads, g.smem, st>>>(xmap, x, w, b, y, g, status);
+    kern<<<units_grid(g.b, num_sms), kCThreads, g.smem, st>>>(xmap, x, w, b, y, pooled, g, status);
     return cudaGetLastError();
 }
 

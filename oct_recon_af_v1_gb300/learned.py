@@ -189,10 +189,14 @@ class BetaFocusNet:
         h = self.img
         for i, (cin, cout) in enumerate(zip(self.chans[:-1], self.chans[1:])):
             w, bias = self.params[2 * i], self.params[2 * i + 1]
-            if fuse_pool and tensor_cores and self.tc_supported(cin, cout, h, h) and h >= 128 and h % 2 == 0:
-                # convolution, ReLU and pooling in one kernel (no pre-activations)
-                self._check(self.lib.octgb_cnn_conv3x3_relu_pool_tc(self.ctx.h, _p(cur), _p(w), _p(bias),
-                                                                    _p(b["pooled"][i]), n, cin, cout, h, h))
+            if tensor_cores and self.tc_supported(cin, cout, h, h) and h >= 128 and h % 2 == 0:
+                # convolution, ReLU and pooling in one kernel (fuse_pool: no pre-activations)
+                if fuse_pool:
+                    self._check(self.lib.octgb_cnn_conv3x3_relu_pool_tc(self.ctx.h, _p(cur), _p(w), _p(bias),
+                                                                        _p(b["pooled"][i]), n, cin, cout, h, h))
+                else:
+                    self._check(self.lib.octgb_cnn_conv3x3_keep_relu_pool_tc(
+                        self.ctx.h, _p(cur), _p(w), _p(bias), _p(b["pre"][i]), _p(b["pooled"][i]), n, cin, cout, h, h))
             else:
                 conv = self.lib.octgb_cnn_conv3x3
                 if tensor_cores and self.tc_supported(cin, cout, h, h):

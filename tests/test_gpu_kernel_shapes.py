@@ -377,3 +377,23 @@ def test_weight_gradient_through_pool(gpu_ctx, n, cin, cout, h, w, shift):
     assert (np.abs(dw.cpu().numpy() - ref) <= 1e-4 * mag).all()
     assert (np.abs(db.cpu().double().numpy() - dy.double().sum((0, 2, 3)).numpy())
             <= 1e-4 * dy.double().abs().sum((0, 2, 3)).numpy()).all()
+
+
+@pytest.mark.parametrize("n,cin,cout,h,w", [(1, 3, 32, 2, 128), (2, 32, 64, 6, 384), (1, 9, 128, 4, 256)])
+def test_conv_with_pool_beside_pre_activations(gpu_ctx, n, cin, cout, h, w):
+    """The one kernel's two outputs equal the two kernels' exactly (the same
+    sums in the same order)."""
+    torch = pytest.importorskip("torch")
+    from oct_recon_af_v1_gb300.learned import _p
+    rng = np.random.default_rng(w + cin)
+    x, wt, b = (torch.tensor(rng.standard_normal(s), dtype=torch.float32, device="cuda")
+                for s in ((n, cin, h, w), (cout, cin, 3, 3), (cout,)))
+    y, y2 = (torch.full((n, cout, h, w), float("nan"), device="cuda") for _ in range(2))
+    p, p2 = (torch.full((n, cout, h // 2, w // 2), float("nan"), device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    L, c = gpu_ctx.lib, gpu_ctx
+    c._check(L.octgb_cnn_conv3x3_tc(c.h, _p(x), _p(wt), _p(b), _p(y), n, cin, cout, h, w))
+    c._check(L.octgb_cnn_relu_pool(c.h, _p(y), _p(p), n * cout, h, w))
+    c._check(L.octgb_cnn_conv3x3_keep_relu_pool_tc(c.h, _p(x), _p(wt), _p(b), _p(y2), _p(p2), n, cin, cout, h, w))
+    c.synchronize()
+    assert torch.isfinite(y).all() and torch.equal(y, y2) and torch.equal(p, p2)
