@@ -361,7 +361,7 @@ void run_spectral(octgb_ctx* c, const void* raw, int dtype, int loc, int B, int 
 // The lines of a batch (any LineMode; exact: kModeReal with the exact
 // background) into `out` (device, 16-byte aligned).
 void run_lines(octgb_ctx* c, const void* raw, int dtype, int loc, int B, int interf, int apod, int mode, float* out_dev,
-               const double* hann = nullptr, const float2* hann2 = nullptr, bool exact = false) {
+               const double* hann = nullptr, const float* hann2 = nullptr, bool exact = false) {
     require_spectral(c);
     if (B == 0) return;
     const int64_t n = static_cast<int64_t>(B) * (interf - apod);
@@ -1629,15 +1629,15 @@ int octgb_disp_load(octgb_ctx* c, const void* raw, int dtype, int loc, int n_bsc
         std::vector<double> hw(kN * 2);
         for (int j = 0; j < kN; ++j) {
             const float hi = static_cast<float>(hann[j]);
-            reinterpret_cast<float*>(hw.data() + kN)[2 * j] = hi;
-            reinterpret_cast<float*>(hw.data() + kN)[2 * j + 1] = static_cast<float>(hann[j] - static_cast<double>(hi));
+            reinterpret_cast<float*>(hw.data() + kN)[j] = hi;
+            reinterpret_cast<float*>(hw.data() + kN)[kN + j] = static_cast<float>(hann[j] - static_cast<double>(hi));
             hw[j] = hann[j];
         }
         ck(c->disp_hann.ensure(kN * 2 * sizeof(double)), "cudaMalloc(hann)");
         ck(cudaMemcpyAsync(c->disp_hann.p, hw.data(), hw.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream),
            "H2D hann");
         run_lines(c, raw, dtype, loc, B, interf, apod, kModeLinHann, c->disp_x.as<float>(), c->disp_hann.as<double>(),
-                  reinterpret_cast<const float2*>(c->disp_hann.as<double>() + kN));
+                  reinterpret_cast<const float*>(c->disp_hann.as<double>() + kN));
         check_status(c);
         c->disp_b = n_bscans;
         c->disp_rep = rep;

@@ -88,33 +88,32 @@ __device__ __forceinline__ void raw4<float>(const float* p, float2& a, float2& b
     b = make_float2(u.z, u.w);
 }
 
-// float32(float64(x) * h) for a float64 h given as float32 hi + lo (h2.x +
-// h2.y, the rest below 2^-48 |h|) without the FP64 pipe: p + e1 = x * hi
+// float32(float64(x) * h), two samples at a time, for float64 h given as float32
+// hi + lo (the rest below 2^-48 |h|) without the FP64 pipe: p + e1 = x * hi
 // exactly (fma), q = x lo + e1 (one rounding), o = p + q rounded once.  The
 // exact product differs from p + q by < 2^-46 |o|; when p + q lies more than
 // 2^-40 |o| from a float32 rounding boundary (r = (p + q) - o exactly, by
-// Fast2Sum), both the product and its float64 rounding round to o.  Otherwise
-// (about one sample in 65 000), and for powers of two (asymmetric boundaries)
-// and tiny values, the float64 product is formed as the reference does.  A
-// window value of exactly zero (the Hann window's end points) gives the exact
-// product x * 0 (signed zero, or NaN) in both forms and needs no float64 step:
-// without this case the two warps holding the end points took the float64 path
-// for every A-scan.
-// The caller forms the float64 product for the lanes whose `safe` is false,
+// Fast2Sum), both the product and its float64 rounding round to o.  |o| of
+// exponent e has its boundaries 2^(e-24) away, a power of two the lower one half
+// as far (hence the exponent of the bits - 1, for both), and 2^-15 of that
+// covers 2^-40 |o|: safe when |r| < 2^(e-24) (1 - 2^-15).  Otherwise (about one
+// sample in 33 000), and for tiny, infinite and NaN values, the float64 product is
+// formed as the reference does: by the caller for the lanes whose `safe` is false,
 // behind a warp vote, so the FP64 pipe only runs in the rare warps that need it.
-__device__ __forceinline__ float mul_window(float x, float2 h2, bool& safe) {
-    const float p = x * h2.x;
-    const float e1 = fmaf(x, h2.x, -p);
-    const float q = fmaf(x, h2.y, e1);
-    const float o = p + q;
-    const float r = q - (o - p);
-    const float ao = fabsf(o);
-    const int bits = __float_as_int(ao);
-    const float half_ulp = __int_as_float((bits & 0x7f800000) - (24 << 23));
-    const bool zero_h = h2.x == 0.f && h2.y == 0.f;
-    safe = zero_h || (ao > 1e-30f && (bits & 0x007fffff) != 0 && fabsf(fabsf(r) - half_ulp) > ao * 9.094947e-13f);
-    // x * 0 keeps x's sign, as the float64 product does (p + q would give +0)
-    return zero_h ? p : o;
+// (One sample at a time, with the distance to the boundary formed per sample, the
+// window was half of the sinc warps' instructions: 274 -> 235 us for 50 000 lines.)
+__device__ __forceinline__ float2 mul_window2(float2 x, float2 hi, float2 lo, float2& p, bool& safe0, bool& safe1) {
+    const float2 nx = make_float2(-x.x, -x.y), nz = make_float2(-0.f, -0.f);
+    p = fma2(x, hi, nz);
+    const float2 nq = fma2(nx, lo, fma2(nx, hi, p));
+    const float2 o = sub2(p, nq);
+    const float2 r = add2(nq, sub2(o, p));                    // -r
+    constexpr float kEdge = 5.9602826e-08f;                   // 2^-24 (1 - 2^-15)
+    const float e0 = __int_as_float((__float_as_int(o.x) - 1) & 0x7f800000) * kEdge;
+    const float e1 = __int_as_float((__float_as_int(o.y) - 1) & 0x7f800000) * kEdge;
+    safe0 = fabsf(r.x) < e0 && fabsf(o.x) > 1e-30f;
+    safe1 = fabsf(r.y) < e1 && fabsf(o.y) > 1e-30f;
+    return o;
 }
 
 template <typename RawT>
@@ -391,6 +390,11 @@ __global__ void __launch_bounds__(kThr, 1) k_lines(const LinesArgs a) {
         wa = __ldg(reinterpret_cast<const float4*>(a.g.win + 4 * tid));
         wb = __ldg(reinterpret_cast<const float4*>(a.g.win + 4 * tid + 2));
     }
+    bool end0 = false, end3 = false;                         // kModeLinHann: window values of exactly zero
+    if (Mode == kModeLinHann) {
+        end0 = a.hann2[4 * tid] == 0.f && a.hann2[kN + 4 * tid] == 0.f;
+        end3 = a.hann2[4 * tid + 3] == 0.f && a.hann2[kN + 4 * tid + 3] == 0.f;
+    }
     __syncthreads();
     pdl_wait();                                              // the previous lines have been read
     pdl_launch();
@@ -455,13 +459,20 @@ __global__ void __launch_bounds__(kThr, 1) k_lines(const LinesArgs a) {
                 o[1] = make_float4(v23.x * wb.x * kN, v23.x * wb.y * kN, v23.y * wb.z * kN, v23.y * wb.w * kN);
             } else {
                 // the plain line (its window is one) times the float64 window, one rounding to float32
-                const float lx[4] = {v01.x, v01.y, v23.x, v23.y};
-                float lh[4];
-                bool lsafe[4];
-#pragma unroll
-                for (int r = 0; r < 4; ++r) lh[r] = mul_window(lx[r], __ldg(a.hann2 + 4 * tid + r), lsafe[r]);
-                const bool all_safe = lsafe[0] && lsafe[1] && lsafe[2] && lsafe[3];
-                if (__any_sync(0xffffffffu, !all_safe)) {
+                const float4 wh = __ldg(reinterpret_cast<const float4*>(a.hann2 + 4 * tid));
+                const float4 wl = __ldg(reinterpret_cast<const float4*>(a.hann2 + kN + 4 * tid));
+                float2 p01, p23;
+                bool ok0, ok1, ok2, ok3;
+                const float2 o01 = mul_window2(v01, make_float2(wh.x, wh.y), make_float2(wl.x, wl.y), p01, ok0, ok1);
+                const float2 o23 = mul_window2(v23, make_float2(wh.z, wh.w), make_float2(wl.z, wl.w), p23, ok2, ok3);
+                // an end point of the window that is exactly zero: x * 0 with x's
+                // sign (or NaN), as the float64 product, for every A-scan
+                float lh[4] = {end0 ? p01.x : o01.x, o01.y, o23.x, end3 ? p23.y : o23.y};
+                ok0 = ok0 || end0;
+                ok3 = ok3 || end3;
+                if (__any_sync(0xffffffffu, !(ok0 && ok1 && ok2 && ok3))) {
+                    const float lx[4] = {v01.x, v01.y, v23.x, v23.y};
+                    const bool lsafe[4] = {ok0, ok1, ok2, ok3};
 #pragma unroll
                     for (int r = 0; r < 4; ++r)
                         if (!lsafe[r])

@@ -115,7 +115,7 @@ struct LinesArgs {
     float* out;               // line l at (l - out_l0) kN (kModeSpec: complex)
     unsigned int out_l0;
     const double* hann;       // kModeLinHann: the float64 window (kN)
-    const float2* hann2;      // kModeLinHann: the window split hi + lo in float32 (kN)
+    const float* hann2;       // kModeLinHann: the window split hi (kN), lo (kN) in float32
     int* status;              // device status word
     uint64_t* ready;          // host: bits of the caller's context, see kernel_ready
 };
