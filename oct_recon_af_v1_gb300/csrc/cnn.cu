@@ -21,12 +21,14 @@
 //   k_relu_pool / k_relu_pool_bwd   ReLU then 2x2 mean, and its gradient
 //   k_gemm          C = A B (+ C) with arbitrary strides, 64x64 tiles
 //   k_bias_relu, k_bias_grad, k_mse, k_adam
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "octgb_internal.h"
 
 namespace octgb {
+namespace cg = cooperative_groups;
 namespace {
 
 constexpr int kImg = 256;
@@ -87,18 +89,27 @@ __global__ void __launch_bounds__(256) k_image_cols(const float* __restrict__ zc
 
 // Sums in float64 of float32 partial sums over 16 pixels (four float4 loads),
 // so the FP64 pipe sees a quarter of an operation per pixel; per_image is a
-// multiple of 4 (probes x 256 x 256).
-__global__ void __launch_bounds__(1024) k_image_norm(float* __restrict__ img, int64_t per_image) {
-    __shared__ double red[32];
-    float* v = img + blockIdx.x * per_image;
+// multiple of 4 (probes x 256 x 256).  A cluster of eight CTAs makes an image (one
+// CTA each left a third of the chip idle at 100 images: 51 -> 37 us): thread t of
+// 1024 sums the pixels that it would in one CTA of 1024, and every CTA adds
+// the 32 warps' sums in that CTA's order, so the result does not depend on the split.
+constexpr int kNormCtas = 8, kNormThreads = 1024 / kNormCtas;
+__global__ void __cluster_dims__(kNormCtas, 1, 1) __launch_bounds__(kNormThreads)
+    k_image_norm(float* __restrict__ img, int64_t per_image) {
+    __shared__ double2 red[kNormThreads / 32];
+    __shared__ double2 total;
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = blockIdx.x % kNormCtas, t = rank * kNormThreads + threadIdx.x;
+    float* v = img + blockIdx.x / kNormCtas * per_image;
     const float4* v4 = reinterpret_cast<const float4*>(v);
     const int64_t n4 = per_image / 4;
     double s = 0.0, s2 = 0.0;
-    for (int64_t i0 = threadIdx.x; i0 < n4; i0 += 4 * static_cast<int64_t>(blockDim.x)) {
+#pragma unroll 2
+    for (int64_t i0 = t; i0 < n4; i0 += 4 * 1024) {
         float fs = 0.f, fs2 = 0.f;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            const int64_t i = i0 + u * static_cast<int64_t>(blockDim.x);
+            const int64_t i = i0 + u * 1024;
             if (i < n4) {
                 const float4 q = v4[i];
                 fs += (q.x + q.y) + (q.z + q.w);
@@ -113,31 +124,26 @@ __global__ void __launch_bounds__(1024) k_image_norm(float* __restrict__ img, in
         s += __shfl_xor_sync(0xffffffffu, s, o);
         s2 += __shfl_xor_sync(0xffffffffu, s2, o);
     }
-    __shared__ double red2[32];
-    if (lane == 0) {
-        red[w] = s;
-        red2[w] = s2;
-    }
-    __syncthreads();
+    if (lane == 0) red[w] = make_double2(s, s2);
+    cl.sync();
     if (w == 0) {
-        s = lane < (blockDim.x >> 5) ? red[lane] : 0.0;
-        s2 = lane < (blockDim.x >> 5) ? red2[lane] : 0.0;
+        const double2 o2 = cl.map_shared_rank(red, lane / (kNormThreads / 32))[lane % (kNormThreads / 32)];
+        s = o2.x;
+        s2 = o2.y;
         for (int o = 16; o > 0; o >>= 1) {
             s += __shfl_xor_sync(0xffffffffu, s, o);
             s2 += __shfl_xor_sync(0xffffffffu, s2, o);
         }
-        if (lane == 0) {
-            red[0] = s;
-            red2[0] = s2;
-        }
+        if (lane == 0) total = make_double2(s, s2);
     }
-    __syncthreads();
-    const double mean = red[0] / per_image;
-    const double var = red2[0] / per_image - mean * mean;
+    cl.sync();                                           // sums read; total visible to the block
+    const double mean = total.x / per_image;
+    const double var = total.y / per_image - mean * mean;
     const float inv = static_cast<float>(1.0 / sqrt(var > 1e-12 ? var : 1e-12));
     const float mf = static_cast<float>(mean);
     float4* w4 = reinterpret_cast<float4*>(v);
-    for (int64_t i = threadIdx.x; i < n4; i += blockDim.x) {
+#pragma unroll 4
+    for (int64_t i = t; i < n4; i += 1024) {
         const float4 q = w4[i];
         w4[i] = make_float4((q.x - mf) * inv, (q.y - mf) * inv, (q.z - mf) * inv, (q.w - mf) * inv);
     }
@@ -331,15 +337,32 @@ __global__ void __launch_bounds__(256) k_gemm(const float* __restrict__ A, int64
     const int kb = blockIdx.z * k_chunk, ke = min(Kd, kb + k_chunk);
     Cm += static_cast<int64_t>(blockIdx.z) * M * ldc;
     const bool a_kfast = sa1 == 1, b_kfast = sb0 == 1;
-    float acc[4][4] = {};
-    for (int k0 = kb; k0 < ke; k0 += kGK) {
-        for (int e = threadIdx.x; e < kGK * kGT; e += 256) {
+    // this thread's elements of a K step: loaded into registers while the step
+    // before is multiplied, so that a step costs its products, not a trip to
+    // memory (128 x 64 x 8192: 48 -> 22 us)
+    constexpr int kE = kGK * kGT / 256;
+    float pa[kE], pb[kE];
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int u = 0; u < kE; ++u) {
+            const int e = threadIdx.x + 256 * u;
             const int kk = a_kfast ? e % kGK : e / kGT, r = a_kfast ? e / kGK : e % kGT;
-            as[kk][r] = (i0 + r < M && k0 + kk < ke) ? A[(i0 + r) * sa0 + (k0 + kk) * sa1] : 0.f;
+            pa[u] = (i0 + r < M && k0 + kk < ke) ? A[(i0 + r) * sa0 + (k0 + kk) * sa1] : 0.f;
             const int kk2 = b_kfast ? e % kGK : e / kGT, r2 = b_kfast ? e / kGK : e % kGT;
-            bs[kk2][r2] = (j0 + r2 < N && k0 + kk2 < ke) ? B[(k0 + kk2) * sb0 + (j0 + r2) * sb1] : 0.f;
+            pb[u] = (j0 + r2 < N && k0 + kk2 < ke) ? B[(k0 + kk2) * sb0 + (j0 + r2) * sb1] : 0.f;
+        }
+    };
+    float acc[4][4] = {};
+    load(kb);
+    for (int k0 = kb; k0 < ke; k0 += kGK) {
+#pragma unroll
+        for (int u = 0; u < kE; ++u) {
+            const int e = threadIdx.x + 256 * u;
+            as[a_kfast ? e % kGK : e / kGT][a_kfast ? e / kGK : e % kGT] = pa[u];
+            bs[b_kfast ? e % kGK : e / kGT][b_kfast ? e / kGK : e % kGT] = pb[u];
         }
         __syncthreads();
+        if (k0 + kGK < ke) load(k0 + kGK);
 #pragma unroll
         for (int kk = 0; kk < kGK; ++kk) {
             float a[4], b[4];
@@ -493,7 +516,7 @@ cudaError_t launch_image_cols(const float* zcol, int n_probe, int nb, int nx, in
 }
 
 cudaError_t launch_image_norm(float* img, int n_images, int64_t per_image, cudaStream_t st) {
-    k_image_norm<<<n_images, 1024, 0, st>>>(img, per_image);
+    k_image_norm<<<n_images * kNormCtas, kNormThreads, 0, st>>>(img, per_image);
     return cudaGetLastError();
 }
 
