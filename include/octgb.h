@@ -432,12 +432,15 @@ int octgb_cnn_conv3x3_bwd(octgb_ctx *ctx, const float *x, const float *w, const 
  * expires is reported by the next synchronising call (OCTGB_ERR_TIMEOUT). */
 int octgb_cnn_conv3x3_bwd_tc(octgb_ctx *ctx, const float *x, const float *w, const float *dy, float *dx, float *dw,
                              float *db, float *w_scratch, int n, int cin, int cout, int h, int wd);
-/* octgb_cnn_relu_pool_bwd followed by octgb_cnn_conv3x3_bwd_tc without dx, in
- * one kernel (the gradient of the pre-activations y never reaches memory): dw,
- * db from x, y (n, cout, h, wd) and dp (n, cout, h/2, wd/2).  Shapes as there,
- * with h even, wd a multiple of 8, and y and dp on 16-byte boundaries. */
-int octgb_cnn_conv3x3_pool_bwd_tc(octgb_ctx *ctx, const float *x, const float *y, const float *dp, float *dw,
-                                  float *db, int n, int cin, int cout, int h, int wd);
+/* octgb_cnn_relu_pool_bwd followed by octgb_cnn_conv3x3_bwd_tc with the
+ * gradient of the pre-activations formed inside the kernels (it never reaches
+ * memory): dw, db and (optional) dx from x, y (n, cout, h, wd) and dp (n, cout,
+ * h/2, wd/2).  Shapes as there, with h even, wd a multiple of 8, y and dp on
+ * 16-byte boundaries; for dx also the shapes of octgb_cnn_conv3x3_tc (cout ->
+ * cin channels) and wd <= 128. */
+int octgb_cnn_conv3x3_pool_bwd_tc(octgb_ctx *ctx, const float *x, const float *w, const float *y, const float *dp,
+                                  float *dx, float *dw, float *db, float *w_scratch, int n, int cin, int cout, int h,
+                                  int wd);
 /* p = 2x2 mean of relu(y) over `planes` planes of h x w (even), and its gradient. */
 int octgb_cnn_relu_pool(octgb_ctx *ctx, const float *y, float *p, int64_t planes, int h, int wd);
 int octgb_cnn_relu_pool_bwd(octgb_ctx *ctx, const float *dp, const float *y, float *dy, int64_t planes, int h,

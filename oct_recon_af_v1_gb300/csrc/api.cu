@@ -2254,7 +2254,7 @@ int octgb_cnn_conv3x3_tc(octgb_ctx* c, const float* x, const float* w, const flo
         require(conv3x3_tc_supported(cin, cout, h, wd),
                 "tensor-core convolution: 1 <= cin <= 32, cout a multiple of 32 up to 128, and the width a "
                 "multiple of 128 or a divisor of 128 whose row count divides the height");
-        ck(launch_conv3x3_tc(x, w, b, y, nullptr, n, cin, cout, h, wd, c->num_sms, c->status_dev, c->stream),
+        ck(launch_conv3x3_tc(x, nullptr, w, b, y, nullptr, n, cin, cout, h, wd, c->num_sms, c->status_dev, c->stream),
            "tensor-core conv kernel");
         c->launches++;
     });
@@ -2268,7 +2268,7 @@ int conv_relu_pool_tc(octgb_ctx* c, const float* x, const float* w, const float*
         require(conv3x3_tc_pool_supported(cin, cout, h, wd),
                 "fused tensor-core convolution + pool: 1 <= cin <= 32, cout a multiple of 32 up to 128, the width "
                 "a multiple of 128 and the height even");
-        ck(launch_conv3x3_tc(x, w, b, y, p, n, cin, cout, h, wd, c->num_sms, c->status_dev, c->stream),
+        ck(launch_conv3x3_tc(x, nullptr, w, b, y, p, n, cin, cout, h, wd, c->num_sms, c->status_dev, c->stream),
            "tensor-core conv + pool kernel");
         c->launches++;
     });
@@ -2326,7 +2326,7 @@ int octgb_cnn_conv3x3_bwd_tc(octgb_ctx* c, const float* x, const float* w, const
             // the data gradient is the convolution of dy with the flipped kernel
             // (cout -> cin channels): BF16 tensor cores where the shape allows
             if (conv3x3_tc_supported(cout, cin, h, wd))
-                ck(launch_conv3x3_tc(dy, w_scratch, nullptr, dx, nullptr, n, cout, cin, h, wd, c->num_sms,
+                ck(launch_conv3x3_tc(dy, nullptr, w_scratch, nullptr, dx, nullptr, n, cout, cin, h, wd, c->num_sms,
                                      c->status_dev, c->stream, true),
                    "tensor-core conv kernel");
             else
@@ -2336,20 +2336,31 @@ int octgb_cnn_conv3x3_bwd_tc(octgb_ctx* c, const float* x, const float* w, const
     });
 }
 
-int octgb_cnn_conv3x3_pool_bwd_tc(octgb_ctx* c, const float* x, const float* y, const float* dp, float* dw, float* db,
-                                  int n, int cin, int cout, int h, int wd) {
+int octgb_cnn_conv3x3_pool_bwd_tc(octgb_ctx* c, const float* x, const float* w, const float* y, const float* dp,
+                                  float* dx, float* dw, float* db, float* w_scratch, int n, int cin, int cout, int h,
+                                  int wd) {
     return guarded(c, [&] {
-        require(x && y && dp && dw && db, "NULL buffer");
+        require(x && w && y && dp && dw && db, "NULL buffer");
         require(n >= 1 && cin >= 1 && cout >= 1 && h >= 1 && wd >= 1, "bad convolution shape");
         const size_t parts = conv3x3_wgrad_tc_partials(n, cin, cout, h, wd, true, c->num_sms);
         require(parts > 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0 && reinterpret_cast<uintptr_t>(dp) % 16 == 0,
                 "tensor-core weight gradient through ReLU + pool: as octgb_cnn_conv3x3_bwd_tc, and the height even, "
                 "the width a multiple of 8, y and dp on 16-byte boundaries");
+        require(dx == nullptr || (w_scratch != nullptr && conv3x3_tc_mask_supported(cout, cin, h, wd)),
+                "the data gradient through ReLU + pool needs w_scratch, the shapes of octgb_cnn_conv3x3_tc (cout -> "
+                "cin channels) and a width up to 128");
         ck(c->wgrad_part.ensure(parts * sizeof(float)), "cudaMalloc(weight-gradient partial sums)");
         ck(launch_conv3x3_wgrad_tc(x, y, dp, dw, db, n, cin, cout, h, wd, c->wgrad_part.as<float>(), c->num_sms,
                                    c->status_dev, c->stream),
            "tensor-core weight-gradient kernel");
         c->launches += 2;
+        if (dx != nullptr) {
+            ck(launch_flip_weights(w, cout, cin, w_scratch, c->stream), "weight flip kernel");
+            ck(launch_conv3x3_tc(y, dp, w_scratch, nullptr, dx, nullptr, n, cout, cin, h, wd, c->num_sms,
+                                 c->status_dev, c->stream, true),
+               "tensor-core conv kernel");
+            c->launches += 2;
+        }
     });
 }
 

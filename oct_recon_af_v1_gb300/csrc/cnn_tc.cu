@@ -185,10 +185,13 @@ __device__ __forceinline__ void stage_slot(const Band& g, const BandAt& o, const
 // are zeros already: what is left of the bounds (the pitch's padding, and column
 // -1 of a slot that holds whole rows) is the same in every band, so the slot
 // offset of each of the thread's pixels is kept in registers (-1: zero).
-template <int kIt>
+// kMask: the slot holds pre-activations, and from float poff0 on the gradient of
+// their ReLU + 2x2 mean (R / 2 + 2 rows from image row y0 / 2 - 1 on; whole rows,
+// y0 even): the pixel is y > 0 ? dp / 4 : 0, k_relu_pool_bwd's value.
+template <int kIt, bool kMask = false>
 struct Pixels {
-    int off[kIt];
-    __device__ __forceinline__ Pixels(const Band& g, int npix, int t, int nt) {
+    int off[kIt], poff[kMask ? kIt : 1];
+    __device__ __forceinline__ Pixels(const Band& g, int npix, int t, int nt, int poff0 = 0) {
         const int sx = g.nseg == 1 ? -1 : 3;               // slot column of staged column 0
 #pragma unroll
         for (int k = 0; k < kIt; ++k) {
@@ -196,17 +199,26 @@ struct Pixels {
             const int r = div_wp(g, i), cc = i - r * g.Wp;
             const bool in = i < npix && r < g.R + 2 && cc < g.Ws + 2 && cc + sx >= 0 && cc + sx < g.rp;
             off[k] = in ? r * g.rp + sx + cc : -1;
+            if (kMask) poff[k] = poff0 + ((r + 1) >> 1) * (g.rp / 2) + ((sx + cc) >> 1);
         }
     }
     template <bool kBf16, bool kAll>
-    __device__ __forceinline__ void stage(const float* raw, int rawp, int nch, uint4* dst, int npix, int t, int nt) const {
+    __device__ __forceinline__ void stage(const float* raw, int rawp, int prawp, int nch, uint4* dst, int npix, int t,
+                                          int nt) const {
 #pragma unroll
         for (int k = 0; k < kIt; ++k) {
             const int i = t + k * nt;
             if (i >= npix) break;
             float v[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) v[e] = off[k] >= 0 && (kAll || e < nch) ? raw[off[k] + e * rawp] : 0.f;
+            for (int e = 0; e < 8; ++e) {
+                const bool in = off[k] >= 0 && (kAll || e < nch);
+                v[e] = in ? raw[off[k] + e * rawp] : 0.f;
+                if (kMask) {
+                    const float d = in ? raw[poff[k] + e * prawp] : 0.f;
+                    v[e] = v[e] > 0.f ? 0.25f * d : 0.f;
+                }
+            }
             dst[i] = make_uint4(pack2<kBf16>(v[0], v[1]), pack2<kBf16>(v[2], v[3]), pack2<kBf16>(v[4], v[5]),
                                 pack2<kBf16>(v[6], v[7]));
         }
@@ -245,6 +257,7 @@ struct ConvGeom {
     int xpix;          // pixels per chunk of a staged block
     int pool, wide;    // wide: W >= 128; pool: 1 = ReLU + mean only, 2 = beside the pre-activations
     int slots, nd;     // raw slots, accumulators
+    int poff, prawp;   // kMask: floats from a slot to its pooled gradient, floats per channel of that
     uint32_t slotb, xbytes, off_x, off_b, smem;
     int tmem_cols;
 };
@@ -278,9 +291,12 @@ __device__ __forceinline__ void conv_mmas(uint32_t d, uint64_t a, uint64_t b, ui
                          b + static_cast<uint64_t>((2 * kKs * tap + 2 * ks) * cout), idesc, tap > 0 || ks > 0 ? 1u : 0u);
 }
 
-template <bool kBf16>
+// kMask (the data gradient through ReLU + 2x2 mean): xmap is of the
+// pre-activations, pmap of the pooled gradient, their product with the mask is
+// formed while it is packed (32 x 128 x 128 at 128 images: 89 + 108 -> 124 us).
+template <bool kBf16, bool kMask>
 __global__ void __launch_bounds__(kCThreads, 1)
-    k_conv3x3_tc(const __grid_constant__ CUtensorMap xmap, const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
+    k_conv3x3_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap pmap, const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
                  float* __restrict__ y, float* __restrict__ pooled, const ConvGeom g, int* status) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ ConvBars S;
@@ -351,9 +367,21 @@ __global__ void __launch_bounds__(kCThreads, 1)
             const BandAt o = band_at(g.b, u);
             for (int c8 = 0; c8 < g.cin8r; ++c8, k.next(g.slots)) {
                 if (k.use > 0 && !(ok = role_wait(&S.empty[k.slot], (k.use - 1) & 1u, &S.abort, status))) break;
-                load_slot(xmap, x, g.b.H, g.b.W, g.b.vec, o.img * g.b.C + 8 * c8, min(8, g.b.C - 8 * c8), o.y0 - 1,
-                          g.b.R + 2, slot_x0(g.b, o), g.b.rp, min(8, g.b.C) * g.b.rawp,
-                          reinterpret_cast<float*>(base + k.slot * g.slotb), &S.full[k.slot]);
+                float* slot = reinterpret_cast<float*>(base + k.slot * g.slotb);
+                if (kMask) {
+                    const int plane = o.img * g.b.C + 8 * c8, nc = min(8, g.b.C);
+                    if (lane == 0) {
+                        mbar_expect_tx(&S.full[k.slot], static_cast<uint32_t>(nc * (g.b.rawp + g.prawp)) * 4u);
+                        tensor_copy(xmap, 0, o.y0 - 1, plane, slot, &S.full[k.slot]);
+                        tensor_copy(pmap, 0, o.y0 / 2 - 1, plane, slot + g.poff, &S.full[k.slot]);
+                    } else {
+                        mbar_arrive(&S.full[k.slot]);
+                    }
+                    __syncwarp();
+                } else {
+                    load_slot(xmap, x, g.b.H, g.b.W, g.b.vec, o.img * g.b.C + 8 * c8, min(8, g.b.C - 8 * c8), o.y0 - 1,
+                              g.b.R + 2, slot_x0(g.b, o), g.b.rp, min(8, g.b.C) * g.b.rawp, slot, &S.full[k.slot]);
+                }
             }
         }
         // no copy may be in flight when the block ends
@@ -402,7 +430,7 @@ __global__ void __launch_bounds__(kCThreads, 1)
     } else if (warp >= kCEpi) {
         // ---- converters
         const int t = tid - 32 * kCEpi;
-        const Pixels<kCPix> px(g.b, (g.b.R + 2) * g.b.Wp, t, 32 * kCConv);
+        const Pixels<kCPix, kMask> px(g.b, (g.b.R + 2) * g.b.Wp, t, 32 * kCConv, g.poff);
         Ring k;
         uint32_t j = 0;
         bool ok = true;
@@ -417,12 +445,12 @@ __global__ void __launch_bounds__(kCThreads, 1)
                 const float* raw = reinterpret_cast<const float*>(base + k.slot * g.slotb);
                 uint4* dst = reinterpret_cast<uint4*>(X + b * g.xbytes) + c8 * g.xpix;
                 const int nch = min(8, g.b.C - 8 * c8), npix = (o.rows + 2) * g.b.Wp;
-                if (!g.b.vec)
+                if (!kMask && !g.b.vec)
                     stage_slot<kBf16>(g.b, o, raw, nch, dst, npix, t, 32 * kCConv);
                 else if (nch == 8)
-                    px.template stage<kBf16, true>(raw, g.b.rawp, 8, dst, npix, t, 32 * kCConv);
+                    px.template stage<kBf16, true>(raw, g.b.rawp, g.prawp, 8, dst, npix, t, 32 * kCConv);
                 else
-                    px.template stage<kBf16, false>(raw, g.b.rawp, nch, dst, npix, t, 32 * kCConv);
+                    px.template stage<kBf16, false>(raw, g.b.rawp, g.prawp, nch, dst, npix, t, 32 * kCConv);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&S.empty[k.slot]);
             }
@@ -750,9 +778,9 @@ __global__ void __launch_bounds__(kWThreads, 1)
                     if (!g.b.vec)
                         stage_slot<true>(g.b, o, raw, nch, dst, g.xpix, t, nt);
                     else if (nch == 8)
-                        px.template stage<true, true>(raw, g.b.rawp, 8, dst, g.xpix, t, nt);
+                        px.template stage<true, true>(raw, g.b.rawp, 0, 8, dst, g.xpix, t, nt);
                     else
-                        px.template stage<true, false>(raw, g.b.rawp, nch, dst, g.xpix, t, nt);
+                        px.template stage<true, false>(raw, g.b.rawp, 0, nch, dst, g.xpix, t, nt);
                 } else {
                     const int ch = 8 * (p - g.cgr) + kk;
                     uint8_t* dd = Ds + d0 + (p - g.cgr) * 128;
@@ -913,7 +941,7 @@ bool band_choose(Band& b, int n, int unit, int col_unit, int num_sms, Fits fits)
 
 int tmem_columns(int cols) { return cols <= 32 ? 32 : (cols <= 64 ? 64 : (cols <= 128 ? 128 : (cols <= 256 ? 256 : 512))); }
 
-bool conv_geom(int n, int cin, int cout, int H, int W, int pool, int num_sms, ConvGeom& g) {
+bool conv_geom(int n, int cin, int cout, int H, int W, int pool, bool mask, int num_sms, ConvGeom& g) {
     g = ConvGeom{};
     g.b.C = cin;
     g.b.H = H;
@@ -927,15 +955,19 @@ bool conv_geom(int n, int cin, int cout, int H, int W, int pool, int num_sms, Co
     g.nd = 512 / cols < 4 ? 512 / cols : 4;
     g.tmem_cols = tmem_columns(g.nd * cols);
     const uint32_t bbytes = 9u * static_cast<uint32_t>(g.cin8) * static_cast<uint32_t>(cout) * 16u;
-    return band_choose(g.b, n, pool ? 2 : 1, kCM, num_sms, [&](int R, int Ws) {
+    return band_choose(g.b, n, pool || mask ? 2 : 1, kCM, num_sms, [&](int R, int Ws) {
         if (g.wide && (Ws % kCM != 0 || W % Ws != 0)) return false;
+        if (mask && (Ws != W || R % 2 != 0)) return false;
         band_set(g.b, n, R, Ws);
         if (g.b.rp > kMaxBox) return false;
         // staged pixels; W < 128: the last tile reads on past them (rows that are not written)
         const int last = (R * g.b.Wp + kCM - 1) / kCM * kCM + 2 * g.b.Wp + 2;
         g.xpix = g.wide ? (R + 2) * g.b.Wp : (last > (R + 2) * g.b.Wp ? last : (R + 2) * g.b.Wp);
         g.xbytes = static_cast<uint32_t>(g.cin8) * g.xpix * 16u;
-        g.slotb = (static_cast<uint32_t>(cin < 8 ? cin : 8) * g.b.rawp * 4u + 127u) & ~127u;
+        const int nc = cin < 8 ? cin : 8;
+        g.poff = (nc * g.b.rawp + 31) / 32 * 32;
+        g.prawp = mask ? (R / 2 + 2) * (g.b.rp / 2) : 0;
+        g.slotb = (static_cast<uint32_t>(mask ? g.poff + nc * g.prawp : nc * g.b.rawp) * 4u + 127u) & ~127u;
         const uint32_t rest = 2u * g.xbytes + bbytes + 1024u;
         if (rest + 3u * g.slotb + sizeof(ConvBars) > kSmemBudget) return false;
         const uint32_t s = (kSmemBudget - static_cast<uint32_t>(sizeof(ConvBars)) - rest) / g.slotb;
@@ -1035,21 +1067,32 @@ bool conv3x3_tc_pool_supported(int cin, int cout, int H, int W) {
     return conv3x3_tc_supported(cin, cout, H, W) && W >= kCM && H % 2 == 0;
 }
 
-cudaError_t launch_conv3x3_tc(const float* x, const float* w, const float* b, float* y, float* pooled, int n, int cin,
-                              int cout, int H, int W, int num_sms, int* status, cudaStream_t st, bool bf16) {
+bool conv3x3_tc_mask_supported(int cin, int cout, int H, int W) {
+    return conv3x3_tc_supported(cin, cout, H, W) && H % 2 == 0 && W % 8 == 0 && W <= kCM;
+}
+
+cudaError_t launch_conv3x3_tc(const float* x, const float* dp, const float* w, const float* b, float* y, float* pooled,
+                              int n, int cin, int cout, int H, int W, int num_sms, int* status, cudaStream_t st,
+                              bool bf16) {
     if (!conv3x3_tc_supported(cin, cout, H, W)) return cudaErrorInvalidValue;
     const int pool = pooled == nullptr ? 0 : (y == nullptr ? 1 : 2);
+    const bool mask = dp != nullptr;
     if (pool && !conv3x3_tc_pool_supported(cin, cout, H, W)) return cudaErrorInvalidValue;
+    if (mask && (!bf16 || !conv3x3_tc_mask_supported(cin, cout, H, W))) return cudaErrorInvalidValue;
     ConvGeom g;
-    if (!conv_geom(n, cin, cout, H, W, pool, num_sms, g)) return cudaErrorInvalidValue;
+    if (!conv_geom(n, cin, cout, H, W, pool, mask, num_sms, g)) return cudaErrorInvalidValue;
     if (g.b.n_units == 0) return cudaSuccess;
-    CUtensorMap xmap{};
-    g.b.vec = aligned_rows(x, W) &&
-              encode_planes(&xmap, x, static_cast<int64_t>(n) * cin, H, W, g.b.rp, g.b.R + 2, cin < 8 ? cin : 8);
-    auto kern = bf16 ? k_conv3x3_tc<true> : k_conv3x3_tc<false>;
+    CUtensorMap xmap{}, pmap{};
+    const int nc = cin < 8 ? cin : 8;
+    const int64_t planes = static_cast<int64_t>(n) * cin;
+    g.b.vec = aligned_rows(x, W) && encode_planes(&xmap, x, planes, H, W, g.b.rp, g.b.R + 2, nc);
+    if (mask && !(g.b.vec && aligned_rows(dp, W / 2) &&
+                  encode_planes(&pmap, dp, planes, H / 2, W / 2, g.b.rp / 2, g.b.R / 2 + 2, nc)))
+        return cudaErrorInvalidValue;
+    const auto kern = mask ? k_conv3x3_tc<true, true> : (bf16 ? k_conv3x3_tc<true, false> : k_conv3x3_tc<false, false>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(g.smem));
     if (e != cudaSuccess) return e;
-    kern<<<units_grid(g.b, num_sms), kCThreads, g.smem, st>>>(xmap, x, w, b, y, pooled, g, status);
+    kern<<<units_grid(g.b, num_sms), kCThreads, g.smem, st>>>(xmap, pmap, x, w, b, y, pooled, g, status);
     return cudaGetLastError();
 }
 

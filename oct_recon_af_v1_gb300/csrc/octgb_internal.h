@@ -299,11 +299,15 @@ cudaError_t launch_image_norm(float* img, int n_images, int64_t per_image, cudaS
 // tensor-core 3x3 convolution (cnn_tc.cu): same contract as launch_conv3x3 for
 // the shapes conv3x3_tc_supported accepts; FP16 operands (BF16 with bf16: the
 // data gradient, whose values span float32's exponent range), float32
-// accumulation (with pooled (n, cout, H/2, W/2): its ReLU + 2x2 mean, y may be NULL)
+// accumulation (with pooled (n, cout, H/2, W/2): its ReLU + 2x2 mean, y may be
+// NULL; with dp (n, cin, H/2, W/2) and bf16, on shapes of
+// conv3x3_tc_mask_supported with x and dp 16-byte aligned: of the gradient of
+// x's ReLU + 2x2 mean whose pooled gradient is dp)
 bool conv3x3_tc_supported(int cin, int cout, int H, int W);
 bool conv3x3_tc_pool_supported(int cin, int cout, int H, int W);
-cudaError_t launch_conv3x3_tc(const float* x, const float* w, const float* b, float* y, float* pooled, int n, int cin,
-                              int cout, int H, int W, int num_sms, int* status, cudaStream_t st, bool bf16 = false);
+bool conv3x3_tc_mask_supported(int cin, int cout, int H, int W);
+cudaError_t launch_conv3x3_tc(const float* x, const float* dp, const float* w, const float* b, float* y, float* pooled,
+                              int n, int cin, int cout, int H, int W, int num_sms, int* status, cudaStream_t st, bool bf16 = false);
 // weight and bias gradients of the 3x3 convolution (cnn_tc.cu; dw on the tensor
 // cores with BF16 operands and float32 accumulation, db from dy in float32):
 // dw (cout, cin, 3, 3) and db (cout) from x (n, cin, H, W) and dy (n, cout, H, W).

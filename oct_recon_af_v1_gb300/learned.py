@@ -153,8 +153,7 @@ class BetaFocusNet:
                  "dout": torch.empty((n, 2), dtype=torch.float32, device=dev),
                  "dh": torch.empty((n, self.hidden), dtype=torch.float32, device=dev),
                  "dflat": torch.empty((n, self.flat), dtype=torch.float32, device=dev),
-                 "dpre": [None if i == 0 and self._fused_first() else torch.empty_like(t)
-                          for i, t in enumerate(pre)],
+                 "dpre": [None if self._fused_bwd(i) else torch.empty_like(t) for i, t in enumerate(pre)],
                  "dpooled": [torch.empty_like(t) for t in pooled[:-1]]}
             self._acts[n] = b
         return b
@@ -166,10 +165,12 @@ class BetaFocusNet:
             return False
         return w % 128 == 0 if w >= 128 else (128 % w == 0 and h % (128 // w) == 0)
 
-    def _fused_first(self) -> bool:
-        """The first layer's gradient straight from its pre-activations
-        (octgb_cnn_conv3x3_pool_bwd_tc: rows of a multiple of 8)."""
-        return self.train_tensor_cores and self.img % 8 == 0
+    def _fused_bwd(self, i: int) -> bool:
+        """Layers whose gradients octgb_cnn_conv3x3_pool_bwd_tc takes straight
+        from the pre-activations."""
+        h = self.img >> i
+        return (self.train_tensor_cores and h % 8 == 0 and
+                (i == 0 or (h <= 128 and self.tc_supported(self.chans[i + 1], self.chans[i], h, h))))
 
     def forward(self, x, tensor_cores: bool = False, fuse_pool=None):
         """x: (n, in_ch, img, img) float32 CUDA tensor -> (n, 2) predictions (a
@@ -235,16 +236,18 @@ class BetaFocusNet:
         for i in reversed(range(len(self.chans) - 1)):
             cin, cout = self.chans[i], self.chans[i + 1]
             xin = self._x if i == 0 else b["pooled"][i - 1]
-            if i == 0 and self._fused_first():
-                # no gradient of the input: ReLU, pooling and the sums in one kernel
-                self._check(self.lib.octgb_cnn_conv3x3_pool_bwd_tc(self.ctx.h, _p(xin), _p(b["pre"][0]), _p(dp),
-                                                                   _p(g[0]), _p(g[1]), n, cin, cout, h, h))
-                break
+            dx = None if i == 0 else b["dpooled"][i - 1]
+            if self._fused_bwd(i):
+                self._check(self.lib.octgb_cnn_conv3x3_pool_bwd_tc(
+                    self.ctx.h, _p(xin), _p(self.params[2 * i]), _p(b["pre"][i]), _p(dp), _p(dx), _p(g[2 * i]),
+                    _p(g[2 * i + 1]), _p(self.wscratch), n, cin, cout, h, h))
+                dp = dx
+                h *= 2
+                continue
             if b["dpre"][i] is None:                        # train_tensor_cores was switched off since
                 b["dpre"][i] = b["pre"][i].new_empty(b["pre"][i].shape)
             self._check(self.lib.octgb_cnn_relu_pool_bwd(self.ctx.h, _p(dp), _p(b["pre"][i]), _p(b["dpre"][i]),
                                                          n * cout, h, h))
-            dx = None if i == 0 else b["dpooled"][i - 1]
             bwd = self.lib.octgb_cnn_conv3x3_bwd_tc if self.train_tensor_cores else self.lib.octgb_cnn_conv3x3_bwd
             self._check(bwd(self.ctx.h, _p(xin), _p(self.params[2 * i]), _p(b["dpre"][i]), _p(dx), _p(g[2 * i]),
                             _p(g[2 * i + 1]), _p(self.wscratch), n, cin, cout, h, h))

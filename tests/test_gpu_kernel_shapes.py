@@ -371,8 +371,8 @@ def test_weight_gradient_through_pool(gpu_ctx, n, cin, cout, h, w, shift):
     xd, yd, dpd = _offset(torch, x.numpy(), shift), y.cuda(), dp.cuda()
     dw, db = torch.full((cout, cin, 3, 3), float("nan"), device="cuda"), torch.full((cout,), float("nan"), device="cuda")
     torch.cuda.synchronize()
-    gpu_ctx._check(gpu_ctx.lib.octgb_cnn_conv3x3_pool_bwd_tc(gpu_ctx.h, _p(xd), _p(yd), _p(dpd), _p(dw), _p(db), n, cin,
-                                                             cout, h, w))
+    gpu_ctx._check(gpu_ctx.lib.octgb_cnn_conv3x3_pool_bwd_tc(gpu_ctx.h, _p(xd), _p(dw), _p(yd), _p(dpd), None, _p(dw),
+                                                             _p(db), None, n, cin, cout, h, w))
     gpu_ctx.synchronize()
     assert (np.abs(dw.cpu().numpy() - ref) <= 1e-4 * mag).all()
     assert (np.abs(db.cpu().double().numpy() - dy.double().sum((0, 2, 3)).numpy())
@@ -397,3 +397,26 @@ def test_conv_with_pool_beside_pre_activations(gpu_ctx, n, cin, cout, h, w):
     c._check(L.octgb_cnn_conv3x3_keep_relu_pool_tc(c.h, _p(x), _p(wt), _p(b), _p(y2), _p(p2), n, cin, cout, h, w))
     c.synchronize()
     assert torch.isfinite(y).all() and torch.equal(y, y2) and torch.equal(p, p2)
+
+
+@pytest.mark.parametrize("n,cin,cout,h,w", [(2, 32, 32, 128, 128), (3, 32, 32, 64, 64), (130, 32, 9, 32, 32),
+                                            (1, 32, 17, 2, 128), (2, 32, 3, 16, 8)])
+def test_data_gradient_through_pool(gpu_ctx, n, cin, cout, h, w):
+    """dx equals, bit for bit, that of the two kernels that put dy in memory
+    (the same products in the same order)."""
+    torch = pytest.importorskip("torch")
+    from oct_recon_af_v1_gb300.learned import _p
+    rng = np.random.default_rng(w + cin)
+    x, wt, y, dp = (torch.tensor(rng.standard_normal(s), dtype=torch.float32, device="cuda")
+                    for s in ((n, cin, h, w), (cout, cin, 3, 3), (n, cout, h, w), (n, cout, h // 2, w // 2)))
+    dy, (dx, dx2) = torch.empty_like(y), (torch.full((n, cin, h, w), float("nan"), device="cuda") for _ in range(2))
+    dw, db, scratch = torch.empty_like(wt), torch.empty(cout, device="cuda"), torch.empty(wt.numel(), device="cuda")
+    torch.cuda.synchronize()
+    L, c = gpu_ctx.lib, gpu_ctx
+    c._check(L.octgb_cnn_relu_pool_bwd(c.h, _p(dp), _p(y), _p(dy), n * cout, h, w))
+    c._check(L.octgb_cnn_conv3x3_bwd_tc(c.h, _p(x), _p(wt), _p(dy), _p(dx), _p(dw), _p(db), _p(scratch), n, cin, cout,
+                                        h, w))
+    c._check(L.octgb_cnn_conv3x3_pool_bwd_tc(c.h, _p(x), _p(wt), _p(y), _p(dp), _p(dx2), _p(dw), _p(db), _p(scratch), n,
+                                             cin, cout, h, w))
+    c.synchronize()
+    assert torch.isfinite(dx).all() and torch.equal(dx, dx2)
