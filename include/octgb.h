@@ -457,6 +457,9 @@ int octgb_cnn_mse(octgb_ctx *ctx, const float *pred, const float *target, int n,
 /* One Adam step (bias-corrected, `step` counted from 1) on n parameters. */
 int octgb_cnn_adam(octgb_ctx *ctx, float *p, const float *g, float *m, float *v, int64_t n, float lr, float beta1,
                    float beta2, float eps, int step);
+/* The same step on `count` tensors in one launch (host arrays of device pointers and of sizes). */
+int octgb_cnn_adam_list(octgb_ctx *ctx, int count, float *const *p, const float *const *g, float *const *m,
+                        float *const *v, const int64_t *n, float lr, float beta1, float beta2, float eps, int step);
 
 /* ---------------------------------------------------------------- allocation-free */
 

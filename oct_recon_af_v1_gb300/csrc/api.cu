@@ -2420,15 +2420,26 @@ int octgb_cnn_mse(octgb_ctx* c, const float* pred, const float* target, int n, f
     });
 }
 
-int octgb_cnn_adam(octgb_ctx* c, float* p, const float* g, float* m, float* v, int64_t n, float lr, float beta1,
-                   float beta2, float eps, int step) {
+int octgb_cnn_adam_list(octgb_ctx* c, int count, float* const* p, const float* const* g, float* const* m,
+                        float* const* v, const int64_t* n, float lr, float beta1, float beta2, float eps, int step) {
     return guarded(c, [&] {
-        require(p && g && m && v && n >= 1 && step >= 1, "bad optimiser arguments");
+        require(p && g && m && v && n && count >= 1 && step >= 1, "bad optimiser arguments");
+        for (int i = 0; i < count; ++i) require(p[i] && g[i] && m[i] && v[i] && n[i] >= 1, "bad optimiser arguments");
         const float c1 = 1.0f - std::pow(beta1, static_cast<float>(step));
         const float c2 = 1.0f - std::pow(beta2, static_cast<float>(step));
-        ck(launch_adam(p, g, m, v, n, lr, beta1, beta2, eps, c1, c2, c->stream), "adam kernel");
-        c->launches++;
+        for (int i0 = 0; i0 < count; i0 += kAdamMost) {
+            AdamList a{};
+            const int k = count - i0 < kAdamMost ? count - i0 : kAdamMost;
+            for (int i = 0; i < k; ++i) a.t[i] = {p[i0 + i], g[i0 + i], m[i0 + i], v[i0 + i], n[i0 + i]};
+            ck(launch_adam(a, k, lr, beta1, beta2, eps, c1, c2, c->stream), "adam kernel");
+            c->launches++;
+        }
     });
+}
+
+int octgb_cnn_adam(octgb_ctx* c, float* p, const float* g, float* m, float* v, int64_t n, float lr, float beta1,
+                   float beta2, float eps, int step) {
+    return octgb_cnn_adam_list(c, 1, &p, &g, &m, &v, &n, lr, beta1, beta2, eps, step);
 }
 
 }  // extern "C"

@@ -340,8 +340,19 @@ cudaError_t launch_bias_relu(float* y, const float* b, int M, int N, float* out,
 cudaError_t launch_bias_grad(const float* g, int Nn, int K, int64_t inner, float* db, float* part, cudaStream_t st);
 cudaError_t launch_relu_bwd(float* g, const float* pre, int64_t n, cudaStream_t st);
 cudaError_t launch_mse(const float* pred, const float* t, int n, float* grad, double* loss, cudaStream_t st);
-cudaError_t launch_adam(float* p, const float* g, float* m, float* v, int64_t n, float lr, float b1, float b2,
-                        float eps, float c1, float c2, cudaStream_t st);
+// one Adam step on up to kAdamMost tensors
+constexpr int kAdamMost = 16;
+struct AdamTensor {
+    float* p;
+    const float* g;
+    float *m, *v;
+    int64_t n;
+};
+struct AdamList {
+    AdamTensor t[kAdamMost];
+};
+cudaError_t launch_adam(const AdamList& a, int count, float lr, float b1, float b2, float eps, float c1, float c2,
+                        cudaStream_t st);
 
 // ordered-uint encoding of float32 for atomic min/max
 __host__ __device__ inline unsigned int f2ord(float f) {

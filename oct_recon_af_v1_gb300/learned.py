@@ -263,9 +263,10 @@ class BetaFocusNet:
 
     def adam(self, lr: float, beta1: float = 0.9, beta2: float = 0.999, eps: float = 1e-8):
         self.step_count += 1
-        for p, g, m, v in zip(self.params, self.grads, self.m, self.v):
-            self._check(self.lib.octgb_cnn_adam(self.ctx.h, _p(p), _p(g), _p(m), _p(v), p.numel(), lr, beta1, beta2,
-                                                eps, self.step_count))
+        n = len(self.params)
+        lists = [(ctypes.c_void_p * n)(*(t.data_ptr() for t in ts)) for ts in (self.params, self.grads, self.m, self.v)]
+        sizes = (ctypes.c_int64 * n)(*(p.numel() for p in self.params))
+        self._check(self.lib.octgb_cnn_adam_list(self.ctx.h, n, *lists, sizes, lr, beta1, beta2, eps, self.step_count))
 
     def train_step(self, x, target, lr: float):
         pred = self.forward(x, tensor_cores=self.train_tensor_cores, fuse_pool=False)

@@ -420,3 +420,25 @@ def test_data_gradient_through_pool(gpu_ctx, n, cin, cout, h, w):
                                              cin, cout, h, w))
     c.synchronize()
     assert torch.isfinite(dx).all() and torch.equal(dx, dx2)
+
+
+def test_adam_list(gpu_ctx):
+    """Tensors of uneven sizes, more than one launch takes, equal those stepped one at a time."""
+    torch = pytest.importorskip("torch")
+    import ctypes
+    from oct_recon_af_v1_gb300.learned import _p
+    sizes = [1, 255, 257, 400_000] + [3] * 13
+    rng = np.random.default_rng(3)
+    one = [[torch.tensor(np.abs(rng.standard_normal(n)), dtype=torch.float32, device="cuda") for n in sizes]
+           for _ in range(4)]
+    many = [[t.clone() for t in ts] for ts in one]
+    torch.cuda.synchronize()
+    for p, g, m, v in zip(*one):
+        gpu_ctx._check(gpu_ctx.lib.octgb_cnn_adam(gpu_ctx.h, _p(p), _p(g), _p(m), _p(v), p.numel(), 1e-3, 0.9, 0.999,
+                                                  1e-8, 3))
+    n = len(sizes)
+    lists = [(ctypes.c_void_p * n)(*(t.data_ptr() for t in ts)) for ts in many]
+    gpu_ctx._check(gpu_ctx.lib.octgb_cnn_adam_list(gpu_ctx.h, n, *lists, (ctypes.c_int64 * n)(*sizes), 1e-3, 0.9, 0.999,
+                                                   1e-8, 3))
+    gpu_ctx.synchronize()
+    assert all(torch.equal(a, b) for x, y in zip(one, many) for a, b in zip(x, y))
