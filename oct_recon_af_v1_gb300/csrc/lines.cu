@@ -485,14 +485,23 @@ __global__ void __launch_bounds__(kThr, 1) k_lines(const LinesArgs a) {
 }
 
 // apodisation mean (cpu_kernels.py:20-25): exact sum, divided in float64,
-// stored float32.  Four samples a thread, five lines in flight.
-constexpr int kApodThreads = 128;                // x 4 samples = a quarter of a row
+// stored float32.  Nine lines in flight: a call of few B-scans is one trip to
+// memory per batch of lines (25 lines of three B-scans: five in flight 6.7 us,
+// nine 5.6, thirteen 5.5 but 2 % slower for 30 B-scans).  Integers: four samples
+// a thread.  Float32 raws: one, since their float64 sums are bound by the SM's
+// FP64 rate and a row then spans four times the SMs (nine B-scans: 14.5 -> 7.0 us).
+constexpr int kApodThreads = 128;
+constexpr int kApodFlight = 9;
+template <typename RawT>
+constexpr int kApodPer = sizeof(RawT) == 2 ? 4 : 1;                          // samples a thread
+template <typename RawT>
+constexpr int kApodParts = kN / (kApodThreads * kApodPer<RawT>);             // CTAs a row
 // Exact: the sums instead, as -S in float32 while that is exact, else as int32.
 template <typename RawT, bool Tiles, bool Exact>
 __global__ void __launch_bounds__(kApodThreads) k_apod_mean(const LinesArgs a, float* __restrict__ out) {
     pdl_launch();                                // the lines kernel loads its weights meanwhile
-    const int row = blockIdx.x >> 2;             // segment * B + b, or the tiles' apod_row0 + b
-    const int j = ((blockIdx.x & 3) * kApodThreads + threadIdx.x) * 4;
+    const int row = blockIdx.x / kApodParts<RawT>;   // segment * B + b, or the tiles' apod_row0 + b
+    const int j = (blockIdx.x % kApodParts<RawT> * kApodThreads + threadIdx.x) * kApodPer<RawT>;
     const RawT* p;
     int apod;
     if (Tiles) {
@@ -509,41 +518,47 @@ __global__ void __launch_bounds__(kApodThreads) k_apod_mean(const LinesArgs a, f
         apod = a.apod;
         p = static_cast<const RawT*>(a.seg[sg]) + static_cast<int64_t>(row - sg * a.B) * a.interf * kN + j;
     }
-    double s[4];
-    if (sizeof(RawT) == 2) {
+    if constexpr (sizeof(RawT) == 2) {
         int acc[4] = {0, 0, 0, 0};
-#pragma unroll 5
-        for (int k = 0; k < apod; ++k) {
-            const uint2 q = __ldg(reinterpret_cast<const uint2*>(p + static_cast<int64_t>(k) * kN));
-            acc[0] += static_cast<int>(static_cast<RawT>(q.x & 0xffffu));
-            acc[1] += static_cast<int>(static_cast<RawT>(q.x >> 16));
-            acc[2] += static_cast<int>(static_cast<RawT>(q.y & 0xffffu));
-            acc[3] += static_cast<int>(static_cast<RawT>(q.y >> 16));
+        for (int k0 = 0; k0 < apod; k0 += kApodFlight) {
+            uint2 q[kApodFlight];
+#pragma unroll
+            for (int i = 0; i < kApodFlight; ++i)
+                q[i] = k0 + i < apod ? __ldg(reinterpret_cast<const uint2*>(p + static_cast<int64_t>(k0 + i) * kN))
+                                     : make_uint2(0u, 0u);
+#pragma unroll
+            for (int i = 0; i < kApodFlight; ++i) {
+                acc[0] += static_cast<int>(static_cast<RawT>(q[i].x & 0xffffu));
+                acc[1] += static_cast<int>(static_cast<RawT>(q[i].x >> 16));
+                acc[2] += static_cast<int>(static_cast<RawT>(q[i].y & 0xffffu));
+                acc[3] += static_cast<int>(static_cast<RawT>(q[i].y >> 16));
+            }
         }
-        if (Exact) {
-            *reinterpret_cast<float4*>(out + static_cast<int64_t>(row) * kN + j) =
-                apod <= kExactFloat ? make_float4(-static_cast<float>(acc[0]), -static_cast<float>(acc[1]),
+        float4 o;
+        if (Exact)
+            o = apod <= kExactFloat ? make_float4(-static_cast<float>(acc[0]), -static_cast<float>(acc[1]),
                                                   -static_cast<float>(acc[2]), -static_cast<float>(acc[3]))
                                     : make_float4(__int_as_float(acc[0]), __int_as_float(acc[1]),
                                                   __int_as_float(acc[2]), __int_as_float(acc[3]));
-            return;
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) s[e] = static_cast<double>(acc[e]);
+        else
+            o = make_float4(static_cast<float>(static_cast<double>(acc[0]) / apod),
+                            static_cast<float>(static_cast<double>(acc[1]) / apod),
+                            static_cast<float>(static_cast<double>(acc[2]) / apod),
+                            static_cast<float>(static_cast<double>(acc[3]) / apod));
+        *reinterpret_cast<float4*>(out + static_cast<int64_t>(row) * kN + j) = o;
     } else {
-        s[0] = s[1] = s[2] = s[3] = 0.0;
-#pragma unroll 5
-        for (int k = 0; k < apod; ++k) {
-            const float4 q = __ldg(reinterpret_cast<const float4*>(p + static_cast<int64_t>(k) * kN));
-            s[0] += static_cast<double>(q.x);
-            s[1] += static_cast<double>(q.y);
-            s[2] += static_cast<double>(q.z);
-            s[3] += static_cast<double>(q.w);
+        double s = 0.0;
+        for (int k0 = 0; k0 < apod; k0 += kApodFlight) {
+            float q[kApodFlight];
+#pragma unroll
+            for (int i = 0; i < kApodFlight; ++i)
+                q[i] = k0 + i < apod ? __ldg(p + static_cast<int64_t>(k0 + i) * kN) : 0.f;
+#pragma unroll
+            for (int i = 0; i < kApodFlight; ++i)
+                if (k0 + i < apod) s += static_cast<double>(q[i]);
         }
+        out[static_cast<int64_t>(row) * kN + j] = static_cast<float>(s / apod);
     }
-    *reinterpret_cast<float4*>(out + static_cast<int64_t>(row) * kN + j) =
-        make_float4(static_cast<float>(s[0] / apod), static_cast<float>(s[1] / apod), static_cast<float>(s[2] / apod),
-                    static_cast<float>(s[3] / apod));
 }
 
 template <typename RawT, int Mode, int U, bool Tiles, bool Exact>
@@ -589,11 +604,11 @@ cudaError_t launch_mode(const LinesArgs& a, int mode, int num_sms, cudaStream_t 
 template <typename RawT>
 void launch_apod_t(const LinesArgs& a, int rows, float* out, cudaStream_t st) {
     if (a.exact)
-        k_apod_mean<RawT, false, true><<<4 * rows, kApodThreads, 0, st>>>(a, out);
+        k_apod_mean<RawT, false, true><<<kApodParts<RawT> * rows, kApodThreads, 0, st>>>(a, out);
     else if (a.qt != nullptr)
-        k_apod_mean<RawT, true, false><<<4 * rows, kApodThreads, 0, st>>>(a, out);
+        k_apod_mean<RawT, true, false><<<kApodParts<RawT> * rows, kApodThreads, 0, st>>>(a, out);
     else
-        k_apod_mean<RawT, false, false><<<4 * rows, kApodThreads, 0, st>>>(a, out);
+        k_apod_mean<RawT, false, false><<<kApodParts<RawT> * rows, kApodThreads, 0, st>>>(a, out);
 }
 
 }  // namespace
