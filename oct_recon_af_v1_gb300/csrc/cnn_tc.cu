@@ -24,10 +24,10 @@
 // pass of its own):
 //   convolution       3 x 256 x 256: 516 -> 270 us (4.3 TB/s), 32 x 128 x 128: 370 -> 108 us (5.0 TB/s)
 //     + ReLU + mean   280 -> 217 us, 265 -> 96 us
-//   gradients of w, b 1100 -> 311 us (3.8 TB/s), 470 -> 233 us (2.3 TB/s)
+//   gradients of w, b 1100 -> 299 us (3.9 TB/s), 470 -> 188 us (2.9 TB/s)
 // What bounds them now: the 1.1 GB stream of the first convolution and its nine
-// MMAs a tile about equally; the MMAs of the gradients at 32 channels (167 us
-// without them), whose M = 128 rows hold 32 output channels.
+// MMAs a tile about equally; of the gradients the converters' instructions and
+// the copies (168 us at 32 x 128 x 128 without MMAs).
 //
 // A staged block holds the band's input rows y0 - 1 .. y0 + R with a zero
 // column before each row and zeros after it up to the row pitch Wp (W + 2
@@ -51,7 +51,7 @@
 namespace octgb {
 namespace {
 
-constexpr int kCM = 128;                    // MMA M: output pixels per tile (convolution), output channels (gradient)
+constexpr int kCM = 128;                    // MMA M of the convolution: output pixels per tile
 constexpr int kMaxSlots = 8;                // raw slots (3 at least: a copy in flight while two are converted)
 constexpr int kMaxBox = 256;                // elements per dimension of a tensor copy
 constexpr uint32_t kSmemBudget = 226u * 1024u;
@@ -567,9 +567,11 @@ __global__ void __launch_bounds__(kCThreads, 1)
 // ---------------------------------------------------------------- weight gradient
 // dw[k][c][ty][tx] = sum over the images and output pixels (oy, ox) of
 //   dy[k](oy, ox) * x[c](oy + ty - 1, ox + tx - 1)          (x zero outside the image)
-// as nine GEMMs that contract over pixels: M = 128 rows = the output channels
-// (rows past cout read in-bounds data of the following chunks into
-// accumulator rows that are never read), N = the input channels rounded up to
+// as nine GEMMs that contract over pixels: M = the output channels, 64 rows or 128
+// (the MMA reads all M rows of A from shared memory, whatever their use: 32
+// channels at M = 128 took 233 us at 32 x 128 x 128, 188 at M = 64; rows past cout
+// read in-bounds data of the following chunks into accumulator rows that are
+// never read), N = the input channels rounded up to
 // 16, K = 16 pixels per MMA; BF16 operands (gradients span float32's exponent
 // range), float32 accumulation.  x is staged as above (the MN-major B operand);
 // dy on the same pitch pixel-contiguous ([8-pixel chunk][output channel][8
@@ -584,7 +586,7 @@ constexpr int kWPix = 4, kWDy = 5;                         // per converter thre
 
 struct WgradGeom {
     Band b;
-    int K;
+    int K, M;            // output channels, MMA M (64 or 128)
     int Q;               // pixels per band (R Wp rounded up to 32)
     int N;               // MMA N: C rounded up to 16
     int cgr, kg;         // channel groups of 8: of x (loaded), of dy
@@ -694,7 +696,7 @@ __global__ void __launch_bounds__(kWThreads, 1)
         }
     } else if (warp == 1) {
         // ---- MMA issue: BF16 A (K-major) and B (MN-major: bit 16)
-        const uint32_t idesc = mma_idesc_f16(kCM, g.fold ? 32 : g.N) | kIdescBf16 | (1u << 16);
+        const uint32_t idesc = mma_idesc_f16(g.M, g.fold ? 32 : g.N) | kIdescBf16 | (1u << 16);
         const uint32_t lbo_a = static_cast<uint32_t>(g.apitch);         // next 8-pixel chunk of dy
         // B is MN-major without swizzle: there the descriptor's leading offset is
         // the step along K (the next 8 pixels, 128 bytes on) and the stride offset
@@ -832,14 +834,15 @@ __global__ void __launch_bounds__(kWThreads, 1)
     __syncthreads();
     tc_fence_after();
     if (S.drained) {
-        // warp w reads TMEM lanes 32 (w % 4) .. + 31 (output channels), 32-column
-        // chunks w / 4, w / 4 + 4, ...; column t * N + c is tap t of channel c
-        const int quarter = warp & 3;
-        const int k = 32 * quarter + lane;
+        // warp w reads TMEM lanes 32 (w % 4) .. + 31 (output channels; M = 64: 16 a
+        // warp, in its lanes 0 .. 15), 32-column chunks w / 4, w / 4 + 4, ...; column
+        // t * N + c is tap t of channel c
+        const int quarter = warp & 3, rows = g.M / 4;
+        const int k = lane < rows ? rows * quarter + lane : g.K;
         const int cols = g.acc_cols;
         const int64_t kc9 = static_cast<int64_t>(g.K) * g.b.C * 9;
         float* mine = part + blockIdx.x * (kc9 + g.K);
-        if (32 * quarter < g.K) {
+        if (rows * quarter < g.K) {
             for (int ch = warp >> 2; 32 * ch < cols; ch += kWThreads / 128) {
                 float v[32];
                 tmem_ld32(tmem + (static_cast<uint32_t>(32 * quarter) << 16) + static_cast<uint32_t>(32 * ch), v);
@@ -987,6 +990,7 @@ bool wgrad_geom(int n, int cin, int cout, int H, int W, bool pool, int num_sms, 
     g.b.H = H;
     g.b.W = W;
     g.K = cout;
+    g.M = cout <= 64 ? 64 : 128;
     g.N = (cin + 15) / 16 * 16;
     g.cgr = (cin + 7) / 8;
     g.kg = (cout + 7) / 8;
