@@ -13,7 +13,7 @@ legacy uint16 quantisation of the volume.
 `--config 0`: one tile, 50 B-scans x (25 + 500) A-scans, z-crop 1000 px:
 spectral stage to dB, global clim, quantisation.
 `--config 2`: the config-1 tiles through the precision form of the spectral
-stage (exact background, tcgen05 split-FP16 sinc), beside the float32 form.
+stage (exact background), beside the float32 form.
 `--config 3`: 64 tiles of uneven size in one call (CUDA graph, autotuned
 order), beside per-tile calls.
 `--config 4`: the learned beta/focus estimator trained on the device (20 k
@@ -52,10 +52,11 @@ sys.path.insert(0, str(ROOT))
 
 METRIC = "A-scans/s on 1 GB300 (fused vs plain FP32; learned vs search β) at ≤1 LSB"
 APOD = 25
-# DRAM bytes per A-scan of the spectral kernel from one ncu capture
-# (profiles/k_spectral_config1_small.md: (49.43 + 7.16) MB over 12 000 A-scans;
-# caches flushed before the kernel, magnitudes partly still in L2 at its end)
-SPECTRAL_DRAM_BYTES_PER_ASCAN = (49.433856e6 + 7.155456e6) / 12000
+# DRAM bytes per A-scan of the spectral stage from one ncu capture
+# (profiles/spectral_and_stitch_config1_small.md: k_apod_mean, k_lines and
+# k_disp_mag over 36 000 A-scans; caches flushed before each kernel, the last
+# lines and magnitudes partly still in L2 at its end)
+SPECTRAL_DRAM_BYTES_PER_ASCAN = (3.7e6 + 385.0e6 + 386.7e6) / 36000
 
 
 # ------------------------------------------------------------------------ workload description
@@ -420,9 +421,8 @@ def gpu_arm(args, rank, world):
 
 
 def precision_leg(ctx, vol, torch, stream, args, sample_bscans=2):
-    """The precision form (exact integer background, tcgen05 split-FP16 sinc,
-    FFT, |.|) over every tile of the resident volume, beside the float32 form
-    (the same tiles through the fused kernel), and the legacy codes of both
+    """The precision form (exact integer background, sinc, FFT, |.|) over every
+    tile of the resident volume, beside the float32 form (the same tiles), and the legacy codes of both
     against the float64 oracle on a sample (B-scans 0..1 of one tile, one
     shared clim)."""
     from oracle import numerics as O
@@ -716,28 +716,20 @@ def gpu_arm_config2(args, rank, world, torch, ctx, stream, dev):
     ms_sinc, _ = timed(sinc_step, args.steps, 1)
     ms_f32, _ = timed(f32_step, args.steps, 1)
     hbm, src = peaks()
-    flops_per_ascan = 32 * 3 * 2 * 64 * 96                     # dense MMA tiles executed per A-scan
     sinc_bytes = ascans * (interf / nxa * 2048 * 2 + 2048 * 4)   # raw in, X out
-    try:
-        tf_peak = float(json.loads((ROOT / "MEASURED_PEAKS.json").read_text()).get("bf16_tflops"))
-    except Exception:
-        tf_peak = 1900.0
     return {"metric": METRIC, "value": ascans / (ms * 1e-3), "unit": "A-scans/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True,
-            "scaling": "weak", "vs_baseline": None, "dtype": "f32 (split-fp16 tensor-core sinc, uint16 in)",
+            "scaling": "weak", "vs_baseline": None, "dtype": "f32 (uint16 in)",
             "data": "synthetic (seeded, generated on device)",
             "config": dict(config1_desc(args.bscans),
                            workload="config2: config-1 tiles (12 x 270 B-scans x 1000 A-scans x 2048 uint16) through "
-                                    "the precision form of the spectral stage (float64 background, tcgen05 "
-                                    "split-FP16 sinc, FFT, |.|), magnitudes out"),
+                                    "the precision form of the spectral stage (exact background, sinc, FFT, |.|), "
+                                    "magnitudes out"),
             "gpu_launches": int(launches),
             "roofline": {"bound": "hbm", "achieved": sinc_bytes / (ms_sinc * 1e-3) / 1e9, "peak": hbm, "unit": "GB/s",
                          "frac": sinc_bytes / (ms_sinc * 1e-3) / 1e9 / hbm, "traffic": None,
-                         "kernel": "precision stage (c): float64 background + split + tcgen05 sinc, raw in / X out",
-                         "ms_per_step": ms_sinc, "peak_source": src + " (burst copy)",
-                         "tensor": {"achieved_tflops": ascans * flops_per_ascan / (ms_sinc * 1e-3) / 1e12,
-                                    "peak_tflops": tf_peak, "flops_per_ascan": flops_per_ascan,
-                                    "note": "dense 128x64x96 MMA tiles x 3 split products; time of the whole stage"}},
+                         "kernel": "precision stage (c): exact background + sinc (k_apod_mean, k_lines), raw in / X out",
+                         "ms_per_step": ms_sinc, "peak_source": src + " (burst copy)"},
             "clocks": clk,
             "float32_form": {"value": ascans / (ms_f32 * 1e-3), "unit": "A-scans/s", "ms_per_step": ms_f32}}
 

@@ -116,22 +116,22 @@ int octgb_db(octgb_ctx *ctx, const void *raw, int raw_dtype, int raw_loc, int B,
  * sum of the numerators), the sinc runs in float64 over the float64 band
  * weights given to octgb_set_geometry, then the float64 window and a float64
  * inverse FFT; |X| (n/2 bins) is rounded once to float32.  raw must be uint16
- * or int16.  Several times slower than octgb_magnitude (GB300's float64 rate is
- * a small fraction of its float32 rate); its codes match the reference's
- * float64 path to within 1 LSB. */
+ * or int16.  The arithmetic runs on pairs of float32 values (GB300's float64
+ * rate is a small fraction of its float32 rate), within ~1e-13 of the line's
+ * scale of float64; its codes match the reference's float64 path to within 1 LSB. */
 int octgb_magnitude_exact(octgb_ctx *ctx, const void *raw, int raw_dtype, int raw_loc, int B, int interf,
                           int apod_size, float *mag, int mag_loc);
 
-/* Precision form of the spectral stage: the sinc k-linearisation as a banded
- * GEMM on the tensor cores (tcgen05.mma, split-FP16 with three products,
- * float32 accumulation in TMEM; 128 A-scans x 64 output samples x a
- * 96-sample source window per block).  The background (apodisation mean, line
+/* Precision form of the spectral stage.  The background (apodisation mean, line
  * mean) is exact (integer sums; float64 for float32 raws): this form is
  * closer to the float64 path than the reference's float32 path, which rounds
- * the apodisation mean to float32 (core/cpu_kernels.py:20-25).  Requires
- * every 64-output block's
+ * the apodisation mean to float32 (core/cpu_kernels.py:20-25).  Integer raws:
+ * the float32 banded sinc of octgb_magnitude in two half sums.  Float32 raws:
+ * the sinc as a banded GEMM on the tensor cores (tcgen05.mma, split-FP16 with
+ * three products, float32 accumulation in TMEM; 128 A-scans x 64 output
+ * samples x a 96-sample source window per block).  Requires every 64-output block's
  * sinc band to fit in 96 source samples (OCTGB_ERR_STATE otherwise) and
- * |raw - apod - mean| < 65504 (the fp16 range).
+ * (float32 raws) |raw - apod - mean| < 65504 (the fp16 range).
  * octgb_linearise_precision: stage (c) only, the linearised interferogram
  *   (B, interf-apod, n) float32 without the window (SpectralProcessor.linearise,
  *   core/spectral.py:118-134);
@@ -426,7 +426,7 @@ int octgb_cnn_conv3x3_bwd(octgb_ctx *ctx, const float *x, const float *w, const 
  * float32 accumulation): dw as nine pixel-contracting GEMMs whose per-CTA
  * partial sums are added in a fixed order; dx as octgb_cnn_conv3x3_tc of dy
  * with the flipped kernel (the float32 kernel where that shape is not
- * supported); db as octgb_cnn_conv3x3_bwd.  Shapes: 1 <= cin <= 48, 1 <= cout
+ * supported); db as octgb_cnn_conv3x3_bwd, summed while dy is packed.  Shapes: 1 <= cin <= 48, 1 <= cout
  * <= 128, and a band of rows dividing h whose staged input fits in shared
  * memory (wd up to about 1000).  Asynchronous; a bounded device wait that
  * expires is reported by the next synchronising call (OCTGB_ERR_TIMEOUT). */
