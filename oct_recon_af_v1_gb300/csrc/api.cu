@@ -24,6 +24,10 @@ using namespace octgb;
 
 namespace {
 
+// the range of no values (ordered uint [max, 0]), copied to reset a range: part
+// of the library image, so that a context needs neither memory nor a copy for it
+static __device__ unsigned int g_empty_range[2] = {0xffffffffu, 0u};
+
 struct DevBuf {
     void* p = nullptr;
     size_t cap = 0;
@@ -156,7 +160,7 @@ struct octgb_ctx {
     DevBuf lines_fixed;          // the allocation-free entry point's own (kMinPass), allocated with the geometry
     // work buffers
     DevBuf raw, apod, out, mm, frames;
-    DevBuf mm_empty;             // the range of no values (ordered uint [max, 0]), copied to reset a range
+    const void* empty_range = nullptr;   // g_empty_range on the context's device
     int* status_host = nullptr;  // mapped pinned status word
     int* status_dev = nullptr;
     // plans and row state
@@ -388,7 +392,7 @@ void copy_out(octgb_ctx* c, void* dst, int loc, const void* src_dev, size_t byte
 }
 
 void reset_minmax(octgb_ctx* c, unsigned int* mm_dev) {
-    ck(cudaMemcpyAsync(mm_dev, c->mm_empty.p, 2 * sizeof(unsigned int), cudaMemcpyDeviceToDevice, c->stream),
+    ck(cudaMemcpyAsync(mm_dev, c->empty_range, 2 * sizeof(unsigned int), cudaMemcpyDeviceToDevice, c->stream),
        "reset range");
 }
 
@@ -631,9 +635,9 @@ int octgb_create(int device, octgb_ctx** out) {
         ck(cudaHostGetDevicePointer(reinterpret_cast<void**>(&c->status_dev), c->status_host, 0),
            "cudaHostGetDevicePointer");
         ck(c->mm.ensure(4096), "cudaMalloc(minmax)");
-        const unsigned int empty[2] = {0xffffffffu, 0u};
-        ck(c->mm_empty.ensure(sizeof(empty)), "cudaMalloc(empty range)");
-        ck(cudaMemcpy(c->mm_empty.p, empty, sizeof(empty), cudaMemcpyHostToDevice), "H2D empty range");
+        void* empty = nullptr;
+        ck(cudaGetSymbolAddress(&empty, g_empty_range), "cudaGetSymbolAddress(empty range)");
+        c->empty_range = empty;
         *out = c;
         g_create_error.clear();
         return OCTGB_OK;
@@ -658,7 +662,7 @@ int octgb_destroy(octgb_ctx* c) {
             delete p;
         }
     }
-    for (DevBuf* b : {&c->start, &c->win, &c->tw, &c->wsh, &c->s0, &c->lines, &c->lines_fixed, &c->raw, &c->apod, &c->out, &c->mm, &c->mm_empty, &c->frames, &c->num,
+    for (DevBuf* b : {&c->start, &c->win, &c->tw, &c->wsh, &c->s0, &c->lines, &c->lines_fixed, &c->raw, &c->apod, &c->out, &c->mm, &c->frames, &c->num,
                       &c->den, &c->plan_table, &c->run_mm, &c->magbuf, &c->dbbuf, &c->planemm, &c->segs, &c->qtable,
                       &c->disp_x, &c->disp_hann, &c->disp_dk2, &c->disp_betas, &c->disp_phase, &c->disp_a, &c->disp_score, &c->xmed,
                       &c->prec_w, &c->prec_kb, &c->prec_hi, &c->prec_lo, &c->prec_m, &c->prec_x, &c->ex_w, &c->ex_win, &c->ex_tw, &c->bias_part, &c->wgrad_part, &c->prep,
