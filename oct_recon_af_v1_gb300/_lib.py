@@ -339,7 +339,7 @@ class Context:
         return out
 
     def magnitude_precision(self, raw, apod_size: int, out=None, raw_dtype=None):
-        """Precision form of magnitude(): tensor-core sinc, then window, FFT, |.|."""
+        """Precision form of magnitude(): exact background, sinc, window, FFT, |.|."""
         raw, p, loc, dt, B, interf = self._raw_args(raw, apod_size, raw_dtype)
         if out is None:
             out = np.empty((B, interf - apod_size, self.n // 2), np.float32)

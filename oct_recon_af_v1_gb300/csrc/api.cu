@@ -303,6 +303,7 @@ void transform_pass(octgb_ctx* c, LinesArgs a, float* scratch, int dtype, unsign
     a.out = scratch;
     ck(launch_lines(a, dtype, kModeReal, c->num_sms, c->stream), "lines kernel");
     DispArgs d{};
+    d.status = c->status_dev;
     d.X = a.out;
     d.phase = a.g.win;
     d.tw = a.g.tw;
@@ -1715,6 +1716,7 @@ int octgb_disp_eval(octgb_ctx* c, int n_beta, const double* betas, int b0, int n
                 A = c->disp_a.as<float>();
             }
             DispArgs a{};
+            a.status = c->status_dev;
             a.X = c->disp_x.as<float>();
             a.phase = c->disp_phase.as<float2>();
             a.tw = c->tw.as<float2>();
@@ -2168,6 +2170,7 @@ int octgb_magnitude_precision(octgb_ctx* c, const void* raw, int dtype, int loc,
         const float* X = precision_linearise(c, raw, dtype, loc, B, interf, apod);
         // window (Hann/rms x dispersion phase / N), inverse FFT, |.|: the scorer's FFT kernel
         DispArgs a{};
+        a.status = c->status_dev;
         a.X = X;
         a.phase = c->win.as<float2>();
         a.tw = c->tw.as<float2>();
@@ -2204,6 +2207,7 @@ int octgb_disp_images(octgb_ctx* c, int n_beta, const double* betas, int b0, int
         const size_t cols = static_cast<size_t>(n_beta) * nb * nx * 256;
         ck(c->disp_a.ensure(cols * sizeof(float)), "cudaMalloc(columns)");
         DispArgs a{};
+        a.status = c->status_dev;
         a.X = c->disp_x.as<float>();
         a.phase = c->disp_phase.as<float2>();
         a.tw = c->tw.as<float2>();

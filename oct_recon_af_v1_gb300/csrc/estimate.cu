@@ -40,14 +40,28 @@ namespace {
 // shared-memory path 54 %, DRAM 32 % (205 000 transforms, 41 betas).  There it
 // takes 823 us; with 128 threads an A-scan, two exchanges and four group
 // barriers the same arithmetic took 967 us.  The next line is prefetched into
-// L2 only: holding it in registers behind the last stage spilled.
+// L2 (holding it in registers behind the last stage spilled), or into shared
+// memory (below).
 constexpr int kDispWarps = 4;
+// Without pooling or repeats shared memory has room for each warp's next line:
+// one CTA of twelve warps shares the twiddles, and a bulk copy brings the line in
+// behind the transform before it, where the warps' loads took a fifth of their
+// time (823 -> 726 us).  Taken from 24 A-scans a warp on (28 a warp: 24 us of a
+// volume's last pass); below, the three smaller CTAs an SM run beside other
+// streams' kernels and end less unevenly (16 a warp: 217 us a call of the
+// precision form against 221).
+constexpr int kLineWarps = 12;
+constexpr int kLineItems = 24;
 
+template <int kWarps, bool kLine>
 struct DispSmem {
     alignas(16) float2 tw[kTwTable];                     // tw2, tw3
-    alignas(16) float2 ex[kDispWarps][kWarpExchange];
-    // followed by [kDispWarps][kHalf] floats (a line's magnitudes) with pooling or repeats
+    alignas(16) float2 ex[kWarps][kWarpExchange];
+    alignas(16) float line[kLine ? kWarps : 1][kLine ? kN : 4];
+    uint64_t bar[kWarps];
+    // followed by [kWarps][kHalf] floats (a line's magnitudes) with pooling or repeats
 };
+static_assert(sizeof(DispSmem<kLineWarps, true>) <= 232448, "k_disp_mag shared memory exceeds 227 KB");
 
 // streamed once: keep L1 for the phase row
 __device__ __forceinline__ float ld_stream(const float* p) {
@@ -57,14 +71,22 @@ __device__ __forceinline__ float ld_stream(const float* p) {
 }
 
 // Pool: probe images; Db: dB of a depth crop; Rep: several B-scan repeats (a.rep > 1)
-template <bool Pool, bool Db, bool Rep>
-__global__ void __launch_bounds__(kDispWarps * 32, 3) k_disp_mag(const DispArgs a) {
+template <bool Pool, bool Db, bool Rep, bool kLine>
+__global__ void __launch_bounds__((kLine ? kLineWarps : kDispWarps) * 32, kLine ? 1 : 3)
+    k_disp_mag(const DispArgs a) {
+    static_assert(!kLine || (!Pool && !Rep), "no room for the lines");
+    constexpr int kWarps = kLine ? kLineWarps : kDispWarps;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    DispSmem& S = *reinterpret_cast<DispSmem*>(smem_raw);
+    using Smem = DispSmem<kWarps, kLine>;
+    Smem& S = *reinterpret_cast<Smem*>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int k = tid; k < kTwTable / 2; k += kDispWarps * 32)
+    for (int k = tid; k < kTwTable / 2; k += kWarps * 32)
         reinterpret_cast<float4*>(S.tw)[k] = __ldg(reinterpret_cast<const float4*>(a.tw) + k);
     const float2 *tw2 = S.tw, *tw3 = S.tw + 256;
+    if (kLine && lane == 0) {
+        mbar_init(&S.bar[warp], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
     __syncthreads();
     pdl_wait();                                          // the lines and phase rows
     pdl_launch();
@@ -73,7 +95,7 @@ __global__ void __launch_bounds__(kDispWarps * 32, 3) k_disp_mag(const DispArgs 
     float* sums = reinterpret_cast<float*>(&S + 1) + warp * kHalf;
     // items < 2^32 - the grid's warps (the launcher checks): 32-bit item arithmetic
     const unsigned int nbx = static_cast<unsigned int>(a.nb) * static_cast<unsigned int>(a.nx);
-    const unsigned int n_items = static_cast<unsigned int>(a.n_beta) * nbx, step = gridDim.x * kDispWarps;
+    const unsigned int n_items = static_cast<unsigned int>(a.n_beta) * nbx, step = gridDim.x * kWarps;
     // repeat 0 of an item: B-scan b0 + bu, A-scan x; repeat rp is rp * nx lines further
     auto line_of = [&](unsigned int item) -> const float* {
         const unsigned int bx = item % nbx;
@@ -81,16 +103,35 @@ __global__ void __launch_bounds__(kDispWarps * 32, 3) k_disp_mag(const DispArgs 
         const unsigned int x = bx - bu * static_cast<unsigned int>(a.nx);
         return a.X + ((static_cast<int64_t>(a.b0 + static_cast<int>(bu)) * a.rep) * a.nx + x) * kN;
     };
-    for (unsigned int item = blockIdx.x * kDispWarps + warp; item < n_items; item += step) {
+    const unsigned int first = blockIdx.x * kWarps + warp;
+    auto copy_line = [&](unsigned int item) {                // by lane 0
+        mbar_expect_tx(&S.bar[warp], kN * sizeof(float));
+        tma_bulk_g2s(S.line[warp], line_of(item), kN * sizeof(float), &S.bar[warp]);
+    };
+    if (kLine && lane == 0 && first < n_items) copy_line(first);
+    uint32_t parity = 0;
+    for (unsigned int item = first; item < n_items; item += step, parity ^= 1u) {
         const float2* ph = a.phase + static_cast<int64_t>(item / nbx) * kN + lane;
         const float* line = line_of(item) + lane;
         float* out = Pool ? sums : a.A + static_cast<int64_t>(item) * (Db ? a.nz : kHalf);
         // the warp's next line into L2 behind this one's transform
-        if (!Rep && lane == 0 && item + step < n_items) bulk_prefetch_l2(line_of(item + step), kN * sizeof(float));
+        if (!kLine && !Rep && lane == 0 && item + step < n_items) bulk_prefetch_l2(line_of(item + step), kN * sizeof(float));
         for (int rp = 0; rp < (Rep ? a.rep : 1); ++rp, line += static_cast<int64_t>(a.nx) * kN) {
             float2 v[64];
 #pragma unroll
-            for (int r = 0; r < 64; ++r) v[r].x = ld_stream(line + 32 * r);
+            for (int r = 0; r < 64; ++r)
+                if (!kLine) v[r].x = ld_stream(line + 32 * r);
+            if (kLine) {
+                const bool ok = mbar_wait_bounded(&S.bar[warp], parity, a.status);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    mbar_wait_bounded(&S.bar[warp], parity, a.status);   // the copy lands before the CTA ends
+                    return;
+                }
+#pragma unroll
+                for (int r = 0; r < 64; ++r) v[r].x = S.line[warp][lane + 32 * r];
+                __syncwarp();
+                if (lane == 0 && item + step < n_items) copy_line(item + step);
+            }
 #pragma unroll
             for (int r = 0; r < 64; ++r) {
                 const float2 p = __ldg(ph + 32 * r);
@@ -541,20 +582,29 @@ cudaError_t launch_xmedian_t(const float* mag, int n_frames, int nx, int nz, int
 }  // namespace
 
 cudaError_t launch_disp_mag(const DispArgs& a, int num_sms, cudaStream_t st) {
-    const size_t smem = sizeof(DispSmem) + (a.zcol != nullptr || a.rep > 1 ? kDispWarps * kHalf * sizeof(float) : 0);
     if (a.mode == kModeDb && (a.rep > 1 || a.zcol != nullptr)) return cudaErrorInvalidValue;
-    const auto kernel = a.mode == kModeDb   ? k_disp_mag<false, true, false>
-                        : a.zcol != nullptr ? (a.rep > 1 ? k_disp_mag<true, false, true> : k_disp_mag<true, false, false>)
-                        : a.rep > 1         ? k_disp_mag<false, false, true>
-                                            : k_disp_mag<false, false, false>;
-    const int bit = a.mode == kModeDb ? 4 : (a.zcol != nullptr ? 2 : 0) + (a.rep > 1 ? 1 : 0);
+    const int64_t items = static_cast<int64_t>(a.n_beta) * a.nb * a.nx;
+    if (items >= (int64_t(1) << 32) - 12 * num_sms) return cudaErrorInvalidValue;   // 32-bit item index
+    const bool extra = a.zcol != nullptr || a.rep > 1;
+    const bool line = !extra && items >= static_cast<int64_t>(kLineItems) * kLineWarps * num_sms;
+    const int warps = line ? kLineWarps : kDispWarps, per_sm = line ? 1 : 3;
+    const size_t smem = line ? sizeof(DispSmem<kLineWarps, true>)
+                             : sizeof(DispSmem<kDispWarps, false>) + (extra ? kDispWarps * kHalf * sizeof(float) : 0);
+    const auto kernel = a.mode == kModeDb   ? (line ? k_disp_mag<false, true, false, true>
+                                                    : k_disp_mag<false, true, false, false>)
+                        : a.zcol != nullptr ? (a.rep > 1 ? k_disp_mag<true, false, true, false>
+                                                         : k_disp_mag<true, false, false, false>)
+                        : a.rep > 1         ? k_disp_mag<false, false, true, false>
+                        : line              ? k_disp_mag<false, false, false, true>
+                                            : k_disp_mag<false, false, false, false>;
+    const int bit = line                  ? (a.mode == kModeDb ? 6 : 5)
+                    : a.mode == kModeDb ? 4
+                                        : (a.zcol != nullptr ? 2 : 0) + (a.rep > 1 ? 1 : 0);
     const cudaError_t e = kernel_ready(a.ready, kReadyDisp + bit, kernel, smem);
     if (e != cudaSuccess) return e;
-    const int64_t items = static_cast<int64_t>(a.n_beta) * a.nb * a.nx;
-    if (items >= (int64_t(1) << 32) - 3 * kDispWarps * num_sms) return cudaErrorInvalidValue;   // 32-bit item index
-    int64_t grid = (items + kDispWarps - 1) / kDispWarps;
-    if (grid > 3 * num_sms) grid = 3 * num_sms;
-    return launch_dependent(kernel, dim3(static_cast<unsigned int>(grid)), dim3(kDispWarps * 32), smem, st, a);
+    const int64_t most = static_cast<int64_t>(per_sm) * num_sms, want = (items + warps - 1) / warps;
+    const unsigned int grid = static_cast<unsigned int>(want < most ? want : most);
+    return launch_dependent(kernel, dim3(grid), dim3(warps * 32), smem, st, a);
 }
 
 cudaError_t launch_phase(const double* betas, const double* dk2, int n, float2* phase, cudaStream_t st) {

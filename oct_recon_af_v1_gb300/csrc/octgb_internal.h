@@ -98,8 +98,8 @@ inline cudaError_t kernel_ready(uint64_t* ready, int bit, Kernel kernel, size_t 
     if (e == cudaSuccess) *ready |= uint64_t(1) << bit;
     return e;
 }
-// bits 0 .. 47: k_lines, 48 .. 52: k_disp_mag, 53 .. 60: k_lines with the exact background
-constexpr int kReadyDisp = 48, kReadyExact = 53;
+// bits 0 .. 47: k_lines, 48 .. 54: k_disp_mag, 55 .. 62: k_lines with the exact background
+constexpr int kReadyDisp = 48, kReadyExact = 55;
 
 // lines.cu: A-scans [l0, l1) of n_seg raw batches of one shape, or of tiles of
 // uneven size (qt), numbered segment by segment, B-scan by B-scan
@@ -230,6 +230,7 @@ struct DispArgs {
     float* zcol;           // (n_beta, nb, nx, 256) depth-pooled sums of |X| (probe images), or null
     int z_keep;            // depths pooled into the 256 image rows
     int n_beta, nb, b0, nx, rep;
+    int* status;           // where a wait that runs out is recorded
     uint64_t* ready;       // host: bits of the caller's context, see kernel_ready
 };
 cudaError_t launch_disp_mag(const DispArgs& a, int num_sms, cudaStream_t st);

@@ -442,3 +442,27 @@ def test_adam_list(gpu_ctx):
                                                    1e-8, 3))
     gpu_ctx.synchronize()
     assert all(torch.equal(a, b) for x, y in zip(one, many) for a, b in zip(x, y))
+
+
+@pytest.mark.parametrize("n", [24 * 12 * 152 - 1, 24 * 12 * 152, 24 * 12 * 152 + 12 * 152 + 5])
+def test_transform_with_lines_in_shared_memory(gpu_ctx, n):
+    """From 24 A-scans a warp on the transform takes its lines from shared
+    memory: every A-scan equals, bit for bit, its magnitudes in a call of few
+    A-scans (the same operations), on either side of the rule."""
+    torch = pytest.importorskip("torch")
+    from oct_recon_af_v1_gb300 import geometry as G
+    from oct_recon_af_v1_gb300 import synthetic
+    sg = G.build_spectral_geometry(synthetic.lambda_nm(), 0.0, 1.33)
+    gpu_ctx.set_geometry(sg.sinc_idx, sg.sinc_w, sg.window)
+    raw = torch.randint(0, 65536, (1, n + 1, 2048), generator=torch.Generator().manual_seed(1)).to(torch.uint16).cuda()
+    mag = torch.full((1, n, 1024), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    gpu_ctx.magnitude(raw, 1, mag, raw_dtype=0)
+    small = torch.empty((1, 500, 1024), device="cuda")
+    for lo in (0, n // 2, n - 500):
+        part = torch.cat([raw[:, :1], raw[:, 1 + lo:501 + lo]], 1).contiguous()
+        torch.cuda.synchronize()
+        gpu_ctx.magnitude(part, 1, small, raw_dtype=0)
+        gpu_ctx.synchronize()
+        assert torch.equal(mag[:, lo:lo + 500], small)
+    assert torch.isfinite(mag).all()
