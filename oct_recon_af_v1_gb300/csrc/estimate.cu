@@ -89,7 +89,9 @@ __global__ void __launch_bounds__((kLine ? kLineWarps : kDispWarps) * 32, kLine 
     }
     __syncthreads();
     pdl_wait();                                          // the lines and phase rows
-    pdl_launch();
+    // kLine: the kernel after this one starts when it ends (started early, the
+    // next pass's lines kernel cost a precision volume's tile 1882 -> 2012 us)
+    if (!kLine) pdl_launch();
     float run_min = __int_as_float(0x7f800000), run_max = -__int_as_float(0x7f800000);
     float2* ex = S.ex[warp];
     float* sums = reinterpret_cast<float*>(&S + 1) + warp * kHalf;
