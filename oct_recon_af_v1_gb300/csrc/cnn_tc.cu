@@ -962,7 +962,8 @@ bool conv_geom(int n, int cin, int cout, int H, int W, int pool, bool mask, int 
         if (g.wide && (Ws % kCM != 0 || W % Ws != 0)) return false;
         if (mask && (Ws != W || R % 2 != 0)) return false;
         band_set(g.b, n, R, Ws);
-        if (g.b.rp > kMaxBox) return false;
+        // (a converter thread takes kCPix pixels of a block)
+        if (g.b.rp > kMaxBox || (R + 2) * g.b.Wp > kCPix * 32 * kCConv) return false;
         // staged pixels; W < 128: the last tile reads on past them (rows that are not written)
         const int last = (R * g.b.Wp + kCM - 1) / kCM * kCM + 2 * g.b.Wp + 2;
         g.xpix = g.wide ? (R + 2) * g.b.Wp : (last > (R + 2) * g.b.Wp ? last : (R + 2) * g.b.Wp);
@@ -1015,6 +1016,9 @@ bool wgrad_geom(int n, int cin, int cout, int H, int W, bool pool, int num_sms, 
         band_set(g.b, n, R, Ws);
         if (g.b.rp > kMaxBox) return false;
         g.stage = stage_bytes(R, g.b.Wp, g.Q, g.xpix, g.xbytes);
+        // (a converter thread takes kWPix pixels of x and kWDy steps of dy; rows of
+        // three pixels are staged eight apart, and 146 of them would be 37 steps of 32)
+        if (g.xpix > kWPix * 32 * kWConv || g.Q > kWDy * 32 * (kWConv / 2)) return false;
         g.rpd = g.b.nseg == 1 ? W : Ws;
         g.rawd = R * g.rpd;
         const int xc = cin < 8 ? cin : 8, dc = cout < 8 ? cout : 8;

@@ -352,6 +352,14 @@ def test_weight_gradient_bands(gpu_ctx, n, cin, cout, h, w, shift):
             <= 1e-4 * dy.double().abs().sum((0, 2, 3)).numpy()).all()
 
 
+@pytest.mark.parametrize("n,cin,cout,h,w", [(304, 3, 8, 146, 3), (400, 9, 16, 141, 3), (152, 1, 1, 292, 3),
+                                            (304, 4, 8, 93, 7), (304, 2, 9, 200, 1)])
+def test_weight_gradient_of_narrow_images(gpu_ctx, n, cin, cout, h, w):
+    """Images a few pixels wide, enough of them that a band holds as many rows
+    as its staging takes: the comparison and tolerance of the test above."""
+    test_weight_gradient_bands(gpu_ctx, n, cin, cout, h, w, 0)
+
+
 @pytest.mark.parametrize("n,cin,cout,h,w,shift", [(1, 3, 32, 6, 640, 0), (2, 16, 40, 2, 264, 1), (3, 33, 9, 10, 128, 0),
                                                   (90, 5, 1, 8, 8, 0), (1, 48, 128, 4, 136, 0), (130, 3, 32, 14, 128, 2)])
 def test_weight_gradient_through_pool(gpu_ctx, n, cin, cout, h, w, shift):
