@@ -116,9 +116,9 @@ int octgb_db(octgb_ctx *ctx, const void *raw, int raw_dtype, int raw_loc, int B,
  * sum of the numerators), the sinc runs in float64 over the float64 band
  * weights given to octgb_set_geometry, then the float64 window and a float64
  * inverse FFT; |X| (n/2 bins) is rounded once to float32.  raw must be uint16
- * or int16.  The arithmetic runs on pairs of float32 values (GB300's float64
- * rate is a small fraction of its float32 rate), within ~1e-13 of the line's
- * scale of float64; its codes match the reference's float64 path to within 1 LSB. */
+ * or int16.  Several times slower than octgb_magnitude (GB300's float64 rate is
+ * a small fraction of its float32 rate); its codes match the reference's
+ * float64 path to within 1 LSB. */
 int octgb_magnitude_exact(octgb_ctx *ctx, const void *raw, int raw_dtype, int raw_loc, int B, int interf,
                           int apod_size, float *mag, int mag_loc);
 

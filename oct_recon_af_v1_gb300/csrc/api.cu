@@ -804,35 +804,24 @@ int octgb_set_geometry(octgb_ctx* c, int n, int taps, const int64_t* idx, const 
            "H2D wsh");
         ck(cudaMemcpyAsync(c->s0.p, s0v.data(), s0v.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream),
            "H2D s0");
-        // float64 form: the band weights as given (tap-major), window / N and
-        // twiddles from float64, each as a pair of float32 (hi + lo)
+        // float64 form: the band weights as given (tap-major), window / N and twiddles in float64
         {
-            auto lo = [](double v) { return static_cast<float>(v - static_cast<double>(static_cast<float>(v))); };
-            auto pair = [&](double re, double im) {
-                return make_float4(static_cast<float>(re), static_cast<float>(im), lo(re), lo(im));
-            };
-            std::vector<float2> wd(static_cast<size_t>(taps) * kN, make_float2(0.f, 0.f));
-            std::vector<float4> wind(kN), rootd(kN), twd(kTwTable);
+            std::vector<double> wd(static_cast<size_t>(taps) * kN, 0.0);
+            std::vector<double2> wind(kN), twd(kN);
             for (int i = 0; i < kN; ++i) {
-                for (int t = 0; t < len[i]; ++t) {
-                    const double v = w[static_cast<size_t>(i) * taps + t];
-                    wd[static_cast<size_t>(t) * kN + i] = make_float2(static_cast<float>(v), lo(v));
-                }
-                wind[i] = pair(window[2 * i] * (1.0 / kN), window[2 * i + 1] * (1.0 / kN));
+                for (int t = 0; t < len[i]; ++t) wd[static_cast<size_t>(t) * kN + i] = w[static_cast<size_t>(i) * taps + t];
+                wind[i] = make_double2(window[2 * i] * (1.0 / kN), window[2 * i + 1] * (1.0 / kN));
                 const double ang = 2.0 * 3.14159265358979323846 * i / kN;
-                rootd[i] = pair(cos(ang), sin(ang));
+                twd[i] = make_double2(cos(ang), sin(ang));
             }
-            for (int k = 0; k < 256; ++k) twd[k] = rootd[(k >> 4) * (k & 15) * (kN / 256) % kN];
-            for (int k = 0; k < 7 * 256; ++k) twd[256 + k] = rootd[((k >> 8) + 1) * (k & 255) % kN];
-            ck(c->ex_w.ensure(wd.size() * sizeof(float2)), "cudaMalloc(float64 weights)");
-            ck(c->ex_win.ensure(wind.size() * sizeof(float4)), "cudaMalloc(float64 window)");
-            ck(c->ex_tw.ensure(twd.size() * sizeof(float4)), "cudaMalloc(float64 twiddles)");
-            ck(cudaMemcpyAsync(c->ex_w.p, wd.data(), wd.size() * sizeof(float2), cudaMemcpyHostToDevice, c->stream),
+            ck(c->ex_w.ensure(wd.size() * sizeof(double)), "cudaMalloc(float64 weights)");
+            ck(c->ex_win.ensure(kN * sizeof(double2)), "cudaMalloc(float64 window)");
+            ck(c->ex_tw.ensure(kN * sizeof(double2)), "cudaMalloc(float64 twiddles)");
+            ck(cudaMemcpyAsync(c->ex_w.p, wd.data(), wd.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream),
                "H2D float64 weights");
-            ck(cudaMemcpyAsync(c->ex_win.p, wind.data(), wind.size() * sizeof(float4), cudaMemcpyHostToDevice,
-                               c->stream),
+            ck(cudaMemcpyAsync(c->ex_win.p, wind.data(), kN * sizeof(double2), cudaMemcpyHostToDevice, c->stream),
                "H2D float64 window");
-            ck(cudaMemcpyAsync(c->ex_tw.p, twd.data(), twd.size() * sizeof(float4), cudaMemcpyHostToDevice, c->stream),
+            ck(cudaMemcpyAsync(c->ex_tw.p, twd.data(), kN * sizeof(double2), cudaMemcpyHostToDevice, c->stream),
                "H2D float64 twiddles");
             ck(cudaStreamSynchronize(c->stream), "sync float64 geometry");
         }
@@ -2136,10 +2125,10 @@ int octgb_magnitude_exact(octgb_ctx* c, const void* raw, int dtype, int loc, int
         a.nx = nx;
         a.n_ascans = static_cast<int64_t>(B) * nx;
         a.start = c->start.as<int>();
-        a.w = c->ex_w.as<float2>();
+        a.w = c->ex_w.as<double>();
         a.taps = c->taps;
-        a.win = c->ex_win.as<float4>();
-        a.tw = c->ex_tw.as<float4>();
+        a.win = c->ex_win.as<double2>();
+        a.tw = c->ex_tw.as<double2>();
         a.mag = dst;
         ck(launch_exact(a, dtype, c->apod.as<int>(), c->num_sms, c->stream), "float64 spectral kernels");
         c->launches += 2;

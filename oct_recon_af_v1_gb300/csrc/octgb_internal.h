@@ -70,12 +70,10 @@ struct ExactArgs {
     int64_t n_ascans;         // B * nx
     const int* apod_sum;      // (B, kN) integer sums of the apodisation lines (filled by launch_exact)
     const int* start;         // [kN] first source sample of each output
-    // pairs of float32, value = first + second (complex: re, im, re low, im low)
-    const float2* w;          // [taps][kN] band weights, tap-major (padding 0)
+    const double* w;          // [taps][kN] float64 band weights, tap-major (padding 0)
     int taps;
-    const float4* win;        // [kN] window / kN
-    const float4* tw;         // [kTwTable] twiddles of the transform
-    float inv_h, inv_l;       // 1 / (2048 apod), set by the launcher
+    const double2* win;       // [kN] window / kN, float64 complex
+    const double2* tw;        // [kN] exp(+2 pi i k / kN), float64
     float* mag;               // (n_ascans, kHalf) |X| rounded to float32
 };
 cudaError_t launch_exact(const ExactArgs& a, int dtype, int* sums, int num_sms, cudaStream_t st);

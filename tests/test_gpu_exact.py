@@ -76,3 +76,26 @@ def test_float64_form_rejects_float_raws(gpu_ctx, case):
     with pytest.raises(_lib.OctgbError) as e:
         gpu_ctx.magnitude_exact(c["raw"][:1].astype(np.float32), 25)
     assert e.value.code == _lib.ERR_ARG and "integer raws" in str(e.value)
+
+
+def test_float64_form_keeps_bins_far_below_the_largest(gpu_ctx):
+    """A ramp of counts under a Hann window, linearised by the identity: its
+    spectrum falls to 1e-9 of the largest bin, and float64 arithmetic resolves
+    that.  Tolerance: the output's rounding, and 2^-53 of the line's largest
+    value: eleven layers' roundings of 2048 values average to sqrt(11 / 2048) =
+    0.07 of that in a bin, the largest of 3072 bins on either side to some
+    ten times more."""
+    n = 2048
+    idx = np.arange(n)[:, None]
+    win = np.hanning(n)
+    gpu_ctx.set_geometry(idx, np.ones((n, 1)), win.astype(complex))
+    raw = np.zeros((1, 4, n), np.uint16)
+    raw[0, 1] = 16 * np.arange(n)
+    raw[0, 2] = 65535
+    raw[0, 3] = raw[0, 1, ::-1]
+    line = raw[0, 1:].astype(np.float64) * win
+    ref = np.abs(np.fft.ifft(line))[:, :n // 2]
+    got = gpu_ctx.magnitude_exact(raw, 1)[0].astype(np.float64)
+    scale = np.abs(line).max(-1, keepdims=True)
+    assert ref.min() < 1e-9 * ref.max()
+    assert (np.abs(got - ref) <= 2.0 ** -24 * ref + 2.0 ** -53 * scale).all()
