@@ -295,6 +295,10 @@ int octgb_graph_launch(octgb_ctx *ctx, int graph_id);
  * OCTGB_ERR_STATE if the wait did not expire; the limit and switch are
  * restored either way and the context stays usable. */
 int octgb_selftest_wait_expiry(octgb_ctx *ctx, int which, int wait_limit_us);
+/* The same for the stitch kernel: one frame of zero magnitudes through a plan
+ * without optical-path correction, each block's first barrier expecting 16
+ * bytes more than its tensor copies deliver. */
+int octgb_selftest_stitch_wait_expiry(octgb_ctx *ctx, int plan_id, int wait_limit_us);
 
 /* Destroy every graph captured on the context (after the work already
  * launched has completed); their ids become invalid and octgb_set_geometry is

@@ -52,6 +52,7 @@ SIGNATURES = {
     "octgb_graphs_release": (c_int, [c_void_p]),
     "octgb_set_stitch_rows": (c_int, [c_void_p, c_int]),
     "octgb_selftest_wait_expiry": (c_int, [c_void_p, c_int, c_int]),
+    "octgb_selftest_stitch_wait_expiry": (c_int, [c_void_p, c_int, c_int]),
     "octgb_magnitude_noalloc": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
     "octgb_batch_process": (c_int, [c_void_p, c_int, c_void_p, c_int, c_float, c_int]),
     "octgb_disp_load": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]),

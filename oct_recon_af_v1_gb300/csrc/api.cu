@@ -2097,6 +2097,47 @@ int octgb_linearise_precision(octgb_ctx* c, const void* raw, int dtype, int loc,
     });
 }
 
+int octgb_selftest_stitch_wait_expiry(octgb_ctx* c, int plan_id, int wait_limit_us) {
+    return guarded(c, [&] {
+        require(plan_id >= 0 && plan_id < static_cast<int>(c->plans.size()), "bad plan id");
+        require(wait_limit_us >= 100 && wait_limit_us <= 2000000, "wait_limit_us must be in [100, 2000000]");
+        const Plan& p = *c->plans[plan_id];
+        require(p.row_table.tma, "the plan's patches are not staged by tensor copies");
+        if (c->capturing) throw Error(OCTGB_ERR_STATE, "self-test during graph capture");
+        // one frame of zero magnitudes
+        const size_t mags = static_cast<size_t>(p.n_tile_x) * kHalf * sizeof(float);
+        const int n_out_x = p.c0 + p.C;
+        ck(c->magbuf.ensure(mags), "cudaMalloc(mag)");
+        ck(c->dbbuf.ensure(static_cast<size_t>(p.n_out_z) * n_out_x * sizeof(float)), "cudaMalloc(db)");
+        ck(cudaMemsetAsync(c->magbuf.p, 0, mags, c->stream), "memset mag");
+        StitchArgs a{};
+        a.tiles.n = 1;
+        a.tiles.id[0] = plan_id;
+        a.mag = c->magbuf.as<float>();
+        stitch_table_args(c, a, p.row_table, p.n_tile_x);
+        a.n_tile_x = p.n_tile_x;
+        a.n_out_z = p.n_out_z;
+        a.n_out_x = n_out_x;
+        a.cblk0 = p.cblk_first;
+        a.db = c->dbbuf.as<float>();
+        a.starve = 16;
+        constexpr unsigned long long kDefaultLimit = 2000000000ull;
+        ck(set_wait_test_stitch(static_cast<unsigned long long>(wait_limit_us) * 1000ull, c->stream),
+           "set wait limit");
+        try {
+            ck(launch_stitch(c->plan_table.as<StitchDev>(), a, p.row_table.smem, p.n_cblk, 1, p.row_rows, c->stream),
+               "stitch kernel");
+            c->launches++;
+            check_status(c);                    // a wait that expired throws OCTGB_ERR_TIMEOUT here
+        } catch (...) {
+            set_wait_test_stitch(kDefaultLimit, c->stream);
+            throw;
+        }
+        ck(set_wait_test_stitch(kDefaultLimit, c->stream), "restore wait limit");
+        throw Error(OCTGB_ERR_STATE, "self-test: the starved wait of the stitch did not expire");
+    });
+}
+
 int octgb_magnitude_exact(octgb_ctx* c, const void* raw, int dtype, int loc, int B, int interf, int apod, float* mag,
                           int mag_loc) {
     return guarded(c, [&] {

@@ -184,6 +184,7 @@ struct StitchArgs {
     int tile_lines;               // lines of `mag` per tile,
     int64_t n_lines;              // and in all
     int* status;                  // device status word (bounded waits)
+    uint32_t starve;              // self-test: bytes the first round's barrier expects beyond its copies
     const float* mag;             // tile t, frame f, A-scan x at t mag_tile_stride + (f n_tile_x + x) kHalf
     int64_t mag_tile_stride;
     int n_tile_x, f0, n_out_z, n_out_x;
@@ -378,6 +379,7 @@ __host__ __device__ inline float ord2f(unsigned int u) {
 // octgb_device.cuh); only octgb_selftest_wait_expiry calls these
 cudaError_t set_wait_test_spectral(unsigned long long limit_ns, int starve, cudaStream_t st);
 cudaError_t set_wait_test_precision(unsigned long long limit_ns, int starve, cudaStream_t st);
+cudaError_t set_wait_test_stitch(unsigned long long limit_ns, cudaStream_t st);
 cudaError_t set_wait_test_cnn(unsigned long long limit_ns, int starve, cudaStream_t st);
 
 }  // namespace octgb

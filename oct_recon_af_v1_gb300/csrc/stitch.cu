@@ -369,7 +369,8 @@ __global__ void __launch_bounds__(kStThreads, kFZ == 128 ? 3 : 5) k_stitch_tma(c
         if (round > 0) __syncthreads();                              // the previous round has been read
         if (warp == 0) {
             if (lane == 0)
-                mbar_expect_tx(&bar, static_cast<uint32_t>(n) * (a.pitch * a.box_lines * 4 + kFZ * 24 + kBlk * 16));
+                mbar_expect_tx(&bar, static_cast<uint32_t>(n) * (a.pitch * a.box_lines * 4 + kFZ * 24 + kBlk * 16) +
+                                         (round == 0 ? a.starve : 0u));
             __syncwarp();
             if (lane < n) {
                 const StitchTmaSlot& s = slot[k0 + lane];
@@ -385,7 +386,10 @@ __global__ void __launch_bounds__(kStThreads, kFZ == 128 ? 3 : 5) k_stitch_tma(c
                 tma_bulk_g2s(d + col_off, s.xcol, kBlk * 16, &bar);
             }
         }
-        if (!mbar_wait_bounded(&bar, round & 1, a.status)) return;
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bar, round & 1, a.status))) {
+            mbar_wait_bounded(&bar, round & 1, a.status);    // the copies land before the CTA ends
+            return;
+        }
         for (int kr = 0; kr < n; ++kr) {
             const StitchTmaSlot& s = slot[k0 + kr];
             const unsigned char* d = sm + kr * a.slot_bytes;
@@ -859,6 +863,10 @@ cudaError_t launch_resample(const QueueTile* qt, int n_qt, unsigned int l0, unsi
     if (l0 == l1) return cudaSuccess;
     k_resample<<<(l1 - l0 + kResLines - 1) / kResLines, kResThreads, 0, st>>>(qt, n_qt, l0, l1, mag, thr, run_mm);
     return cudaGetLastError();
+}
+
+cudaError_t set_wait_test_stitch(unsigned long long limit_ns, cudaStream_t st) {
+    return set_wait_test_here(limit_ns, 0, st);
 }
 
 cudaError_t launch_minmax_init(unsigned int* mm, int count, cudaStream_t st) {
