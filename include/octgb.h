@@ -310,6 +310,14 @@ int octgb_graphs_release(octgb_ctx *ctx);
  * autotuner picks the fastest for a workload.  Graphs already captured keep
  * the shape they were captured with.  Not during graph capture. */
 int octgb_set_stitch_rows(octgb_ctx *ctx, int rows);
+/* A-scans of one pass of the spectral stage at most (64 .. 91 200, 0: the
+ * default of 91 200).  A pass keeps 8 KiB of linearised spectrum per A-scan
+ * (the batched form 12 KiB) on the device, so a lower value bounds the
+ * context's scratch; scratch beyond it is given back unless a captured graph may
+ * hold it.  Results do not depend on it.  octgb_set_geometry makes room for
+ * 29 184 + 3648 A-scans (256 MiB) at most, calls of more A-scans for up to 91 200
+ * (712 MiB); a device short of memory holds fewer and takes more passes. */
+int octgb_set_pass_lines(octgb_ctx *ctx, int lines);
 
 /* ---------------------------------------------------------------- batched form */
 

@@ -50,6 +50,7 @@ SIGNATURES = {
     "octgb_graph_end": (c_int, [c_void_p, POINTER(c_int)]),
     "octgb_graph_launch": (c_int, [c_void_p, c_int]),
     "octgb_graphs_release": (c_int, [c_void_p]),
+    "octgb_set_pass_lines": (c_int, [c_void_p, c_int]),
     "octgb_set_stitch_rows": (c_int, [c_void_p, c_int]),
     "octgb_selftest_wait_expiry": (c_int, [c_void_p, c_int, c_int]),
     "octgb_selftest_stitch_wait_expiry": (c_int, [c_void_p, c_int, c_int]),
@@ -580,6 +581,11 @@ class Context:
     def set_stitch_rows(self, rows: int):
         """Output rows per block of frames_process's stitch kernel (32, 64 or 128; results do not depend on it)."""
         self._check(self.lib.octgb_set_stitch_rows(self.h, int(rows)))
+
+    def set_pass_lines(self, lines: int = 0):
+        """A-scans of one pass of the spectral stage at most (64 to 91 200, 0: the default), which bounds
+        the context's scratch; results do not depend on it."""
+        self._check(self.lib.octgb_set_pass_lines(self.h, int(lines)))
 
     # -------------------------------------------------------------- batched form
     def batch_process(self, tiles, threshold: float, grab: int = 4, raw_dtype: int = U16):

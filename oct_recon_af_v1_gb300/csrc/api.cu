@@ -46,6 +46,20 @@ struct DevBuf {
         if (e == cudaSuccess) cap = bytes;
         return e;
     }
+    // grows while the old allocation stands: without room it is kept as it is
+    bool try_grow(size_t bytes) {
+        void* q = nullptr;
+        if (cudaMalloc(&q, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (p) {
+            if (keep_old) retired.push_back(p); else cudaFree(p);
+        }
+        p = q;
+        cap = bytes;
+        return true;
+    }
     void release() {
         if (p) cudaFree(p);
         for (void* q : retired) cudaFree(q);
@@ -145,6 +159,7 @@ struct octgb_ctx {
     int device = 0;
     int num_sms = 0;
     int stitch_rows = kStitchRows;           // frame-batch stitch block height (octgb_set_stitch_rows)
+    int pass_limit = kMaxPass;               // A-scans of a pass at most (octgb_set_pass_lines)
     cudaStream_t own = nullptr;
     cudaStream_t stream = nullptr;
     std::string err;
@@ -287,11 +302,29 @@ LinesArgs lines_args(octgb_ctx* c, const void* const* segs, int n_seg, int B, in
     return a;
 }
 
-// A-scans of a pass of a call of `total`; the scratch grows to hold them.
+// Rows (of `row` floats) of a pass of `want` that `buf` holds, grown to hold
+// them: to no more than a quarter of the free memory, and where that is not to
+// be had to half as many, and so on.  A buffer that holds a shortest pass does
+// not grow during a capture (nodes captured before may hold its address).
+unsigned int scratch_rows(octgb_ctx* c, DevBuf& buf, unsigned int want, size_t row, const char* what) {
+    const size_t bytes = row * sizeof(float);
+    want = std::min(want, static_cast<unsigned int>(c->pass_limit));
+    const unsigned int least = std::min<unsigned int>(want, kLeastPass);
+    const unsigned int have = static_cast<unsigned int>(std::min<size_t>(buf.cap / bytes, want));
+    if (have == want || (c->capturing && have >= least)) return have;
+    size_t free_bytes = 0, all = 0;
+    ck(cudaMemGetInfo(&free_bytes, &all), "cudaMemGetInfo");
+    unsigned int rows = static_cast<unsigned int>(std::min<size_t>(want, std::max<size_t>(least, free_bytes / 4 / bytes)));
+    while (rows > have && !buf.try_grow(rows * bytes)) {
+        if (rows == least) throw Error(OCTGB_ERR_CUDA, std::string("no device memory: ") + what);
+        rows = std::max(rows / 2, least);
+    }
+    return std::max(rows, have);
+}
+
+// A-scans of a pass of a call of `total`
 unsigned int pass_lines(octgb_ctx* c, unsigned int total) {
-    const unsigned int pass = std::min<unsigned int>(total, kMaxPass);
-    ck(c->lines.ensure(static_cast<size_t>(pass) * kN * sizeof(float)), "cudaMalloc(lines)");
-    return pass;
+    return scratch_rows(c, c->lines, std::min<unsigned int>(total, kMaxPass), kN, "cudaMalloc(lines)");
 }
 
 // Linearised lines of A-scans [l0, l1) into `scratch`, then their transform:
@@ -338,7 +371,10 @@ void launch_spectral_segs(octgb_ctx* c, const void* const* segs, int n_seg, int 
     a.exact = exact;
     ck(launch_apod_mean(a, dtype, n_seg * B, apod_mean, c->stream), "apod kernel");
     c->launches++;
-    const unsigned int total = static_cast<unsigned int>(n), pass = fixed ? kMinPass : pass_lines(c, total);
+    const unsigned int total = static_cast<unsigned int>(n);
+    const unsigned int pass =
+        !fixed ? pass_lines(c, total)
+               : static_cast<unsigned int>(std::min<size_t>(c->lines_fixed.cap / (kN * sizeof(float)), c->pass_limit));
     float* scratch = (fixed ? c->lines_fixed : c->lines).as<float>();
     const int64_t row = mode == kModeDb ? nz : kHalf;
     for (unsigned int l0 = 0, l1; l0 < total; l0 = l1) {
@@ -790,8 +826,9 @@ int octgb_set_geometry(octgb_ctx* c, int n, int taps, const int64_t* idx, const 
         // tw2[16 r + j] = w^(r j N/256), tw3[256 (r - 1) + j] = w^(r j), w = e^(2 pi i / N)
         for (int k = 0; k < 256; ++k) tw[k] = root[(k >> 4) * (k & 15) * (kN / 256) % kN];
         for (int k = 0; k < 7 * 256; ++k) tw[256 + k] = root[((k >> 8) + 1) * (k & 255) % kN];
-        ck(c->lines.ensure(static_cast<size_t>(kFirstPass) * kN * sizeof(float)), "cudaMalloc(lines)");
-        ck(c->lines_fixed.ensure(static_cast<size_t>(kMinPass) * kN * sizeof(float)), "cudaMalloc(lines)");
+        c->lines_fixed.keep_old = true;          // the caller's own graphs may hold it
+        scratch_rows(c, c->lines_fixed, kMinPass, kN, "cudaMalloc(lines)");
+        scratch_rows(c, c->lines, kFirstPass, kN, "cudaMalloc(lines)");
         ck(c->start.ensure(kN * sizeof(int)), "cudaMalloc(start)");
         ck(c->win.ensure(kN * sizeof(float2)), "cudaMalloc(win)");
         ck(c->tw.ensure(kTwTable * sizeof(float2)), "cudaMalloc(tw)");
@@ -1518,6 +1555,17 @@ int octgb_graphs_release(octgb_ctx* c) {
     });
 }
 
+int octgb_set_pass_lines(octgb_ctx* c, int lines) {
+    return guarded(c, [&] {
+        if (c->capturing) throw Error(OCTGB_ERR_STATE, "octgb_set_pass_lines during graph capture");
+        require(lines == 0 || (lines >= 64 && lines <= kMaxPass), "pass lines must be 0 (default) or in [64, 91200]");
+        c->pass_limit = lines == 0 ? kMaxPass : lines;
+        // scratch beyond the limit goes back (unless a graph may hold it)
+        if (c->lines.cap > static_cast<size_t>(c->pass_limit) * kN * sizeof(float) && !c->lines.keep_old)
+            c->lines.release();
+    });
+}
+
 int octgb_set_stitch_rows(octgb_ctx* c, int rows) {
     return guarded(c, [&] {
         if (c->capturing) throw Error(OCTGB_ERR_STATE, "octgb_set_stitch_rows during graph capture");
@@ -1572,8 +1620,7 @@ int octgb_batch_process(octgb_ctx* c, int n_tiles, const octgb_tile* tiles, int 
         a.n_qt = n_tiles;
         ck(launch_apod_mean(a, dtype, rows, c->apod.as<float>(), c->stream), "apod kernel");
         c->launches++;
-        const unsigned int pass = pass_lines(c, lines);
-        ck(c->magbuf.ensure(static_cast<size_t>(pass) * kHalf * sizeof(float)), "cudaMalloc(mag)");
+        const unsigned int pass = scratch_rows(c, c->magbuf, pass_lines(c, lines), kHalf, "cudaMalloc(mag)");
         // passes of whole B-scans (the lateral blend reads neighbours of the same
         // B-scan); one longer than a pass is cut between groups of four
         int t = 0;

@@ -17,8 +17,10 @@ constexpr int kSincThreads = 512; // threads of the banded sinc, four outputs ea
 // 324 000 A-scans stitched took 4043, 3685, 3479, 3356 and 3290 us with 24,
 // 48, 96, 192 and 600 per SM.  set_geometry makes room for kFirstPass (228
 // MiB: a first call of up to 29 184 A-scans allocates nothing), longer calls
-// grow it; the allocation-free entry point has its own of kMinPass.
-constexpr int kMaxPass = 152 * 600, kFirstPass = 152 * 192, kMinPass = 152 * 24;
+// grow it; the allocation-free entry point has its own of kMinPass.  A device
+// short of memory holds less of each, down to kLeastPass: the calls then take
+// more passes.
+constexpr int kMaxPass = 152 * 600, kFirstPass = 152 * 192, kMinPass = 152 * 24, kLeastPass = 152;
 constexpr int kTwTable = 256 + 7 * 256;   // the transform's twiddles tw2, tw3
 
 // device-side status word values

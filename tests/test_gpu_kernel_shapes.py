@@ -171,6 +171,56 @@ def test_batched_tiles_equal_single_tiles_across_passes(gpu_ctx):
         ctx.close()
 
 
+@pytest.mark.parametrize("pass_lines", [64, 101, 1000, 1266, 3797, 3800])
+def test_batched_tiles_do_not_depend_on_the_pass(pass_lines):
+    """Passes that end at a B-scan's start, inside a B-scan longer than a pass,
+    at and among its last four A-scans, against one pass for everything: the same
+    bits and range.  The lateral operator blends neighbours wherever a group of
+    four allows it."""
+    torch = pytest.importorskip("torch")
+    from oct_recon_af_v1_gb300 import _lib
+    from oct_recon_af_v1_gb300 import geometry as G
+    from oct_recon_af_v1_gb300 import stitching as S
+    from oct_recon_af_v1_gb300 import synthetic
+    ctx = _lib.Context(0)
+    try:
+        ctx.follow_torch_stream()
+        sg = G.build_spectral_geometry(synthetic.lambda_nm(), 0.0, 1.33)
+        ctx.set_geometry(sg.sinc_idx, sg.sinc_w, sg.window)
+        tiles = []
+        for k, (b, nx, rows) in enumerate(((2, 3, 50), (1, 3801, 33), (3, 130, 257), (1, 64, 9), (2, 1003, 20))):
+            lay = S.ScanLayout(np.array([0.0]), np.array([0.0]), np.array([0.0]), nx, b, nx * 1e-3, b * 1e-3)
+            z = S.tiled_geometry(lay, sg.z_um, [np.nan], 1.0).out_z_mm
+            tg = S.tiled_geometry(lay, sg.z_um, [np.nan], 1.0, (z[10] - 1e-9, z[9 + rows] + 1e-9))
+            st = S.TileStitcher.build(tg, 0.0, 0.0, np.nan, 80.0)
+            assert st.c0 == 0 and st.c1 == nx
+            for x in range(0, nx - 8, 2):
+                st.WxT[x:x + 2, x:x + 2] = ((0.75, 0.25), (0.25, 0.75))
+            raw = torch.from_numpy(synthetic.generate_numpy(b, nx, 25, seed=k).view(np.int16)).cuda()
+            tiles.append((raw, 25, st.upload(ctx), torch.empty((b, nx, len(tg.out_z_mm)), device="cuda")))
+        thr = S.min_weight_threshold(np.float32)
+
+        def run():
+            ctx.clim_reset()
+            for t in tiles:
+                t[3].fill_(7.0)
+            ctx.batch_process(tiles, thr)
+            return [t[3].clone() for t in tiles], ctx.clim_get()
+        whole, clim = run()
+        ctx.set_pass_lines(pass_lines)
+        parts, clim2 = run()
+        assert clim2 == clim
+        assert all(torch.isfinite(w).all() and torch.equal(w, p) for w, p in zip(whole, parts))
+        small, raw = torch.empty((2, 1003, 1024), device="cuda"), tiles[4][0]       # and the magnitudes
+        ctx.magnitude(raw, 25, small, raw_dtype=0)
+        ctx.set_pass_lines()
+        assert torch.equal(small, ctx.magnitude(raw, 25, torch.empty_like(small), raw_dtype=0))
+        for bad in (-1, 63, 91_201):
+            assert ctx.lib.octgb_set_pass_lines(ctx.h, bad) == _lib.ERR_ARG
+    finally:
+        ctx.close()
+
+
 @pytest.mark.parametrize("nx,frames,tiles_x,depths,fraction", [(7, 1, 1, 1, 0.0), (33, 2, 2, 3, 0.0), (64, 3, 2, 2, 0.5),
                                                                (301, 2, 2, 3, 0.3), (1000, 1, 2, 3, 0.0)])
 def test_stitched_frames_against_oracle_and_row_interface(gpu_ctx, nx, frames, tiles_x, depths, fraction):

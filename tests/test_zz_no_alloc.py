@@ -75,3 +75,37 @@ def test_noalloc_matches_magnitude_on_consecutive_calls(spectral_case):
         assert b"allocation-free limit" in lib.octgb_last_error(ctx.h)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("bscans,nx,dtype", [(2, 2000, "int16"), (64, 115, "float32"), (1, 3649, "int16"),
+                                             (1, 3648, "int16")])
+def test_noalloc_in_several_passes(bscans, nx, dtype):
+    """Calls longer than its scratch of 3648 A-scans, up to the last A-scan:
+    the ordinary entry point's bits (the same operations on each A-scan)."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import oct_recon_af_v1_gb300 as pkg
+    pkg.build()
+    from oct_recon_af_v1_gb300 import _lib, geometry, synthetic
+    sg = geometry.build_spectral_geometry(synthetic.lambda_nm(), synthetic.beta_ref_from_px(1e-5), 1.33)
+    ctx = _lib.Context(0)
+    try:
+        ctx.follow_torch_stream()
+        ctx.set_geometry(sg.sinc_idx, sg.sinc_w, sg.window)
+        raw = torch.randint(0, 30000, (bscans, 25 + nx, 2048), generator=torch.Generator().manual_seed(nx)).to(
+            getattr(torch, dtype)).cuda()
+        ref = ctx.magnitude(raw, 25, torch.empty((bscans, nx, 1024), device="cuda"))
+        out = torch.full_like(ref, float("nan"))
+        torch.cuda.synchronize()
+        free0 = torch.cuda.mem_get_info()[0]
+        for _ in range(2):
+            rc = ctx.lib.octgb_magnitude_noalloc(ctx.h, ctypes.c_void_p(raw.data_ptr()),
+                                                 _lib.I16 if dtype == "int16" else _lib.F32, bscans, 25 + nx, 25,
+                                                 ctypes.c_void_p(out.data_ptr()))
+            assert rc == _lib.OK, ctx.lib.octgb_last_error(ctx.h)
+            torch.cuda.synchronize()
+        assert torch.cuda.mem_get_info()[0] == free0
+        assert torch.isfinite(ref).all() and torch.equal(out, ref)
+    finally:
+        ctx.close()
