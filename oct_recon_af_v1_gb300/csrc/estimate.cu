@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(kMedThreads) k_xmedian(const float* __restrict
             for (int i = lane; i < nx; i += 32) {
                 const float v = s[i * kPitch];
                 nn += isnan(v);
-                if (!isnan(v) && !isinf(v)) acc += static_cast<double>(v);
+                if (!isnan(v)) acc += static_cast<double>(v);
             }
             nn = __reduce_add_sync(0xffffffffu, nn);
             for (int d = 16; d > 0; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);

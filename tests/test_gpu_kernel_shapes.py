@@ -105,6 +105,24 @@ def test_x_profiles_equal_numpy(gpu_ctx, nx, nz):
                                       np.nanmedian(mag.astype(np.float64), axis=1))
 
 
+@pytest.mark.parametrize("nx,nz", [(1, 3), (33, 20), (1025, 9)])
+def test_x_mean_with_infinities_and_nan(gpu_ctx, nx, nz):
+    """NaN is left out, an infinity is not: numpy.nanmean's values (1e-12, as
+    above), infinite columns, opposite infinities and columns of NaN included."""
+    rng = np.random.default_rng(nx)
+    mag = rng.normal(size=(3, nx, nz)).astype(np.float32)
+    mag[0, rng.integers(0, nx, nx // 3), rng.integers(0, nz, nx // 3)] = np.nan
+    mag[0, nx // 2, 0] = np.inf
+    mag[1, 0, nz - 1] = -np.inf
+    mag[1, :, 1] = np.nan
+    mag[2, 0, 2], mag[2, -1, 2] = np.inf, -np.inf
+    with np.errstate(all="ignore"):
+        import warnings
+        warnings.simplefilter("ignore", RuntimeWarning)
+        np.testing.assert_allclose(gpu_ctx.xmean(mag), np.nanmean(mag.astype(np.float64), axis=1), rtol=1e-12,
+                                   atol=1e-12)
+
+
 @pytest.mark.parametrize("dtype", [np.uint16, np.int16, np.float32])
 @pytest.mark.parametrize("bscans,nx", [(1, 1), (1, 2), (3, 1), (2, 7), (1, 305), (5, 123)])
 def test_lines_and_magnitudes_of_ragged_batches(gpu_ctx, dtype, bscans, nx):
