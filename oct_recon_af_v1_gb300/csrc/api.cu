@@ -1904,10 +1904,14 @@ int octgb_prepare_raw(octgb_ctx* c, const void* raw, int dtype, int loc, int B, 
         prep_args(a, raw, B, n_lines, apod, binning, apod_mode, apod_group);
         *out_lines = a.a_out + a.n_kept;
         if (B == 0) return;
-        const bool direct = out_loc == OCTGB_DEVICE && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+        // straight into the caller's buffer, unless it shares memory with the raws
+        const size_t in_bytes = static_cast<size_t>(B) * n_lines * kN * raw_elem(dtype);
+        const size_t out_bytes = static_cast<size_t>(B) * (a.a_out + a.n_kept) * kN * sizeof(float);
+        const uintptr_t r = reinterpret_cast<uintptr_t>(raw), o = reinterpret_cast<uintptr_t>(out);
+        const bool shared = loc == OCTGB_DEVICE && r < o + out_bytes && o < r + in_bytes;
+        const bool direct = out_loc == OCTGB_DEVICE && (o & 15u) == 0 && !shared;
         run_prepare(c, a, dtype, loc, direct ? out : nullptr);
-        if (!direct)
-            copy_out(c, out, out_loc, c->prep.p, static_cast<size_t>(B) * (a.a_out + a.n_kept) * kN * sizeof(float));
+        if (!direct) copy_out(c, out, out_loc, c->prep.p, out_bytes);
         check_status(c);
     });
 }

@@ -170,3 +170,27 @@ def test_spectral_processor_prepares_rare_formats(ctx):
         dev = sp.magnitude(torch.from_numpy(raw.view(np.int16)).cuda())
         torch.cuda.synchronize()
         np.testing.assert_array_equal(dev.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("dtype,binning,mode,shift", [("float32", 2, 0, 0), ("float32", 3, 1, 4096), ("int16", 1, 0, 0),
+                                                      ("int16", 2, 0, 8192)])
+def test_prepare_into_the_memory_of_the_raws(gpu_ctx, dtype, binning, mode, shift):
+    """The prepared batch may overlap the raws it is made of: the values of a
+    separate output."""
+    torch = pytest.importorskip("torch")
+    from oct_recon_af_v1_gb300 import geometry as G
+    from oct_recon_af_v1_gb300 import synthetic
+    sg = G.build_spectral_geometry(synthetic.lambda_nm(), 0.0, 1.33)
+    gpu_ctx.set_geometry(sg.sinc_idx, sg.sinc_w, sg.window)
+    raw = torch.from_numpy(synthetic.generate_numpy(3, 200, 25, seed=binning).astype(dtype)).cuda()
+    lines = gpu_ctx.prepared_lines(raw, 25, binning, mode, 1)
+    ref = torch.empty((3, lines, 2048), device="cuda")
+    torch.cuda.synchronize()
+    gpu_ctx.prepare_raw(raw, 25, binning, mode, 1, out=ref)
+    buf = torch.empty(shift + max(ref.numel() * 4, raw.numel() * raw.element_size()), dtype=torch.uint8, device="cuda")
+    inside = buf[:raw.numel() * raw.element_size()].view(getattr(torch, dtype)).view(raw.shape)
+    inside.copy_(raw)
+    out = buf[shift:shift + ref.numel() * 4].view(torch.float32).view(ref.shape)
+    torch.cuda.synchronize()
+    gpu_ctx.prepare_raw(inside, 25, binning, mode, 1, out=out)
+    assert torch.equal(out, ref)
