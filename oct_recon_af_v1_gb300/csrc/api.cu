@@ -202,7 +202,8 @@ struct octgb_ctx {
     bool win_is_one = false;                 // geometry window is exactly 1 (plain linearisation)
     DevBuf disp_x, disp_hann, disp_dk2, disp_betas, disp_phase, disp_a, disp_score, xmed;
     int disp_b = 0, disp_rep = 0, disp_nx = 0;
-    bool has_dk2 = false;
+    std::vector<double> dk2;                 // as given; on the device (disp_dk2) from the first use on
+    bool dk2_uploaded = false;
     std::vector<QTable*> qtables;            // batched form: device tile tables by content
     uint64_t qtable_clock = 0;
     std::vector<SlotTable*> slot_tables;
@@ -1699,16 +1700,21 @@ int octgb_disp_lines(octgb_ctx* c, float* out, int out_loc) {
 int octgb_disp_set_dk2(octgb_ctx* c, const double* dk2) {
     return guarded(c, [&] {
         require(dk2 != nullptr, "dk2 is NULL");
-        ck(c->disp_dk2.ensure(kN * sizeof(double)), "cudaMalloc(dk2)");
-        ck(cudaMemcpyAsync(c->disp_dk2.p, dk2, kN * sizeof(double), cudaMemcpyHostToDevice, c->stream), "H2D dk2");
-        ck(cudaStreamSynchronize(c->stream), "sync dk2");
-        c->has_dk2 = true;
+        c->dk2.assign(dk2, dk2 + kN);
+        c->dk2_uploaded = false;
     });
 }
 
 namespace {
 // phase rows of `n` betas into c->disp_phase (sized for `cap` rows)
 void disp_phase_rows(octgb_ctx* c, const double* betas, int n, int cap) {
+    if (!c->dk2_uploaded) {
+        ck(c->disp_dk2.ensure(kN * sizeof(double)), "cudaMalloc(dk2)");
+        ck(cudaMemcpyAsync(c->disp_dk2.p, c->dk2.data(), kN * sizeof(double), cudaMemcpyHostToDevice, c->stream),
+           "H2D dk2");
+        ck(cudaStreamSynchronize(c->stream), "sync dk2");
+        c->dk2_uploaded = true;
+    }
     ck(c->disp_betas.ensure(static_cast<size_t>(cap) * sizeof(double)), "cudaMalloc(betas)");
     ck(c->disp_phase.ensure(static_cast<size_t>(cap) * kN * sizeof(float2)), "cudaMalloc(phase)");
     ck(cudaMemcpyAsync(c->disp_betas.p, betas, static_cast<size_t>(n) * sizeof(double), cudaMemcpyHostToDevice,
@@ -1724,7 +1730,7 @@ int octgb_disp_eval(octgb_ctx* c, int n_beta, const double* betas, int b0, int n
                     int z_min, double* scores, float* mag, int mag_loc) {
     return guarded(c, [&] {
         require(c->disp_b > 0, "octgb_disp_load has not been called");
-        require(c->has_dk2, "octgb_disp_set_dk2 has not been called");
+        require(!c->dk2.empty(), "octgb_disp_set_dk2 has not been called");
         require(n_beta >= 1 && betas != nullptr, "no betas");
         require(b0 >= 0 && nb >= 1 && b0 + nb <= c->disp_b, "B-scan range outside the loaded B-scans");
         require(metric >= 0 && metric <= 4, "metric must be 0 (none) .. 4");
@@ -2277,7 +2283,7 @@ int octgb_disp_images(octgb_ctx* c, int n_beta, const double* betas, int b0, int
                       int normalise) {
     return guarded(c, [&] {
         require(c->disp_b > 0, "octgb_disp_load has not been called");
-        require(c->has_dk2, "octgb_disp_set_dk2 has not been called");
+        require(!c->dk2.empty(), "octgb_disp_set_dk2 has not been called");
         require(n_beta >= 1 && betas != nullptr, "no betas");
         require(b0 >= 0 && nb >= 1 && b0 + nb <= c->disp_b, "B-scan range outside the loaded B-scans");
         require(z_keep >= 1 && z_keep <= kHalf, "z_keep must be in [1, N/2]");

@@ -193,3 +193,44 @@ def test_windowed_lines_bit_exact(built):
         np.testing.assert_array_equal(got.view(np.int32), ref.view(np.int32))
     finally:
         ctx.close()
+
+
+def test_dk2_set_during_a_capture(gpu_ctx):
+    """octgb_disp_set_dk2 only keeps its values: it may come between the calls
+    that a graph captures, and counts from then on."""
+    torch = pytest.importorskip("torch")
+    from oct_recon_af_v1_gb300 import estimation as E
+    from oct_recon_af_v1_gb300 import geometry as G
+    from oct_recon_af_v1_gb300 import synthetic
+    sg = G.build_spectral_geometry(synthetic.lambda_nm(), 0.0, 1.33)
+    gpu_ctx.set_geometry(sg.sinc_idx, sg.sinc_w, np.ones(2048, np.complex128))
+    dk2 = G.dispersion_dk2(sg)
+    raw = torch.from_numpy(synthetic.generate_numpy(1, 40, 25, seed=2).view(np.int16)).cuda()
+    mag = torch.empty((1, 40, 1024), device="cuda")
+    gpu_ctx.disp_load(raw, 25, 1, 1, E.hann_rms(2048), raw_dtype=0)
+    gpu_ctx.disp_set_dk2(dk2)
+    ref = gpu_ctx.disp_eval([2e7], 0, 1, 1, 100)
+    gpu_ctx.disp_set_dk2(0.0 * dk2)
+    zero = gpu_ctx.disp_eval([2e7], 0, 1, 1, 100)
+    gpu_ctx.magnitude(raw, 25, mag, raw_dtype=0)
+    gpu_ctx.synchronize()
+    whole = mag.clone()
+    stream = torch.cuda.Stream()
+    gpu_ctx.set_stream(stream.cuda_stream)
+    try:
+        torch.cuda.synchronize()
+        gpu_ctx.graph_begin()
+        try:
+            gpu_ctx.magnitude(raw, 25, mag, raw_dtype=0)
+            gpu_ctx.disp_set_dk2(dk2)
+        finally:
+            gid = gpu_ctx.graph_end()
+        mag.zero_()
+        torch.cuda.synchronize()
+        gpu_ctx.graph_launch(gid)
+        gpu_ctx.synchronize()
+        assert torch.equal(mag, whole)
+        assert gpu_ctx.disp_eval([2e7], 0, 1, 1, 100) == ref and ref != zero
+    finally:
+        gpu_ctx.set_stream(None)
+        gpu_ctx.graphs_release()
