@@ -159,18 +159,20 @@ def _ptr(a):
     raise TypeError(f"unsupported array type {type(a)!r}")
 
 
-_TORCH_DTYPE: dict = {}          # torch dtype -> raw_dtype, filled when the first tensor comes
+_TORCH_DTYPE: dict = {}          # torch dtype -> raw_dtype, made when the first tensor comes
 
 
 def _raw_dtype(a) -> int:
     if isinstance(a, np.ndarray):
         code = _DTYPE.get(a.dtype)
     else:
-        if not _TORCH_DTYPE:
+        global _TORCH_DTYPE
+        if not _TORCH_DTYPE:                                 # (whole at once: other threads may look it up meanwhile)
             import torch
-            _TORCH_DTYPE.update({torch.int16: I16, torch.float32: F32})
+            codes = {torch.int16: I16, torch.float32: F32}
             if hasattr(torch, "uint16"):
-                _TORCH_DTYPE[torch.uint16] = U16
+                codes[torch.uint16] = U16
+            _TORCH_DTYPE = codes
         code = _TORCH_DTYPE.get(a.dtype)
     if code is None:
         raise TypeError(f"raw spectra must be uint16, int16 or float32, got {a.dtype}")

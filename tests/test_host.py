@@ -7,6 +7,7 @@ reference's, which the fixtures store.
 from __future__ import annotations
 
 import numpy as np
+import pytest
 
 from oct_recon_af_v1_gb300 import geometry as G
 from oct_recon_af_v1_gb300 import stitching as S
@@ -84,3 +85,27 @@ def test_synthetic_generator_shapes_and_range():
     assert abs(raw[:, :25, 1024].mean() - env[1024]) < 30    # background line ~ envelope
     lam = synthetic.lambda_nm()
     assert abs(lam[0] - 796.0) < 1e-9 and abs(lam[-1] - 1010.0) < 1e-9
+
+
+def test_raw_dtype_codes_appear_at_once(monkeypatch):
+    """A thread that meets its first tensor while another makes the table of
+    dtype codes finds it whole or not at all."""
+    torch = pytest.importorskip("torch")
+    if not hasattr(torch, "uint16"):
+        pytest.skip("no torch.uint16")
+    import sys
+    import types
+    from oct_recon_af_v1_gb300 import _lib
+    counts = torch.zeros(1, dtype=torch.int32).to(torch.uint16)
+    seen = []
+
+    class Torch(types.ModuleType):
+        def __getattr__(self, name):
+            if name == "uint16" and not seen:
+                seen.append(None)
+                seen[0] = _lib._raw_dtype(counts)            # the other thread, at this point
+            return getattr(torch, name)
+    monkeypatch.setattr(_lib, "_TORCH_DTYPE", {})
+    monkeypatch.setitem(sys.modules, "torch", Torch("torch"))
+    assert _lib._raw_dtype(counts) == _lib.U16
+    assert seen == [_lib.U16]
