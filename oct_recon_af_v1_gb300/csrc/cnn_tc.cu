@@ -13,9 +13,11 @@
 // segment where whole rows would not fit) of one image.  Specialised warps
 // hand a band on through mbarriers:
 //   producer   copies the band's rows, eight channels at a time, into a ring of
-//              raw slots (one tensor copy a slot; 4-byte cp.async where the rows
-//              are not on 16-byte boundaries);
-//   converters pack a slot's rows to 16-bit operands in one of two staged blocks;
+//              raw slots (one tensor copy a slot);
+//   converters pack a slot's rows to 16-bit operands in one of two staged blocks
+//              (kDirect, rows off 16-byte boundaries: from memory, all channels at
+//              once; a form of its own, since both in one kernel cost the slots'
+//              form up to 18 %);
 //   MMA        one warp issues the band's tcgen05.mma;
 //   epilogue   (convolution) drains the accumulators to global memory.
 // Copies of later bands are in flight throughout, so no phase waits for the
@@ -129,55 +131,58 @@ __device__ __forceinline__ void tensor_copy(const CUtensorMap& map, int x0, int 
         : "memory");
 }
 
-// Producer warp: nch channels from plane `plane` on, rows y0 .. y0 + rows - 1 and
-// columns x0 .. x0 + cols - 1, into a raw slot.  One tensor copy (box: the whole
-// slot, zeros outside the planes), or 4-byte copies of the part inside the image
-// where the rows are not on 16-byte boundaries; either way the slot's barrier
-// counts the 32 lanes.  (One bulk copy per channel and
+// Producer warp: a box of eight channels from plane `plane` on, of rows from y0
+// and columns from x0 on, into a raw slot by one tensor copy (zeros outside the
+// planes); the slot's barrier counts the 32 lanes.  (One bulk copy per channel and
 // row of 512 bytes measured 100 cycles a copy: 751 us for 1.1 GB, copies alone.)
-__device__ __forceinline__ void load_slot(const CUtensorMap& map, const float* src, int H, int W, int vec, int plane,
-                                          int nch, int y0, int rows, int x0, int cols, int box_floats, float* slot,
+__device__ __forceinline__ void load_slot(const CUtensorMap& map, int plane, int y0, int x0, int box_floats, float* slot,
                                           uint64_t* bar) {
-    const int lane = threadIdx.x & 31;
-    if (vec) {
-        if (lane == 0) {
-            mbar_expect_tx(bar, static_cast<uint32_t>(box_floats) * 4u);
-            tensor_copy(map, x0, y0, plane, slot, bar);
-        } else {
-            mbar_arrive(bar);
-        }
-        __syncwarp();
+    if ((threadIdx.x & 31) == 0) {
+        mbar_expect_tx(bar, static_cast<uint32_t>(box_floats) * 4u);
+        tensor_copy(map, x0, y0, plane, slot, bar);
     } else {
-        const int r0 = max(0, -y0), r1 = min(rows, H - y0), c0 = max(0, -x0), c1 = min(cols, W - x0);
-        for (int c = 0; c < nch; ++c)
-            for (int r = r0; r < r1; ++r) {
-                const float* p = src + (static_cast<int64_t>(plane + c) * H + y0 + r) * W + x0;
-                for (int i = c0 + lane; i < c1; i += 32)
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(slot + (c * rows + r) * cols + i)),
-                                 "l"(p + i)
-                                 : "memory");
-            }
-        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+        mbar_arrive(bar);
+    }
+    __syncwarp();
+}
+
+// converter thread t of nt, rows off 16-byte boundaries: nch channels, rows y0 ..
+// y0 + rows - 1 and columns x0 .. x0 + cols - 1 into L2 (of the band after this one)
+__device__ __forceinline__ void prefetch_planes(const float* src, int H, int W, int plane, int nch, int y0, int rows,
+                                                int x0, int cols, int t, int nt) {
+    const int r0 = max(0, -y0), r1 = min(rows, H - y0), c0 = max(0, -x0), c1 = min(cols, W - x0);
+    const bool whole = c1 - c0 == W;                           // a channel's rows are one run
+    const int runs = whole ? 1 : r1 - r0, lines = ((whole ? (r1 - r0) * W : c1 - c0) + 31) / 32;
+    for (int k = t; k < nch * runs * lines; k += nt) {
+        const int c = k / (runs * lines), m = k - c * (runs * lines), r = m / lines, l = m - r * lines;
+        const float* p = src + (static_cast<int64_t>(plane + c) * H + y0 + r0 + r) * W + x0 + c0 + 32 * l;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
     }
 }
 
-// converter thread t of nt: a raw slot's pixels as 16-byte groups of 8
-// channels, zero outside the image
+// converter thread t of nt: a band's pixels from memory, as 16-byte groups of 8
+// channels, zero outside the image.  (Rows off 16-byte boundaries: all warps' plain
+// loads over all channels at once.  Taken through the raw slots by one warp's
+// 4-byte copies, the gradients of 64 images of 32 -> 32 channels, 64 x 30, took
+// 341 us, so 42.)
 template <bool kBf16>
-__device__ __forceinline__ void stage_slot(const Band& g, const BandAt& o, const float* raw, int nch, uint4* dst,
-                                           int npix, int t, int nt) {
-    const int sx = o.x0 - 1 - slot_x0(g, o);               // slot column of staged column 0
-#pragma unroll 2
-    for (int i = t; i < npix; i += nt) {
+__device__ __forceinline__ void stage_planes(const Band& g, const BandAt& o, const float* __restrict__ x, int groups,
+                                             uint4* dst, int xpix, int npix, int t, int nt) {
+    const int64_t hw = static_cast<int64_t>(g.H) * g.W;
+    const float* img = x + static_cast<int64_t>(o.img) * g.C * hw;
+#pragma unroll 4
+    for (int k = t; k < groups * npix; k += nt) {
+        const int p = k / npix, i = k - p * npix;
         const int r = div_wp(g, i), cc = i - r * g.Wp;
         const int iy = o.y0 - 1 + r, ix = o.x0 - 1 + cc;
         const bool in = r < o.rows + 2 && cc < g.Ws + 2 && iy >= 0 && iy < g.H && ix >= 0 && ix < g.W;
-        const float* p = raw + (in ? r * g.rp + sx + cc : 0);
+        const float* q = img + (in ? 8 * p * hw + static_cast<int64_t>(iy) * g.W + ix : 0);
+        const int nch = g.C - 8 * p;
         float v[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = in && e < nch ? p[e * g.rawp] : 0.f;
-        dst[i] = make_uint4(pack2<kBf16>(v[0], v[1]), pack2<kBf16>(v[2], v[3]), pack2<kBf16>(v[4], v[5]),
-                            pack2<kBf16>(v[6], v[7]));
+        for (int e = 0; e < 8; ++e) v[e] = in && e < nch ? __ldg(q + e * hw) : 0.f;
+        dst[p * xpix + i] = make_uint4(pack2<kBf16>(v[0], v[1]), pack2<kBf16>(v[2], v[3]), pack2<kBf16>(v[4], v[5]),
+                                       pack2<kBf16>(v[6], v[7]));
     }
 }
 
@@ -294,7 +299,7 @@ __device__ __forceinline__ void conv_mmas(uint32_t d, uint64_t a, uint64_t b, ui
 // kMask (the data gradient through ReLU + 2x2 mean): xmap is of the
 // pre-activations, pmap of the pooled gradient, their product with the mask is
 // formed while it is packed (32 x 128 x 128 at 128 images: 89 + 108 -> 124 us).
-template <bool kBf16, bool kMask>
+template <bool kBf16, bool kMask, bool kDirect>
 __global__ void __launch_bounds__(kCThreads, 1)
     k_conv3x3_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap pmap, const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
                  float* __restrict__ y, float* __restrict__ pooled, const ConvGeom g, int* status) {
@@ -333,19 +338,39 @@ __global__ void __launch_bounds__(kCThreads, 1)
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     for (int co = tid; co < g.cout; co += kCThreads) S.bias[co] = bias != nullptr ? bias[co] : 0.f;
-    // weights: B[tap][c8][co] = 8 values of channels 8 c8 .. 8 c8 + 7 (zero past cin)
-    for (int i = tid; i < 9 * g.cin8 * g.cout; i += kCThreads) {
-        const int kb = i / g.cout, co = i - kb * g.cout;
-        const int tap = kb / g.cin8, c8 = kb - tap * g.cin8;
-        float v[8];
+    // weights: B[tap][c8][co] = 8 values of channels 8 c8 .. 8 c8 + 7 (zero past cin).
+    // Where they fit in the L1 that the shared memory leaves, a thread gathers the
+    // eight values of an operand row 36 bytes apart; else they are read along memory
+    // (24 -> 128 channels, two rows of 128: 29 us a call gathered, 17 so; with
+    // little shared memory, 16 x 16: 13.5 gathered, 15.3 so).
+    if (static_cast<uint32_t>(9 * g.b.C * g.cout * 4) + g.smem <= 240 * 1024) {
+        for (int i = tid; i < 9 * g.cin8 * g.cout; i += kCThreads) {
+            const int kb = i / g.cout, co = i - kb * g.cout;
+            const int tap = kb / g.cin8, c8 = kb - tap * g.cin8;
+            float v[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const int c = 8 * c8 + e;
-            v[e] = c < g.b.C ? w[(static_cast<int64_t>(co) * g.b.C + c) * 9 + tap] : 0.f;
+            for (int e = 0; e < 8; ++e) {
+                const int c = 8 * c8 + e;
+                v[e] = c < g.b.C ? w[(static_cast<int64_t>(co) * g.b.C + c) * 9 + tap] : 0.f;
+            }
+            *reinterpret_cast<uint4*>(B + static_cast<uint32_t>(kb) * b_chunk + co * 16) =
+                make_uint4(pack2<kBf16>(v[0], v[1]), pack2<kBf16>(v[2], v[3]), pack2<kBf16>(v[4], v[5]),
+                           pack2<kBf16>(v[6], v[7]));
         }
-        *reinterpret_cast<uint4*>(B + static_cast<uint32_t>(kb) * b_chunk + co * 16) =
-            make_uint4(pack2<kBf16>(v[0], v[1]), pack2<kBf16>(v[2], v[3]), pack2<kBf16>(v[4], v[5]),
-                       pack2<kBf16>(v[6], v[7]));
+    } else {
+        const auto at = [&](int tap, int c, int co) {
+            return reinterpret_cast<uint16_t*>(B + static_cast<uint32_t>(tap * g.cin8 + c / 8) * b_chunk + co * 16 + c % 8 * 2);
+        };
+        const int per_co = 9 * g.b.C;
+#pragma unroll 8
+        for (int i = tid; i < g.cout * per_co; i += kCThreads) {
+            const int co = i / per_co, k = i - co * per_co, c = k / 9;
+            *at(k - 9 * c, c, co) = static_cast<uint16_t>(pack2<kBf16>(w[i], 0.f));
+        }
+        for (int i = tid; i < 9 * (8 * g.cin8 - g.b.C) * g.cout; i += kCThreads) {
+            const int k = i / g.cout, co = i - k * g.cout;
+            *at(k % 9, g.b.C + k / 9, co) = 0;
+        }
     }
     // the padding chunk of both staged blocks (never rewritten)
     if (g.cin8 > g.cin8r)
@@ -362,7 +387,7 @@ __global__ void __launch_bounds__(kCThreads, 1)
     if (warp == kCEpi + kCConv) {
         // ---- producer
         Ring k;
-        bool ok = true;
+        bool ok = !kDirect;                                // else nothing goes through the slots
         for (int64_t u = blockIdx.x; u < g.b.n_units && ok; u += gridDim.x) {
             const BandAt o = band_at(g.b, u);
             for (int c8 = 0; c8 < g.cin8r; ++c8, k.next(g.slots)) {
@@ -379,8 +404,8 @@ __global__ void __launch_bounds__(kCThreads, 1)
                     }
                     __syncwarp();
                 } else {
-                    load_slot(xmap, x, g.b.H, g.b.W, g.b.vec, o.img * g.b.C + 8 * c8, min(8, g.b.C - 8 * c8), o.y0 - 1,
-                              g.b.R + 2, slot_x0(g.b, o), g.b.rp, min(8, g.b.C) * g.b.rawp, slot, &S.full[k.slot]);
+                    load_slot(xmap, o.img * g.b.C + 8 * c8, o.y0 - 1, slot_x0(g.b, o), min(8, g.b.C) * g.b.rawp, slot,
+                              &S.full[k.slot]);
                 }
             }
         }
@@ -430,7 +455,7 @@ __global__ void __launch_bounds__(kCThreads, 1)
     } else if (warp >= kCEpi) {
         // ---- converters
         const int t = tid - 32 * kCEpi;
-        const Pixels<kCPix, kMask> px(g.b, (g.b.R + 2) * g.b.Wp, t, 32 * kCConv, g.poff);
+        const Pixels<kDirect ? 1 : kCPix, kMask> px(g.b, (g.b.R + 2) * g.b.Wp, t, 32 * kCConv, g.poff);
         Ring k;
         uint32_t j = 0;
         bool ok = true;
@@ -439,15 +464,23 @@ __global__ void __launch_bounds__(kCThreads, 1)
             const uint32_t b = j & 1u;
             // the MMAs of the band two before have read block b
             if (j >= 2 && !(ok = role_wait(&S.sempty[b], ((j >> 1) - 1) & 1u, &S.abort, status))) break;
-            for (int c8 = 0; c8 < g.cin8r; ++c8, k.next(g.slots)) {
+            const int npix = (o.rows + 2) * g.b.Wp;
+            if (kDirect) {
+                if (u + gridDim.x < g.b.n_units) {
+                    const BandAt q = band_at(g.b, u + gridDim.x);
+                    prefetch_planes(x, g.b.H, g.b.W, q.img * g.b.C, g.b.C, q.y0 - 1, g.b.R + 2, slot_x0(g.b, q), g.b.rp,
+                                    t, 32 * kCConv);
+                }
+                stage_planes<kBf16>(g.b, o, x, g.cin8r, reinterpret_cast<uint4*>(X + b * g.xbytes), g.xpix, npix, t,
+                                    32 * kCConv);
+            }
+            for (int c8 = 0; !kDirect && c8 < g.cin8r; ++c8, k.next(g.slots)) {
                 ok = role_wait(&S.full[k.slot], k.use & 1u, &S.abort, status);
                 if (!ok) break;
                 const float* raw = reinterpret_cast<const float*>(base + k.slot * g.slotb);
                 uint4* dst = reinterpret_cast<uint4*>(X + b * g.xbytes) + c8 * g.xpix;
-                const int nch = min(8, g.b.C - 8 * c8), npix = (o.rows + 2) * g.b.Wp;
-                if (!kMask && !g.b.vec)
-                    stage_slot<kBf16>(g.b, o, raw, nch, dst, npix, t, 32 * kCConv);
-                else if (nch == 8)
+                const int nch = min(8, g.b.C - 8 * c8);
+                if (nch == 8)
                     px.template stage<kBf16, true>(raw, g.b.rawp, g.prawp, 8, dst, npix, t, 32 * kCConv);
                 else
                     px.template stage<kBf16, false>(raw, g.b.rawp, g.prawp, nch, dst, npix, t, 32 * kCConv);
@@ -614,7 +647,7 @@ struct WgradBars {
 // gradient dp of their ReLU + 2x2 mean, and dy = y > 0 ? dp / 4 : 0 is formed while
 // it is packed (k_relu_pool_bwd's value).  That saves writing and reading dy, of
 // the first layer's 1.1 GB each at 128 images: 339 + 307 us -> 340 us.
-template <bool kPool>
+template <bool kPool, bool kDirect>
 __global__ void __launch_bounds__(kWThreads, 1)
     k_conv3x3_wgrad_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap dmap,
                        const __grid_constant__ CUtensorMap pmap, const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ part,
@@ -623,6 +656,7 @@ __global__ void __launch_bounds__(kWThreads, 1)
     __shared__ WgradBars S;
     uint8_t* base = smem_raw + align_up_smem(smem_raw, 1024);    // raw slots, then the staged blocks
     uint8_t* stages = base + g.slots * g.slotb;
+    const bool xdirect = kDirect && !g.b.vec, ddirect = kDirect && !kPool && !g.dvec;
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);          // uniform: the roles are warps
 
@@ -662,17 +696,18 @@ __global__ void __launch_bounds__(kWThreads, 1)
     const uint32_t tmem = __shfl_sync(0xffffffffu, S.tmem, 0);
 
     if (warp == 0) {
-        // ---- producer: per band the channel groups of x, then of dy
+        // ---- producer: per band the channel groups of x, then of dy (of those that
+        // go through the slots)
         Ring k;
         bool ok = true;
         for (int64_t u = blockIdx.x; u < g.b.n_units && ok; u += gridDim.x) {
             const BandAt o = band_at(g.b, u);
-            for (int p = 0; p < g.cgr + g.kg; ++p, k.next(g.slots)) {
+            for (int p = xdirect ? g.cgr : 0; p < g.cgr + (ddirect ? 0 : g.kg); ++p, k.next(g.slots)) {
                 if (k.use > 0 && !(ok = role_wait(&S.empty[k.slot], (k.use - 1) & 1u, &S.abort, status))) break;
                 float* slot = reinterpret_cast<float*>(base + k.slot * g.slotb);
                 if (p < g.cgr)
-                    load_slot(xmap, x, g.b.H, g.b.W, g.b.vec, o.img * g.b.C + 8 * p, min(8, g.b.C - 8 * p), o.y0 - 1,
-                              g.b.R + 2, slot_x0(g.b, o), g.b.rp, min(8, g.b.C) * g.b.rawp, slot, &S.full[k.slot]);
+                    load_slot(xmap, o.img * g.b.C + 8 * p, o.y0 - 1, slot_x0(g.b, o), min(8, g.b.C) * g.b.rawp, slot,
+                              &S.full[k.slot]);
                 else if (kPool) {
                     const int plane = o.img * g.K + 8 * (p - g.cgr), nd = min(8, g.K);
                     if (lane == 0) {
@@ -684,8 +719,7 @@ __global__ void __launch_bounds__(kWThreads, 1)
                     }
                     __syncwarp();
                 } else
-                    load_slot(dmap, dy, g.b.H, g.b.W, g.dvec, o.img * g.K + 8 * (p - g.cgr),
-                              min(8, g.K - 8 * (p - g.cgr)), o.y0, g.b.R, o.x0, g.rpd, min(8, g.K) * g.rawd, slot,
+                    load_slot(dmap, o.img * g.K + 8 * (p - g.cgr), o.y0, o.x0, min(8, g.K) * g.rawd, slot,
                               &S.full[k.slot]);
             }
         }
@@ -769,17 +803,46 @@ __global__ void __launch_bounds__(kWThreads, 1)
             uint8_t* Ds = Xs + g.xbytes;
             // the MMAs of the band staged in block b before have read it
             if (use > 0 && !(ok = role_wait(&S.sempty[b], (use - 1) & 1u, &S.abort, status))) break;
-            for (int p = 0; p < g.cgr + g.kg; ++p, k.next(g.slots)) {
+            const int t = tid - 64, nt = 32 * kWConv;
+            if (kDirect && u + gridDim.x < g.b.n_units) {
+                const BandAt q = band_at(g.b, u + gridDim.x);
+                if (xdirect)
+                    prefetch_planes(x, g.b.H, g.b.W, q.img * g.b.C, g.b.C, q.y0 - 1, g.b.R + 2, slot_x0(g.b, q), g.b.rp,
+                                    t, nt);
+                if (ddirect) prefetch_planes(dy, g.b.H, g.b.W, q.img * g.K, g.K, q.y0, g.b.R, q.x0, g.rpd, t, nt);
+            }
+            if (xdirect) stage_planes<true>(g.b, o, x, g.cgr, reinterpret_cast<uint4*>(Xs), g.xpix, g.xpix, t, nt);
+            if (ddirect) {
+                const int64_t hw = static_cast<int64_t>(g.b.H) * g.b.W;
+                // dy from memory: the groups and steps of the band in one sequence
+                const int steps = g.Q / 32;
+                const float* img = dy + static_cast<int64_t>(o.img) * g.K * hw;
+#pragma unroll 8
+                for (int it = cw >> 1; it < g.kg * steps; it += kWConv / 2) {
+                    const int p = it / steps, hb = it - p * steps, ch = 8 * p + kk;
+                    const int q = 32 * hb + 4 * (lane & 7);
+                    const int r = div_wp(g.b, q), ox = q - r * g.b.Wp;
+                    const int nx = ch < g.K && r < o.rows ? min(g.b.Ws - ox, g.b.W - o.x0 - ox) : 0;
+                    const float* pr = img + (nx > 0 ? ch * hw + static_cast<int64_t>(o.y0 + r) * g.b.W + o.x0 + ox : 0);
+                    const float4 f = make_float4(nx > 0 ? __ldg(pr) : 0.f, nx > 1 ? __ldg(pr + 1) : 0.f,
+                                                 nx > 2 ? __ldg(pr + 2) : 0.f, nx > 3 ? __ldg(pr + 3) : 0.f);
+                    *reinterpret_cast<uint2*>(Ds + (4 * hb + ((lane & 7) >> 1)) * g.apitch + kk * 16 + (lane & 1) * 8 + p * 128) =
+                        make_uint2(pack_bf2(f.x, f.y), pack_bf2(f.z, f.w));
+                    float sum = (f.x + f.y) + (f.z + f.w);
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+                    if ((lane & 7) == 0) S.bias[cw][ch] += sum;
+                }
+            }
+            for (int p = xdirect ? g.cgr : 0; p < g.cgr + (ddirect ? 0 : g.kg); ++p, k.next(g.slots)) {
                 ok = role_wait(&S.full[k.slot], k.use & 1u, &S.abort, status);
                 if (!ok) break;
                 const float* raw = reinterpret_cast<const float*>(base + k.slot * g.slotb);
                 if (p < g.cgr) {
                     uint4* dst = reinterpret_cast<uint4*>(Xs) + p * g.xpix;
                     const int nch = min(8, g.b.C - 8 * p);
-                    const int t = tid - 64, nt = 32 * kWConv;
-                    if (!g.b.vec)
-                        stage_slot<true>(g.b, o, raw, nch, dst, g.xpix, t, nt);
-                    else if (nch == 8)
+                    if (nch == 8)
                         px.template stage<true, true>(raw, g.b.rawp, 0, 8, dst, g.xpix, t, nt);
                     else
                         px.template stage<true, false>(raw, g.b.rawp, 0, nch, dst, g.xpix, t, nt);
@@ -792,25 +855,14 @@ __global__ void __launch_bounds__(kWThreads, 1)
                         const int hb = (cw >> 1) + kWConv / 2 * i;
                         if (hb >= g.Q / 32) break;
                         float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (kPool || g.dvec) {
-                            if (doff[i] >= 0 && ch < g.K) {
-                                f = *reinterpret_cast<const float4*>(raw + doff[i]);
-                                if (kPool) {
-                                    const float2 d = *reinterpret_cast<const float2*>(raw + poff[i]);
-                                    const float g0 = 0.25f * d.x, g1 = 0.25f * d.y;
-                                    f = make_float4(f.x > 0.f ? g0 : 0.f, f.y > 0.f ? g0 : 0.f, f.z > 0.f ? g1 : 0.f,
-                                                    f.w > 0.f ? g1 : 0.f);
-                                }
+                        if (doff[i] >= 0 && ch < g.K) {
+                            f = *reinterpret_cast<const float4*>(raw + doff[i]);
+                            if (kPool) {
+                                const float2 d = *reinterpret_cast<const float2*>(raw + poff[i]);
+                                const float g0 = 0.25f * d.x, g1 = 0.25f * d.y;
+                                f = make_float4(f.x > 0.f ? g0 : 0.f, f.y > 0.f ? g0 : 0.f, f.z > 0.f ? g1 : 0.f,
+                                                f.w > 0.f ? g1 : 0.f);
                             }
-                        } else {
-                            const int q = 32 * hb + 4 * (lane & 7);
-                            const int r = div_wp(g.b, q), ox = q - r * g.b.Wp;
-                            const int nx = ch < g.K && r < o.rows ? min(g.b.Ws - ox, g.b.W - o.x0 - ox) : 0;
-                            const float* pr = raw + kk * g.rawd + r * g.rpd + ox;
-                            if (nx > 0) f.x = pr[0];
-                            if (nx > 1) f.y = pr[1];
-                            if (nx > 2) f.z = pr[2];
-                            if (nx > 3) f.w = pr[3];
                         }
                         *reinterpret_cast<uint2*>(dd + i * (2 * kWConv * g.apitch)) =
                             make_uint2(pack_bf2(f.x, f.y), pack_bf2(f.z, f.w));
@@ -918,11 +970,13 @@ void band_set(Band& b, int n, int R, int Ws) {
 
 // Rows per band: as many as leave three raw slots beside the staged blocks (the
 // halo rows are read and packed once per band), up to 1024 pixels (more brings
-// nothing), and few enough that every SM has two bands where the work allows.
+// nothing), and few enough that every SM has two bands where the work allows, but
+// no fewer than `least` staged pixels (the convolution of narrow images: half an
+// MMA tile; 16 images of 32 channels, 64 x 2: 12.7 us, 74 in bands of three rows).
 // Columns: whole rows where a band of two of them fits, else the longest
 // segment for which it does.  fits(R, Ws) lays the geometry out.
 template <class Fits>
-bool band_choose(Band& b, int n, int unit, int col_unit, int num_sms, Fits fits) {
+bool band_choose(Band& b, int n, int unit, int col_unit, int least, int num_sms, Fits fits) {
     for (int nseg = 1;; ++nseg) {
         const int Ws = (b.W + nseg - 1) / nseg;
         const int Wu = nseg == 1 ? b.W : (Ws + col_unit - 1) / col_unit * col_unit;
@@ -930,7 +984,8 @@ bool band_choose(Band& b, int n, int unit, int col_unit, int num_sms, Fits fits)
         if (fits(need, Wu)) {
             int R = need;
             for (int r = need + unit; r <= b.H && r * (Wu + 4) <= kBandPix; r += unit) {
-                if (static_cast<int64_t>(n) * ((b.H + r - 1) / r) * nseg < 2ll * num_sms || !fits(r, Wu)) break;
+                if (static_cast<int64_t>(n) * ((b.H + r - 1) / r) * nseg < 2ll * num_sms && R * (Wu + 4) >= least) break;
+                if (!fits(r, Wu)) break;
                 R = r;
             }
             const int nband = (b.H + R - 1) / R;
@@ -958,7 +1013,7 @@ bool conv_geom(int n, int cin, int cout, int H, int W, int pool, bool mask, int 
     g.nd = 512 / cols < 4 ? 512 / cols : 4;
     g.tmem_cols = tmem_columns(g.nd * cols);
     const uint32_t bbytes = 9u * static_cast<uint32_t>(g.cin8) * static_cast<uint32_t>(cout) * 16u;
-    return band_choose(g.b, n, pool || mask ? 2 : 1, kCM, num_sms, [&](int R, int Ws) {
+    return band_choose(g.b, n, pool || mask ? 2 : 1, kCM, g.wide ? 0 : kCM / 2, num_sms, [&](int R, int Ws) {
         if (g.wide && (Ws % kCM != 0 || W % Ws != 0)) return false;
         if (mask && (Ws != W || R % 2 != 0)) return false;
         band_set(g.b, n, R, Ws);
@@ -1011,7 +1066,7 @@ bool wgrad_geom(int n, int cin, int cout, int H, int W, bool pool, int num_sms, 
         const uint32_t Wp = (W + 2 + 3) / 4 * 4, Q = (Wp + 31) / 32 * 32, xpix = (Q + 2 * Wp + 2 + 7) / 8 * 8;
         if ((((g.fold ? 4 : xgroups) * xpix * 16u + Q * g.kg * 16u + 127u) & ~127u) + 3072u > 227u * 1024u) return false;
     }
-    return band_choose(g.b, n, pool ? 2 : 1, pool ? 8 : 4, num_sms, [&](int R, int Ws) {
+    return band_choose(g.b, n, pool ? 2 : 1, pool ? 8 : 4, 0, num_sms, [&](int R, int Ws) {
         if (pool && R % 2 != 0) return false;
         band_set(g.b, n, R, Ws);
         if (g.b.rp > kMaxBox) return false;
@@ -1097,7 +1152,9 @@ cudaError_t launch_conv3x3_tc(const float* x, const float* dp, const float* w, c
     if (mask && !(g.b.vec && aligned_rows(dp, W / 2) &&
                   encode_planes(&pmap, dp, planes, H / 2, W / 2, g.b.rp / 2, g.b.R / 2 + 2, nc)))
         return cudaErrorInvalidValue;
-    const auto kern = mask ? k_conv3x3_tc<true, true> : (bf16 ? k_conv3x3_tc<true, false> : k_conv3x3_tc<false, false>);
+    const auto kern = mask      ? k_conv3x3_tc<true, true, false>
+                      : g.b.vec ? (bf16 ? k_conv3x3_tc<true, false, false> : k_conv3x3_tc<false, false, false>)
+                                : (bf16 ? k_conv3x3_tc<true, false, true> : k_conv3x3_tc<false, false, true>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(g.smem));
     if (e != cudaSuccess) return e;
     kern<<<units_grid(g.b, num_sms), kCThreads, g.smem, st>>>(xmap, pmap, x, w, b, y, pooled, g, status);
@@ -1125,7 +1182,8 @@ cudaError_t launch_conv3x3_wgrad_tc(const float* x, const float* dy, const float
     if (pool && !(g.dvec && aligned_rows(dp, W / 2) &&
                   encode_planes(&pmap, dp, planes, H / 2, W / 2, g.rpd / 2, g.b.R / 2, dc)))
         return cudaErrorInvalidValue;
-    const auto kern = pool ? k_conv3x3_wgrad_tc<true> : k_conv3x3_wgrad_tc<false>;
+    const auto kern = pool ? (g.b.vec ? k_conv3x3_wgrad_tc<true, false> : k_conv3x3_wgrad_tc<true, true>)
+                           : (g.b.vec && g.dvec ? k_conv3x3_wgrad_tc<false, false> : k_conv3x3_wgrad_tc<false, true>);
     const int grid = units_grid(g.b, num_sms);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(g.smem));
     if (e != cudaSuccess) return e;

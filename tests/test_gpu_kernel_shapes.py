@@ -455,6 +455,34 @@ def test_weight_gradient_through_pool(gpu_ctx, n, cin, cout, h, w, shift):
             <= 1e-4 * dy.double().abs().sum((0, 2, 3)).numpy()).all()
 
 
+@pytest.mark.parametrize("n,cin,cout,h,w,shift", [(3, 32, 32, 5, 128, 1), (2, 9, 96, 7, 256, 2), (160, 17, 32, 16, 16, 3),
+                                                  (2, 24, 128, 4, 384, 1)])
+def test_rows_off_boundaries_equal_aligned_rows(gpu_ctx, n, cin, cout, h, w, shift):
+    """Forward, weight and data gradients read rows off 16-byte boundaries from
+    memory: the bits of aligned rows (the same products in the same order), but
+    for the bias gradient's order of sums (1e-5 of its terms' magnitudes)."""
+    torch = pytest.importorskip("torch")
+    from oct_recon_af_v1_gb300.learned import _p
+    rng = np.random.default_rng(h * w + cin)
+    x, dy = (rng.standard_normal((n, c, h, w)).astype(np.float32) for c in (cin, cout))
+    wt = torch.tensor(rng.standard_normal((cout, cin, 3, 3)), dtype=torch.float32, device="cuda")
+    L, c, out = gpu_ctx.lib, gpu_ctx, []
+    for k in (0, shift):
+        xd, dyd = _offset(torch, x, k), _offset(torch, dy, k)
+        y, dx = torch.full_like(dyd, float("nan")), torch.full_like(xd, float("nan"))
+        dw, db, scratch = torch.empty_like(wt), torch.empty(cout, device="cuda"), torch.empty_like(wt)
+        torch.cuda.synchronize()
+        c._check(L.octgb_cnn_conv3x3_tc(c.h, _p(xd), _p(wt), None, _p(y), n, cin, cout, h, w))
+        c._check(L.octgb_cnn_conv3x3_bwd_tc(c.h, _p(xd), _p(wt), _p(dyd), _p(dx), _p(dw), _p(db), _p(scratch), n, cin,
+                                            cout, h, w))
+        c.synchronize()
+        assert all(torch.isfinite(t).all() for t in (y, dx, dw, db))
+        out.append((y.contiguous(), dx.contiguous(), dw, db))
+    assert all(torch.equal(a, b) for a, b in zip(out[0][:3], out[1][:3]))
+    bound = 1e-5 * torch.tensor(np.abs(dy).sum((0, 2, 3)), device="cuda")
+    assert ((out[0][3] - out[1][3]).abs() <= bound).all()
+
+
 @pytest.mark.parametrize("n,cin,cout,h,w", [(1, 3, 32, 2, 128), (2, 32, 64, 6, 384), (1, 9, 128, 4, 256)])
 def test_conv_with_pool_beside_pre_activations(gpu_ctx, n, cin, cout, h, w):
     """The one kernel's two outputs equal the two kernels' exactly (the same
