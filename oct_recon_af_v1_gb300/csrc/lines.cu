@@ -53,8 +53,18 @@ namespace octgb {
 namespace {
 
 constexpr int kSincWarps = 16;                   // 512 threads x 4 outputs
-constexpr int kBgWarps = 4;
-constexpr int kThr = (kSincWarps + kBgWarps) * 32;
+// Wide windows (U > 18): a sinc thread's 4 U weights do not fit its 96 registers
+// (17 to 20 warps are five on a scheduler, so fewer background warps give it no
+// more).  The compiler kept what did not fit in local memory, which the L1 beside
+// 160 KB and more of shared memory does not hold either: 100 000 A-scans to
+// magnitudes with U = 22 took 1622 us (uint16) and 1912 (float32).  The weights of
+// the window's steps from kRegSteps on now lie in shared memory, eight bytes a
+// thread and bank-conflict free: 797 and 827 us (U = 26: 1784 and 1857, now 904 and
+// 1000).  Two background warps leave the room for them.
+constexpr int kRegSteps = 16;
+constexpr int bg_warps(int U) { return U <= 18 ? 4 : 2; }
+constexpr int reg_steps(int U) { return U <= 18 ? U : kRegSteps; }
+constexpr int lines_threads(int U) { return (kSincWarps + bg_warps(U)) * 32; }
 constexpr int kRing = 8;                         // background-free lines in shared memory
 constexpr int kDLine = kN + kTail;               // line incl. zero tail (16-byte rows)
 
@@ -116,16 +126,18 @@ __device__ __forceinline__ float2 mul_window2(float2 x, float2 hi, float2 lo, fl
     return o;
 }
 
-template <typename RawT>
+template <typename RawT, int U>
 struct LinesSmem {
+    static constexpr int kBgWarps = bg_warps(U);
     uint64_t raw_full[kBgWarps][2], full[kRing], empty[kRing];
     int abort;
     float mval[kRing];
     alignas(16) RawT raw[kBgWarps][2][kN];
     alignas(16) float apod[kBgWarps][2][kN];
     alignas(16) float d[kRing][kDLine];
+    float2 w[U > reg_steps(U) ? U - reg_steps(U) : 1][2][U > reg_steps(U) ? kSincWarps * 32 : 1];   // weights of steps reg_steps(U) .. U - 1
 };
-static_assert(sizeof(LinesSmem<float>) <= 232448, "k_lines shared memory exceeds 227 KB");
+static_assert(sizeof(LinesSmem<float, 18>) <= 232448 && sizeof(LinesSmem<float, 26>) <= 232448, "k_lines shared memory exceeds 227 KB");
 
 // the place of one A-scan: segment (or tile), B-scan, column
 struct LinePos {
@@ -144,9 +156,10 @@ __device__ __forceinline__ int add_pair(uint32_t w, int c) {
 constexpr int kExactFloat = 255;
 
 template <typename RawT, int Mode, int U, bool Tiles, bool Exact>
-__global__ void __launch_bounds__(kThr, 1) k_lines(const LinesArgs a) {
+__global__ void __launch_bounds__(lines_threads(U), 1) k_lines(const LinesArgs a) {
+    constexpr int kBgWarps = bg_warps(U), kThr = lines_threads(U);
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    using Smem = LinesSmem<RawT>;
+    using Smem = LinesSmem<RawT, U>;
     Smem& S = *reinterpret_cast<Smem*>(smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // this CTA's A-scans
@@ -377,11 +390,15 @@ __global__ void __launch_bounds__(kThr, 1) k_lines(const LinesArgs a) {
     // ---------------------------------------------------- sinc
     // the weights of outputs 4t, 4t + 1 (4t + 2, 4t + 3) at window step u form
     // one packed pair wp[0][u] (wp[1][u]): two outputs per f32x2 fma
-    float2 wp[2][U];
+    constexpr int kReg = reg_steps(U);
+    float2 wp[2][kReg];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        for (int u = kReg; u < U; ++u) S.w[u - kReg][h][tid] = __ldg(a.g.wsh + (h * U + u) * (kSincWarps * 32) + tid);
 #pragma unroll
     for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int u = 0; u < U; ++u) wp[h][u] = __ldg(a.g.wsh + (h * U + u) * (kSincWarps * 32) + tid);
+        for (int u = 0; u < kReg; ++u) wp[h][u] = __ldg(a.g.wsh + (h * U + u) * (kSincWarps * 32) + tid);
     const int s0 = __ldg(a.g.s0 + tid);
     const int wrot = s0 % U;                                 // window samples before s0 wrap to the next period
     const int wbase = s0 - wrot;
@@ -426,11 +443,13 @@ __global__ void __launch_bounds__(kThr, 1) k_lines(const LinesArgs a) {
                         acc[h][e] = make_float2(0.f, 0.f);
                     }
             }
+            const float2 w0 = u < kReg ? wp[0][u < kReg ? u : 0] : S.w[u < kReg ? 0 : u - kReg][0][tid];
+            const float2 w1 = u < kReg ? wp[1][u < kReg ? u : 0] : S.w[u < kReg ? 0 : u - kReg][1][tid];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const float x = p[h * kDLine];
-                acc[h][0] = fma2(wp[0][u], make_float2(x, x), acc[h][0]);
-                acc[h][1] = fma2(wp[1][u], make_float2(x, x), acc[h][1]);
+                acc[h][0] = fma2(w0, make_float2(x, x), acc[h][0]);
+                acc[h][1] = fma2(w1, make_float2(x, x), acc[h][1]);
             }
         }
         if (Exact) {
@@ -563,7 +582,7 @@ __global__ void __launch_bounds__(kApodThreads) k_apod_mean(const LinesArgs a, f
 
 template <typename RawT, int Mode, int U, bool Tiles, bool Exact>
 cudaError_t launch_t(const LinesArgs& a, int num_sms, cudaStream_t st) {
-    const size_t smem = sizeof(LinesSmem<RawT>);
+    const size_t smem = sizeof(LinesSmem<RawT, U>);
     const auto kernel = k_lines<RawT, Mode, U, Tiles, Exact>;
     constexpr int kType = sizeof(RawT) == 4 ? 2 : static_cast<RawT>(-1) < 0 ? 1 : 0;
     constexpr int kBit = Exact ? kReadyExact + kType * 4 + (U - 14) / 4
@@ -573,10 +592,10 @@ cudaError_t launch_t(const LinesArgs& a, int num_sms, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     const unsigned int n = a.l1 - a.l0;
     const unsigned int grid = n < static_cast<unsigned int>(num_sms) ? n : static_cast<unsigned int>(num_sms);
-    return launch_dependent(kernel, dim3(grid), dim3(kThr), smem, st, a);
+    return launch_dependent(kernel, dim3(grid), dim3(lines_threads(U)), smem, st, a);
 }
 
-// (wider windows than 14 spill a few weights: five warps a scheduler have 96 registers a thread)
+// (five warps a scheduler have 96 registers a thread: windows of 18 spill a few weights)
 template <typename RawT, int Mode, bool Tiles, bool Exact>
 cudaError_t launch_u(const LinesArgs& a, int num_sms, cudaStream_t st) {
     switch (a.g.U) {

@@ -148,6 +148,30 @@ def test_lines_and_magnitudes_of_ragged_batches(gpu_ctx, dtype, bscans, nx):
     assert np.abs(gpu_ctx.fused_pre_fft(raw, 25) - spec).max() < 2e-6 * np.abs(spec).max()
 
 
+@pytest.mark.parametrize("dtype", [np.uint16, np.float32])
+@pytest.mark.parametrize("span_nm,bscans,nx", [(300.0, 2, 7), (600.0, 1, 1), (600.0, 3, 305), (800.0, 1, 154), (800.0, 5, 61)])
+def test_lines_of_wide_windows(gpu_ctx, dtype, span_nm, bscans, nx):
+    """Spectrometers whose four neighbouring outputs read up to 18, 22 and 26
+    source samples: magnitudes against the oracle's float32 restatement (4e-6 of
+    the largest: a band of up to twenty products and the transform's eleven
+    layers), the scorer's lines exactly (the plain line times the float64 window,
+    rounded once)."""
+    from oracle import numerics as O
+    from oct_recon_af_v1_gb300 import estimation as E
+    from oct_recon_af_v1_gb300 import geometry as G
+    from oct_recon_af_v1_gb300 import synthetic
+    lam = np.linspace(1300 - span_nm / 2, 1300 + span_nm / 2, 2048)
+    sg, og = G.build_spectral_geometry(lam, 0.0, 1.33), O.spectral_geometry(lam, 0.0, 1.33)
+    gpu_ctx.set_geometry(sg.sinc_idx, sg.sinc_w, sg.window)
+    raw = synthetic.generate_numpy(bscans, nx, 25, seed=nx).astype(dtype)
+    ref = O.magnitude_numba(raw, og, 25)
+    assert np.abs(gpu_ctx.magnitude(raw, 25) - ref).max() < 4e-6 * np.abs(ref).max()
+    gpu_ctx.set_geometry(sg.sinc_idx, sg.sinc_w, np.ones(2048, np.complex128))
+    line = gpu_ctx.fused_pre_fft(raw, 25).real.astype(np.float64)
+    gpu_ctx.disp_load(raw, 25, bscans, 1, E.hann_rms(2048))
+    np.testing.assert_array_equal(gpu_ctx.disp_lines(), (line * E.hann_rms(2048)).astype(np.float32))
+
+
 def test_batched_tiles_equal_single_tiles_across_passes(gpu_ctx):
     """Tiles of uneven size (an empty one, B-scans shorter than a group of
     four, one B-scan longer than the smallest pass) in one call against one
