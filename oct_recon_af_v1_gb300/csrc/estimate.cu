@@ -487,7 +487,9 @@ constexpr int kMedMaxReg = 1024;                  // columns of up to this many 
 // bits: 32 times the warp counts its keys below a candidate (kReg keys a lane
 // in registers; kReg = 0 reads them from shared memory each time).  Issue-bound:
 // ~2 instructions a key and bit.  9216 columns of 333 A-scans take 29 us; the
-// bitonic sort of a column per warp in shared memory before it took 169 us.
+// bitonic sort of a column per warp in shared memory before it took 169 us.  Up
+// to 32 A-scans a column is one key a lane and sorted by shuffles (a whole call of
+// 200 frames of 32: 80 us, 264 by bisection, 162 before it).
 // mean_mode: the float64 mean of the non-NaN values instead of the median.
 template <int kCols, int kReg>
 __global__ void __launch_bounds__(kMedThreads) k_xmedian(const float* __restrict__ mag, int nx, int nz,
@@ -545,6 +547,21 @@ __global__ void __launch_bounds__(kMedThreads) k_xmedian(const float* __restrict
         }
         // the key of rank k0 (the middle one, or the lower of the two)
         const int k0 = (n - 1) / 2;
+        if (kReg == 1) {
+            // one key a lane: sorted by a bitonic network of shuffles
+            unsigned int v = key[0];
+#pragma unroll
+            for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+                for (int j = k >> 1; j > 0; j >>= 1) {
+                    const unsigned int u = __shfl_xor_sync(0xffffffffu, v, j);
+                    v = ((lane & j) == 0) == ((lane & k) == 0) ? min(v, u) : max(v, u);
+                }
+            const double lo = static_cast<double>(ord2f(__shfl_sync(0xffffffffu, v, k0)));
+            const double hi = static_cast<double>(ord2f(__shfl_sync(0xffffffffu, v, n / 2)));
+            if (lane == 0) *o = (n & 1) ? lo : (lo + hi) / 2.0;
+            continue;
+        }
         unsigned int med = 0u;
 #pragma unroll 1
         for (int bit = 31; bit >= 0; --bit) {
@@ -644,11 +661,14 @@ cudaError_t launch_xmedian(const float* mag, int n_frames, int nx, int nz, int i
                            double* out, cudaStream_t st) {
     if (nx > kMedMaxX) return cudaErrorInvalidValue;
     // 16 columns (64-byte rows) while their tile leaves several blocks an SM,
-    // 8 for long columns (147 KB at 4096 A-scans)
-    const auto f = nx <= 256            ? launch_xmedian_t<16, 8>
-                   : nx <= 512          ? launch_xmedian_t<16, 16>
-                   : nx <= kMedMaxReg   ? launch_xmedian_t<16, 32>
-                                        : launch_xmedian_t<8, 0>;
+    // 8 for long columns (147 KB at 4096 A-scans) and where 16 would leave SMs idle
+    // (one frame of 32 A-scans, a whole call: mean 27 -> 21 us)
+    const bool few = static_cast<int64_t>(n_frames) * ((nz + 15) / 16) < 152;
+    const auto f = nx <= 32           ? (few ? launch_xmedian_t<8, 1> : launch_xmedian_t<16, 1>)
+                   : nx <= 256        ? (few ? launch_xmedian_t<8, 8> : launch_xmedian_t<16, 8>)
+                   : nx <= 512        ? (few ? launch_xmedian_t<8, 16> : launch_xmedian_t<16, 16>)
+                   : nx <= kMedMaxReg ? (few ? launch_xmedian_t<8, 32> : launch_xmedian_t<16, 32>)
+                                      : launch_xmedian_t<8, 0>;
     return f(mag, n_frames, nx, nz, ignore_nan, mean_mode, out, st);
 }
 

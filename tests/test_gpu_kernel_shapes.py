@@ -105,6 +105,12 @@ def test_x_profiles_equal_numpy(gpu_ctx, nx, nz):
                                       np.nanmedian(mag.astype(np.float64), axis=1))
 
 
+@pytest.mark.parametrize("nx", [1, 2, 31, 32, 33, 257, 513])
+def test_x_profiles_of_many_columns(gpu_ctx, nx):
+    """The same where the columns fill the GPU sixteen to a block (a ragged last one)."""
+    test_x_profiles_equal_numpy(gpu_ctx, nx, 1305)
+
+
 @pytest.mark.parametrize("nx,nz", [(1, 3), (33, 20), (1025, 9)])
 def test_x_mean_with_infinities_and_nan(gpu_ctx, nx, nz):
     """NaN is left out, an infinity is not: numpy.nanmean's values (1e-12, as
