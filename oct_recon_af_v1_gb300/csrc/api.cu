@@ -1860,6 +1860,8 @@ int octgb_quantise_double(octgb_ctx* c, const float* db, int64_t n, int db_loc, 
     });
 }
 
+constexpr size_t kPackSmall = 64 * 1024;    // bytes of slots
+
 int octgb_packbits(octgb_ctx* c, const uint16_t* img, int img_loc, int rows, int cols, uint8_t* out,
                    int64_t capacity, int* row_sizes, int64_t* total) {
     return guarded(c, [&] {
@@ -1877,23 +1879,40 @@ int octgb_packbits(octgb_ctx* c, const uint16_t* img, int img_loc, int rows, int
         }
         const size_t cap = static_cast<size_t>(rows) * packbits_slot(cols);
         ck(c->enc_slots.ensure(cap), "cudaMalloc(slots)");
-        ck(c->enc_packed.ensure(cap), "cudaMalloc(packed rows)");
         ck(c->enc_sizes.ensure(static_cast<size_t>(rows) * sizeof(int)), "cudaMalloc(sizes)");
-        ck(c->enc_offsets.ensure((static_cast<size_t>(rows) + 1) * sizeof(long long)), "cudaMalloc(row offsets)");
+        // a small image's slots cross as they are, beside the sizes: one wait (a call of
+        // 20 x 40 takes 31 us, 45 with the rows put together on the device and their bytes
+        // asked for; 150 x 200: 39 and 50; from 64 KB on the two are even)
+        const bool small = cap <= kPackSmall;
+        if (!small) {
+            ck(c->enc_packed.ensure(cap), "cudaMalloc(packed rows)");
+            ck(c->enc_offsets.ensure((static_cast<size_t>(rows) + 1) * sizeof(long long)), "cudaMalloc(row offsets)");
+        }
         ck(launch_packbits(src, rows, cols, c->enc_slots.as<uint8_t>(), c->enc_sizes.as<int>(),
-                           c->enc_offsets.as<long long>(), c->enc_packed.as<uint8_t>(), c->stream),
+                           c->enc_offsets.as<long long>(), small ? nullptr : c->enc_packed.as<uint8_t>(), c->stream),
            "packbits kernels");
-        c->launches += 3;
+        c->launches += small ? 1 : 3;
         ck(cudaMemcpyAsync(row_sizes, c->enc_sizes.p, static_cast<size_t>(rows) * sizeof(int), cudaMemcpyDeviceToHost,
                            c->stream),
            "D2H sizes");
+        std::vector<uint8_t> slots(small ? cap : 0);
+        if (small)
+            ck(cudaMemcpyAsync(slots.data(), c->enc_slots.p, cap, cudaMemcpyDeviceToHost, c->stream), "D2H slots");
         check_status(c);
         int64_t bytes = 0;
         for (int r = 0; r < rows; ++r) bytes += row_sizes[r];
         require(bytes <= capacity, "output capacity too small for the packed image");
-        ck(cudaMemcpyAsync(out, c->enc_packed.p, static_cast<size_t>(bytes), cudaMemcpyDeviceToHost, c->stream),
-           "D2H packed rows");
-        check_status(c);
+        if (small) {
+            uint8_t* o = out;
+            for (int r = 0; r < rows; ++r) {
+                memcpy(o, slots.data() + static_cast<size_t>(r) * packbits_slot(cols), row_sizes[r]);
+                o += row_sizes[r];
+            }
+        } else {
+            ck(cudaMemcpyAsync(out, c->enc_packed.p, static_cast<size_t>(bytes), cudaMemcpyDeviceToHost, c->stream),
+               "D2H packed rows");
+            check_status(c);
+        }
         *total = bytes;
     });
 }

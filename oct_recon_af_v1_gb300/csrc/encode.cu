@@ -179,6 +179,7 @@ cudaError_t launch_packbits(const uint16_t* img, int rows, int cols, uint8_t* sl
     const int slot = packbits_slot(cols);
     k_packbits_rows<<<(rows + kPackWarps - 1) / kPackWarps, kPackWarps * 32, 0, st>>>(img, rows, cols, slots, slot,
                                                                                       sizes);
+    if (out == nullptr) return cudaGetLastError();
     k_row_offsets<<<1, 1024, 0, st>>>(sizes, rows, offsets);
     k_pack_rows<<<rows, 128, 0, st>>>(slots, slot, sizes, offsets, out);
     return cudaGetLastError();

@@ -266,6 +266,7 @@ cudaError_t launch_requant(uint16_t* bits, int64_t n, double p1, double p2, doub
                            cudaStream_t st);
 int packbits_slot(int cols);
 // slots: rows x packbits_slot(cols) bytes of scratch; offsets: rows + 1; out: the rows' bytes, one after the other
+// (NULL: slots and sizes only, offsets not used)
 cudaError_t launch_packbits(const uint16_t* img, int rows, int cols, uint8_t* slots, int* sizes, long long* offsets,
                             uint8_t* out, cudaStream_t st);
 

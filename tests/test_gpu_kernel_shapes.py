@@ -82,6 +82,12 @@ def test_packbits_rows(gpu_ctx, rows, cols):
     assert packed == b"".join(ref)
 
 
+@pytest.mark.parametrize("rows,cols", [(1030, 130), (33, 2000), (3000, 7), (1, 33000)])
+def test_packbits_rows_put_together_on_the_device(gpu_ctx, rows, cols):
+    """The same for images whose rows are gathered on the device (more than 64 KB)."""
+    test_packbits_rows(gpu_ctx, rows, cols)
+
+
 @pytest.mark.parametrize("nx,nz", [(1, 1), (2, 17), (31, 16), (32, 5), (33, 40), (256, 20), (257, 20), (512, 9),
                                    (1024, 33), (1025, 9), (4096, 3)])
 def test_x_profiles_equal_numpy(gpu_ctx, nx, nz):
