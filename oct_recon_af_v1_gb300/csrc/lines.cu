@@ -509,14 +509,18 @@ __global__ void __launch_bounds__(lines_threads(U), 1) k_lines(const LinesArgs a
 // nine 5.6, thirteen 5.5 but 2 % slower for 30 B-scans).  Integers: four samples
 // a thread.  Float32 raws: one, since their float64 sums are bound by the SM's
 // FP64 rate and a row then spans four times the SMs (nine B-scans: 14.5 -> 7.0 us).
+// Many lines take 24 in flight (10 B-scans of 400 A-scans and 700 lines to
+// magnitudes: 77.5 -> 63.7 us; 2000 float32 lines: 346 -> 319, 700: 118 -> 121).
 constexpr int kApodThreads = 128;
-constexpr int kApodFlight = 9;
+constexpr int kApodFlight = 9, kApodFlightMany = 24;
+template <typename RawT>
+constexpr int kApodMany = sizeof(RawT) == 2 ? 128 : 1024;
 template <typename RawT>
 constexpr int kApodPer = sizeof(RawT) == 2 ? 4 : 1;                          // samples a thread
 template <typename RawT>
 constexpr int kApodParts = kN / (kApodThreads * kApodPer<RawT>);             // CTAs a row
 // Exact: the sums instead, as -S in float32 while that is exact, else as int32.
-template <typename RawT, bool Tiles, bool Exact>
+template <typename RawT, bool Tiles, bool Exact, int kFlight>
 __global__ void __launch_bounds__(kApodThreads) k_apod_mean(const LinesArgs a, float* __restrict__ out) {
     pdl_launch();                                // the lines kernel loads its weights meanwhile
     const int row = blockIdx.x / kApodParts<RawT>;   // segment * B + b, or the tiles' apod_row0 + b
@@ -539,14 +543,14 @@ __global__ void __launch_bounds__(kApodThreads) k_apod_mean(const LinesArgs a, f
     }
     if constexpr (sizeof(RawT) == 2) {
         int acc[4] = {0, 0, 0, 0};
-        for (int k0 = 0; k0 < apod; k0 += kApodFlight) {
-            uint2 q[kApodFlight];
+        for (int k0 = 0; k0 < apod; k0 += kFlight) {
+            uint2 q[kFlight];
 #pragma unroll
-            for (int i = 0; i < kApodFlight; ++i)
+            for (int i = 0; i < kFlight; ++i)
                 q[i] = k0 + i < apod ? __ldg(reinterpret_cast<const uint2*>(p + static_cast<int64_t>(k0 + i) * kN))
                                      : make_uint2(0u, 0u);
 #pragma unroll
-            for (int i = 0; i < kApodFlight; ++i) {
+            for (int i = 0; i < kFlight; ++i) {
                 acc[0] += static_cast<int>(static_cast<RawT>(q[i].x & 0xffffu));
                 acc[1] += static_cast<int>(static_cast<RawT>(q[i].x >> 16));
                 acc[2] += static_cast<int>(static_cast<RawT>(q[i].y & 0xffffu));
@@ -567,13 +571,13 @@ __global__ void __launch_bounds__(kApodThreads) k_apod_mean(const LinesArgs a, f
         *reinterpret_cast<float4*>(out + static_cast<int64_t>(row) * kN + j) = o;
     } else {
         double s = 0.0;
-        for (int k0 = 0; k0 < apod; k0 += kApodFlight) {
-            float q[kApodFlight];
+        for (int k0 = 0; k0 < apod; k0 += kFlight) {
+            float q[kFlight];
 #pragma unroll
-            for (int i = 0; i < kApodFlight; ++i)
+            for (int i = 0; i < kFlight; ++i)
                 q[i] = k0 + i < apod ? __ldg(p + static_cast<int64_t>(k0 + i) * kN) : 0.f;
 #pragma unroll
-            for (int i = 0; i < kApodFlight; ++i)
+            for (int i = 0; i < kFlight; ++i)
                 if (k0 + i < apod) s += static_cast<double>(q[i]);
         }
         out[static_cast<int64_t>(row) * kN + j] = static_cast<float>(s / apod);
@@ -620,14 +624,20 @@ cudaError_t launch_mode(const LinesArgs& a, int mode, int num_sms, cudaStream_t 
     }
 }
 
-template <typename RawT>
+template <typename RawT, int kFlight>
 void launch_apod_t(const LinesArgs& a, int rows, float* out, cudaStream_t st) {
-    if (a.exact)
-        k_apod_mean<RawT, false, true><<<kApodParts<RawT> * rows, kApodThreads, 0, st>>>(a, out);
-    else if (a.qt != nullptr)
-        k_apod_mean<RawT, true, false><<<kApodParts<RawT> * rows, kApodThreads, 0, st>>>(a, out);
+    const auto kernel = a.exact           ? k_apod_mean<RawT, false, true, kFlight>
+                        : a.qt != nullptr ? k_apod_mean<RawT, true, false, kFlight>
+                                          : k_apod_mean<RawT, false, false, kFlight>;
+    kernel<<<kApodParts<RawT> * rows, kApodThreads, 0, st>>>(a, out);
+}
+
+template <typename RawT>
+void launch_apod_f(const LinesArgs& a, int rows, float* out, cudaStream_t st) {
+    if (a.qt == nullptr && a.apod >= kApodMany<RawT>)
+        launch_apod_t<RawT, kApodFlightMany>(a, rows, out, st);
     else
-        k_apod_mean<RawT, false, false><<<kApodParts<RawT> * rows, kApodThreads, 0, st>>>(a, out);
+        launch_apod_t<RawT, kApodFlight>(a, rows, out, st);
 }
 
 }  // namespace
@@ -635,11 +645,11 @@ void launch_apod_t(const LinesArgs& a, int rows, float* out, cudaStream_t st) {
 cudaError_t launch_apod_mean(const LinesArgs& a, int dtype, int rows, float* out, cudaStream_t st) {
     if (rows == 0) return cudaSuccess;
     if (dtype == 0)
-        launch_apod_t<uint16_t>(a, rows, out, st);
+        launch_apod_f<uint16_t>(a, rows, out, st);
     else if (dtype == 1)
-        launch_apod_t<int16_t>(a, rows, out, st);
+        launch_apod_f<int16_t>(a, rows, out, st);
     else
-        launch_apod_t<float>(a, rows, out, st);
+        launch_apod_f<float>(a, rows, out, st);
     return cudaGetLastError();
 }
 

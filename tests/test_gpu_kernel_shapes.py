@@ -160,6 +160,24 @@ def test_lines_and_magnitudes_of_ragged_batches(gpu_ctx, dtype, bscans, nx):
     assert np.abs(gpu_ctx.fused_pre_fft(raw, 25) - spec).max() < 2e-6 * np.abs(spec).max()
 
 
+@pytest.mark.parametrize("dtype", [np.uint16, np.int16, np.float32])
+@pytest.mark.parametrize("apod", [9, 10, 127, 128, 144, 145, 1024, 1057])
+def test_apodisation_mean_of_many_lines(gpu_ctx, dtype, apod):
+    """Line counts around the batches in flight and where they grow: with equal
+    scan lines of zero the linearised spectrum is minus the mean's, exactly that
+    of a call with the mean as its one float32 line."""
+    from oct_recon_af_v1_gb300 import geometry as G
+    from oct_recon_af_v1_gb300 import synthetic
+    sg = G.build_spectral_geometry(synthetic.lambda_nm(), 0.0, 1.33)
+    gpu_ctx.set_geometry(sg.sinc_idx, sg.sinc_w, sg.window)
+    rng = np.random.default_rng(apod)
+    raw = np.zeros((3, apod + 2, 2048), dtype)
+    raw[:, :apod] = rng.integers(0, 30000, (3, apod, 2048))
+    mean = np.zeros((3, 3, 2048), np.float32)
+    mean[:, 0] = raw[:, :apod].astype(np.float64).sum(1) / apod
+    np.testing.assert_array_equal(gpu_ctx.fused_pre_fft(raw, apod), gpu_ctx.fused_pre_fft(mean, 1))
+
+
 @pytest.mark.parametrize("dtype", [np.uint16, np.float32])
 @pytest.mark.parametrize("span_nm,bscans,nx", [(300.0, 2, 7), (600.0, 1, 1), (600.0, 3, 305), (800.0, 1, 154), (800.0, 5, 61)])
 def test_lines_of_wide_windows(gpu_ctx, dtype, span_nm, bscans, nx):
