@@ -285,7 +285,7 @@ int octgb_graph_end(octgb_ctx *ctx, int *graph_id);
 int octgb_graph_launch(octgb_ctx *ctx, int graph_id);
 /* Self-test of the bounded device waits (no counterpart in the reference):
  * runs the lines kernel (which = 0) or the precision form's tensor-core
- * sinc (which = 1, integer raws; needs a geometry with precision tiles) on a
+ * sinc (which = 1, float32 raws; needs a geometry with precision tiles) on a
  * small internal batch of zero raws, with the waits' limit cut to
  * wait_limit_us (100 .. 2 000 000) and each CTA's first row-copy barrier
  * expecting 16 bytes more than its copies deliver.  Every copy still lands;
@@ -439,8 +439,8 @@ int octgb_cnn_conv3x3_bwd(octgb_ctx *ctx, const float *x, const float *w, const 
  * partial sums are added in a fixed order; dx as octgb_cnn_conv3x3_tc of dy
  * with the flipped kernel (the float32 kernel where that shape is not
  * supported); db as octgb_cnn_conv3x3_bwd, summed while dy is packed.  Shapes: 1 <= cin <= 48, 1 <= cout
- * <= 128, and a band of rows dividing h whose staged input fits in shared
- * memory (wd up to about 1000).  Asynchronous; a bounded device wait that
+ * <= 128, and a width of which one staged row fits in shared memory (up to
+ * 1000 and more with few channels, 700 with 24 -> 128 not).  Asynchronous; a bounded device wait that
  * expires is reported by the next synchronising call (OCTGB_ERR_TIMEOUT). */
 int octgb_cnn_conv3x3_bwd_tc(octgb_ctx *ctx, const float *x, const float *w, const float *dy, float *dx, float *dw,
                              float *db, float *w_scratch, int n, int cin, int cout, int h, int wd);

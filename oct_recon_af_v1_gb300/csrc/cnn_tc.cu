@@ -24,9 +24,9 @@
 // memory latency.  Measured at 128 images, against kernels that staged each tile
 // with plain loads between two block barriers (and summed the bias gradient in a
 // pass of its own):
-//   convolution       3 x 256 x 256: 516 -> 270 us (4.3 TB/s), 32 x 128 x 128: 370 -> 108 us (5.0 TB/s)
-//     + ReLU + mean   280 -> 217 us, 265 -> 96 us
-//   gradients of w, b 1100 -> 299 us (3.9 TB/s), 470 -> 188 us (2.9 TB/s)
+//   convolution       3 x 256 x 256: 516 -> 270 us (4.3 TB/s), 32 x 128 x 128: 370 -> 104 us (5.2 TB/s)
+//     + ReLU + mean   280 -> 217 us, 265 -> 88 us
+//   gradients of w, b 1100 -> 274 us (4.2 TB/s), 470 -> 180 us (3.0 TB/s)
 // What bounds them now: the 1.1 GB stream of the first convolution and its nine
 // MMAs a tile about equally; of the gradients the converters' instructions and
 // the copies (168 us at 32 x 128 x 128 without MMAs).
@@ -298,7 +298,8 @@ __device__ __forceinline__ void conv_mmas(uint32_t d, uint64_t a, uint64_t b, ui
 
 // kMask (the data gradient through ReLU + 2x2 mean): xmap is of the
 // pre-activations, pmap of the pooled gradient, their product with the mask is
-// formed while it is packed (32 x 128 x 128 at 128 images: 89 + 108 -> 124 us).
+// formed while it is packed (32 x 128 x 128 at 128 images: 89 + 108 -> 124 us when it
+// was made so; the three layers' data gradients of a training step take 182).
 template <bool kBf16, bool kMask, bool kDirect>
 __global__ void __launch_bounds__(kCThreads, 1)
     k_conv3x3_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap pmap, const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
@@ -602,7 +603,7 @@ __global__ void __launch_bounds__(kCThreads, 1)
 //   dy[k](oy, ox) * x[c](oy + ty - 1, ox + tx - 1)          (x zero outside the image)
 // as nine GEMMs that contract over pixels: M = the output channels, 64 rows or 128
 // (the MMA reads all M rows of A from shared memory, whatever their use: 32
-// channels at M = 128 took 233 us at 32 x 128 x 128, 188 at M = 64; rows past cout
+// channels at M = 128 took 233 us at 32 x 128 x 128, 188 at M = 64 then; rows past cout
 // read in-bounds data of the following chunks into accumulator rows that are
 // never read), N = the input channels rounded up to
 // 16, K = 16 pixels per MMA; BF16 operands (gradients span float32's exponent
@@ -646,7 +647,7 @@ struct WgradBars {
 // kPool: dy is not in memory: dmap is then of the pre-activations y and pmap of the
 // gradient dp of their ReLU + 2x2 mean, and dy = y > 0 ? dp / 4 : 0 is formed while
 // it is packed (k_relu_pool_bwd's value).  That saves writing and reading dy, of
-// the first layer's 1.1 GB each at 128 images: 339 + 307 us -> 340 us.
+// the first layer's 1.1 GB each at 128 images: 339 + 307 us -> 297 us.
 template <bool kPool, bool kDirect>
 __global__ void __launch_bounds__(kWThreads, 1)
     k_conv3x3_wgrad_tc(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap dmap,
