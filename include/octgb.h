@@ -177,8 +177,10 @@ int octgb_minmax(octgb_ctx *ctx, const float *db, int64_t n, int db_loc, double 
  * (n_tile_x, c1-c0) are the reference's dense linear-interpolation operators
  * restricted to the rows/columns that receive data; each row of Wz and each
  * column of WxT has at most two adjacent non-zeros (MATLAB linear
- * interpolation), which the library verifies and stores in compact form.
- * fz (r1-r0): focus weight.  shift/pdz (n_y, n_tile_x): optical-path
+ * interpolation), which the library verifies and stores in compact form.  An
+ * A-scan whose weight in a column is zero is not read for it where all columns of
+ * a block of 32 take one A-scan: an infinite or NaN magnitude then stays in its
+ * own column.  fz (r1-r0): focus weight.  shift/pdz (n_y, n_tile_x): optical-path
  * correction (OpticalPathCorrection, stitching.py:54-78), or NULL/NULL when it
  * is off.  n_rows: depth samples per A-scan (n/2).  Returns a plan id. */
 int octgb_stitch_plan(octgb_ctx *ctx, int n_rows, int r0, int r1, int c0, int c1, int n_out_z, int n_tile_x,
@@ -438,10 +440,11 @@ int octgb_cnn_conv3x3_bwd(octgb_ctx *ctx, const float *x, const float *w, const 
  * float32 accumulation): dw as nine pixel-contracting GEMMs whose per-CTA
  * partial sums are added in a fixed order; dx as octgb_cnn_conv3x3_tc of dy
  * with the flipped kernel (the float32 kernel where that shape is not
- * supported); db as octgb_cnn_conv3x3_bwd, summed while dy is packed.  Shapes: 1 <= cin <= 48, 1 <= cout
- * <= 128, and a width of which one staged row fits in shared memory (up to
- * 1000 and more with few channels, 700 with 24 -> 128 not).  Asynchronous; a bounded device wait that
- * expires is reported by the next synchronising call (OCTGB_ERR_TIMEOUT). */
+ * supported); db as octgb_cnn_conv3x3_bwd, summed while dy is packed.
+ * Shapes: 1 <= cin <= 48, 1 <= cout <= 128, and a width of which one staged row fits in shared memory (up to 1086
+ * for 1 -> 1 channels, 890 for 3 -> 32 and 32 -> 32, 506 for 24 -> 128).
+ * Asynchronous; a bounded device wait that expires is reported by the next
+ * synchronising call (OCTGB_ERR_TIMEOUT). */
 int octgb_cnn_conv3x3_bwd_tc(octgb_ctx *ctx, const float *x, const float *w, const float *dy, float *dx, float *dw,
                              float *db, float *w_scratch, int n, int cin, int cout, int h, int wd);
 /* octgb_cnn_relu_pool_bwd followed by octgb_cnn_conv3x3_bwd_tc with the

@@ -2427,8 +2427,8 @@ int octgb_cnn_conv3x3_bwd_tc(octgb_ctx* c, const float* x, const float* w, const
         require(x && w && dy && dw && db, "NULL buffer");
         require(n >= 1 && cin >= 1 && cout >= 1 && h >= 1 && wd >= 1, "bad convolution shape");
         const size_t parts = conv3x3_wgrad_tc_partials(n, cin, cout, h, wd, false, c->num_sms);
-        require(parts > 0, "tensor-core weight gradient: 1 <= cin <= 48, 1 <= cout <= 128 and a band of rows "
-                           "dividing the height whose staged input fits in shared memory");
+        require(parts > 0, "tensor-core weight gradient: 1 <= cin <= 48, 1 <= cout <= 128 and a width "
+                           "of which one staged row fits in shared memory");
         ck(c->wgrad_part.ensure(parts * sizeof(float)), "cudaMalloc(weight-gradient partial sums)");
         ck(launch_conv3x3_wgrad_tc(x, dy, nullptr, dw, db, n, cin, cout, h, wd, c->wgrad_part.as<float>(),
                                    c->num_sms, c->status_dev, c->stream),
