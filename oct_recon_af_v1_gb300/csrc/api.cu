@@ -1524,7 +1524,7 @@ int octgb_graph_end(octgb_ctx* c, int* graph_id) {
         for (DevBuf* b : {&c->lines, &c->raw, &c->apod, &c->out, &c->mm, &c->frames, &c->num, &c->den, &c->plan_table,
                           &c->run_mm, &c->magbuf, &c->dbbuf, &c->planemm, &c->segs, &c->qtable,
                           &c->disp_x, &c->disp_hann, &c->disp_dk2, &c->disp_betas, &c->disp_phase, &c->disp_a, &c->disp_score, &c->xmed,
-                          &c->prec_hi, &c->prec_lo, &c->prec_m, &c->prec_x, &c->prep, &c->prep_apod,
+                          &c->prec_hi, &c->prec_lo, &c->prec_m, &c->prec_x, &c->prep, &c->prep_apod, &c->bias_part, &c->wgrad_part,
                           &c->magrep, &c->srr, &c->gemm_part, &c->enc_bits, &c->enc_lut, &c->enc_slots, &c->enc_sizes, &c->enc_offsets, &c->enc_packed})
             b->keep_old = true;
         for (int k = 0; k < octgb_ctx::kRing; ++k) c->ring[k].keep_old = true;

@@ -624,3 +624,47 @@ def test_transform_with_lines_in_shared_memory(gpu_ctx, n):
         gpu_ctx.synchronize()
         assert torch.equal(mag[:, lo:lo + 500], small)
     assert torch.isfinite(mag).all()
+
+
+def test_captured_gradients_after_larger_ones():
+    """A graph over a weight gradient replays after a call that needs more room
+    for its partial sums (the float32 form's bias gradient likewise)."""
+    torch = pytest.importorskip("torch")
+    from oct_recon_af_v1_gb300 import _lib
+    from oct_recon_af_v1_gb300.learned import _p
+    ctx = _lib.Context(0)
+    try:
+        stream = torch.cuda.Stream()
+        ctx.set_stream(stream.cuda_stream)
+        g = torch.Generator(device="cuda").manual_seed(4)
+
+        def buffers(n, h):
+            x, dy, w = (torch.randn(s, device="cuda", generator=g) for s in ((n, 8, h, h), (n, 32, h, h), (32, 8, 3, 3)))
+            return x, w, dy, torch.empty_like(w), torch.empty(32, device="cuda")
+
+        def run(f, b):
+            x, w, dy, dw, db = b
+            ctx._check(f(ctx.h, _p(x), _p(w), _p(dy), None, _p(dw), _p(db), None, x.shape[0], 8, 32, x.shape[2], x.shape[3]))
+        small, large = buffers(1, 16), buffers(300, 32)
+        torch.cuda.synchronize()
+        for f in (ctx.lib.octgb_cnn_conv3x3_bwd_tc, ctx.lib.octgb_cnn_conv3x3_bwd):
+            run(f, small)
+            ctx.synchronize()
+            ref = [t.clone() for t in small[3:]]
+            torch.cuda.synchronize()
+            ctx.graph_begin()
+            run(f, small)
+            gid = ctx.graph_end()
+            run(f, large)
+            ctx.synchronize()
+            fill = torch.empty(1 << 24, device="cuda").fill_(3.0)       # what was freed is in use again
+            for t in small[3:]:
+                t.zero_()
+            torch.cuda.synchronize()
+            ctx.graph_launch(gid)
+            ctx.synchronize()
+            assert (fill == 3.0).all()
+            for t, r in zip(small[3:], ref):
+                assert (t - r).abs().max() <= 1e-5 * r.abs().max()
+    finally:
+        ctx.close()
